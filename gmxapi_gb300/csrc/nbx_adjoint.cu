@@ -103,7 +103,7 @@ __device__ __forceinline__ void adj_pair(const DeviceView& v, const float2* __re
         int_bit  = 1.0f;
     }
     r2                   = fmaxf(r2, kMinDist2);
-    float       rinv     = rsqrtf(r2);
+    float       rinv     = fast_rsqrt(r2);
     rinv                 = rinv * (1.5f - 0.5f * r2 * rinv * rinv);
     const float  rinv2   = rinv * rinv;
     const float2 lj      = nbfp_s[ti * nt1 + tj];

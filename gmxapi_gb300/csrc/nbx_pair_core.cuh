@@ -32,6 +32,15 @@ __device__ __forceinline__ float fast_rcp(float x)
     return r;
 }
 
+// 1/sqrt without the denormal scaling that rsqrtf() adds around it (six instructions a pair): r^2 is
+// at least kMinDist2 here, and for normal arguments the result is the same bits.
+__device__ __forceinline__ float fast_rsqrt(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 __device__ __forceinline__ float fast_ex2(float x)
 {
     float r;
@@ -242,7 +251,7 @@ __device__ __forceinline__ void process_half(const DeviceView& v, const SysPtrs&
             }
             const bool in_range = kExcl ? (mask != 0.0f) : (r2 < rc2);
             r2         = fmaxf(r2, kMinDist2);
-            float rinv = rsqrtf(r2);
+            float rinv = fast_rsqrt(r2);
             if (kEnergy)
             {
                 // one Newton step: rsqrt.approx -> ~correctly rounded, unbiased for the energy sums

@@ -47,6 +47,14 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
     return *reinterpret_cast<float2*>(&rd);
 }
+// Compensated (Kahan) accumulation of two sums at once, the steps of kahan_add in packed arithmetic.
+__device__ __forceinline__ void kahan_add2(float2& sum, float2& c, float2 v)
+{
+    const float2 y = sub2(v, c);
+    const float2 t = add2(sum, y);
+    c              = sub2(sub2(t, sum), y);
+    sum            = t;
+}
 // The erfc expansion polynomial of erfc_poly (nbx_internal.cuh), same coefficients, evaluated by
 // Estrin's scheme: (c0 + c1 t) + (c2 + c3 t) t^2 + ((c4 + c5 t) + (c6 + c7 t) t^2) t^4 -- a
 // dependency depth of 4 instead of Horner's 7, for two more multiplications (the pair loop is
@@ -238,7 +246,7 @@ __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* 
     const bool    inA = g.inA, inB = g.inB;
     const float   intA = g.intA, intB = g.intB;
     float2        r2   = make_float2(fmaxf(g.r2.x, kMinDist2), fmaxf(g.r2.y, kMinDist2));
-    float2        rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+    float2        rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
     if (kEnergy)
     {
         // one Newton step: rsqrt.approx -> ~correctly rounded, unbiased for the energy sums;
@@ -416,7 +424,7 @@ __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2&
                                          const float* __restrict__ jx,
                                          float4* __restrict__ lane_rec, int cj_lane, unsigned m0, unsigned m1,
                                          unsigned wA, unsigned wB, int sci, bool central, int ii, int jj,
-                                         float& acc_el, float& cmp_el, float& acc_lj, float& cmp_lj)
+                                         float2& acc, float2& cmp)
 {
     const unsigned full = 0xffffffffu;
     const unsigned u    = m0 | m1;
@@ -453,28 +461,26 @@ __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2&
         }
         if (kEnergy)
         {
-            kahan_add(acc_el, cmp_el, qj.x * ejel.x);
-            kahan_add(acc_el, cmp_el, qj.y * ejel.y);
-            kahan_add(acc_lj, cmp_lj, ejlj.x + ejlj.y);
+            // {Coulomb, LJ} of this j-cluster into the compensated per-lane totals, both in one chain
+            kahan_add2(acc, cmp, make_float2(fmaf(qj.x, ejel.x, qj.y * ejel.y), ejlj.x + ejlj.y));
         }
         // j forces: sum over the 8 i-lanes, reduce-scatter on the first level so that lanes
         // ii < 4 end with the half-0 atom (jj) and lanes ii >= 4 with the half-1 atom (jj + 4)
         const bool hi = (ii & 4) != 0;
-        float      kx = hi ? fjx.y : fjx.x, ky = hi ? fjy.y : fjy.x, kz = hi ? fjz.y : fjz.x;
+        float2     kxy = make_float2(hi ? fjx.y : fjx.x, hi ? fjy.y : fjy.x);
+        float      kz  = hi ? fjz.y : fjz.x;
         const float sx = hi ? fjx.x : fjx.y, sy = hi ? fjy.x : fjy.y, sz = hi ? fjz.x : fjz.y;
-        kx += __shfl_xor_sync(full, sx, 4);
-        ky += __shfl_xor_sync(full, sy, 4);
+        kxy = add2(kxy, make_float2(__shfl_xor_sync(full, sx, 4), __shfl_xor_sync(full, sy, 4)));
         kz += __shfl_xor_sync(full, sz, 4);
 #pragma unroll
         for (int o = 2; o > 0; o >>= 1)
         {
-            kx += __shfl_xor_sync(full, kx, o);
-            ky += __shfl_xor_sync(full, ky, o);
+            kxy = add2(kxy, make_float2(__shfl_xor_sync(full, kxy.x, o), __shfl_xor_sync(full, kxy.y, o)));
             kz += __shfl_xor_sync(full, kz, o);
         }
         if ((ii & 3) == 0)
         {
-            red_add_v4(&p.fnb[cj * kCl + jj + (hi ? 4 : 0)], -kx, -ky, -kz);
+            red_add_v4(&p.fnb[cj * kCl + jj + (hi ? 4 : 0)], -kxy.x, -kxy.y, -kz);
         }
     }
 }
@@ -520,7 +526,7 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
         lane_rec[c * kCl * kIRecF4 + 2 + jj] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     __syncwarp();
-    float acc_el = 0.0f, cmp_el = 0.0f, acc_lj = 0.0f, cmp_lj = 0.0f;
+    float2 acc = f2(0.0f), cmp = f2(0.0f);  // {Coulomb, LJ} and their compensations
     // pipeline over the cj4 groups: kDepth - 1 groups' copies in flight ahead of the one computed
     // (with each group's record and, where it has exclusion masks, the lane's exclusion words,
     // so their load latency is hidden behind the groups computed before)
@@ -585,12 +591,12 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
         if ((ime.y | ime.w) == 0)
         {
             group_x2<kEnergy, kCoul, false>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, ~0u, ~0u, s.sci, central,
-                                             ii, jj, acc_el, cmp_el, acc_lj, cmp_lj);
+                                             ii, jj, acc, cmp);
         }
         else
         {
             group_x2<kEnergy, kCoul, true>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, wAB.x, wAB.y, s.sci,
-                                            central, ii, jj, acc_el, cmp_el, acc_lj, cmp_lj);
+                                            central, ii, jj, acc, cmp);
         }
     }
     // i forces: reduce over the 4 j-lanes of each i-atom
@@ -616,8 +622,8 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
     }
     if (kEnergy)
     {
-        e_el_acc += (double)acc_el - (double)cmp_el;
-        e_lj_acc += (double)acc_lj - (double)cmp_lj;
+        e_el_acc += (double)acc.x - (double)cmp.x;
+        e_lj_acc += (double)acc.y - (double)cmp.y;
     }
     if (!central)
     {
