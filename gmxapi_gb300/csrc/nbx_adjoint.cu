@@ -104,7 +104,7 @@ __device__ __forceinline__ void adj_pair(const DeviceView& v, const float2* __re
     }
     r2                   = fmaxf(r2, kMinDist2);
     float       rinv     = fast_rsqrt(r2);
-    rinv                 = rinv * (1.5f - 0.5f * r2 * rinv * rinv);
+    rinv                 = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
     const float  rinv2   = rinv * rinv;
     const float2 lj      = nbfp_s[ti * nt1 + tj];
     float        rinv6   = rinv2 * rinv2 * rinv2;

@@ -255,7 +255,7 @@ __device__ __forceinline__ void process_half(const DeviceView& v, const SysPtrs&
             if (kEnergy)
             {
                 // one Newton step: rsqrt.approx -> ~correctly rounded, unbiased for the energy sums
-                rinv = rinv * (1.5f - 0.5f * r2 * rinv * rinv);
+                rinv = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
             }
             const float  rinv2 = rinv * rinv;
             float4       lj;

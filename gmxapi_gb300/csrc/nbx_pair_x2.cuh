@@ -47,12 +47,12 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
     return *reinterpret_cast<float2*>(&rd);
 }
-// Compensated (Kahan) accumulation of two sums at once, the steps of kahan_add in packed arithmetic.
-__device__ __forceinline__ void kahan_add2(float2& sum, float2& c, float2 v)
+// Compensated (Kahan) accumulation of two sums at once in packed arithmetic; y: the addend plus the
+// carried correction c (the negated compensation of kahan_add).
+__device__ __forceinline__ void kahan_add2(float2& sum, float2& c, float2 y)
 {
-    const float2 y = sub2(v, c);
     const float2 t = add2(sum, y);
-    c              = sub2(sub2(t, sum), y);
+    c              = sub2(y, sub2(t, sum));
     sum            = t;
 }
 // The erfc expansion polynomial of erfc_poly (nbx_internal.cuh), same coefficients, evaluated by
@@ -197,6 +197,12 @@ struct SysPtrsX2
     double*       fshift;
 };
 
+// Per-lane energies of one list entry, {half 0, half 1}: Coulomb and LJ sums and their corrections.
+struct EnergySumsX2
+{
+    float2 el, cel, lj, clj;
+};
+
 // Constants of the pair loop, read once per entry.
 struct PairConstsX2
 {
@@ -250,9 +256,10 @@ __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* 
     if (kEnergy)
     {
         // one Newton step: rsqrt.approx -> ~correctly rounded, unbiased for the energy sums;
-        // y (1.5 - (r^2 / 2) y^2) with -r^2 / 2 formed beside the rsqrt
+        // y + y (1/2 - (r^2 / 2) y^2) with -r^2 / 2 formed beside the rsqrt (the small correction is
+        // added in one rounding, where y times a factor near 1 rounds the factor as well)
         const float2 r2h = mul2(r2, f2(-0.5f));
-        rinv             = mul2(rinv, fma2(r2h, mul2(rinv, rinv), f2(1.5f)));
+        rinv             = fma2(rinv, fma2(r2h, mul2(rinv, rinv), f2(0.5f)), rinv);
     }
     // pairs outside the cut-off (or of a pruned half, or the diagonal's lower triangle) get
     // 1/r = 0: every force term below carries 1/r^2 and vanishes
@@ -424,7 +431,7 @@ __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2&
                                          const float* __restrict__ jx,
                                          float4* __restrict__ lane_rec, int cj_lane, unsigned m0, unsigned m1,
                                          unsigned wA, unsigned wB, int sci, bool central, int ii, int jj,
-                                         float2& acc, float2& cmp)
+                                         EnergySumsX2& es)
 {
     const unsigned full = 0xffffffffu;
     const unsigned u    = m0 | m1;
@@ -461,8 +468,11 @@ __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2&
         }
         if (kEnergy)
         {
-            // {Coulomb, LJ} of this j-cluster into the compensated per-lane totals, both in one chain
-            kahan_add2(acc, cmp, make_float2(fmaf(qj.x, ejel.x, qj.y * ejel.y), ejlj.x + ejlj.y));
+            // this j-cluster's sums into the compensated per-lane totals of the two halves; q_j times the
+            // Coulomb sum enters unrounded (a rounded product is off alike for every atom of a charge
+            // class, and the cancelling total amplifies that)
+            kahan_add2(es.el, es.cel, fma2(qj, ejel, es.cel));
+            kahan_add2(es.lj, es.clj, add2(ejlj, es.clj));
         }
         // j forces: sum over the 8 i-lanes, reduce-scatter on the first level so that lanes
         // ii < 4 end with the half-0 atom (jj) and lanes ii >= 4 with the half-1 atom (jj + 4)
@@ -526,7 +536,7 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
         lane_rec[c * kCl * kIRecF4 + 2 + jj] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     __syncwarp();
-    float2 acc = f2(0.0f), cmp = f2(0.0f);  // {Coulomb, LJ} and their compensations
+    EnergySumsX2 es = { f2(0.0f), f2(0.0f), f2(0.0f), f2(0.0f) };
     // pipeline over the cj4 groups: kDepth - 1 groups' copies in flight ahead of the one computed
     // (with each group's record and, where it has exclusion masks, the lane's exclusion words,
     // so their load latency is hidden behind the groups computed before)
@@ -591,12 +601,12 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
         if ((ime.y | ime.w) == 0)
         {
             group_x2<kEnergy, kCoul, false>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, ~0u, ~0u, s.sci, central,
-                                             ii, jj, acc, cmp);
+                                             ii, jj, es);
         }
         else
         {
             group_x2<kEnergy, kCoul, true>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, wAB.x, wAB.y, s.sci,
-                                            central, ii, jj, acc, cmp);
+                                            central, ii, jj, es);
         }
     }
     // i forces: reduce over the 4 j-lanes of each i-atom
@@ -622,8 +632,8 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
     }
     if (kEnergy)
     {
-        e_el_acc += (double)acc.x - (double)cmp.x;
-        e_lj_acc += (double)acc.y - (double)cmp.y;
+        e_el_acc += ((double)es.el.x + (double)es.cel.x) + ((double)es.el.y + (double)es.cel.y);
+        e_lj_acc += ((double)es.lj.x + (double)es.clj.x) + ((double)es.lj.y + (double)es.clj.y);
     }
     if (!central)
     {
