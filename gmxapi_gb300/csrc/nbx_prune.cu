@@ -8,11 +8,9 @@
 //    any pair is within rlistInner;
 //  - rolling pass: only bits in (outer XOR inner) are re-tested and may be
 //    added to the inner mask.
-// Fresh pass: one block per list entry, its warps taking the entry's cj4 groups
-// in turn; lane (ip, jj) holds the shifted i-atoms ip and ip + 4 of the 8
-// i-clusters in registers and tests both against j-atom jj in packed FP32x2
-// arithmetic; the in-range flags of a j-cluster's 8 i-clusters become per-lane
-// bit masks, ORed over the warp with one reduction per j-cluster.
+// Fresh pass: one warp per list entry, lane = one cluster pair of the cj4 group
+// in hand; minima of packed squared distances decide, and the few that lie
+// within rounding of a radius are recomputed exactly.
 // Rolling pass: one warp per list entry; the few bits to re-test are numbered
 // over the warp and each lane tests whole bits (32 atom pairs).  Compiled with
 // --fmad=false; r^2 = fma(dz, dz, fma(dy, dy, dx dx)) is written out with
@@ -26,8 +24,7 @@ namespace nbx
 namespace
 {
 
-// warps per block: 4 for the rolling pass (a warp per list entry), 4 for the fresh pass (a block per
-// list entry, every bit tested, compute-bound)
+// warps per block (a warp per list entry in both passes)
 constexpr int kPruneWarpsRolling = 4;
 constexpr int kPruneWarpsFresh   = 4;
 
@@ -42,133 +39,222 @@ __device__ __forceinline__ float2 p_sub(float2 a, float2 b)
     return *reinterpret_cast<float2*>(&rd);
 }
 
-// Fresh prune of one list entry: each warp of the block takes cj4 groups warp, warp + W, ... on its
-// own (no block barrier).  Lane (ip, jj), ip = lane & 3 and jj = lane >> 2, holds the shifted i-atoms
-// ip and ip + 4 of the entry's 8 i-clusters in registers as pairs {x_ip, x_ip+4}, ... and tests
-// both against j-atom jj of a j-cluster in one packed operation, so both results belong to the same
-// warp half (jj / 4) and the lane keeps their minimum.  The in-range flags of the 8 i-clusters are
-// collected as per-lane bit masks, inner and outer, placed by warp half in one word and ORed over the
-// warp with one reduction per j-cluster; j-clusters without bits are skipped.
-template<int kPruneWarps>
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Squared distance with the rounding of the reference's norm2 in its prune kernel.
+__device__ __forceinline__ float exact_r2(float dx, float dy, float dz)
+{
+    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+}
+
+// The smallest squared distance between the 8 atoms at xi (shifted by s*) and the 4 at xj, each
+// rounded as the CPU restatement rounds it.
+__device__ __noinline__ float exact_min_r2(const float4* __restrict__ xi, const float4* __restrict__ xj, float sx,
+                                           float sy, float sz)
+{
+    unsigned m = 0xffffffffu;
+    for (int b = 0; b < kCl / kSplit; b++)
+    {
+        const float4 q = xj[b];
+        for (int a = 0; a < kCl; a++)
+        {
+            const float4 p = xi[a];
+            m = min(m, __float_as_uint(exact_r2((p.x + sx) - q.x, (p.y + sy) - q.y, (p.z + sz) - q.z)));
+        }
+    }
+    return __uint_as_float(m);
+}
+
+// Per-warp shared memory of the fresh pass: x, y and z of three groups' four packed records.
+constexpr int kFreshDepth = 3;
+struct FreshSmem
+{
+    float4 x[kFreshDepth][kJg][6];
+};
+
+// Lanes (jm, part), part < 6, copy the coordinates (96 of the record's 160 bytes) of j-cluster cj into
+// buffer b, if there is one, and close the copy group.
+__device__ __forceinline__ void fresh_copy(FreshSmem& sm, int b, int cj, bool any, const float* xqp, int lane)
+{
+    if (any && (lane & 7) < 6)
+    {
+        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(&sm.x[b][lane >> 3][lane & 7]));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                     "l"(xqp + (size_t)cj * kPackWords + 4 * (lane & 7))
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// Fresh prune of one list entry by one warp.  Lane (c, jm) = (lane & 7, lane >> 3) takes the cluster
+// pair of i-cluster c and j-cluster jm of each cj4 group, so its flags sit at the mask bit of the
+// lane's own number and four ballots make the group's masks.  The pass is bound by the FMA pipe
+// (64 squared distances per cluster pair), so they are formed as |x_j|^2 - 2 x_i.x_j + |x_i|^2 about
+// the entry's first atom: three packed multiply-adds per two pairs (the two halves' atoms a, a + 4
+// in one operation, from the cluster-packed records) instead of six operations, and three-input
+// minima.  That form rounds differently: with coordinates up to A from the origin and a radius R
+// its error is below 10 2^-24 (3 A + R)^2 (three coordinate roundings, the two norms and four
+// additions, each of terms below (|x_i| + |x_j|)^2).  A minimum within 16 2^-24 (3 A + R)^2 of a
+// radius, about one in 10^4, is therefore recomputed by exact_min_r2, and the masks equal the
+// exact ones bit for bit.  Fillers: an i-filler's norm is 1e9 (never in range), a j-filler is far
+// away by itself, and two fillers are as far apart as their shift (ff_in, ff_out).
+// 960k-atom water list (523k groups, cold caches): 330 us with the exact form on all 64 pairs and a
+// block per entry, 247 us now (FMA pipe 49 %; the rest is latency at 16 warps of 128 registers per SM --
+// the i-atoms read from shared memory instead, at 24 warps, took 272 us).
 __device__ void prune_entry_fresh(const Sci& s, const Cj4* cj4, unsigned* imask_outer, const float4* xq,
-                                  const float* shiftvec, float outer2, float inner2)
+                                  const float* xqp, const float* shiftvec, float outer2, float inner2, FreshSmem& sm)
 {
     const int      lane = threadIdx.x & 31;
-    const int      warp = threadIdx.x >> 5;
-    const int      ip   = lane & 3;
-    const int      jj   = lane >> 2;
+    const int      c    = lane & 7;
+    const int      jm   = lane >> 3;
     const unsigned full = 0xffffffffu;
-    // the next group's record is loaded while the current one is tested
-    Cj4 c4n{};
-    if (s.cj4_start + warp < s.cj4_end)
-    {
-        c4n = cj4[s.cj4_start + warp];
-    }
-    const float sx = shiftvec[3 * s.shift], sy = shiftvec[3 * s.shift + 1], sz = shiftvec[3 * s.shift + 2];
-    // the j-atoms of the entry's j-clusters are fetched into L2 by the whole block (thread t: group
-    // t / 4, j-cluster t % 4), so that only each warp's first group waits for device memory
-    for (int q = threadIdx.x; q < (s.cj4_end - s.cj4_start) * kJg; q += blockDim.x)
-    {
-        const int cj = cj4[s.cj4_start + q / kJg].cj[q % kJg];
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(xq + (size_t)cj * kCl)));
-    }
-    if (s.cj4_start + warp >= s.cj4_end)
+    if (s.cj4_start >= s.cj4_end)
     {
         return;
     }
-    float2 xi[kNcl], yi[kNcl], zi[kNcl];
-#pragma unroll
-    for (int c = 0; c < kNcl; c++)
+    // three groups' coordinates in shared memory, one computed and two groups' copies in flight; the
+    // lane's j-cluster indices are loaded one group further ahead
+    Cj4*       g   = const_cast<Cj4*>(cj4) + s.cj4_start;
+    Cj4* const end = const_cast<Cj4*>(cj4) + s.cj4_end;
+    unsigned*  om  = imask_outer + 2 * (size_t)s.cj4_start;
+    int        cj0 = g->cj[jm], cj1 = 0, cj2 = 0;
+    int4       imn = *reinterpret_cast<const int4*>(&g->imei[0]);
+    if (g + 1 < end)
     {
-        const float4 a = xq[s.sci * kSc + c * kCl + ip];
-        const float4 b = xq[s.sci * kSc + c * kCl + ip + 4];
-        xi[c]          = make_float2(a.x + sx, b.x + sx);
-        yi[c]          = make_float2(a.y + sy, b.y + sy);
-        zi[c]          = make_float2(a.z + sz, b.z + sz);
+        cj1 = g[1].cj[jm];
     }
-    // this lane's flags go to bits 0-15 (half 0) or 16-31 (half 1) of the reduced word
-    const int    hshift   = 16 * (jj >> 2);
-    const float2 inner2x2 = make_float2(inner2, inner2), outer2x2 = make_float2(outer2, outer2);
-    for (int j4 = s.cj4_start + warp; j4 < s.cj4_end; j4 += kPruneWarps)
+    if (g + 2 < end)
     {
-        const Cj4 c4 = c4n;
-        if (j4 + kPruneWarps < s.cj4_end)
+        cj2 = g[2].cj[jm];
+    }
+    __syncwarp();  // the readers of the last entry's shared memory are done
+    fresh_copy(sm, 0, cj0, g < end, xqp, lane);
+    fresh_copy(sm, 1, cj1, g + 1 < end, xqp, lane);
+    const float sx = shiftvec[3 * s.shift], sy = shiftvec[3 * s.shift + 1], sz = shiftvec[3 * s.shift + 2];
+    const float4* const xi = xq + (size_t)s.sci * kSc + c * kCl;
+    const float4        o4 = xq[(size_t)s.sci * kSc];
+    const float         ox = o4.x + sx, oy = o4.y + sy, oz = o4.z + sz;
+    float2              xm[kCl], ym[kCl], zm[kCl], ni[kCl];  // {-2 x, -2 x}, ..., {|x|^2, |x|^2}
+    float               amax     = 0.0f;
+    bool                has_fill = false;
+#pragma unroll
+    for (int a = 0; a < kCl; a++)
+    {
+        const float4 p    = xi[a];
+        const bool   fill = p.x == kFarAway;
+        const float  x = (p.x + sx) - ox, y = (p.y + sy) - oy, z = (p.z + sz) - oz;
+        const float  n = exact_r2(x, y, z);
+        const float  m = fill ? 0.0f : -2.0f, nf = fill ? 1.0e9f : n;
+        amax           = fmaxf(amax, fill ? 0.0f : n);
+        has_fill |= fill;
+        ni[a] = make_float2(nf, nf);
+        xm[a] = make_float2(m * x, m * x);
+        ym[a] = make_float2(m * y, m * y);
+        zm[a] = make_float2(m * z, m * z);
+    }
+    amax              = __uint_as_float(__reduce_max_sync(full, __float_as_uint(amax)));
+    const float reach = 3.0f * sqrtf(amax) + sqrtf(outer2);
+    const float eps   = 9.5367432e-7f * reach * reach;
+    // two fillers of this shift: the exact arithmetic on their coordinates
+    const float  ff = exact_r2((kFarAway + sx) - kFarAway, (kFarAway + sy) - kFarAway, (kFarAway + sz) - kFarAway);
+    const bool   any_ff = ff < outer2 && __any_sync(full, has_fill);
+    const float2 ox2 = make_float2(ox, ox), oy2 = make_float2(oy, oy), oz2 = make_float2(oz, oz);
+    int          b   = 0;
+    for (; g < end; g++, om += 2, b = (b == kFreshDepth - 1) ? 0 : b + 1)
+    {
+        const unsigned check0 = (unsigned)imn.x, check1 = (unsigned)imn.z;
+        const int      cj_own = cj0;
+        __syncwarp();  // the readers of the buffer two ahead (the group before this one) are done
+        fresh_copy(sm, (b == 0) ? kFreshDepth - 1 : b - 1, cj2, g + 2 < end, xqp, lane);
+        cj0 = cj1;
+        cj1 = cj2;
+        if (g + 1 < end)
         {
-            c4n = cj4[j4 + kPruneWarps];
+            imn = *reinterpret_cast<const int4*>(&g[1].imei[0]);
         }
-        // per half: the bits to test (all set bits), the outer mask kept so far, the inner mask
-        const unsigned check[kSplit]  = { c4.imei[0].imask, c4.imei[1].imask };
-        unsigned       full_m[kSplit] = { check[0], check[1] };
-        unsigned       nw[kSplit]     = { 0u, 0u };
-        const unsigned either         = check[0] | check[1];
-        if (!either)
+        if (g + 3 < end)
+        {
+            cj2 = g[3].cj[jm];
+        }
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncwarp();
+        if (!(check0 | check1))
         {
             continue;
         }
-        // the j-atoms of the group's j-clusters with bits to test, all loaded before any is tested
-        // (one memory latency per group instead of one per j-cluster)
-        float4 xj[kJg];
+        const float4* const rec = sm.x[b][jm];
+        float2              xj[4], yj[4], zj[4], m[4];
 #pragma unroll
-        for (int jm = 0; jm < kJg; jm++)
+        for (int h = 0; h < 2; h++)
         {
-            if ((either >> (jm * kNcl)) & 0xffu)
+            const float4 x = rec[h], y = rec[2 + h], z = rec[4 + h];
+            xj[2 * h]     = p_sub(make_float2(x.x, x.y), ox2);
+            xj[2 * h + 1] = p_sub(make_float2(x.z, x.w), ox2);
+            yj[2 * h]     = p_sub(make_float2(y.x, y.y), oy2);
+            yj[2 * h + 1] = p_sub(make_float2(y.z, y.w), oy2);
+            zj[2 * h]     = p_sub(make_float2(z.x, z.y), oz2);
+            zj[2 * h + 1] = p_sub(make_float2(z.z, z.w), oz2);
+            m[2 * h] = m[2 * h + 1] = make_float2(3.0e38f, 3.0e38f);
+        }
+#pragma unroll
+        for (int a = 0; a < kCl; a += 2)
+        {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
             {
-                xj[jm] = xq[c4.cj[jm] * kCl + jj];
+                const float2 t = __ffma2_rn(xm[a], xj[q], __ffma2_rn(ym[a], yj[q], __ffma2_rn(zm[a], zj[q], ni[a])));
+                const float2 u = __ffma2_rn(
+                        xm[a + 1], xj[q], __ffma2_rn(ym[a + 1], yj[q], __ffma2_rn(zm[a + 1], zj[q], ni[a + 1])));
+                m[q] = make_float2(min3(m[q].x, t.x, u.x), min3(m[q].y, t.y, u.y));
             }
         }
 #pragma unroll
-        for (int jm = 0; jm < kJg; jm++)
+        for (int q = 0; q < 4; q++)
         {
-            const unsigned sh  = jm * kNcl;
-            const unsigned sel = (either >> sh) & 0xffu;
-            if (!sel)
-            {
-                continue;
-            }
-            const float2 xjj = make_float2(xj[jm].x, xj[jm].x);
-            const float2 yjj = make_float2(xj[jm].y, xj[jm].y);
-            const float2 zjj = make_float2(xj[jm].z, xj[jm].z);
-            // per lane: bit i set when one of this lane's two pairs with i-cluster i is in range,
-            // shifted in from the top i-cluster down.  All 8 i-clusters are tested (no per-cluster
-            // branch); the flag is the sign of r^2 - cutoff^2 for the smaller r^2 of the two (the
-            // difference of two floats is negative exactly when the first is smaller), taken for
-            // two i-clusters at once in packed arithmetic.  r^2 = fma(dz, dz, fma(dy, dy, dx dx)),
-            // the contraction of the reference's norm2 in its prune kernel.
-            unsigned fin = 0u, fout = 0u;
-#pragma unroll
-            for (int i = kNcl - 1; i >= 0; i -= 2)
-            {
-                float mm[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++)
-                {
-                    const float2   dx = p_sub(xi[i - u], xjj);
-                    const float2   dy = p_sub(yi[i - u], yjj);
-                    const float2   dz = p_sub(zi[i - u], zjj);
-                    const float2   r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                    mm[u]             = __uint_as_float(min(__float_as_uint(r2.x), __float_as_uint(r2.y)));
-                }
-                const float2 m2   = make_float2(mm[0], mm[1]);
-                const float2 din  = p_sub(m2, inner2x2);
-                const float2 dout = p_sub(m2, outer2x2);
-                fin               = __funnelshift_l(__float_as_uint(din.x), fin, 1);
-                fin               = __funnelshift_l(__float_as_uint(din.y), fin, 1);
-                fout              = __funnelshift_l(__float_as_uint(dout.x), fout, 1);
-                fout              = __funnelshift_l(__float_as_uint(dout.y), fout, 1);
-            }
-            // any pair of the (i-cluster, half) within range: one OR over the lanes of
-            // {inner half 0, outer half 0, inner half 1, outer half 1}, 8 bits each
-            const unsigned w  = __reduce_or_sync(full, (fin | (fout << 8)) << hshift);
-            const unsigned t0 = check[0] & (0xffu << sh), t1 = check[1] & (0xffu << sh);
-            nw[0] |= ((w & 0xffu) << sh) & t0;
-            nw[1] |= (((w >> 16) & 0xffu) << sh) & t1;
-            full_m[0] &= ~(t0 & ~(((w >> 8) & 0xffu) << sh));
-            full_m[1] &= ~(t1 & ~((w >> 24) << sh));
+            m[q] = __fadd2_rn(m[q], __ffma2_rn(zj[q], zj[q], __ffma2_rn(yj[q], yj[q], __fmul2_rn(xj[q], xj[q]))));
         }
-        if (lane < kSplit)
+        float m0 = fminf(min3(m[0].x, m[1].x, m[2].x), m[3].x);
+        float m1 = fminf(min3(m[0].y, m[1].y, m[2].y), m[3].y);
+        // distances of the minima from the radii (of unset bits too: one vote for all)
+        const float d0 = fminf(fabsf(m0 - inner2), fabsf(m0 - outer2));
+        const float d1 = fminf(fabsf(m1 - inner2), fabsf(m1 - outer2));
+        if (__any_sync(full, fminf(d0, d1) <= eps))
         {
-            imask_outer[2 * j4 + lane]                 = lane == 0 ? full_m[0] : full_m[1];
-            const_cast<Cj4*>(cj4)[j4].imei[lane].imask = lane == 0 ? nw[0] : nw[1];
+            if (d0 <= eps)
+            {
+                m0 = exact_min_r2(xi, xq + (size_t)cj_own * kCl, sx, sy, sz);
+            }
+            if (d1 <= eps)
+            {
+                m1 = exact_min_r2(xi, xq + (size_t)cj_own * kCl + kCl / kSplit, sx, sy, sz);
+            }
+        }
+        if (any_ff)
+        {
+            const float4 xa = rec[0], xb = rec[1];
+            if (has_fill && (xa.x == kFarAway || xa.z == kFarAway || xb.x == kFarAway || xb.z == kFarAway))
+            {
+                m0 = fminf(m0, ff);
+            }
+            if (has_fill && (xa.y == kFarAway || xa.w == kFarAway || xb.y == kFarAway || xb.w == kFarAway))
+            {
+                m1 = fminf(m1, ff);
+            }
+        }
+        const unsigned nw0 = check0 & __ballot_sync(full, m0 < inner2);
+        const unsigned nw1 = check1 & __ballot_sync(full, m1 < inner2);
+        const unsigned ou0 = check0 & __ballot_sync(full, m0 < outer2);
+        const unsigned ou1 = check1 & __ballot_sync(full, m1 < outer2);
+        if (lane == 0)
+        {
+            *reinterpret_cast<uint2*>(om) = make_uint2(ou0, ou1);
+            g->imei[0].imask              = nw0;
+            g->imei[1].imask              = nw1;
         }
     }
 }
@@ -328,12 +414,12 @@ __device__ void prune_entry_rolling(const Sci& s, const Cj4* cj4, const unsigned
     }
 }
 
-// Fresh prune: a block per list entry, its warps over the entry's groups.  Rolling prune: a warp
-// per list entry.
+// A warp per list entry in both passes.
 template<int kPruneWarps, bool kFresh>
 __global__ void __launch_bounds__(32 * kPruneWarps, kFresh ? 4 : 6) k_prune(DeviceView v, int part, int nparts)
 {
-    __shared__ RollSmem rsm[kFresh ? 1 : kPruneWarps];
+    __shared__ RollSmem  rsm[kFresh ? 1 : kPruneWarps];
+    __shared__ FreshSmem fsm[kFresh ? kPruneWarps : 1];
     const int           numSci = v.hdr->num_sci;
     if (v.hdr->status & (kStatusListOverflow | kStatusExclOverflow))
     {
@@ -342,19 +428,22 @@ __global__ void __launch_bounds__(32 * kPruneWarps, kFresh ? 4 : 6) k_prune(Devi
     if constexpr (kFresh)
     {
         // the next entry's record is loaded while the current entry is pruned
-        Sci sn{};
-        if (blockIdx.x < numSci)
+        const int stride = gridDim.x * kPruneWarps;
+        int       e      = blockIdx.x * kPruneWarps + (threadIdx.x >> 5);
+        Sci       sn{};
+        if (e < numSci)
         {
-            sn = v.sci[blockIdx.x];
+            sn = v.sci[e];
         }
-        for (int e = blockIdx.x; e < numSci; e += gridDim.x)
+        for (; e < numSci; e += stride)
         {
             const Sci s = sn;
-            if (e + gridDim.x < numSci)
+            if (e + stride < numSci)
             {
-                sn = v.sci[e + gridDim.x];
+                sn = v.sci[e + stride];
             }
-            prune_entry_fresh<kPruneWarps>(s, v.cj4, v.imask_outer, v.xq, v.shiftvec, v.rlist2, v.rlist_inner2);
+            prune_entry_fresh(s, v.cj4, v.imask_outer, v.xq, v.xqp, v.shiftvec, v.rlist2, v.rlist_inner2,
+                              fsm[threadIdx.x >> 5]);
         }
     }
     else
@@ -396,16 +485,17 @@ __global__ void __launch_bounds__(32 * kPruneWarps)
         k_batch_prune(const BatchSys* sys, const int* entry_prefix, int nsys, float outer2, float inner2, int part,
                       int nparts)
 {
-    __shared__ RollSmem rsm[kFresh ? 1 : kPruneWarps];
+    __shared__ RollSmem  rsm[kFresh ? 1 : kPruneWarps];
+    __shared__ FreshSmem fsm[kFresh ? kPruneWarps : 1];
     const int           total = entry_prefix[nsys];
     if constexpr (kFresh)
     {
-        for (int e = blockIdx.x; e < total; e += gridDim.x)
+        for (int e = blockIdx.x * kPruneWarps + (threadIdx.x >> 5); e < total; e += gridDim.x * kPruneWarps)
         {
             const int       k = batch_system_of(entry_prefix, nsys, e);
             const BatchSys& b = sys[k];
-            prune_entry_fresh<kPruneWarps>(b.sci[e - entry_prefix[k]], b.cj4, b.imask_outer, b.xq, b.shiftvec,
-                                           outer2, inner2);
+            prune_entry_fresh(b.sci[e - entry_prefix[k]], b.cj4, b.imask_outer, b.xq, b.xqp, b.shiftvec, outer2,
+                              inner2, fsm[threadIdx.x >> 5]);
         }
     }
     else

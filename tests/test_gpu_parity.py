@@ -155,6 +155,40 @@ def test_fresh_prune_masks_bit_exact(name):
     assert outer_sets(pg) == outer_sets(po)
 
 
+def _sparse(n=150, edge=9.0):
+    # clusters several nm wide, most slots of the cells filled up: coordinates far from the cell's first atom
+    return systems.spc_water(n // 3, edge, seed=21)
+
+
+def _masks(p, outer=True):
+    rows = []
+    for sc, sh, c0, c1 in p["sci"]:
+        rows += [(sc, sh, *p["cj4"][j][:4], *p["cj4"][j][[4, 6]].view(np.uint32),
+                  *(p["imask_outer"][j] if outer else ())) for j in range(c0, c1)]
+    return sorted(tuple(int(v) for v in r) for r in rows)
+
+
+@pytest.mark.parametrize("inner", [0.9, 0.95, 0.9999])
+@pytest.mark.parametrize("name", ["water_tiny", "water_small_box", "lj_liquid", "sparse"])
+def test_fresh_prune_masks_forms(name, inner):
+    """Inner and outer masks equal the oracle's bit for bit on boxes with partly filled clusters, boxes
+    shorter than two list radii and clusters several nm wide; then the inner masks for atoms that moved
+    (a second full prune: the oracle keeps the outer mask of a half without inner bits, the engine
+    clears it)."""
+    s = _sparse() if name == "sparse" else SYSTEMS[name]()
+    calc, o = _pair(s, rlist_inner=inner, prune=10)
+    o.prune(fresh=True)
+    assert _masks(calc.pairlist()) == _masks(o.pairlist())
+    x = systems.perturb(s.x, np.random.default_rng(5), 0.05)
+    calc.compute(x)
+    calc.prune_device(-1)
+    calc.synchronize()
+    o.set_x(x)
+    o.prune(fresh=True)
+    assert _masks(calc.pairlist(), False) == _masks(o.pairlist(), False)
+    calc.close()
+
+
 @pytest.mark.parametrize("name", list(SYSTEMS))
 @pytest.mark.parametrize("coulomb", [nblib.CoulombType.Pme, nblib.CoulombType.ReactionField])
 def test_forces_energies_virial_vs_oracle(name, coulomb):
