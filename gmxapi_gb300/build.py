@@ -35,6 +35,12 @@ UNITS = {
     "nbx_md.cu": [],
     "nbx_fep.cu": [],
     "nbx_fft.cu": [],
+    "nbx_fft_len0.cu": [],
+    "nbx_fft_len1.cu": [],
+    "nbx_fft_len2.cu": [],
+    "nbx_fft_len3.cu": [],
+    "nbx_fft_len4.cu": [],
+    "nbx_fft_len5.cu": [],
 }
 
 

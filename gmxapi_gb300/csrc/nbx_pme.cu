@@ -16,8 +16,8 @@
 //    src/gromacs/ewald/pme_solve.cpp:332-587);
 //  - the force gather (gather_f_bsplines / do_fspline,
 //    src/gromacs/ewald/pme_gather.cpp:78-360).
-// The 3-D real<->complex transforms are hand-written (nbx_fft.cu: one warp per line, Stockham
-// stages; unnormalised both ways, like the reference's).  Spreading accumulates with float atomics (16-byte vector reductions
+// The 3-D real<->complex transforms are hand-written (nbx_fft_len.cuh, nbx_fft.cu; unnormalised
+// both ways, like the reference's).  Spreading accumulates with float atomics (16-byte vector reductions
 // when nz is a multiple of 4); the energy and the virial terms are summed per warp in
 // float and across the grid in FP64.
 //
@@ -28,12 +28,12 @@
 #include "nbx_internal.cuh"
 
 #include "nbx_fft.cuh"
+#include "nbx_pme_solve.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <string>
-#include <type_traits>
 #include <vector>
 
 namespace
@@ -41,11 +41,9 @@ namespace
 
 constexpr int kOrder = 4;  // pme_order (grid points per dimension and atom)
 
-struct PmeDims
-{
-    int   n[3];
-    float rec[3];  // recipbox diagonal: 1 / box edge (invertBoxMatrix, math/invertmatrix.cpp:62-64)
-};
+using nbx::PmeDims;
+using nbx::solve_finish;
+using nbx::solve_point;
 
 // CALC_SPLINE(4) for the fraction dr: weights th[0..3] and derivatives dth[0..3]
 __device__ __forceinline__ void bspline4(float dr, float th[4], float dth[4])
@@ -205,138 +203,12 @@ constexpr int kSolveMaxBlocks = 4096;  // one point per thread up to 1M points, 
 // counter, and thousands of same-address atomics would serialise in L2.
 constexpr int kSolveEnergyBlocksPerSm = 4;
 
-// The solve's energy / virial sums: per warp in float, per block in FP64 into partials[block][8];
-// the last block to finish (completion counter) adds the partials in FP64 and writes
-// energy = 0.5 sum, virial = 0.25 sum.
-__device__ void solve_finish(const float acc[7], double* partials, unsigned int* done, double* energy_out,
-                             double* virial_out)
-{
-    __shared__ double red[7][kSolveThreads / 32];
-    __shared__ bool   last;
-    const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < 7; k++)
-    {
-        float v = acc[k];
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            v += __shfl_xor_sync(0xffffffffu, v, o);
-        }
-        if (lane == 0)
-        {
-            red[k][warp] = (double)v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 7)
-    {
-        double v = 0.0;
-        for (int w = 0; w < kSolveThreads / 32; w++)
-        {
-            v += red[threadIdx.x][w];
-        }
-        partials[blockIdx.x * 8 + threadIdx.x] = v;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last)
-    {
-        return;
-    }
-    // the last block: FP64 sum of every block's partials
-    __threadfence();
-    double sum[7] = { 0, 0, 0, 0, 0, 0, 0 };
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-    {
-        for (int k = 0; k < 7; k++)
-        {
-            sum[k] += __ldcg(&partials[b * 8 + k]);
-        }
-    }
-    __syncthreads();
-    for (int k = 0; k < 7; k++)
-    {
-        double v = sum[k];
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            v += __shfl_xor_sync(0xffffffffu, v, o);
-        }
-        if (lane == 0)
-        {
-            red[k][warp] = v;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        double tot[7];
-        for (int k = 0; k < 7; k++)
-        {
-            tot[k] = 0.0;
-            for (int w = 0; w < kSolveThreads / 32; w++)
-            {
-                tot[k] += red[k][w];
-            }
-        }
-        if (energy_out)
-        {
-            energy_out[0] = 0.5 * tot[0];
-        }
-        if (virial_out)
-        {
-            virial_out[0]                 = 0.25 * tot[1];
-            virial_out[1] = virial_out[3] = 0.25 * tot[2];
-            virial_out[2] = virial_out[6] = 0.25 * tot[3];
-            virial_out[4]                 = 0.25 * tot[4];
-            virial_out[5] = virial_out[7] = 0.25 * tot[5];
-            virial_out[8]                 = 0.25 * tot[6];
-        }
-        *done = 0u;  // ready for the next solve on this stream
-    }
-}
-
-// One point (kx, ky, kz) != 0 of solve_pme_yzx (pme_solve.cpp:332-587): scales c by eterm and, with
-// energies, adds its energy and virial terms to acc.
-__device__ __forceinline__ void solve_point(const PmeDims& d, const float* __restrict__ bsp, float elfac, float factor,
-                                            float pivol, int kx, int ky, int kz, bool energy, float2& c, float acc[7])
-{
-    const int   mx    = kx < (d.n[0] + 1) / 2 ? kx : kx - d.n[0];
-    const int   my    = ky < (d.n[1] + 1) / 2 ? ky : ky - d.n[1];
-    const float mhx   = (float)mx * d.rec[0];
-    const float mhy   = (float)my * d.rec[1];
-    const float mhz   = (float)kz * d.rec[2];
-    const float m2    = mhx * mhx + mhy * mhy + mhz * mhz;
-    const float by    = pivol * bsp[d.n[0] + ky];
-    const float den   = m2 * bsp[d.n[0] + d.n[1] + kz] * by * bsp[kx];
-    const float eterm = elfac / den * expf(-factor * m2);
-    if (energy)
-    {
-        const float corner  = (kz == 0 || kz == (d.n[2] + 1) / 2) ? 0.5f : 1.0f;
-        const float struct2 = 2.0f * (c.x * c.x + c.y * c.y);
-        const float ets2    = corner * eterm * struct2;
-        const float ets2vf  = ets2 * ((factor * m2 + 1.0f) * 2.0f / m2);
-        acc[0] += ets2;
-        acc[1] += ets2vf * mhx * mhx - ets2;
-        acc[2] += ets2vf * mhx * mhy;
-        acc[3] += ets2vf * mhx * mhz;
-        acc[4] += ets2vf * mhy * mhy - ets2;
-        acc[5] += ets2vf * mhy * mhz;
-        acc[6] += ets2vf * mhz * mhz - ets2;
-    }
-    c.x *= eterm;
-    c.y *= eterm;
-}
-
 // The x transform of the forward FFT, the solve and the x transform of the backward FFT in one
 // pass over the half-complex grid (the x lines are the last forward and the first backward
 // transform): block (ky, z-tile) loads the tile [nx][T] of x lines, warp c transforms column c,
 // solves its points (kx, ky, kz = tile * T + c) and transforms it back; energy and virial sums as
-// k_pme_solve's.
-template<bool kEnergy, int kN>
+// k_pme_solve's.  Lengths without a compile-time transform (nbx_fft_len.cuh).
+template<bool kEnergy>
 __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAxis ax, PmeDims d, float2* cgrid,
                                                                    const float* __restrict__ bsp, float elfac,
                                                                    float factor, float pivol, int ntiles, double* partials,
@@ -345,7 +217,7 @@ __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAx
 {
     constexpr int T    = nbx::kFftTile;
     extern __shared__ float2 xsm[];
-    const int     n    = kN > 0 ? kN : ax.n;  // nx
+    const int     n    = ax.n;  // nx
     const int     nzc  = d.n[2] / 2 + 1;
     float2*       W    = xsm;
     float2*       tile = xsm + n;                  // [n][T + 1]
@@ -373,7 +245,7 @@ __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAx
         float2*   s   = scr + (size_t)warp * n;
         const int kz  = t * T + warp;
         // forward along x, then the solve on the column wherever the transform left it
-        const bool in_s = nbx::fft_line_any<kN, false>(col, T + 1, s, 1, W, ax, lane);
+        const bool in_s = nbx::fft_line<false>(col, T + 1, s, 1, W, ax, lane);
         float2*    v    = in_s ? s : col;
         const int  vs   = in_s ? 1 : T + 1;
         for (int kx = lane; kx < n; kx += 32)
@@ -389,7 +261,7 @@ __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAx
         // backward along x
         float2*    other = in_s ? col : s;
         const int  os    = in_s ? T + 1 : 1;
-        const bool moved = nbx::fft_line_any<kN, true>(v, vs, other, os, W, ax, lane);
+        const bool moved = nbx::fft_line<true>(v, vs, other, os, W, ax, lane);
         // the result is in `other` when moved; bring it to the tile column
         if (moved != in_s)
         {
@@ -417,9 +289,8 @@ __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAx
 
 // solve_pme_yzx over the half-complex grid: scales each element by eterm and sums the
 // energy and virial terms (energy = 0.5 sum, virial = 0.25 sum).  Per-point terms and
-// per-thread / per-warp sums are float (the reference sums them in `real`); each block
-// writes its 7 sums in FP64 to partials[block][8] and the last block to finish sums the
-// partials in FP64 (no same-address atomics on the sums).
+// per-thread / per-warp sums are float (the reference sums them in `real`), per block and
+// across blocks FP64 (solve_finish).
 __global__ void __launch_bounds__(kSolveThreads) k_pme_solve(PmeDims d, float2* cgrid, const float* __restrict__ bsp,
                                                              float elfac, float factor, float pivol, double* partials,
                                                              unsigned int* done, double* energy_out,
@@ -666,7 +537,7 @@ struct nbx_pme
     float*       grid      = nullptr;  // real grid [nx][ny][nz]
     float2*      cgrid     = nullptr;  // half-complex grid [nx][ny][nz/2+1]
     float*       bsp       = nullptr;  // spline moduli x | y | z
-    double*      sums      = nullptr;  // solve partials [kSolveMaxBlocks][8]: energy + 6 virial terms
+    double*      sums      = nullptr;  // solve sums [kSolveReplicas][8]: energy + 6 virial terms, zero between solves
     unsigned*    done      = nullptr;  // blocks of the running solve that have written their partials
     int          num_sms   = 1;
     nbx::FftPlan3 fft{};  // the hand-written 3D real <-> half-complex transform (nbx_fft.cu)
@@ -743,17 +614,10 @@ cudaError_t launch_solve(nbx_pme* p, float2* cgrid, double* d_energy, double* d_
     return cudaGetLastError();
 }
 
-// The fused x pass + Coulomb solve: one block per (ky, z-tile), the solve's partials sized for
-// kSolveMaxBlocks blocks.
-int x_solve_blocks(const nbx_pme* p)
-{
-    const int nzc = p->d.n[2] / 2 + 1;
-    return p->d.n[1] * ((nzc + nbx::kFftTile - 1) / nbx::kFftTile);
-}
-
+// The x pass and the Coulomb solve in one kernel (any length whose line fits the shared memory).
 bool fused_x_solve(const nbx_pme* p)
 {
-    return !p->lj && p->d.n[0] > 1 && x_solve_blocks(p) <= kSolveMaxBlocks && p->fused_smem_ok;
+    return !p->lj && p->d.n[0] > 1 && (p->fft.len[0] || p->fused_smem_ok);
 }
 
 cudaError_t launch_x_solve(nbx_pme* p, double* d_energy, double* d_virial)
@@ -762,32 +626,26 @@ cudaError_t launch_x_solve(nbx_pme* p, double* d_energy, double* d_virial)
     const float  factor = (float)(M_PI * M_PI) / (p->beta * p->beta);
     const float  elfac  = (float)nbx::one_4pi_eps0() / p->epsilon_r;
     const float  pivol  = (float)M_PI * (float)vol;
+    if (p->fft.len[0])
+    {
+        const nbx::PmeSolve ps = { p->d, p->bsp, elfac, factor, pivol, p->sums, p->done, d_energy, d_virial };
+        p->fft.len[0]->x_solve(p->fft.ax[0].roots, p->cgrid, ps, p->stream);
+        return cudaGetLastError();
+    }
     const int    nzc    = p->d.n[2] / 2 + 1;
     const int    ntiles = (nzc + nbx::kFftTile - 1) / nbx::kFftTile;
     const size_t smem   = nbx::fft_tiled_smem(p->d.n[0]);
-    const bool   energy = d_energy || d_virial;
-    auto         go     = [&](auto kn) {
-        constexpr int kN = decltype(kn)::value;
-        if (energy)
-        {
-            k_pme_fft_x_solve<true, kN><<<x_solve_blocks(p), kSolveThreads, smem, p->stream>>>(
-                    p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums, p->done, d_energy,
-                    d_virial);
-        }
-        else
-        {
-            k_pme_fft_x_solve<false, kN><<<x_solve_blocks(p), kSolveThreads, smem, p->stream>>>(
-                    p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums, p->done, nullptr,
-                    nullptr);
-        }
-    };
-    switch (p->d.n[0])
+    if (d_energy || d_virial)
     {
-#define NBX_FFT_CASE(L)                                                                                                \
-    case L: go(std::integral_constant<int, L>{}); break;
-        NBX_FFT_FIXED_LENGTHS(NBX_FFT_CASE)
-#undef NBX_FFT_CASE
-        default: go(std::integral_constant<int, 0>{}); break;
+        k_pme_fft_x_solve<true><<<p->d.n[1] * ntiles, kSolveThreads, smem, p->stream>>>(
+                p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums, p->done, d_energy,
+                d_virial);
+    }
+    else
+    {
+        k_pme_fft_x_solve<false><<<p->d.n[1] * ntiles, kSolveThreads, smem, p->stream>>>(
+                p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums, p->done, nullptr,
+                nullptr);
     }
     return cudaGetLastError();
 }
@@ -883,7 +741,8 @@ int nbx_pme_create(const float* box, const int* grid, float ewaldcoeff_q, float 
     if (e == cudaSuccess) e = cudaMalloc(&p->grid, sizeof(float) * real_points(p));
     if (e == cudaSuccess) e = cudaMalloc(&p->cgrid, sizeof(float2) * complex_points(p));
     if (e == cudaSuccess) e = cudaMalloc(&p->bsp, sizeof(float) * (grid[0] + grid[1] + grid[2]));
-    if (e == cudaSuccess) e = cudaMalloc(&p->sums, sizeof(double) * 8 * kSolveMaxBlocks);
+    if (e == cudaSuccess) e = cudaMalloc(&p->sums, sizeof(double) * 8 * nbx::kSolveReplicas);
+    if (e == cudaSuccess) e = cudaMemset(p->sums, 0, sizeof(double) * 8 * nbx::kSolveReplicas);
     if (e == cudaSuccess) e = cudaMalloc(&p->done, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(p->done, 0, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, device);
@@ -907,9 +766,9 @@ int nbx_pme_create(const float* box, const int* grid, float ewaldcoeff_q, float 
     {
         const size_t xs  = nbx::fft_tiled_smem(grid[0]);
         p->fused_smem_ok = xs <= 48 * 1024
-                           || (cudaFuncSetAttribute(k_pme_fft_x_solve<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           || (cudaFuncSetAttribute(k_pme_fft_x_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)xs) == cudaSuccess
-                               && cudaFuncSetAttribute(k_pme_fft_x_solve<false, 0>,
+                               && cudaFuncSetAttribute(k_pme_fft_x_solve<false>,
                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs) == cudaSuccess);
     }
     if (!p->plan)
