@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(round32(kCols* Shape<R1, R2>::threads))
     }
     if (kEnergy)
     {
-        solve_finish(acc, ps.partials, ps.done, ps.energy_out, ps.virial_out);
+        solve_add(acc, ps.partials);
     }
 }
 
@@ -508,7 +508,7 @@ template<int R1, int R2>
 void launch_x_solve(const float2* roots, float2* cgrid, const PmeSolve& ps, cudaStream_t s)
 {
     const int ntiles = (ps.d.n[2] / 2 + 1 + kCols - 1) / kCols, threads = round32(kCols * Shape<R1, R2>::threads);
-    if (ps.energy_out || ps.virial_out)
+    if (ps.partials)
     {
         k_x_solve<R1, R2, true><<<ps.d.n[1] * ntiles, threads, 0, s>>>(roots, cgrid, ps, ntiles);
     }

@@ -13,32 +13,34 @@ struct PmeDims
     float rec[3];  // recipbox diagonal: 1 / box edge (invertBoxMatrix, math/invertmatrix.cpp:62-64)
 };
 
-// What a Coulomb solve needs besides the grid: spline moduli x | y | z, the three scalars of
-// solve_pme_yzx, and where the energy and virial sums go.
+// What the Coulomb solve of the x pass needs besides the grid: spline moduli x | y | z, the three scalars
+// of solve_pme_yzx, and the energy and virial sums.
 struct PmeSolve
 {
     PmeDims      d;
     const float* bsp;
     float        elfac, factor, pivol;
-    double*      partials;  // [kSolveReplicas][8], zero between solves
-    unsigned*    done;      // blocks that have added their sums, zero between solves
-    double*      energy_out;
-    double*      virial_out;
+    double*      partials;  // [kSolveReplicas][8], zero between solves; nullptr: no energy or virial
+};
+
+// Where the kernel that ends an evaluation (the gather) writes the solve's energy and virial.  Its first
+// warp sums the replicas: at 120^3 a completion counter and a last block in the x pass cost 8 us.
+struct PmeTotals
+{
+    double* partials;  // nullptr: nothing to write
+    double* energy_out;
+    double* virial_out;
 };
 
 // Copies of the 7 sums that blocks add to (block b to copy b mod 32): FP64 adds on one address
-// serialise in L2, and the last block then reads 32 copies instead of one per block (960 blocks'
-// partials read by one block took about 8 us at 120^3).
+// serialise in L2.
 constexpr int kSolveReplicas = 32;
 
-// The solve's energy / virial sums: per warp in float, per block in FP64 added to one of the
-// replicas; the last block to finish (completion counter) sums the replicas, clears them and writes
-// energy = 0.5 sum, virial = 0.25 sum.  Blocks of at most 256 threads, a multiple of 32.
-__device__ __forceinline__ void solve_finish(const float acc[7], double* partials, unsigned int* done,
-                                             double* energy_out, double* virial_out)
+// The block's energy / virial sums: per warp in float, per block in FP64 added to one of the replicas.
+// Blocks of at most 256 threads, a multiple of 32.
+__device__ __forceinline__ void solve_add(const float acc[7], double* partials)
 {
     __shared__ double red[7][8];
-    __shared__ bool   last;
     const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     for (int k = 0; k < 7; k++)
     {
@@ -61,24 +63,18 @@ __device__ __forceinline__ void solve_finish(const float acc[7], double* partial
             v += red[threadIdx.x][w];
         }
         atomicAdd(&partials[(blockIdx.x % kSolveReplicas) * 8 + threadIdx.x], v);
-        __threadfence();
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last || warp != 0)
-    {
-        return;
-    }
-    // the last block: lane r sums replica r over the lanes of warp 0, per term
-    __threadfence();
-    double tot[7];
+}
+
+// One warp: the replicas' sums (complete: of an earlier kernel, or behind a completion counter), which
+// are cleared for the next solve; energy = 0.5 sum, virial = 0.25 sum.
+__device__ __forceinline__ void solve_total(double* partials, double* energy_out, double* virial_out)
+{
+    const int lane = threadIdx.x & 31;
+    double    tot[7];
     for (int k = 0; k < 7; k++)
     {
-        double v                  = __ldcg(&partials[lane * 8 + k]);
+        double v               = __ldcg(&partials[lane * 8 + k]);
         partials[lane * 8 + k] = 0.0;
         for (int o = 16; o > 0; o >>= 1)
         {
@@ -101,7 +97,33 @@ __device__ __forceinline__ void solve_finish(const float acc[7], double* partial
             virial_out[5] = virial_out[7] = 0.25 * tot[5];
             virial_out[8]                 = 0.25 * tot[6];
         }
-        *done = 0u;  // ready for the next solve on this stream
+    }
+}
+
+// A solve on its own (no gather follows): the last block to finish writes the totals.
+__device__ __forceinline__ void solve_finish(const float acc[7], double* partials, unsigned int* done,
+                                             double* energy_out, double* virial_out)
+{
+    __shared__ bool last;
+    solve_add(acc, partials);
+    if (threadIdx.x < 7)
+    {
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last && threadIdx.x < 32)
+    {
+        __threadfence();
+        solve_total(partials, energy_out, virial_out);
+        if (threadIdx.x == 0)
+        {
+            *done = 0u;  // ready for the next solve on this stream
+        }
     }
 }
 

@@ -310,3 +310,33 @@ def test_water_288k_matches_oracle(pm):
     net = f.astype(np.float64).sum(0)
     assert np.abs(net - ref_f.sum(0)).max() <= 1e-5 * np.abs(ref_f).max() * np.sqrt(s.n)
     p.close()
+
+
+@pytest.mark.parametrize("layout,grid", [("uniform", (48, 48, 48)), ("images", (44, 52, 28)), ("crowded", (40, 36, 60)),
+                                         ("one_brick", (32, 32, 32))])
+def test_filed_atoms_match_oracle(pm, layout, grid):
+    """Enough atoms per grid point for the passes that file them by 8 x 8 x 8 brick: grids that are no
+    multiples of 8, atoms in other images, some without charge, and boxes whose atoms crowd into a few
+    bricks (more than a brick holds).  Twice, so that the second call meets the first one's workspace."""
+    rng = np.random.default_rng(17)
+    box = (2.9, 3.1, 3.3)
+    n = 17001
+    frac = rng.random((n, 3))
+    if layout == "crowded":
+        frac = 0.4 * frac + 0.75
+    elif layout == "one_brick":
+        frac = 0.2 * frac + 0.01
+    elif layout == "images":
+        frac += rng.integers(-1, 2, size=(n, 3))
+    x = (frac * np.array(box)).astype(np.float32)
+    q = rng.normal(0.0, 0.4, n).astype(np.float32)
+    q[::7] = 0.0
+    p = pm.Pme(box, grid, 3.0, device=0)
+    for _ in range(2):
+        f = p.compute(x, q)
+        ref, energy, vir = P.compute(x, q, box, grid, 3.0, single=True)
+        assert rel_rms(f, ref) <= FORCE_RTOL
+        assert abs(p.energy - energy) <= ENERGY_RTOL * abs(energy)
+        assert np.abs(p.virial - vir).max() <= ENERGY_RTOL * np.abs(vir).max()
+        x = np.roll(x, 5, axis=0)
+    p.close()
