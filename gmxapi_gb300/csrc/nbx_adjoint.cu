@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         k_backward(DeviceView v, const float4* __restrict__ gnb, float4* dnb, double* gnbfp, int* work_counter,
                    const double* __restrict__ gE)
 {
+    pdl_begin();
     AdjConsts k{ 0.0f, 0.0f };
     if (gE)
     {
@@ -475,6 +476,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         k_batch_backward(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
                          double* gnbfp, int* work_counter, const double* __restrict__ gE)
 {
+    pdl_begin();
     __shared__ float2 nbfp_s[kAdjMaxTypes1 * kAdjMaxTypes1];
     __shared__ double gsum_s[2 * kAdjMaxTypes1 * kAdjMaxTypes1];
     // dynamic: per warp the i-side accumulators (64 i-atoms x 4 lane slots), then the type-pair
@@ -525,6 +527,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
 __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const float* __restrict__ gF, int* counter,
                                     double* gnbfp, int n_gnbfp)
 {
+    pdl_begin();
     // block (0, 0) also clears the work queue and the FP64 type-pair gradient table
     if (blockIdx.x == 0 && blockIdx.y == 0)
     {
@@ -553,6 +556,7 @@ __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const floa
 __global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ sys, const double* __restrict__ gE,
                                    float* gx, float* gq)
 {
+    pdl_begin();
     const BatchSys& b = sys[blockIdx.y];
     const int       a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= b.n)
@@ -580,6 +584,7 @@ __global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ s
 // Charges of all systems (concatenated atom order) into xq.w and each system's q.
 __global__ void k_batch_set_q(const BatchSys* __restrict__ sys, const float* __restrict__ q)
 {
+    pdl_begin();
     const BatchSys& b = sys[blockIdx.y];
     const int       k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= b.hdr->num_cells * kSc)
@@ -599,6 +604,7 @@ __global__ void k_batch_set_q(const BatchSys* __restrict__ sys, const float* __r
 __global__ void k_match_loss(const float* __restrict__ f, const float* __restrict__ ft, size_t n3, float* gF,
                              double* loss)
 {
+    pdl_begin();
     double acc = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x)
     {
@@ -624,6 +630,7 @@ __global__ void k_match_loss(const float* __restrict__ f, const float* __restric
 __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const float* __restrict__ gF, float4* gnb,
                               float4* dnb, int* counter, double* gnbfp, int n_gnbfp)
 {
+    pdl_begin();
     if (blockIdx.x == 0)
     {
         for (int i = threadIdx.x; i < n_gnbfp; i += blockDim.x)
@@ -663,6 +670,7 @@ __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const f
 __global__ void k_adj_finish(DeviceView v, const float4* __restrict__ dnb, const double* __restrict__ gE, float* gx,
                              float* gq, const double* __restrict__ gpad, double* gout)
 {
+    pdl_begin();
     if (gout && blockIdx.x == 0)
     {
         const int nt = v.ntypes1 - 1;
@@ -701,6 +709,7 @@ __global__ void k_adj_finish(DeviceView v, const float4* __restrict__ dnb, const
 // C12 = 4 eps s^12 (the combination nblib applies, api/nblib/gmxsetup.cpp:143-166).
 __global__ void k_lb_table(const double* __restrict__ sig, const double* __restrict__ eps, int nt, double* table)
 {
+    pdl_begin();
     for (int m = threadIdx.x; m < nt * nt; m += blockDim.x)
     {
         const int    i = m / nt, j = m - (m / nt) * nt;
@@ -720,6 +729,7 @@ __global__ void k_lb_table(const double* __restrict__ sig, const double* __restr
 __global__ void k_lb_table_backward(const double* __restrict__ sig, const double* __restrict__ eps, int nt,
                                     const double* __restrict__ gt, double* gsig, double* geps)
 {
+    pdl_begin();
     extern __shared__ double lbs[];  // [2][nt * nt]: d L / d sigma_ij, d L / d epsilon_ij
     double* gs = lbs;
     double* ge = lbs + nt * nt;
@@ -761,14 +771,14 @@ int adjoint_max_types1()
 
 cudaError_t launch_lb_table(const double* sig, const double* eps, int nt, double* table, cudaStream_t s)
 {
-    k_lb_table<<<1, 256, 0, s>>>(sig, eps, nt, table);
+    launch_pdl(k_lb_table, 1, 256, 0, s, sig, eps, nt, table);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lb_table_backward(const double* sig, const double* eps, int nt, const double* gtable,
                                      double* gsig, double* geps, cudaStream_t s)
 {
-    k_lb_table_backward<<<1, 256, 2 * sizeof(double) * nt * nt, s>>>(sig, eps, nt, gtable, gsig, geps);
+    launch_pdl(k_lb_table_backward, 1, 256, 2 * sizeof(double) * nt * nt, s, sig, eps, nt, gtable, gsig, geps);
     return cudaGetLastError();
 }
 
@@ -803,25 +813,28 @@ cudaError_t launch_backward(const DeviceView& v, const float* d_x, const float* 
 {
     const int tb    = 256;
     const int slots = v.g.cells_capacity * kSc;
-    k_adj_prepare<<<(slots + tb - 1) / tb, tb, 0, s>>>(v, d_x, d_gF, gnb, dnb, counter, d_gnbfp,
-                                                       2 * v.ntypes1 * v.ntypes1);
+    launch_pdl(k_adj_prepare, (slots + tb - 1) / tb, tb, 0, s, v, d_x, d_gF, gnb, dnb, counter, d_gnbfp,
+               2 * v.ntypes1 * v.ntypes1);
     const size_t dyn = adj_table_bytes(v.ntypes1);
     cudaError_t  e   = cudaSuccess;
     if (v.coulomb == 0)
     {
         e = adj_optin<k_backward<true>>(dyn);
-        k_backward<true><<<num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s>>>(v, gnb, dnb, d_gnbfp, counter, d_gE);
+        launch_pdl(k_backward<true>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, v, gnb, dnb, d_gnbfp, counter,
+                   d_gE);
     }
     else
     {
         e = adj_optin<k_backward<false>>(dyn);
-        k_backward<false><<<num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s>>>(v, gnb, dnb, d_gnbfp, counter, d_gE);
+        launch_pdl(k_backward<false>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, v, gnb, dnb, d_gnbfp, counter,
+                   d_gE);
     }
     if (e != cudaSuccess)
     {
         return e;
     }
-    k_adj_finish<<<std::max(1, (v.n + tb - 1) / tb), tb, 0, s>>>(v, dnb, d_gE, d_gx, d_gq, d_gnbfp, d_gnbfp_out);
+    launch_pdl(k_adj_finish, std::max(1, (v.n + tb - 1) / tb), tb, 0, s, v, dnb, d_gE, d_gx, d_gq, d_gnbfp,
+               d_gnbfp_out);
     return cudaGetLastError();
 }
 
@@ -830,32 +843,34 @@ cudaError_t launch_batch_backward(const DeviceView& cv, const BatchSys* sys, con
                                   double* d_gnbfp, int* counter, float* d_gx, float* d_gq, int num_sms, cudaStream_t s)
 {
     const int tb = 256;
-    k_batch_adj_prepare<<<dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s>>>(sys, d_gF, counter, d_gnbfp,
-                                                                             2 * cv.ntypes1 * cv.ntypes1);
+    launch_pdl(k_batch_adj_prepare, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_gF, counter, d_gnbfp,
+               2 * cv.ntypes1 * cv.ntypes1);
     const size_t dyn = adj_table_bytes(cv.ntypes1);
     cudaError_t  e   = cudaSuccess;
     if (cv.coulomb == 0)
     {
         e = adj_optin<k_batch_backward<true>>(dyn);
-        k_batch_backward<true><<<num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s>>>(cv, sys, prefix, nsys, d_gnbfp, counter, d_gE);
+        launch_pdl(k_batch_backward<true>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, cv, sys, prefix, nsys,
+                   d_gnbfp, counter, d_gE);
     }
     else
     {
         e = adj_optin<k_batch_backward<false>>(dyn);
-        k_batch_backward<false><<<num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s>>>(cv, sys, prefix, nsys, d_gnbfp, counter, d_gE);
+        launch_pdl(k_batch_backward<false>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, cv, sys, prefix, nsys,
+                   d_gnbfp, counter, d_gE);
     }
     if (e != cudaSuccess)
     {
         return e;
     }
-    k_batch_adj_finish<<<dim3((max_atoms + tb - 1) / tb, nsys), tb, 0, s>>>(cv, sys, d_gE, d_gx, d_gq);
+    launch_pdl(k_batch_adj_finish, dim3((max_atoms + tb - 1) / tb, nsys), tb, 0, s, cv, sys, d_gE, d_gx, d_gq);
     return cudaGetLastError();
 }
 
 cudaError_t launch_batch_set_q(const BatchSys* sys, int nsys, int max_slots, const float* d_q, cudaStream_t s)
 {
     const int tb = 256;
-    k_batch_set_q<<<dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s>>>(sys, d_q);
+    launch_pdl(k_batch_set_q, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_q);
     return cudaGetLastError();
 }
 
@@ -863,7 +878,7 @@ cudaError_t launch_match_loss(const float* d_f, const float* d_ft, size_t n3, fl
                               int num_sms, cudaStream_t s)
 {
     cudaMemsetAsync(d_loss, 0, sizeof(double), s);
-    k_match_loss<<<num_sms * 4, 256, 0, s>>>(d_f, d_ft, n3, d_gF, d_loss);
+    launch_pdl(k_match_loss, num_sms * 4, 256, 0, s, d_f, d_ft, n3, d_gF, d_loss);
     return cudaGetLastError();
 }
 
@@ -876,6 +891,7 @@ cudaError_t launch_set_nbfp(const DeviceView& v, const float* d_nbfp, cudaStream
 // nbfp table (with the all-zero filler type); the self energy follows the charges.
 __global__ void k_set_q(DeviceView v, const float* __restrict__ q)
 {
+    pdl_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= v.hdr->num_cells * kSc)
     {
@@ -890,6 +906,7 @@ __global__ void k_set_q(DeviceView v, const float* __restrict__ q)
 
 __global__ void k_set_nbfp(float2* nbfp, const float* __restrict__ src, int nt)
 {
+    pdl_begin();
     const int m   = blockIdx.x * blockDim.x + threadIdx.x;
     const int nt1 = nt + 1;
     if (m >= nt1 * nt1)
@@ -903,6 +920,7 @@ __global__ void k_set_nbfp(float2* nbfp, const float* __restrict__ src, int nt)
 
 __global__ void k_compact_gnbfp(const double* padded, double* out, int nt)
 {
+    pdl_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nt * nt)
     {
@@ -915,7 +933,7 @@ __global__ void k_compact_gnbfp(const double* padded, double* out, int nt)
 
 cudaError_t launch_compact_gnbfp(const double* padded, double* out, int nt, cudaStream_t s)
 {
-    k_compact_gnbfp<<<(nt * nt + 255) / 256, 256, 0, s>>>(padded, out, nt);
+    launch_pdl(k_compact_gnbfp, (nt * nt + 255) / 256, 256, 0, s, padded, out, nt);
     return cudaGetLastError();
 }
 
@@ -925,12 +943,13 @@ cudaError_t launch_set_parameters(const DeviceView& v, const float* d_q, const f
     if (d_q)
     {
         cudaMemcpyAsync(const_cast<float*>(v.q), d_q, sizeof(float) * v.n, cudaMemcpyDeviceToDevice, s);
-        k_set_q<<<(v.g.cells_capacity * kSc + tb - 1) / tb, tb, 0, s>>>(v, d_q);
+        launch_pdl(k_set_q, (v.g.cells_capacity * kSc + tb - 1) / tb, tb, 0, s, v, d_q);
     }
     if (d_nbfp)
     {
         const int nt = v.ntypes1 - 1;
-        k_set_nbfp<<<(v.ntypes1 * v.ntypes1 + tb - 1) / tb, tb, 0, s>>>(const_cast<float2*>(v.nbfp), d_nbfp, nt);
+        launch_pdl(k_set_nbfp, (v.ntypes1 * v.ntypes1 + tb - 1) / tb, tb, 0, s, const_cast<float2*>(v.nbfp), d_nbfp,
+                   nt);
     }
     return cudaGetLastError();
 }

@@ -105,6 +105,7 @@ __device__ int split_entry(const unsigned char* __restrict__ grp_pairs, Sci e, i
 
 __global__ void k_balance_count(DeviceView v, int min_ci_balanced)
 {
+    pdl_begin();
     const ListHeader* hdr = v.hdr;
     if (hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
     {
@@ -128,6 +129,7 @@ __global__ void k_balance_count(DeviceView v, int min_ci_balanced)
 // total goes to num_sci_split.
 __global__ void __launch_bounds__(1024) k_balance_scan(DeviceView v)
 {
+    pdl_begin();
     __shared__ int    warp_sums[32];
     const ListHeader* hdr = v.hdr;
     if (hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(1024) k_balance_scan(DeviceView v)
 
 __global__ void k_balance_write(DeviceView v)
 {
+    pdl_begin();
     const ListHeader* hdr = v.hdr;
     if (hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
     {
@@ -229,6 +232,7 @@ __global__ void k_balance_write(DeviceView v)
 // the rank among equal classes of a batch of 32 from __match_any_sync.
 __global__ void __launch_bounds__(kSortThreads) k_sort_entries(DeviceView v)
 {
+    pdl_begin();
     __shared__ int hist[kSortWarps][kMaxSizeClass + 1];  // counts, then each warp's first position
     ListHeader*    hdr = v.hdr;
     if (hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
@@ -355,10 +359,10 @@ cudaError_t launch_balance(const DeviceView& v, int min_ci_balanced, cudaStream_
 {
     const int tb     = 256;
     const int blocks = (v.sci_cap + tb - 1) / tb;
-    k_balance_count<<<blocks, tb, 0, s>>>(v, min_ci_balanced);
-    k_balance_scan<<<1, 1024, 0, s>>>(v);
-    k_balance_write<<<blocks, tb, 0, s>>>(v);
-    k_sort_entries<<<1, kSortThreads, 0, s>>>(v);
+    launch_pdl(k_balance_count, blocks, tb, 0, s, v, min_ci_balanced);
+    launch_pdl(k_balance_scan, 1, 1024, 0, s, v);
+    launch_pdl(k_balance_write, blocks, tb, 0, s, v);
+    launch_pdl(k_sort_entries, 1, kSortThreads, 0, s, v);
     return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@ namespace
 // and are flagged.
 __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsigned* status)
 {
+    pdl_begin();
     if (threadIdx.x != 0)
     {
         return;
@@ -52,6 +53,7 @@ __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsig
 // clears the grid-order force accumulators, so no per-system memset is needed.
 __global__ void k_batch_convert(const BatchSys* __restrict__ sys, const float* __restrict__ x)
 {
+    pdl_begin();
     const BatchSys& b = sys[blockIdx.y];
     const int       k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= b.hdr->num_cells * kSc)
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(256) k_batch_excl_energy(DeviceView cv, const 
                                                            const int* __restrict__ prefix, int nsys,
                                                            double* energies)
 {
+    pdl_begin();
     const int* chunk_prefix = prefix + nsys + 1;
     const int  total        = chunk_prefix[nsys];
     const int  lane         = threadIdx.x & 31;
@@ -118,6 +121,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         k_batch_force(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
                       int* work_counter, double* energies, double* fshift)
 {
+    pdl_begin();
     extern __shared__ float4 nbfp_s[];
     const int nt1 = cv.ntypes1;
     for (int k = threadIdx.x; k < nt1 * nt1; k += blockDim.x)
@@ -186,6 +190,7 @@ constexpr int kBatchReduceAtoms = 8;
 __global__ void k_batch_reduce(const BatchSys* __restrict__ sys, float* __restrict__ f, double* virial,
                                int do_virial)
 {
+    pdl_begin();
     const BatchSys& b = sys[blockIdx.y];
     float           w[9];
 #pragma unroll
@@ -264,6 +269,7 @@ __global__ void k_batch_reduce(const BatchSys* __restrict__ sys, float* __restri
 __global__ void k_batch_finish(const BatchSys* __restrict__ sys, int nsys, const double* energies,
                                const double* fshift, const double* virial, double* d_e, double* d_vir)
 {
+    pdl_begin();
     const int s = blockIdx.x;
     const int t = threadIdx.x;
     if (s >= nsys)
@@ -291,7 +297,7 @@ void launch_batch_force_t(const DeviceView& cv, const BatchSys* sys, const int* 
                           double* en, double* fs, int num_sms, cudaStream_t s)
 {
     const size_t smem = sizeof(float4) * (size_t)cv.ntypes1 * cv.ntypes1 + (size_t)(kT / 32) * kStageSmemPerWarp;
-    k_batch_force<kE, kW, kT, kM><<<num_sms * kM, kT, smem, s>>>(cv, sys, prefix, nsys, ctr, en, fs);
+    launch_pdl(k_batch_force<kE, kW, kT, kM>, num_sms * kM, kT, smem, s, cv, sys, prefix, nsys, ctr, en, fs);
 }
 
 template<bool kE, bool kW, int kT, int kM>
@@ -329,7 +335,7 @@ void launch_batch_force_variant(int variant, const DeviceView& cv, const BatchSy
 
 cudaError_t launch_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsigned* status, cudaStream_t s)
 {
-    k_batch_prefix<<<1, 32, 0, s>>>(sys, nsys, prefix, status);
+    launch_pdl(k_batch_prefix, 1, 32, 0, s, sys, nsys, prefix, status);
     return cudaGetLastError();
 }
 
@@ -337,7 +343,7 @@ cudaError_t launch_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsi
 cudaError_t launch_batch_convert(const BatchSys* sys, int nsys, int max_slots, const float* d_x, cudaStream_t s)
 {
     const int tb = 256;
-    k_batch_convert<<<dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s>>>(sys, d_x);
+    launch_pdl(k_batch_convert, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_x);
     return cudaGetLastError();
 }
 
@@ -354,10 +360,10 @@ cudaError_t launch_batch_compute(const DeviceView& cv, const BatchSys* sys, cons
     cudaError_t e      = cudaMemsetAsync(sums, 0, sums_bytes, s);
     const int  tb      = 256;
     dim3       gconv((max_slots + tb - 1) / tb, nsys);
-    k_batch_convert<<<gconv, tb, 0, s>>>(sys, d_x);
+    launch_pdl(k_batch_convert, gconv, tb, 0, s, sys, d_x);
     if (energy)
     {
-        k_batch_excl_energy<<<num_sms * 8, 256, 0, s>>>(cv, sys, prefix, nsys, en);
+        launch_pdl(k_batch_excl_energy, num_sms * 8, 256, 0, s, cv, sys, prefix, nsys, en);
     }
     const bool ewald = (cv.coulomb == 0);
     if (variant & 4)
@@ -385,10 +391,10 @@ cudaError_t launch_batch_compute(const DeviceView& cv, const BatchSys* sys, cons
             launch_batch_force_variant<false, false>(variant, cv, sys, prefix, nsys, counter, en, fs, num_sms, s);
     }
     dim3 gred((max_atoms + tb * kBatchReduceAtoms - 1) / (tb * kBatchReduceAtoms), nsys);
-    k_batch_reduce<<<gred, tb, 0, s>>>(sys, d_f, vir, d_vir ? 1 : 0);
+    launch_pdl(k_batch_reduce, gred, tb, 0, s, sys, d_f, vir, d_vir ? 1 : 0);
     if (energy)
     {
-        k_batch_finish<<<nsys, 32, 0, s>>>(sys, nsys, en, fs, vir, d_e, d_vir);
+        launch_pdl(k_batch_finish, nsys, 32, 0, s, sys, nsys, en, fs, vir, d_e, d_vir);
     }
     return e == cudaSuccess ? cudaGetLastError() : e;
 }

@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         k_batch_force_x2(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
                          int* work_counter, double* energies, double* fshift)
 {
+    pdl_begin();
     // {-6*C6, 12*C12, LJ energy shift of the pair, 0} per type pair (kernel_gpu_ref.cpp:327-336)
     extern __shared__ float4 smem_bx2[];
     float4*   nbfp_s = smem_bx2;
@@ -97,8 +98,8 @@ template<bool kE, int kW, int kT, int kM, int kD>
 cudaError_t launch_t(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys, int* ctr, double* en,
                      double* fs, int num_sms, cudaStream_t s)
 {
-    k_batch_force_x2<kE, kW, kT, kM, kD><<<num_sms * kM, kT, batch_x2_smem<kT, kD>(cv.ntypes1), s>>>(
-            cv, sys, prefix, nsys, ctr, en, fs);
+    launch_pdl(k_batch_force_x2<kE, kW, kT, kM, kD>, num_sms * kM, kT, batch_x2_smem<kT, kD>(cv.ntypes1), s, cv, sys,
+               prefix, nsys, ctr, en, fs);
     return cudaGetLastError();
 }
 

@@ -239,6 +239,7 @@ __device__ __forceinline__ int min_image(const DeviceView& v, float4 xi, float4 
 template<bool kEwald>
 __global__ void __launch_bounds__(kFepWarps * 32) k_fep(DeviceView v, FepView fp, int energy)
 {
+    pdl_begin();
     __shared__ float  fsh[kNShift * 3];
     __shared__ int    exl[kFepMaxExcl];
     __shared__ double esum[kFepWarps][4];
@@ -451,11 +452,11 @@ cudaError_t launch_fep(const DeviceView& v, const FepView& fp, bool energy, cuda
     }
     if (v.coulomb == 0)
     {
-        k_fep<true><<<fp.np, kFepWarps * 32, 0, s>>>(v, fp, energy ? 1 : 0);
+        launch_pdl(k_fep<true>, fp.np, kFepWarps * 32, 0, s, v, fp, energy ? 1 : 0);
     }
     else
     {
-        k_fep<false><<<fp.np, kFepWarps * 32, 0, s>>>(v, fp, energy ? 1 : 0);
+        launch_pdl(k_fep<false>, fp.np, kFepWarps * 32, 0, s, v, fp, energy ? 1 : 0);
     }
     return cudaGetLastError();
 }

@@ -2,6 +2,7 @@
 // nbx_fft.cuh.  Real grid [n0][n1][n2] (z fastest), half-complex [n0][n1][n2/2 + 1], unnormalised,
 // exp(-2 pi i ...) forward and exp(+2 pi i ...) backward, as the reference's FFT wrapper
 // (src/gromacs/fft/fft.h: gmx_fft_3d_real) and cuFFT's R2C / C2R define them.
+#include "nbx_internal.cuh"
 #include "nbx_fft.cuh"
 
 #include <cmath>
@@ -48,6 +49,7 @@ __device__ __forceinline__ void load_roots(float2* W, const FftAxis& ax)
 __global__ void __launch_bounds__(kZWarps * 32) k_fft_z_r2c(FftAxis ax, const float* __restrict__ real,
                                                             float2* __restrict__ cplx, int nlines)
 {
+    pdl_begin();
     extern __shared__ float2 fsm[];
     float2*   W    = fsm;
     const int n    = ax.n;
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(kZWarps * 32) k_fft_z_r2c(FftAxis ax, const fl
 __global__ void __launch_bounds__(kZWarps * 32) k_fft_z_c2r(FftAxis ax, const float2* __restrict__ cplx,
                                                             float* __restrict__ real, int nlines)
 {
+    pdl_begin();
     extern __shared__ float2 fsm[];
     float2*   W    = fsm;
     const int n    = ax.n;
@@ -142,6 +145,7 @@ template<bool kInv>
 __global__ void __launch_bounds__(kFftTile * 32) k_fft_strided(FftAxis ax, float2* __restrict__ data, int elem_stride,
                                                                int outer_stride, int ntiles, int nzc)
 {
+    pdl_begin();
     extern __shared__ float2 fsm[];
     float2*   W    = fsm;
     const int n    = ax.n;
@@ -202,8 +206,8 @@ cudaError_t strided_pass(const FftPlan3& p, int axis, float2* cplx, cudaStream_t
     }
     else
     {
-        k_fft_strided<kInv><<<nouter * ntiles, kFftTile * 32, strided_smem(ax.n), s>>>(ax, cplx, elem, outer, ntiles,
-                                                                                       nzc);
+        launch_pdl(k_fft_strided<kInv>, nouter * ntiles, kFftTile * 32, strided_smem(ax.n), s, ax, cplx, elem, outer,
+                   ntiles, nzc);
     }
     return cudaGetLastError();
 }
@@ -225,11 +229,11 @@ cudaError_t z_pass(bool inv, const FftPlan3& p, const float* real_in, float* rea
     }
     else if (inv)
     {
-        k_fft_z_c2r<<<z_blocks(nlines), kZWarps * 32, z_smem(p.n[2]), s>>>(ax, cplx, real_out, nlines);
+        launch_pdl(k_fft_z_c2r, z_blocks(nlines), kZWarps * 32, z_smem(p.n[2]), s, ax, cplx, real_out, nlines);
     }
     else
     {
-        k_fft_z_r2c<<<z_blocks(nlines), kZWarps * 32, z_smem(p.n[2]), s>>>(ax, real_in, cplx, nlines);
+        launch_pdl(k_fft_z_r2c, z_blocks(nlines), kZWarps * 32, z_smem(p.n[2]), s, ax, real_in, cplx, nlines);
     }
     return cudaGetLastError();
 }

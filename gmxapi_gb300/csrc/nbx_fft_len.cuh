@@ -12,6 +12,7 @@
 // (j, c) with c fastest, so global rows of 64 bytes are read and written whole, without staging.
 #pragma once
 
+#include "nbx_internal.cuh"
 #include "nbx_fft.cuh"
 #include "nbx_pme_solve.cuh"
 
@@ -218,6 +219,7 @@ template<int R1, int R2>
 __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
         k_z_r2c(const float2* __restrict__ roots, const float* __restrict__ real, float2* __restrict__ cplx, int nlines)
 {
+    pdl_begin();
     using S              = Shape<R1, R2>;
     constexpr int n      = S::n, nzc = n / 2 + 1;
     constexpr int kLine  = R1 * S::row;
@@ -283,6 +285,7 @@ template<int R1, int R2>
 __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
         k_z_c2r(const float2* __restrict__ roots, const float2* __restrict__ cplx, float* __restrict__ real, int nlines)
 {
+    pdl_begin();
     using S              = Shape<R1, R2>;
     constexpr int n      = S::n, nzc = n / 2 + 1;
     constexpr int kLine  = R1 * S::row;
@@ -349,6 +352,7 @@ __global__ void __launch_bounds__(round32(kCols* Shape<R1, R2>::threads))
         k_strided(const float2* __restrict__ roots, float2* __restrict__ data, int elem_stride, int outer_stride,
                   int ntiles, int nzc)
 {
+    pdl_begin();
     using S = Shape<R1, R2>;
     __shared__ float2 sm[R1 * S::row * kCols];
     const int         o = blockIdx.x / ntiles, t = blockIdx.x - o * ntiles;
@@ -396,6 +400,7 @@ template<int R1, int R2, bool kEnergy>
 __global__ void __launch_bounds__(round32(kCols* Shape<R1, R2>::threads))
         k_x_solve(const float2* __restrict__ roots, float2* cgrid, PmeSolve ps, int ntiles)
 {
+    pdl_begin();
     using S = Shape<R1, R2>;
     __shared__ float2 sm[R1 * S::row * kCols];
     const int         nzc = ps.d.n[2] / 2 + 1;
@@ -479,14 +484,14 @@ template<int R1, int R2>
 void launch_z_r2c(const float2* roots, const float* real, float2* cplx, int nlines, cudaStream_t s)
 {
     const int blocks = (nlines + 2 * kZPairs - 1) / (2 * kZPairs);
-    k_z_r2c<R1, R2><<<blocks, round32(kZPairs * Shape<R1, R2>::threads), 0, s>>>(roots, real, cplx, nlines);
+    launch_pdl(k_z_r2c<R1, R2>, blocks, round32(kZPairs * Shape<R1, R2>::threads), 0, s, roots, real, cplx, nlines);
 }
 
 template<int R1, int R2>
 void launch_z_c2r(const float2* roots, const float2* cplx, float* real, int nlines, cudaStream_t s)
 {
     const int blocks = (nlines + 2 * kZPairs - 1) / (2 * kZPairs);
-    k_z_c2r<R1, R2><<<blocks, round32(kZPairs * Shape<R1, R2>::threads), 0, s>>>(roots, cplx, real, nlines);
+    launch_pdl(k_z_c2r<R1, R2>, blocks, round32(kZPairs * Shape<R1, R2>::threads), 0, s, roots, cplx, real, nlines);
 }
 
 template<int R1, int R2>
@@ -496,11 +501,11 @@ void launch_strided(bool inv, const float2* roots, float2* data, int nouter, int
     const int ntiles = (nzc + kCols - 1) / kCols, threads = round32(kCols * Shape<R1, R2>::threads);
     if (inv)
     {
-        k_strided<R1, R2, true><<<nouter * ntiles, threads, 0, s>>>(roots, data, elem, outer, ntiles, nzc);
+        launch_pdl(k_strided<R1, R2, true>, nouter * ntiles, threads, 0, s, roots, data, elem, outer, ntiles, nzc);
     }
     else
     {
-        k_strided<R1, R2, false><<<nouter * ntiles, threads, 0, s>>>(roots, data, elem, outer, ntiles, nzc);
+        launch_pdl(k_strided<R1, R2, false>, nouter * ntiles, threads, 0, s, roots, data, elem, outer, ntiles, nzc);
     }
 }
 
@@ -510,11 +515,11 @@ void launch_x_solve(const float2* roots, float2* cgrid, const PmeSolve& ps, cuda
     const int ntiles = (ps.d.n[2] / 2 + 1 + kCols - 1) / kCols, threads = round32(kCols * Shape<R1, R2>::threads);
     if (ps.partials)
     {
-        k_x_solve<R1, R2, true><<<ps.d.n[1] * ntiles, threads, 0, s>>>(roots, cgrid, ps, ntiles);
+        launch_pdl(k_x_solve<R1, R2, true>, ps.d.n[1] * ntiles, threads, 0, s, roots, cgrid, ps, ntiles);
     }
     else
     {
-        k_x_solve<R1, R2, false><<<ps.d.n[1] * ntiles, threads, 0, s>>>(roots, cgrid, ps, ntiles);
+        launch_pdl(k_x_solve<R1, R2, false>, ps.d.n[1] * ntiles, threads, 0, s, roots, cgrid, ps, ntiles);
     }
 }
 

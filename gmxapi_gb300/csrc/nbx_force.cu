@@ -63,6 +63,7 @@ constexpr int kExclBlocksPerSm = 4;
 template<bool kEnergy, bool kEwald, int kLj = 0>
 __global__ void __launch_bounds__(kForceThreads, kForceMinBlocks) k_force(DeviceView v, int* work_counter)
 {
+    pdl_begin();
     // {6*C6, 12*C12, LJ energy shift of the pair, LJ-PME grid 6*C6 (geometric)} per type pair
     extern __shared__ float4 nbfp_s[];
     const int nt1 = v.ntypes1;
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(kForceThreads, kForceMinBlocks) k_force(Device
 
 __global__ void __launch_bounds__(kExclThreads) k_excl_energy(DeviceView v)
 {
+    pdl_begin();
     double    acc    = 0.0;
     double    acc_lj = 0.0;  // LJ-PME: the grid part of excluded pairs
     double    acc_s  = 0.0;  // Ewald: sum of q_i q_j S(beta^2 r^2) over excluded pairs
@@ -244,6 +246,7 @@ constexpr int kReduceThreads = 256;
 __global__ void __launch_bounds__(kReduceThreads)
         k_reduce_f(DeviceView v, float* __restrict__ f, int do_virial, double* d_energies, double* d_virial, int stage)
 {
+    pdl_begin();
     float w[9];
 #pragma unroll
     for (int k = 0; k < 9; k++)
@@ -444,11 +447,13 @@ __global__ void __launch_bounds__(kReduceThreads)
 // (mdlib/sim_util.cpp:157-176, calcvir.cpp:103-145).
 __global__ void k_finish(DeviceView v, double* d_energies, double* d_virial)
 {
+    pdl_begin();
     finish_sums(v, d_energies, d_virial, threadIdx.x);
 }
 
 __global__ void k_pair_count(DeviceView v, unsigned long long* out)
 {
+    pdl_begin();
     const int          j   = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long cnt = 0;
     if (j < v.hdr->num_cj4)
@@ -467,6 +472,7 @@ __global__ void k_pair_count(DeviceView v, unsigned long long* out)
 
 __global__ void k_noalloc_init(ListHeader* hdr, int num_sci, int num_cells)
 {
+    pdl_begin();
     hdr->num_sci      = num_sci;
     hdr->num_cells    = num_cells;
     hdr->status       = 0u;
@@ -507,7 +513,7 @@ void launch_k_force(const DeviceView& v, int blocks, size_t smem, cudaStream_t s
     {
         return;  // the launch error is reported by cudaGetLastError
     }
-    k_force<kEnergy, kEwald, kLj><<<blocks, kForceThreads, smem, s>>>(v, counter);
+    launch_pdl(k_force<kEnergy, kEwald, kLj>, blocks, kForceThreads, smem, s, v, counter);
 }
 
 // Marks the outputs of an allocation-free evaluation whose device status word is non-zero (a
@@ -515,6 +521,7 @@ void launch_k_force(const DeviceView& v, int blocks, size_t smem, cudaStream_t s
 // and the virial become NaN, so a failed evaluation cannot pass for a correct one.
 __global__ void k_noalloc_check(const ListHeader* hdr, float* f, int n3, double* d_energies, double* d_virial)
 {
+    pdl_begin();
     if (__ldcg(&hdr->status) == 0u)
     {
         return;
@@ -559,7 +566,7 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
     kv.excl_chunks = 0;
     if (energy && v.vdw_mod == NBX_VDW_LJPME)
     {
-        k_excl_energy<<<excl_blocks(v.n, num_sms), kExclThreads, 0, s>>>(v);
+        launch_pdl(k_excl_energy, excl_blocks(v.n, num_sms), kExclThreads, 0, s, v);
     }
     else if (energy)
     {
@@ -607,15 +614,15 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
 cudaError_t launch_reduce_f(const DeviceView& v, float* d_f, double* d_e, double* d_vir, cudaStream_t s, bool stage)
 {
     const int per_block = kReduceThreads * kReduceAtoms;
-    k_reduce_f<<<(v.n + per_block - 1) / per_block, kReduceThreads, 0, s>>>(v, d_f, d_vir ? 1 : 0, d_e, d_vir,
-                                                                           stage ? 1 : 0);
+    launch_pdl(k_reduce_f, (v.n + per_block - 1) / per_block, kReduceThreads, 0, s, v, d_f, d_vir ? 1 : 0, d_e,
+               d_vir, stage ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pair_count(const DeviceView& v, unsigned long long* d_out, cudaStream_t s)
 {
     cudaMemsetAsync(d_out, 0, sizeof(unsigned long long), s);
-    k_pair_count<<<(v.cj4_cap + 255) / 256, 256, 0, s>>>(v, d_out);
+    launch_pdl(k_pair_count, (v.cj4_cap + 255) / 256, 256, 0, s, v, d_out);
     return cudaGetLastError();
 }
 
@@ -808,7 +815,7 @@ extern "C" int nbx_compute_noalloc(const nbx_noalloc_args* a, float* d_f, double
         }
     }
     // the array keeps the previous call's contents: clear what must start at zero
-    k_noalloc_init<<<1, 1, 0, s>>>(v.hdr, a->num_sci, a->num_slots / kSc);
+    launch_pdl(k_noalloc_init, 1, 1, 0, s, v.hdr, a->num_sci, a->num_slots / kSc);
     cudaError_t e = cudaMemsetAsync(v.fnb, 0, sizeof(float4) * (size_t)a->num_slots, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(sums, 0, kNoAllocSumsBytes, s);
     int num_sms = 0, dev = 0;
@@ -821,7 +828,7 @@ extern "C" int nbx_compute_noalloc(const nbx_noalloc_args* a, float* d_f, double
         int*         ctr    = &v.hdr->work_counter;
         if (energy)
         {
-            k_excl_energy<<<excl_blocks(v.n, num_sms), kExclThreads, 0, s>>>(v);
+            launch_pdl(k_excl_energy, excl_blocks(v.n, num_sms), kExclThreads, 0, s, v);
             if (v.coulomb == 0)
             {
                 launch_k_force<true, true, 0>(v, blocks, smem, s, ctr);
@@ -839,14 +846,14 @@ extern "C" int nbx_compute_noalloc(const nbx_noalloc_args* a, float* d_f, double
         {
             launch_k_force<false, false, 0>(v, blocks, smem, s, ctr);
         }
-        k_reduce_f<<<(v.n + kReduceThreads * kReduceAtoms - 1) / (kReduceThreads * kReduceAtoms), kReduceThreads, 0, s>>>(
-                v, d_f, d_virial ? 1 : 0, nullptr, nullptr, 0);
+        launch_pdl(k_reduce_f, (v.n + kReduceThreads * kReduceAtoms - 1) / (kReduceThreads * kReduceAtoms),
+                   kReduceThreads, 0, s, v, d_f, d_virial ? 1 : 0, nullptr, nullptr, 0);
         if (energy)
         {
-            k_finish<<<1, 32, 0, s>>>(v, d_energies, d_virial);
+            launch_pdl(k_finish, 1, 32, 0, s, v, d_energies, d_virial);
         }
-        k_noalloc_check<<<std::min(num_sms, (3 * v.n + 255) / 256), 256, 0, s>>>(v.hdr, d_f, 3 * v.n, d_energies,
-                                                                                 d_virial);
+        launch_pdl(k_noalloc_check, std::min(num_sms, (3 * v.n + 255) / 256), 256, 0, s, v.hdr, d_f, 3 * v.n,
+                   d_energies, d_virial);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? NBX_OK : NBX_ERR_CUDA;

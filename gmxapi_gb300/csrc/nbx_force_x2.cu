@@ -23,6 +23,7 @@ constexpr int kForceThreads = 256;
 template<bool kEnergy, int kCoul, int kDepth, int kBlocks>
 __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force_x2(DeviceView v, int* work_counter)
 {
+    pdl_begin();
     // {-6*C6, 12*C12, LJ energy shift of the pair, 0} per type pair
     extern __shared__ float4 smem_x2[];
     float4*   nbfp_s = smem_x2;
@@ -127,7 +128,7 @@ cudaError_t launch_x2(const DeviceView& v, cudaStream_t s, int num_sms, int* cou
     {
         return e;
     }
-    k_force_x2<kEnergy, kCoul, kDepth, kBlocks><<<num_sms * kBlocks, kForceThreads, smem, s>>>(v, counter);
+    launch_pdl(k_force_x2<kEnergy, kCoul, kDepth, kBlocks>, num_sms * kBlocks, kForceThreads, smem, s, v, counter);
     return cudaGetLastError();
 }
 

@@ -71,6 +71,7 @@ constexpr int kMaxSmemCols    = 8192;  // column counters kept in shared memory 
 // atomic, so a column sees one global atomic per block instead of one per atom.
 __global__ void __launch_bounds__(kGridThreads) k_wrap_column(DeviceView v, float* x, int write_back)
 {
+    pdl_begin();
     extern __shared__ int s_cnt[];  // [ncol]: counts, then the block's base slot per column
     const int  ncol     = v.g.ncol;
     const bool use_smem = ncol <= kMaxSmemCols;
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kGridThreads) k_wrap_column(DeviceView v, floa
 // Cells per column and their prefix sum (grid.cpp:1300-1330), one block.
 __global__ void k_column_scan(DeviceView v)
 {
+    pdl_begin();
     __shared__ int warp_sums[32];
     const int      ncol     = v.g.ncol;
     const int      nthreads = blockDim.x;
@@ -213,6 +215,7 @@ __global__ void k_column_scan(DeviceView v)
 
 __global__ void k_scatter(DeviceView v)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.n || v.hdr->num_cells == 0)
     {
@@ -352,6 +355,7 @@ constexpr int kSmemSortItems = 4096;
 // One block per grid column: z sort, per-slab y and x sorts, fill (fillCell).
 __global__ void __launch_bounds__(kSortThreads) k_sort_fill(DeviceView v, unsigned long long* scratch)
 {
+    pdl_begin();
     __shared__ unsigned long long skeys[kSmemSortItems];
     __shared__ int                slab[kSortThreads / 32][32];
     const int                     cxy = blockIdx.x;
@@ -500,6 +504,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_fill(DeviceView v, unsign
 // counter), in place of separate memsets before the force kernel.
 __global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear, int atom_order)
 {
+    pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (clear)
     {
@@ -572,6 +577,7 @@ __global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear
 // conversion rewrites only the slots that hold atoms).
 __global__ void k_pack_slots(DeviceView v)
 {
+    pdl_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= v.hdr->num_cells * kSc)
     {
@@ -592,11 +598,11 @@ cudaError_t launch_grid(const DeviceView& v, float* d_x, int write_back, cudaStr
     const int tb = 256;
     const int per_block = kGridThreads * kAtomsPerThread;
     const size_t smem   = v.g.ncol <= kMaxSmemCols ? sizeof(int) * (size_t)v.g.ncol : 0;
-    k_wrap_column<<<(v.n + per_block - 1) / per_block, kGridThreads, smem, s>>>(v, d_x, write_back);
-    k_column_scan<<<1, 1024, 0, s>>>(v);
-    k_scatter<<<(v.n + tb - 1) / tb, tb, 0, s>>>(v);
-    k_sort_fill<<<v.g.ncol, kSortThreads, 0, s>>>(v, reinterpret_cast<unsigned long long*>(v.fnb));
-    k_pack_slots<<<(v.g.cells_capacity * kSc + tb - 1) / tb, tb, 0, s>>>(v);
+    launch_pdl(k_wrap_column, (v.n + per_block - 1) / per_block, kGridThreads, smem, s, v, d_x, write_back);
+    launch_pdl(k_column_scan, 1, 1024, 0, s, v);
+    launch_pdl(k_scatter, (v.n + tb - 1) / tb, tb, 0, s, v);
+    launch_pdl(k_sort_fill, v.g.ncol, kSortThreads, 0, s, v, reinterpret_cast<unsigned long long*>(v.fnb));
+    launch_pdl(k_pack_slots, (v.g.cells_capacity * kSc + tb - 1) / tb, tb, 0, s, v);
     return cudaGetLastError();
 }
 
@@ -605,7 +611,8 @@ cudaError_t launch_convert_x(const DeviceView& v, const float* d_x, cudaStream_t
     const int tb      = 256;
     const int items   = atom_order ? v.n : v.g.cells_capacity * kSc;
     const int threads = clear ? std::max(items, v.g.cells_capacity * kSc) : items;
-    k_convert_x<<<threads > 0 ? (threads + tb - 1) / tb : 1, tb, 0, s>>>(v, d_x, clear ? 1 : 0, atom_order ? 1 : 0);
+    launch_pdl(k_convert_x, threads > 0 ? (threads + tb - 1) / tb : 1, tb, 0, s, v, d_x, clear ? 1 : 0,
+               atom_order ? 1 : 0);
     return cudaGetLastError();
 }
 

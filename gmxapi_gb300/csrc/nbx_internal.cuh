@@ -9,6 +9,33 @@
 namespace nbx
 {
 
+// Every kernel is launched as a programmatic dependent of the kernel before it on its stream: its blocks
+// may take their places while that kernel still runs, and wait in pdl_begin (the first statement of
+// every kernel, before any access to memory) until it has ended and its writes are visible.  An
+// evaluation is a chain of kernels of a few microseconds, so their launch latencies and block start-up
+// were a large part of it (3,000 atoms: 3 kernels for the forces, 7 for PME).
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+}
+
+template<class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute pdl;
+    pdl.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg                         = {};
+    cfg.gridDim                                    = grid;
+    cfg.blockDim                                   = block;
+    cfg.dynamicSmemBytes                           = smem;
+    cfg.stream                                     = stream;
+    cfg.attrs                                      = &pdl;
+    cfg.numAttrs                                   = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Cluster geometry of the GPU pair list (src/gromacs/nbnxm/pairlistparams.h:60-89,
 // pairlist.h:146-171): 8-atom clusters, 8 clusters (2x2x2) per 64-atom cell,
 // j-clusters in groups of 4, each 8x8 cluster pair split in two warp halves.

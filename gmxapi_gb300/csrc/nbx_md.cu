@@ -16,7 +16,7 @@
 // search steps (the update right before one), not every step as nblib's LeapFrog does.
 #include "../../include/nbnxm_gb300.h"
 
-#include <cuda_runtime.h>
+#include "nbx_internal.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(kLfThreads) k_leapfrog(int n, float dt, const 
                                                          const float* __restrict__ f, float3 box, int wrap,
                                                          double* partials, unsigned* done, double* ekin_out)
 {
+    nbx::pdl_begin();
     double ke2 = 0.0;  // sum of m v^2 over the old and the new half-step velocities
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x)
     {
@@ -186,9 +187,8 @@ int launch_leapfrog(nbx_leapfrog* p, float dt, float* d_x, float* d_v, const flo
         return NBX_OK;
     }
     cudaSetDevice(p->device);
-    k_leapfrog<<<lf_blocks(p), kLfThreads, 0, p->stream>>>(p->n, dt, p->inv_mass, d_x, d_v, d_f,
-                                                           make_float3(p->box[0], p->box[1], p->box[2]), wrap,
-                                                           p->partials, p->done, d_ekin);
+    nbx::launch_pdl(k_leapfrog, lf_blocks(p), kLfThreads, 0, p->stream, p->n, dt, p->inv_mass, d_x, d_v, d_f,
+                    make_float3(p->box[0], p->box[1], p->box[2]), wrap, p->partials, p->done, d_ekin);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? NBX_OK : md_error(p, NBX_ERR_CUDA, cudaGetErrorString(e));
 }

@@ -101,6 +101,7 @@ __device__ __forceinline__ int wrap_once(int i, int n)
 __global__ void k_pme_splines(PmeDims d, int natoms, const float* __restrict__ x, int* idx, float* theta,
                               float* dtheta)
 {
+    nbx::pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= natoms)
     {
@@ -198,6 +199,7 @@ template<bool kVec>
 __global__ void k_pme_spread(PmeDims d, int natoms, const float* __restrict__ x, const float* __restrict__ q,
                              float* grid)
 {
+    nbx::pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if ((t >> 2) < natoms)
     {
@@ -243,6 +245,7 @@ __device__ __forceinline__ int brick_count(const Bricks& b)
 __global__ void __launch_bounds__(256) k_pme_file(PmeDims d, Bricks b, int natoms, const float* __restrict__ x,
                                                   const float* __restrict__ q, float4* grid4, int n4)
 {
+    nbx::pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = t; i < n4; i += gridDim.x * blockDim.x)
     {
@@ -305,6 +308,7 @@ struct SpreadWarp
 __global__ void __launch_bounds__(32 * kBrickWarps)
         k_pme_spread_bricks(PmeDims d, Bricks b, const float* __restrict__ x, const float* __restrict__ q, float* grid)
 {
+    nbx::pdl_begin();
     extern __shared__ float4 spread_smem[];
     SpreadWarp& w     = reinterpret_cast<SpreadWarp*>(spread_smem)[threadIdx.x >> 5];
     const int   lane  = threadIdx.x & 31;
@@ -412,6 +416,7 @@ __global__ void __launch_bounds__(kSolveThreads, 6) k_pme_fft_x_solve(nbx::FftAx
                                                                    const float* __restrict__ bsp, float elfac,
                                                                    float factor, float pivol, int ntiles, double* partials)
 {
+    nbx::pdl_begin();
     constexpr int T    = nbx::kFftTile;
     extern __shared__ float2 xsm[];
     const int     n    = ax.n;  // nx
@@ -493,6 +498,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_pme_solve(PmeDims d, float2* 
                                                              unsigned int* done, double* energy_out,
                                                              double* virial_out)
 {
+    nbx::pdl_begin();
     const bool energy = energy_out || virial_out;
     const int  nzc    = d.n[2] / 2 + 1;
     const int  total  = d.n[0] * d.n[1] * nzc;
@@ -541,6 +547,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_pme_solve_lj(PmeDims d, float
                                                                 float by_pref, double* partials, unsigned int* done,
                                                                 double* energy_out, double* virial_out)
 {
+    nbx::pdl_begin();
     const bool energy = energy_out || virial_out;
     const int  nzc    = d.n[2] / 2 + 1;
     const int  total  = d.n[0] * d.n[1] * nzc;
@@ -643,6 +650,7 @@ __device__ __forceinline__ void gather_atom(const PmeDims& d, int a, float qa, c
 __global__ void k_pme_gather(PmeDims d, int natoms, const float* __restrict__ x, const float* __restrict__ q,
                              const float* __restrict__ grid, float* f, PmeTotals tot)
 {
+    nbx::pdl_begin();
     if (tot.partials && blockIdx.x == 0 && threadIdx.x < 32)
     {
         nbx::solve_total(tot.partials, tot.energy_out, tot.virial_out);
@@ -665,6 +673,7 @@ __global__ void __launch_bounds__(kGatherThreads, 10)
         k_pme_gather_bricks(PmeDims d, Bricks b, const float* __restrict__ x, const float* __restrict__ q,
                             const float* __restrict__ grid, float* f, PmeTotals tot)
 {
+    nbx::pdl_begin();
     __shared__ float tile[kTileFloats];
     const int        nbr = brick_count(b), brick = blockIdx.x;
     const int        n     = min(b.count[brick], b.cap);
@@ -751,6 +760,7 @@ __global__ void __launch_bounds__(kGatherThreads, 10)
 // The solve's totals alone (an evaluation without atoms has no gather).
 __global__ void k_pme_totals(PmeTotals tot)
 {
+    nbx::pdl_begin();
     nbx::solve_total(tot.partials, tot.energy_out, tot.virial_out);
 }
 
@@ -886,11 +896,11 @@ cudaError_t launch_spread(nbx_pme* p, int natoms, const float* d_x, const float*
     const bool vec    = p->d.n[2] % 4 == 0 && (reinterpret_cast<uintptr_t>(grid) & 15) == 0;
     if (vec)
     {
-        k_pme_spread<true><<<blocks, 256, 0, p->stream>>>(p->d, natoms, d_x, d_q, grid);
+        nbx::launch_pdl(k_pme_spread<true>, blocks, 256, 0, p->stream, p->d, natoms, d_x, d_q, grid);
     }
     else
     {
-        k_pme_spread<false><<<blocks, 256, 0, p->stream>>>(p->d, natoms, d_x, d_q, grid);
+        nbx::launch_pdl(k_pme_spread<false>, blocks, 256, 0, p->stream, p->d, natoms, d_x, d_q, grid);
     }
     return cudaGetLastError();
 }
@@ -985,10 +995,10 @@ cudaError_t launch_spread_bricks(nbx_pme* p, int natoms, const float* d_x, const
         }
     }
     p->filed = true;
-    k_pme_file<<<(natoms + 255) / 256, 256, 0, p->stream>>>(p->d, b, natoms, d_x, d_q, reinterpret_cast<float4*>(grid),
-                                                            (int)(real_points(p) / 4));
-    k_pme_spread_bricks<<<(nbr + kBrickWarps - 1) / kBrickWarps, 32 * kBrickWarps, sizeof(SpreadWarp) * kBrickWarps,
-                          p->stream>>>(p->d, b, d_x, d_q, grid);
+    nbx::launch_pdl(k_pme_file, (natoms + 255) / 256, 256, 0, p->stream, p->d, b, natoms, d_x, d_q,
+                    reinterpret_cast<float4*>(grid), (int)(real_points(p) / 4));
+    nbx::launch_pdl(k_pme_spread_bricks, (nbr + kBrickWarps - 1) / kBrickWarps, 32 * kBrickWarps,
+                    sizeof(SpreadWarp) * kBrickWarps, p->stream, p->d, b, d_x, d_q, grid);
     return cudaGetLastError();
 }
 
@@ -997,7 +1007,7 @@ cudaError_t launch_gather_bricks(nbx_pme* p, const float* d_x, const float* d_q,
 {
     const Bricks& b   = p->bricks;
     const int     nbr = b.nb[0] * b.nb[1] * b.nb[2];
-    k_pme_gather_bricks<<<nbr, kGatherThreads, 0, p->stream>>>(p->d, b, d_x, d_q, grid, d_f, tot);
+    nbx::launch_pdl(k_pme_gather_bricks, nbr, kGatherThreads, 0, p->stream, p->d, b, d_x, d_q, grid, d_f, tot);
     const cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
     {
@@ -1018,15 +1028,15 @@ cudaError_t launch_solve(nbx_pme* p, float2* cgrid, double* d_energy, double* d_
     {
         // by = 3 V B_y / (pi sqrt(pi) beta^3) (pme_solve.cpp:664)
         const float by_pref = (float)(3.0 * vol / (M_PI * std::sqrt(M_PI) * (double)p->beta * p->beta * p->beta));
-        k_pme_solve_lj<<<nblocks, kSolveThreads, 0, p->stream>>>(p->d, cgrid, p->bsp, factor, by_pref, p->sums,
-                                                                 p->done, d_energy, d_virial);
+        nbx::launch_pdl(k_pme_solve_lj, nblocks, kSolveThreads, 0, p->stream, p->d, cgrid, p->bsp, factor, by_pref,
+                        p->sums, p->done, d_energy, d_virial);
         return cudaGetLastError();
     }
     // elfac = ONE_4PI_EPS0 / epsilon_r (pme_solve.cpp:354)
     const float elfac = (float)nbx::one_4pi_eps0() / p->epsilon_r;
     const float pivol = (float)M_PI * (float)vol;
-    k_pme_solve<<<nblocks, kSolveThreads, 0, p->stream>>>(p->d, cgrid, p->bsp, elfac, factor, pivol, p->sums,
-                                                          p->done, d_energy, d_virial);
+    nbx::launch_pdl(k_pme_solve, nblocks, kSolveThreads, 0, p->stream, p->d, cgrid, p->bsp, elfac, factor, pivol,
+                    p->sums, p->done, d_energy, d_virial);
     return cudaGetLastError();
 }
 
@@ -1053,13 +1063,13 @@ cudaError_t launch_x_solve(nbx_pme* p, double* d_energy, double* d_virial)
     const size_t smem   = nbx::fft_tiled_smem(p->d.n[0]);
     if (d_energy || d_virial)
     {
-        k_pme_fft_x_solve<true><<<p->d.n[1] * ntiles, kSolveThreads, smem, p->stream>>>(
-                p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums);
+        nbx::launch_pdl(k_pme_fft_x_solve<true>, p->d.n[1] * ntiles, kSolveThreads, smem, p->stream, p->fft.ax[0],
+                        p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums);
     }
     else
     {
-        k_pme_fft_x_solve<false><<<p->d.n[1] * ntiles, kSolveThreads, smem, p->stream>>>(
-                p->fft.ax[0], p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums);
+        nbx::launch_pdl(k_pme_fft_x_solve<false>, p->d.n[1] * ntiles, kSolveThreads, smem, p->stream, p->fft.ax[0],
+                        p->d, p->cgrid, p->bsp, elfac, factor, pivol, ntiles, p->sums);
     }
     return cudaGetLastError();
 }
@@ -1069,11 +1079,12 @@ cudaError_t launch_gather(nbx_pme* p, int natoms, const float* d_x, const float*
 {
     if (natoms > 0)
     {
-        k_pme_gather<<<(natoms + 127) / 128, 128, 0, p->stream>>>(p->d, natoms, d_x, d_q, grid, d_f, tot);
+        nbx::launch_pdl(k_pme_gather, (natoms + 127) / 128, 128, 0, p->stream, p->d, natoms, d_x, d_q, grid, d_f,
+                        tot);
     }
     else if (tot.partials)
     {
-        k_pme_totals<<<1, 32, 0, p->stream>>>(tot);
+        nbx::launch_pdl(k_pme_totals, 1, 32, 0, p->stream, tot);
     }
     return cudaGetLastError();
 }
@@ -1332,7 +1343,8 @@ int nbx_pme_splines_device(nbx_pme* p, int natoms, const float* d_x, int* d_idx,
     {
         return NBX_OK;
     }
-    k_pme_splines<<<(natoms + 127) / 128, 128, 0, p->stream>>>(p->d, natoms, d_x, d_idx, d_theta, d_dtheta);
+    nbx::launch_pdl(k_pme_splines, (natoms + 127) / 128, 128, 0, p->stream, p->d, natoms, d_x, d_idx, d_theta,
+                    d_dtheta);
     return cuda_status(p, cudaGetLastError());
 }
 

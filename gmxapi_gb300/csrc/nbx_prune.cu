@@ -418,6 +418,7 @@ __device__ void prune_entry_rolling(const Sci& s, const Cj4* cj4, const unsigned
 template<int kPruneWarps, bool kFresh>
 __global__ void __launch_bounds__(32 * kPruneWarps, kFresh ? 4 : 6) k_prune(DeviceView v, int part, int nparts)
 {
+    pdl_begin();
     __shared__ RollSmem  rsm[kFresh ? 1 : kPruneWarps];
     __shared__ FreshSmem fsm[kFresh ? kPruneWarps : 1];
     const int           numSci = v.hdr->num_sci;
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(32 * kPruneWarps)
         k_batch_prune(const BatchSys* sys, const int* entry_prefix, int nsys, float outer2, float inner2, int part,
                       int nparts)
 {
+    pdl_begin();
     __shared__ RollSmem  rsm[kFresh ? 1 : kPruneWarps];
     __shared__ FreshSmem fsm[kFresh ? kPruneWarps : 1];
     const int           total = entry_prefix[nsys];
@@ -541,14 +543,14 @@ cudaError_t launch_batch_prune(const BatchSys* sys, const int* entry_prefix, int
     if (fresh)
     {
         constexpr auto kKernel = k_batch_prune<kPruneWarpsFresh, true>;
-        kKernel<<<resident_grid<kKernel, 32 * kPruneWarpsFresh>(), 32 * kPruneWarpsFresh, 0, s>>>(
-                sys, entry_prefix, nsys, outer2, inner2, part, 1);
+        launch_pdl(kKernel, resident_grid<kKernel, 32 * kPruneWarpsFresh>(), 32 * kPruneWarpsFresh, 0, s, sys,
+                   entry_prefix, nsys, outer2, inner2, part, 1);
     }
     else
     {
         constexpr auto kKernel = k_batch_prune<kPruneWarpsRolling, false>;
-        kKernel<<<resident_grid<kKernel, 32 * kPruneWarpsRolling>(), 32 * kPruneWarpsRolling, 0, s>>>(
-                sys, entry_prefix, nsys, outer2, inner2, part, nparts);
+        launch_pdl(kKernel, resident_grid<kKernel, 32 * kPruneWarpsRolling>(), 32 * kPruneWarpsRolling, 0, s, sys,
+                   entry_prefix, nsys, outer2, inner2, part, nparts);
     }
     return cudaGetLastError();
 }
@@ -558,13 +560,13 @@ cudaError_t launch_prune(const DeviceView& v, int fresh, int part, int nparts, c
     if (fresh)
     {
         constexpr auto kKernel = k_prune<kPruneWarpsFresh, true>;
-        kKernel<<<resident_grid<kKernel, 32 * kPruneWarpsFresh>(), 32 * kPruneWarpsFresh, 0, s>>>(v, 0, 1);
+        launch_pdl(kKernel, resident_grid<kKernel, 32 * kPruneWarpsFresh>(), 32 * kPruneWarpsFresh, 0, s, v, 0, 1);
     }
     else
     {
         constexpr auto kKernel = k_prune<kPruneWarpsRolling, false>;
-        kKernel<<<resident_grid<kKernel, 32 * kPruneWarpsRolling>(), 32 * kPruneWarpsRolling, 0, s>>>(v, part,
-                                                                                                      nparts);
+        launch_pdl(kKernel, resident_grid<kKernel, 32 * kPruneWarpsRolling>(), 32 * kPruneWarpsRolling, 0, s, v,
+                   part, nparts);
     }
     return cudaGetLastError();
 }

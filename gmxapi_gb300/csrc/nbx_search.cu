@@ -96,6 +96,7 @@ struct CountSmem
 
 __global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) k_search_count(DeviceView v)
 {
+    pdl_begin();
     __shared__ CountSmem wsm[kWarpsPerBlock];
     const int           lane = threadIdx.x & 31;
     const int           wib  = threadIdx.x >> 5;
@@ -491,6 +492,7 @@ struct EmitSmem
 // (setExclusionsForIEntry).
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView v)
 {
+    pdl_begin();
     __shared__ EmitSmem wsm[kWarpsPerBlock];
     const int           lane = threadIdx.x & 31;
     const int           wib  = threadIdx.x >> 5;
@@ -849,6 +851,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView 
 // Exclusive prefix sums of the per-cell entry and cj4 counts, one block.
 __global__ void k_scan_counts(DeviceView v)
 {
+    pdl_begin();
     __shared__ int ws[2][32];
     const int      n        = v.hdr->num_cells;
     const int      nthreads = blockDim.x;
@@ -957,8 +960,8 @@ cudaError_t launch_search_count(const DeviceView& v, cudaStream_t s)
     // num_subpairs .. rec_need: accumulated by the count pass or set by balancing
     cudaMemsetAsync(&v.hdr->num_subpairs, 0,
                     offsetof(ListHeader, rec_need) + sizeof(int) - offsetof(ListHeader, num_subpairs), s);
-    k_search_count<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(v);
-    k_scan_counts<<<1, 1024, 0, s>>>(v);
+    launch_pdl(k_search_count, blocks, 32 * kWarpsPerBlock, 0, s, v);
+    launch_pdl(k_scan_counts, 1, 1024, 0, s, v);
     return cudaGetLastError();
 }
 
@@ -967,7 +970,7 @@ cudaError_t launch_search_write(const DeviceView& v, int num_entries, cudaStream
     if (num_entries > 0)
     {
         const int blocks = (num_entries + kWarpsPerBlock - 1) / kWarpsPerBlock;
-        k_search_emit<<<blocks, 32 * kWarpsPerBlock, 0, s>>>(v);
+        launch_pdl(k_search_emit, blocks, 32 * kWarpsPerBlock, 0, s, v);
     }
     return cudaGetLastError();
 }
