@@ -45,44 +45,69 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     k.k_rf     = cv.k_rf;
     k.c_rf     = cv.c_rf;
     k.epsfac   = cv.epsfac;
-    for (;;)
-    {
-        int e = 0;
+    // per-lane FP64 energies of the system in hand, added to its sums when the warp's entries move on to
+    // another system (the queue hands out entries in system order)
+    __shared__ double e_acc_s[2][kThreads];
+    double&           e_lj_acc = e_acc_s[0][threadIdx.x];
+    double&           e_el_acc = e_acc_s[1][threadIdx.x];
+    e_lj_acc                   = 0.0;
+    e_el_acc                   = 0.0;
+    auto flush = [&](int sidx) {
+        double elj = e_lj_acc, eel = e_el_acc;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            elj += __shfl_xor_sync(full, elj, o);
+            eel += __shfl_xor_sync(full, eel, o);
+        }
+        if (lane == 0)
+        {
+            atomicAdd(&energies[2 * sidx], elj);
+            atomicAdd(&energies[2 * sidx + 1], eel * cv.epsfac_d);
+        }
+        e_lj_acc = 0.0;
+        e_el_acc = 0.0;
+    };
+    int  e = 0, next = -1;  // the work item and its system
+    Sci  s{};
+    auto claim = [&]() {
         if (lane == 0)
         {
             e = atomicAdd(work_counter, 1);
         }
+    };
+    auto fetch = [&]() {
         e = __shfl_sync(full, e, 0);
-        if (e >= total)
+        if (e < total)
         {
-            break;
+            next = find_system(prefix, nsys, e);
+            s    = sys[next].sci[e - prefix[next]];
         }
-        const int       sidx = find_system(prefix, nsys, e);
-        const BatchSys& b    = sys[sidx];
-        const Sci       s    = b.sci[e - prefix[sidx]];
-        const SysPtrsX2 p    = { b.xq, b.tgrid, b.xqp, b.fnb, b.cj4, b.excl, b.shiftvec,
-                                 fshift + (size_t)kNShift * 3 * sidx };
-        double          elj = 0.0, eel = 0.0;
-        if (!process_entry_x2<kEnergy, kCoul, kDepth>(k, p, s, reinterpret_cast<const char*>(nbfp_s), js, w, nt1,
-                                                       lane, cv.wait_test_bytes, elj, eel))
+    };
+    claim();
+    fetch();
+    int sidx = next;
+    while (e < total)
+    {
+        if (kEnergy && next != sidx)
+        {
+            flush(sidx);
+        }
+        sidx              = next;
+        const BatchSys& b = sys[sidx];
+        const Sci       si = s;
+        const SysPtrsX2 p  = { b.xq, b.tgrid, b.xqp, b.fnb, b.cj4, b.excl, b.shiftvec,
+                               fshift + (size_t)kNShift * 3 * sidx };
+        if (!process_entry_x2<kEnergy, kCoul, kDepth>(k, p, si, reinterpret_cast<const char*>(nbfp_s), js, w, nt1,
+                                                       lane, cv.wait_test_bytes, e_lj_acc, e_el_acc, claim, fetch))
         {
             stage_timeout_x2(js, const_cast<unsigned*>(&b.hdr->status), lane);
             break;
         }
-        if (kEnergy)
-        {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                elj += __shfl_xor_sync(full, elj, o);
-                eel += __shfl_xor_sync(full, eel, o);
-            }
-            if (lane == 0)
-            {
-                atomicAdd(&energies[2 * sidx], elj);
-                atomicAdd(&energies[2 * sidx + 1], eel * cv.epsfac_d);
-            }
-        }
+    }
+    if (kEnergy && sidx >= 0)
+    {
+        flush(sidx);
     }
 }
 

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kForceThreads, kForceMinBlocks) k_force(Device
             {
                 const double beta2  = (double)v.beta * (double)v.beta;
                 double       excl_s = 0.0;  // Ewald series sums of this item
-                for (int i = e * kExclChunkAtoms + lane; i < min(v.n, (e + 1) * kExclChunkAtoms); i += 32)
+                for (int i = e * v.excl_atoms + lane; i < min(v.n, (e + 1) * v.excl_atoms); i += 32)
                 {
                     double dummy_lj = 0.0;
                     excl_atom(v, v, i, false, beta2, e_el_acc, excl_s, dummy_lj);
@@ -570,7 +570,11 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
     }
     else if (energy)
     {
-        kv.excl_chunks = (v.n + kExclChunkAtoms - 1) / kExclChunkAtoms;
+        // an atom's exclusions are a chain of dependent loads: one atom per lane while that leaves fewer items
+        // than the list has entries (24k atoms: about 750 beside 6,700), four where items would only add
+        // queue traffic
+        kv.excl_atoms  = v.n < 65536 ? 32 : kExclChunkAtoms;
+        kv.excl_chunks = (v.n + kv.excl_atoms - 1) / kv.excl_atoms;
     }
     if (ev0)
     {

@@ -65,36 +65,48 @@ __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force_x2(DeviceView 
     e_lj_acc                   = 0.0;
     e_el_acc                   = 0.0;
     const int numChunks = kEnergy ? v.excl_chunks : 0;
-    for (;;)
-    {
-        int t = 0;
+    // the work item in hand: list entry e with its record s, or exclusion chunk e
+    int  t = 0, e = 0;
+    bool chunk = false;
+    Sci  s{};
+    auto claim = [&]() {
         if (lane == 0)
         {
             t = atomicAdd(work_counter, 1);
         }
+    };
+    auto fetch = [&]() {
         t = __shfl_sync(full, t, 0);
-        if (t >= numSci + numChunks)
+        if (t < numSci + numChunks)
         {
-            break;
-        }
-        int e;
-        if (item_is_chunk(t, numSci, numChunks, e))
-        {
-            if (kEnergy)
+            chunk = item_is_chunk(t, numSci, numChunks, e);
+            if (!chunk)
             {
-                const double beta2  = (double)v.beta * (double)v.beta;
-                double       excl_s = 0.0;
-                for (int i = e * kExclChunkAtoms + lane; i < min(v.n, (e + 1) * kExclChunkAtoms); i += 32)
-                {
-                    double dummy_lj = 0.0;
-                    excl_atom(v, v, i, false, beta2, e_el_acc, excl_s, dummy_lj);
-                }
-                e_el_acc = fma(excl_s, -(double)v.beta * 1.1283791670955125739, e_el_acc);
+                s = v.sci[e];
             }
+        }
+    };
+    claim();
+    fetch();
+    while (t < numSci + numChunks)
+    {
+        if (kEnergy && chunk)
+        {
+            const double beta2  = (double)v.beta * (double)v.beta;
+            double       excl_s = 0.0;
+            for (int i = e * v.excl_atoms + lane; i < min(v.n, (e + 1) * v.excl_atoms); i += 32)
+            {
+                double dummy_lj = 0.0;
+                excl_atom(v, v, i, false, beta2, e_el_acc, excl_s, dummy_lj);
+            }
+            e_el_acc = fma(excl_s, -(double)v.beta * 1.1283791670955125739, e_el_acc);
+            claim();
+            fetch();
             continue;
         }
-        if (!process_entry_x2<kEnergy, kCoul, kDepth>(k, p, v.sci[e], reinterpret_cast<const char*>(nbfp_s), js, w,
-                                                        nt1, lane, v.wait_test_bytes, e_lj_acc, e_el_acc))
+        const Sci si = s;
+        if (!process_entry_x2<kEnergy, kCoul, kDepth>(k, p, si, reinterpret_cast<const char*>(nbfp_s), js, w, nt1, lane,
+                                                       v.wait_test_bytes, e_lj_acc, e_el_acc, claim, fetch))
         {
             stage_timeout_x2(js, &v.hdr->status, lane);
             break;
@@ -102,17 +114,26 @@ __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force_x2(DeviceView 
     }
     if (kEnergy)
     {
-        double elj = e_lj_acc, eel = e_el_acc;
+        // one add per block and energy: all blocks' adds fall on two addresses, where FP64 adds serialise
+        // (an add per warp cost about 4 us at the end of every launch)
+        __syncthreads();
+        if (threadIdx.x < 64)
+        {
+            const double* acc = e_acc_s[threadIdx.x >> 5];
+            double        sum = 0.0;
+            for (int i = lane; i < kForceThreads; i += 32)
+            {
+                sum += acc[i];
+            }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            elj += __shfl_xor_sync(full, elj, o);
-            eel += __shfl_xor_sync(full, eel, o);
-        }
-        if (lane == 0)
-        {
-            atomicAdd(&v.energy[0], elj);
-            atomicAdd(&v.energy[1], eel * v.epsfac_d);
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                sum += __shfl_xor_sync(full, sum, o);
+            }
+            if (lane == 0 && sum != 0.0)
+            {
+                atomicAdd(&v.energy[threadIdx.x >> 5], threadIdx.x < 32 ? sum : sum * v.epsfac_d);
+            }
         }
     }
 }

@@ -253,8 +253,9 @@ struct DeviceView
     // (nbnxn_gpu_add_nbat_f_to_f_kernel<accumulateForce = true>); 0: overwrites it
     int accumulate_f;
     // > 0: the energy flavours of k_force also compute the excluded-pair and self energies, as
-    // this many work items of kExclChunkAtoms atoms interleaved with the list entries
+    // this many work items of excl_atoms atoms interleaved with the list entries
     int excl_chunks;
+    int excl_atoms;
     // force kernel tile: 1 = packed core (two pairs per lane, FP32x2 arithmetic; potential-shift
     // or plain cut-off LJ), 0 = scalar core (one pair per lane); j-stage buffers per warp (2, 3)
     int pair_core;
