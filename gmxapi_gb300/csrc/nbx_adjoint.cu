@@ -15,15 +15,24 @@
 // excluded pair), whose derivative is psi' = -(1.5 psi + (2b/sqrt(pi)) b^2
 // e^{-b^2 r^2}) / r^2 for normal and excluded pairs alike.
 //
-// Layout: as the forward kernel (persistent warps, one list entry per warp,
-// lane = j-atom-of-half * 8 + i-atom); the entry's shifted i-atoms and their
-// upstream gradients are staged in shared memory, the per-lane i accumulators
-// (dx, dy, dz, dq per i-cluster) stay in registers; j accumulators are reduced
-// over the 8 i-lanes and added with one vector red per j-atom.  Type-pair
-// gradients go to a warp-private shared table and are flushed to FP64 global
-// sums after every entry.
+// Layout: persistent warps, one list entry per warp, an 8x8 cluster pair per step: lane (j, ip) =
+// (lane >> 2, lane & 3) computes j-atom j against the i-atoms ip and ip + 4 in one FP32x2 instruction
+// stream.  The entry's i-atoms and their upstream gradients sit in shared memory as packed pairs, the
+// lane's i-side sums beside them (one slot per lane and i-cluster: no conflicts); the j-side sums stay in
+// registers and end in one add per lane.
+//
+// Type-pair gradients.  d6 / d12 of a step are 8x8 matrices G over (i-atom, j-atom), and the table gradient
+// is sum_steps P_i^T G P_j with one-hot type matrices P: a contraction, so it runs on the tensor cores.
+// The lane mapping above is the B fragment of mma.m16n8k8 (k = i-atom, n = j-atom), P_i^T is its A
+// fragment, and the products are exact: a one-hot factor times a float split into three tf32 parts
+// (11 + 11 + 2 bits).  The high parts and the lower ones are summed in accumulators of their own over the
+// at most 8 steps of a j-cluster, then a second product with P_j gives the types (a, b), added in FP32 over
+// the entry and in FP64 beyond it.  (Float atomics on per-warp tables in shared memory, which this
+// replaces, are compare-and-swap loops.)  The kernel is bound by instruction issue and latency.
+// 24,000-atom 8-type liquid: 91.6 us with one pair per lane and table atomics; 16 liquids of 2,000 to
+// 50,000 atoms: 758 us.
 #include "nbx_internal.cuh"
-#include "nbx_pair_core.cuh"
+#include "nbx_pair_x2.cuh"
 
 #include <algorithm>
 
@@ -32,406 +41,569 @@ namespace nbx
 namespace
 {
 
-constexpr int kAdjThreads    = 256;
-constexpr int kAdjBlocksPerSm = 2;  // 16 warps per SM (128 registers a thread, no spills)
-constexpr int kAdjWarps      = kAdjThreads / 32;
-constexpr int kAdjMaxTypes1  = 16;
-// Up to this many types (+ the dummy type) every warp keeps one type-pair gradient table per
-// i-atom lane index (8 replicas): the lanes that add into one table in the same instruction then
-// share their i-atom, so two of them hit the same entry only when their j-atoms have the same type.
-constexpr int kAdjRepTypes1  = 10;
-constexpr int kAdjReplicas   = kCl;
+constexpr int kAdjThreads     = 256;
+constexpr int kAdjBlocksPerSm = 2;  // 16 warps per SM
+constexpr int kAdjWarps       = kAdjThreads / 32;
+constexpr int kAdjMaxTypes1   = 16;
+constexpr int kAdjRow         = 16;  // type-pair rows of 16 entries in shared memory
 
-// Type-pair gradient tables of one warp: replicas x (nt1^2 + 1) float2, each replica planar (its
-// nt1^2 + 1 dc6 sums, then its nt1^2 + 1 dc12 sums; the +1 staggers the replicas over the
-// shared-memory banks).
-__host__ __device__ __forceinline__ int adj_table_replicas(int nt1)
-{
-    return nt1 <= kAdjRepTypes1 ? kAdjReplicas : 1;
-}
-__host__ __device__ __forceinline__ int adj_table_stride(int nt1)
-{
-    return nt1 * nt1 + 1;
-}
-
+// Constants of the pair loop; gE_*: upstream energy gradients (0 in the flavours without them).
 struct AdjConsts
 {
-    float gE_lj, gE_c;  // upstream energy gradients
+    float rc2, pbeta, nbeta2l2, c2b, nb2c2b, sh_ewald, nk_rf2, k_rf, c_rf, epsfac, cpot6, cpot12;
+    float gE_lj, gE_c;
+    int   filler;  // the type of empty slots
 };
+
+__device__ __forceinline__ AdjConsts adj_consts(const DeviceView& v)
+{
+    AdjConsts k;
+    k.rc2      = v.rc2;
+    k.pbeta    = v.pbeta;
+    k.nbeta2l2 = -v.beta2l2;
+    k.c2b      = v.c2b;
+    k.nb2c2b   = -v.beta * v.beta * v.c2b;
+    k.sh_ewald = v.sh_ewald;
+    k.nk_rf2   = -2.0f * v.k_rf;
+    k.k_rf     = v.k_rf;
+    k.c_rf     = v.c_rf;
+    k.epsfac   = v.epsfac;
+    k.cpot6    = v.cpot6 * (1.0f / 6.0f);
+    k.cpot12   = v.cpot12 * (1.0f / 12.0f);
+    k.gE_lj    = 0.0f;
+    k.gE_c     = 0.0f;
+    k.filler   = v.ntypes1 - 1;
+    return k;
+}
 
 // The per-system arrays one list entry of the adjoint touches.
 struct AdjPtrs
 {
     const float4* xq;
-    const int*    tgrid;
     const Cj4*    cj4;
     const Excl*   excl;
     const float*  shiftvec;
-    const float4* gnb;
+    const float4* gnb;  // upstream gradient and type (int bits) per slot
     float4*       dnb;
 };
 
-// One atom pair (i-atom ii of i-cluster c, the lane's j-atom): recomputes the pair terms, adds
-// the i-side gradients to the lane's accumulator slot acc[(c * 8 + ii) * 4 + jj] (shared memory,
-// one slot per lane and i-atom: no conflicts), the j-side ones to dj*, and the type-pair gradient
-// to the lane's table.
-template<bool kEwald, bool kExcl>
-__device__ __forceinline__ void adj_pair(const DeviceView& v, const float2* __restrict__ nbfp_s, float2* ttab,
-                                         const float4* __restrict__ xis, const float4* __restrict__ gis, float4* acc,
-                                         int c, const float4 xj, const float4 gj, int tj, unsigned wj, bool diag_cj,
-                                         int h, int ii, int jj, const AdjConsts& k, float pbeta, float beta2l2,
-                                         float c2b, float b2c2b, float& djx, float& djy, float& djz, float& djq)
+// Shared memory of one warp.
+struct AdjWarp
 {
-    const int    nt1 = v.ntypes1;
-    const float4 xi  = xis[c * kCl + ii];
-    const float4 gi  = gis[c * kCl + ii];
-    const int    ti  = __float_as_int(gi.w);
-    const float  dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    float        r2 = dx * dx + dy * dy + dz * dz;
-    bool         in_range;
-    float        int_bit;
-    if (kExcl)
+    // per i-cluster and ip: {x, x', y, y'}, {z, z', q, q'}, {gx, gx', gy, gy'}, {gz, gz', type, type'} of
+    // the atoms ip and ip + 4
+    float4 irec[kNcl][4][4];
+    // per i-cluster and lane: {x, x', y, y'}, {z, z', q, q'} sums (rows padded by four entries: the
+    // reduction reads eight lanes' sums of two clusters at a time)
+    float4 acc[kNcl][2 * 32 + 4];
+    float4 jx[32], jg[32];
+};
+
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], float b0, float b1)
+{
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+                 "{%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+
+// The leading 11 significant bits of x (a tf32 value).
+__device__ __forceinline__ float tf32_head(float x)
+{
+    return __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+}
+
+// d_hi, d_lo += A {b0, b1} with b split into three tf32 parts, exactly representable each.
+__device__ __forceinline__ void mma_split_b(float (&d_hi)[4], float (&d_lo)[4], const unsigned (&a)[4], float b0,
+                                            float b1)
+{
+    const float h0 = tf32_head(b0), h1 = tf32_head(b1);
+    const float r0 = b0 - h0, r1 = b1 - h1;
+    const float m0 = tf32_head(r0), m1 = tf32_head(r1);
+    mma_tf32(d_hi, a, h0, h1);
+    mma_tf32(d_lo, a, m0, m1);
+    mma_tf32(d_lo, a, r0 - m0, r1 - m1);
+}
+
+// The same with the split factor as A (rows 8.. only with kBig) and a one-hot B; the sum is returned in d.
+template<bool kBig>
+__device__ __forceinline__ void mma_split_a(float (&d)[4], const float (&x)[4], float b0, float b1)
+{
+    float    lo[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+    unsigned h[4], m[4], l[4];
+    // C fragment (row, 2 l), (row, 2 l + 1), (row + 8, ...) as the A fragment with columns in that order
+    const float c[4] = { x[0], x[2], x[1], x[3] };
+#pragma unroll
+    for (int i = 0; i < 4; i++)
     {
-        // the diagonal cluster pair counts j > i only
-        const bool self_lower = diag_cj && (c == (int)(wj >> 24)) && (h * (kCl / kSplit) + jj <= ii);
-        in_range              = (r2 < v.rc2) && !self_lower;
-        int_bit               = (wj & (1u << c)) ? 1.0f : 0.0f;
-    }
-    else
-    {
-        in_range = r2 < v.rc2;
-        int_bit  = 1.0f;
-    }
-    r2                   = fmaxf(r2, kMinDist2);
-    float       rinv     = fast_rsqrt(r2);
-    rinv                 = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
-    const float  rinv2   = rinv * rinv;
-    const float2 lj      = nbfp_s[ti * nt1 + tj];
-    float        rinv6   = rinv2 * rinv2 * rinv2;
-    if (kExcl)
-    {
-        rinv6 *= int_bit;
-    }
-    const float vrep    = lj.y * rinv6 * rinv6;
-    const float vdisp   = lj.x * rinv6;
-    const float phi_lj  = (vrep - vdisp) * rinv2;
-    const float dphi_lj = (4.0f * vdisp - 7.0f * vrep) * rinv2 * rinv2;
-    float       psi, dpsi, hq;  // Coulomb phi / qq, its s-derivative, energy / qq
-    if (kEwald)
-    {
-        const float r    = r2 * rinv;
-        const float t    = fast_rcp(fmaf(pbeta, r, 1.0f));
-        const float poly = erfc_poly(t);
-        const float expm = fast_ex2(-beta2l2 * r2);
-        const float tp   = t * poly;
-        psi              = expm * fmaf(tp, rinv, c2b) * rinv2;
-        hq               = tp * expm * rinv - int_bit * v.sh_ewald;
-        if (kExcl)
+        if (!kBig && (i & 1))
         {
-            psi -= (1.0f - int_bit) * rinv * rinv2;
-            hq -= (1.0f - int_bit) * rinv;
+            h[i] = m[i] = l[i] = 0u;
+            continue;
         }
-        dpsi = -(1.5f * psi + b2c2b * expm) * rinv2;
+        const float hi = tf32_head(c[i]);
+        const float r  = c[i] - hi;
+        const float mi = tf32_head(r);
+        h[i]           = __float_as_uint(hi);
+        m[i]           = __float_as_uint(mi);
+        l[i]           = __float_as_uint(r - mi);
     }
-    else
+    d[0] = d[1] = d[2] = d[3] = 0.0f;
+    mma_tf32(d, h, b0, b1);
+    mma_tf32(lo, m, b0, b1);
+    mma_tf32(lo, l, b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
     {
-        const float r3 = rinv * rinv2;
-        psi            = int_bit * r3 - 2.0f * v.k_rf;
-        dpsi           = -1.5f * int_bit * r3 * rinv2;
-        hq             = int_bit * rinv + v.k_rf * r2 - v.c_rf;
-    }
-    const float qq   = v.epsfac * xi.w * xj.w;
-    const float phi  = fmaf(qq, psi, phi_lj);
-    const float dphi = fmaf(qq, dpsi, dphi_lj);
-    const float gx = gi.x - gj.x, gy = gi.y - gj.y, gz = gi.z - gj.z;
-    const float gr   = gx * dx + gy * dy + gz * dz;
-    const float coef = 2.0f * dphi * gr - fmaf(k.gE_c * qq, psi, k.gE_lj * phi_lj);
-    float       ux   = fmaf(phi, gx, coef * dx);
-    float       uy   = fmaf(phi, gy, coef * dy);
-    float       uz   = fmaf(phi, gz, coef * dz);
-    float       wq   = v.epsfac * fmaf(psi, gr, k.gE_c * hq);
-    ux               = in_range ? ux : 0.0f;
-    uy               = in_range ? uy : 0.0f;
-    uz               = in_range ? uz : 0.0f;
-    wq               = in_range ? wq : 0.0f;
-    float4* const ai = &acc[(c * kCl + ii) * 4 + jj];
-    float4        av = *ai;
-    av.x += ux;
-    av.y += uy;
-    av.z += uz;
-    av.w = fmaf(wq, xj.w, av.w);
-    *ai  = av;
-    djx -= ux;
-    djy -= uy;
-    djz -= uz;
-    djq = fmaf(wq, xi.w, djq);
-    // dL/d(6C6), dL/d(12C12) of this type pair
-    if (in_range && int_bit != 0.0f)
-    {
-        const float dc12 = fmaf(gr * rinv6, rinv6 * rinv2, k.gE_lj * (rinv6 * rinv6 + v.cpot12) * (1.0f / 12.0f));
-        const float dc6  = -fmaf(gr * rinv6, rinv2, k.gE_lj * (rinv6 + v.cpot6) * (1.0f / 6.0f));
-        // planar replica: the dc6 sums, then (one table stride on) the dc12 sums, so that a warp's
-        // 32 atomics spread over all banks instead of the even ones of interleaved pairs
-        float* const slot = reinterpret_cast<float*>(ttab) + ti * nt1 + tj;
-        atomicAdd(slot, dc6);
-        atomicAdd(slot + adj_table_stride(nt1), dc12);
+        d[i] += lo[i];
     }
 }
 
-// One warp half's j-clusters of a cj4 group: per j-cluster with set bits, the set i-clusters are
-// visited two at a time (two independent pair computations in one basic block), the j-side sums
-// reduced over the 8 i-lanes and added with one vector red per j-atom.
-template<bool kEwald, bool kExcl>
-__device__ __forceinline__ void adj_half(const DeviceView& v, const float4* __restrict__ jx,
-                                         const float4* __restrict__ jg, const float2* __restrict__ nbfp_s,
-                                         float2* ttab, const float4* __restrict__ xis, const float4* __restrict__ gis,
-                                         float4* acc, float4* dnb, const int cj_lane, unsigned im, unsigned wexcl,
-                                         int h, int sci, bool central, int ii, int jj, const AdjConsts& k,
-                                         float pbeta, float beta2l2, float c2b, float b2c2b)
+// j-side sums of the lane's j-atom over its two i-atoms' slots, and the type-pair products of one j-cluster.
+struct AdjJ
+{
+    float2 x, y, z, q;
+    float  h6[4], l6[4], h12[4], l12[4];
+};
+
+// One step: i-cluster c against the lane's j-atom.  okA / okB: the pair's mask bit (and, on the diagonal,
+// j > i); intA / intB: its exclusion bit as 0 / 1.
+template<bool kEwald, bool kGE, bool kBig, bool kExcl>
+__device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w, int c,
+                                         int lane, const float4 xj, const float4 gj, float qje, int tjb, bool okA,
+                                         bool okB, float intA, float intB, AdjJ& dj)
+{
+    const int     ip = lane & 3;
+    const float4  i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
+    const int     tA = __float_as_int(i3.z), tB = __float_as_int(i3.w);
+    const float2  dx = sub2(make_float2(i0.x, i0.y), f2(xj.x));
+    const float2  dy = sub2(make_float2(i0.z, i0.w), f2(xj.y));
+    const float2  dz = sub2(make_float2(i1.x, i1.y), f2(xj.z));
+    float2        r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+    const bool    inA = okA && r2.x < k.rc2, inB = okB && r2.y < k.rc2;
+    r2                = make_float2(fmaxf(r2.x, kMinDist2), fmaxf(r2.y, kMinDist2));
+    float2       rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
+    rinv              = fma2(rinv, fma2(mul2(r2, f2(-0.5f)), mul2(rinv, rinv), f2(0.5f)), rinv);
+    // 1/r = 0 for pairs out of range: every term below then vanishes, but for the constants, which have
+    // their own masks
+    rinv               = make_float2(inA ? rinv.x : 0.0f, inB ? rinv.y : 0.0f);
+    const float2 rinv2 = mul2(rinv, rinv);
+    const float2 ljA   = *reinterpret_cast<const float2*>(nbfp_b + (tA << 7) + tjb);
+    const float2 ljB   = *reinterpret_cast<const float2*>(nbfp_b + (tB << 7) + tjb);
+    float2       rinv6 = mul2(mul2(rinv2, rinv2), rinv2);
+    if (kExcl)
+    {
+        rinv6 = mul2(rinv6, make_float2(intA, intB));
+    }
+    const float2 vdisp   = make_float2(ljA.x * rinv6.x, ljB.x * rinv6.y);
+    const float2 vrep    = make_float2(ljA.y * rinv6.x * rinv6.x, ljB.y * rinv6.y * rinv6.y);
+    const float2 phi_lj  = mul2(sub2(vrep, vdisp), rinv2);
+    const float2 dphi_lj = mul2(fma2(f2(-7.0f), vrep, mul2(f2(4.0f), vdisp)), mul2(rinv2, rinv2));
+    float2       psi, dpsi, hq = f2(0.0f);  // Coulomb phi / qq, its s-derivative, energy / qq
+    if (kEwald)
+    {
+        const float2 tt   = fma2(f2(k.pbeta), mul2(r2, rinv), f2(1.0f));
+        const float2 t    = make_float2(fast_rcp(tt.x), fast_rcp(tt.y));
+        const float2 earg = mul2(f2(k.nbeta2l2), r2);
+        const float2 expm = make_float2(fast_ex2(earg.x), fast_ex2(earg.y));
+        const float2 tp   = mul2(mul2(t, erfc_poly2(t)), rinv);  // erfc(beta r) / r = tp expm
+        psi               = mul2(mul2(expm, add2(tp, f2(k.c2b))), rinv2);
+        if (kGE)
+        {
+            hq = fma2(tp, expm, make_float2(inA ? -intA * k.sh_ewald : 0.0f, inB ? -intB * k.sh_ewald : 0.0f));
+        }
+        if (kExcl)
+        {
+            const float2 ex = mul2(make_float2(intA - 1.0f, intB - 1.0f), rinv);  // -(1 - int) / r
+            psi             = fma2(ex, rinv2, psi);
+            if (kGE)
+            {
+                hq = add2(hq, ex);
+            }
+        }
+        dpsi = mul2(fma2(f2(-1.5f), psi, mul2(f2(k.nb2c2b), expm)), rinv2);
+    }
+    else
+    {
+        const float2 r3 = kExcl ? mul2(mul2(rinv, rinv2), make_float2(intA, intB)) : mul2(rinv, rinv2);
+        psi             = add2(r3, make_float2(inA ? k.nk_rf2 : 0.0f, inB ? k.nk_rf2 : 0.0f));
+        dpsi            = mul2(mul2(f2(-1.5f), r3), rinv2);
+        if (kGE)
+        {
+            const float2 h = fma2(f2(k.k_rf), r2, sub2(mul2(rinv, make_float2(intA, intB)), f2(k.c_rf)));
+            hq             = make_float2(inA ? h.x : 0.0f, inB ? h.y : 0.0f);
+        }
+    }
+    const float2 qi   = make_float2(i1.z, i1.w);
+    const float2 qq   = mul2(qi, f2(qje));
+    const float2 phi  = fma2(qq, psi, phi_lj);
+    const float2 dphi = fma2(qq, dpsi, dphi_lj);
+    const float2 gx   = sub2(make_float2(i2.x, i2.y), f2(gj.x));
+    const float2 gy   = sub2(make_float2(i2.z, i2.w), f2(gj.y));
+    const float2 gz   = sub2(make_float2(i3.x, i3.y), f2(gj.z));
+    const float2 gr   = fma2(gz, dz, fma2(gy, dy, mul2(gx, dx)));
+    float2       coef = mul2(mul2(f2(2.0f), dphi), gr);
+    float2       wq   = mul2(psi, gr);  // dL/d(q_i q_j) / epsfac
+    if (kGE)
+    {
+        coef = sub2(coef, fma2(f2(k.gE_c), mul2(qq, psi), mul2(f2(k.gE_lj), phi_lj)));
+        wq   = fma2(f2(k.gE_c), hq, wq);
+    }
+    const float2 ux = fma2(phi, gx, mul2(coef, dx));
+    const float2 uy = fma2(phi, gy, mul2(coef, dy));
+    const float2 uz = fma2(phi, gz, mul2(coef, dz));
+    float4* const pa = &w.acc[c][lane];
+    float4 a0 = pa[0], a1 = pa[32];
+    const float2 sx = add2(make_float2(a0.x, a0.y), ux), sy = add2(make_float2(a0.z, a0.w), uy);
+    const float2 sz = add2(make_float2(a1.x, a1.y), uz), sq = fma2(wq, f2(qje), make_float2(a1.z, a1.w));
+    pa[0]  = make_float4(sx.x, sx.y, sy.x, sy.y);
+    pa[32] = make_float4(sz.x, sz.y, sq.x, sq.y);
+    dj.x   = add2(dj.x, ux);
+    dj.y   = add2(dj.y, uy);
+    dj.z   = add2(dj.z, uz);
+    dj.q   = fma2(wq, qi, dj.q);
+    // dL/d(6C6) and dL/d(12C12) of the pairs, by i type
+    float2 d6  = mul2(gr, mul2(rinv6, rinv2));
+    float2 d12 = mul2(d6, rinv6);
+    if (kGE)
+    {
+        const bool   cA = inA && (!kExcl || intA != 0.0f), cB = inB && (!kExcl || intB != 0.0f);
+        const float2 e6 = fma2(rinv6, f2(1.0f / 6.0f), make_float2(cA ? k.cpot6 : 0.0f, cB ? k.cpot6 : 0.0f));
+        const float2 e12 =
+                fma2(mul2(rinv6, rinv6), f2(1.0f / 12.0f), make_float2(cA ? k.cpot12 : 0.0f, cB ? k.cpot12 : 0.0f));
+        d6  = fma2(f2(k.gE_lj), e6, d6);
+        d12 = fma2(f2(k.gE_lj), e12, d12);
+    }
+    const int      row   = lane >> 2;
+    const unsigned one   = 0x3f800000u;
+    const unsigned hot[4] = { tA == row ? one : 0u, kBig && tA == row + 8 ? one : 0u, tB == row ? one : 0u,
+                              kBig && tB == row + 8 ? one : 0u };
+    mma_split_b(dj.h6, dj.l6, hot, d6.x, d6.y);
+    mma_split_b(dj.h12, dj.l12, hot, d12.x, d12.y);
+}
+
+// Type-pair sums of an entry: C fragments (type rows lane >> 2 (+ 8), columns 2 (lane & 3) + {0, 1} of
+// column tile n) of dL/d(6C6) (negated) and dL/d(12C12).
+template<bool kBig>
+struct AdjTypes
+{
+    float s6[kBig ? 2 : 1][4], s12[kBig ? 2 : 1][4];
+};
+
+// All set cluster pairs of one cj4 group.  m: the mask of the lane's half; u: both halves' masks; wA / wB:
+// the lane's exclusion words (i-atoms ip and ip + 4).
+template<bool kEwald, bool kGE, bool kBig, bool kExcl>
+__device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w,
+                                          float4* __restrict__ dnb, int cj_lane, unsigned m, unsigned u, unsigned wA,
+                                          unsigned wB, int sci, bool central, int lane, AdjTypes<kBig>& types)
 {
     const unsigned full = 0xffffffffu;
+    const int      j = lane >> 2, ip = lane & 3;
 #pragma unroll 1
     for (int jm = 0; jm < kJg; jm++)
     {
-        unsigned   rem = (im >> (jm * kNcl)) & 0xffu;
-        const int  cj  = __shfl_sync(full, cj_lane, jm);
+        unsigned  rem = (u >> (jm * kNcl)) & 0xffu;
+        const int cj  = __shfl_sync(full, cj_lane, jm);
         if (!rem)
         {
             continue;
         }
-        const int    aj = cj * kCl + h * (kCl / kSplit) + jj;
-        // the cj4 group's 32 j-atoms are staged in shared memory (slot jm * 8 + atom)
-        const int    sj = jm * kCl + h * (kCl / kSplit) + jj;
-        const float4 xj = jx[sj];
-        const float4 gj = jg[sj];
-        const int    tj = __float_as_int(gj.w);
-        // exclusion bits of this j-cluster's i-clusters; bits 24.. carry the diagonal i-cluster
-        const bool     diag_cj = kExcl && central && (cj >= sci * kNcl) && (cj < sci * kNcl + kNcl);
-        const unsigned wj      = kExcl ? (((wexcl >> (jm * kNcl)) & 0xffu) | ((unsigned)(cj - sci * kNcl) << 24)) : 0u;
-        float          djx = 0.0f, djy = 0.0f, djz = 0.0f, djq = 0.0f;
+        const float4   xj   = w.jx[jm * kCl + j], gj = w.jg[jm * kCl + j];
+        const int      tj   = __float_as_int(gj.w);
+        const float    qje  = xj.w * k.epsfac;
+        // an empty slot has no pairs: two empty slots coincide, and the huge powers of their 1/r must not meet
+        // the zeros of the one-hot factors
+        const unsigned mj   = tj == k.filler ? 0u : m >> (jm * kNcl);
+        const unsigned xA   = wA >> (jm * kNcl), xB = wB >> (jm * kNcl);
+        const int      diag = kExcl && central ? cj - sci * kNcl : -1;  // the diagonal i-cluster, if in 0 .. 7
+        AdjJ           dj;
+        dj.x = dj.y = dj.z = dj.q = f2(0.0f);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+        {
+            dj.h6[i] = dj.l6[i] = dj.h12[i] = dj.l12[i] = 0.0f;
+        }
+        auto step = [&](int c) {
+            bool  okA = (mj >> c) & 1u, okB = okA;
+            float intA = 1.0f, intB = 1.0f;
+            if (kExcl)
+            {
+                // the diagonal cluster pair counts j > i only
+                okA  = okA && !(c == diag && j <= ip);
+                okB  = okB && !(c == diag && j <= ip + 4);
+                intA = ((xA >> c) & 1u) ? 1.0f : 0.0f;
+                intB = ((xB >> c) & 1u) ? 1.0f : 0.0f;
+            }
+            adj_step<kEwald, kGE, kBig, kExcl>(k, nbfp_b, w, c, lane, xj, gj, qje, tj * 8, okA, okB, intA, intB, dj);
+        };
+#pragma unroll 1
         while (rem)
         {
             const int ca = __ffs(rem) - 1;
             rem &= rem - 1;
             if (rem)
             {
+                // two independent steps share a basic block
                 const int cb = __ffs(rem) - 1;
                 rem &= rem - 1;
-                adj_pair<kEwald, kExcl>(v, nbfp_s, ttab, xis, gis, acc, ca, xj, gj, tj, wj, diag_cj, h, ii, jj, k,
-                                        pbeta, beta2l2, c2b, b2c2b, djx, djy, djz, djq);
-                adj_pair<kEwald, kExcl>(v, nbfp_s, ttab, xis, gis, acc, cb, xj, gj, tj, wj, diag_cj, h, ii, jj, k,
-                                        pbeta, beta2l2, c2b, b2c2b, djx, djy, djz, djq);
+                step(ca);
+                step(cb);
             }
             else
             {
-                adj_pair<kEwald, kExcl>(v, nbfp_s, ttab, xis, gis, acc, ca, xj, gj, tj, wj, diag_cj, h, ii, jj, k,
-                                        pbeta, beta2l2, c2b, b2c2b, djx, djy, djz, djq);
+                step(ca);
             }
         }
+        // j side: the two slots, then the four ip lanes reduce-scattered to one component each
+        float2      xy = make_float2(dj.x.x + dj.x.y, dj.y.x + dj.y.y);
+        float2      zq = make_float2(dj.z.x + dj.z.y, -k.epsfac * (dj.q.x + dj.q.y));
+        const bool  o1 = lane & 1, o2 = lane & 2;
+        float2      keep = o2 ? zq : xy, send = o2 ? xy : zq;
+        keep.x += __shfl_xor_sync(full, send.x, 2);
+        keep.y += __shfl_xor_sync(full, send.y, 2);
+        float one = (o1 ? keep.y : keep.x) + __shfl_xor_sync(full, o1 ? keep.x : keep.y, 1);
+        atomicAdd(reinterpret_cast<float*>(&dnb[cj * kCl + j]) + ip, -one);
+        // type pairs: columns j = 2 ip, 2 ip + 1 of the products times the one-hot j types
+        const int t0 = __shfl_sync(full, tj, 8 * ip), t1 = __shfl_sync(full, tj, 8 * ip + 4);
+        float     c6[4], c12[4];
 #pragma unroll
-        for (int o = 1; o < kCl; o <<= 1)
+        for (int i = 0; i < 4; i++)
         {
-            djx += __shfl_xor_sync(full, djx, o);
-            djy += __shfl_xor_sync(full, djy, o);
-            djz += __shfl_xor_sync(full, djz, o);
-            djq += __shfl_xor_sync(full, djq, o);
+            c6[i]  = dj.h6[i] + dj.l6[i];
+            c12[i] = dj.h12[i] + dj.l12[i];
         }
-        if (ii == 0)
+#pragma unroll
+        for (int n = 0; n < (kBig ? 2 : 1); n++)
         {
-            red_add_v4(&dnb[aj], djx, djy, djz, djq);
+            const float b0 = t0 == j + 8 * n ? 1.0f : 0.0f, b1 = t1 == j + 8 * n ? 1.0f : 0.0f;
+            float       d[4];
+            mma_split_a<kBig>(d, c6, b0, b1);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+                types.s6[n][i] += d[i];
+            }
+            mma_split_a<kBig>(d, c12, b0, b1);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+                types.s12[n][i] += d[i];
+            }
         }
     }
 }
 
-// One list entry: its 64 shifted i-atoms and their upstream gradients go to the
-// warp's shared-memory slots, all cj4 groups are processed, then the i-side sums
-// and the entry's type-pair table are flushed (vector reds / FP64 atomics).
-template<bool kEwald>
-__device__ __forceinline__ void adj_entry(const DeviceView& v, const AdjPtrs& p, const Sci& s,
-                                          const float2* __restrict__ nbfp_s, float2* ttab, float4* xis, float4* gis,
-                                          float4* jx, float4* jg, float4* acc, int lane, const AdjConsts& k,
-                                          float pbeta, float beta2l2, float c2b, float b2c2b, double* gnbfp)
+// FP64 sums per lane: (column tile, C fragment element, {6C6, 12C12})
+template<bool kBig>
+__host__ __device__ constexpr int adj_lane_sums()
+{
+    return kBig ? 16 : 4;
+}
+
+// Copies of the lanes' sums in a block: one per warp, or with 16 values a lane (32 KB for 8 warps, which
+// would leave room for one block per SM) one that the warps add to atomically.
+template<bool kBig>
+__host__ __device__ constexpr int adj_sum_copies()
+{
+    return kBig ? 1 : kAdjWarps;
+}
+
+// One list entry.  gsum: the lane's FP64 type-pair sums (shared memory, stride 32).
+template<bool kEwald, bool kGE, bool kBig>
+__device__ __forceinline__ void adj_entry(const AdjConsts& k, const AdjPtrs& p, const Sci& s,
+                                          const char* __restrict__ nbfp_b, AdjWarp& w, double* gsum, int lane)
 {
     const unsigned full    = 0xffffffffu;
-    const int      ii      = lane & 7;
-    const int      jj      = lane >> 3;
-    const int      nt1     = v.ntypes1;
     const float    sx = p.shiftvec[3 * s.shift], sy = p.shiftvec[3 * s.shift + 1], sz = p.shiftvec[3 * s.shift + 2];
     const bool     central = (s.shift == kCentral);
-    const int      reps    = adj_table_replicas(nt1);
-    const int      tstride = adj_table_stride(nt1);
-    float2* const  ttab_lane = ttab + (reps > 1 ? ii : 0) * tstride;
     __syncwarp();
-    for (int m = lane; m < kSc; m += 32)
+    // lane (c, ip) fills the records of the i-atoms ip and ip + 4 of i-cluster c
     {
-        const int    a = s.sci * kSc + m;
-        const float4 x = p.xq[a];
-        const float4 g = p.gnb[a];
-        xis[m]         = make_float4(x.x + sx, x.y + sy, x.z + sz, x.w);
-        gis[m]         = make_float4(g.x, g.y, g.z, __int_as_float(p.tgrid[a]));
+        const int    c = lane >> 2, ip = lane & 3;
+        const int    a = s.sci * kSc + c * kCl + ip;
+        const float4 x0 = p.xq[a], x1 = p.xq[a + 4], g0 = p.gnb[a], g1 = p.gnb[a + 4];
+        w.irec[c][0][ip] = make_float4(x0.x + sx, x1.x + sx, x0.y + sy, x1.y + sy);
+        w.irec[c][1][ip] = make_float4(x0.z + sz, x1.z + sz, x0.w, x1.w);
+        w.irec[c][2][ip] = make_float4(g0.x, g1.x, g0.y, g1.y);
+        w.irec[c][3][ip] = make_float4(g0.z, g1.z, g0.w, g1.w);
     }
-    for (int m = lane; m < kSc * 4; m += 32)
+#pragma unroll
+    for (int c = 0; c < kNcl; c++)
     {
-        acc[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w.acc[c][lane]      = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w.acc[c][32 + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    __syncwarp();
-    // software pipeline over the cj4 groups, as in the force kernel: the next group's
-    // record is loaded when a group starts, its 32 j-atoms after the group's first half
+    AdjTypes<kBig> types;
+#pragma unroll
+    for (int n = 0; n < (kBig ? 2 : 1); n++)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+        {
+            types.s6[n][i] = types.s12[n][i] = 0.0f;
+        }
+    }
+    // the next group's record and j-atoms are loaded while a group is computed
     int4   rec_ime{};
     int    rec_cj = 0;
     float4 xr{}, gr{};
-    if (s.cj4_start < s.cj4_end)
-    {
-        rec_ime     = *reinterpret_cast<const int4*>(&p.cj4[s.cj4_start].imei[0]);
-        rec_cj      = (lane < kJg) ? p.cj4[s.cj4_start].cj[lane] : 0;
+    auto load_record = [&](int g) {
+        rec_ime = *reinterpret_cast<const int4*>(&p.cj4[g].imei[0]);
+        rec_cj  = (lane < kJg) ? p.cj4[g].cj[lane] : 0;
+    };
+    auto load_atoms = [&]() {
         const int a = __shfl_sync(full, rec_cj, lane >> 3) * kCl + (lane & (kCl - 1));
         xr          = p.xq[a];
         gr          = p.gnb[a];
-        gr.w        = __int_as_float(p.tgrid[a]);
+    };
+    if (s.cj4_start < s.cj4_end)
+    {
+        load_record(s.cj4_start);
+        load_atoms();
     }
     for (int j4 = s.cj4_start; j4 < s.cj4_end; j4++)
     {
         const int4 ime     = rec_ime;
         const int  cj_lane = rec_cj;
         __syncwarp();
-        jx[lane] = xr;
-        jg[lane] = gr;
+        w.jx[lane] = xr;
+        w.jg[lane] = gr;
         __syncwarp();
-        const bool more = j4 + 1 < s.cj4_end;
-        if (more)
+        if (j4 + 1 < s.cj4_end)
         {
-            rec_ime = *reinterpret_cast<const int4*>(&p.cj4[j4 + 1].imei[0]);
-            rec_cj  = (lane < kJg) ? p.cj4[j4 + 1].cj[lane] : 0;
+            load_record(j4 + 1);
+            load_atoms();
         }
-#pragma unroll 1
-        for (int h = 0; h < kSplit; h++)
+        const unsigned m0 = (unsigned)ime.x, m1 = (unsigned)ime.z;
+        const unsigned m  = lane < 16 ? m0 : m1;
+        if ((ime.y | ime.w) == 0)
         {
-            if (h == 1 && more)
+            adj_group<kEwald, kGE, kBig, false>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, ~0u, ~0u, s.sci, central,
+                                                lane, types);
+        }
+        else
+        {
+            const unsigned* pair = p.excl[lane < 16 ? ime.y : ime.w].pair;
+            const int       at   = ((lane >> 2) & 3) * kCl + (lane & 3);
+            adj_group<kEwald, kGE, kBig, true>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, pair[at], pair[at + 4], s.sci,
+                                               central, lane, types);
+        }
+    }
+    // the i-side sums: lane (c, ip) adds the eight j-lanes' slots of the atoms ip and ip + 4
+    __syncwarp();
+    {
+        const int c = lane >> 2, ip = lane & 3;
+        float4    t0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), t1 = t0;
+#pragma unroll
+        for (int j = 0; j < kCl; j++)
+        {
+            const float4 a = w.acc[c][4 * j + ip], b = w.acc[c][32 + 4 * j + ip];
+            t0.x += a.x;
+            t0.y += a.y;
+            t0.z += a.z;
+            t0.w += a.w;
+            t1.x += b.x;
+            t1.y += b.y;
+            t1.z += b.z;
+            t1.w += b.w;
+        }
+        const int at = s.sci * kSc + c * kCl + ip;
+        red_add_v4(&p.dnb[at], t0.x, t0.z, t1.x, t1.z);
+        red_add_v4(&p.dnb[at + 4], t0.y, t0.w, t1.y, t1.w);
+    }
+#pragma unroll
+    for (int n = 0; n < (kBig ? 2 : 1); n++)
+    {
+#pragma unroll
+        for (int i = 0; i < (kBig ? 4 : 2); i++)
+        {
+            const int v = n * 4 + i;
+            if (kBig)
             {
-                const int a = __shfl_sync(full, rec_cj, lane >> 3) * kCl + (lane & (kCl - 1));
-                xr          = p.xq[a];
-                gr          = p.gnb[a];
-                gr.w        = __int_as_float(p.tgrid[a]);
-            }
-            const unsigned im  = (h == 0) ? (unsigned)ime.x : (unsigned)ime.z;
-            const int      exi = (h == 0) ? ime.y : ime.w;
-            if (!im)
-            {
-                continue;
-            }
-            if (exi == 0)
-            {
-                adj_half<kEwald, false>(v, jx, jg, nbfp_s, ttab_lane, xis, gis, acc, p.dnb, cj_lane, im, 0u, h, s.sci,
-                                        central, ii, jj, k, pbeta, beta2l2, c2b, b2c2b);
+                atomicAdd(&gsum[32 * (2 * v)], -(double)types.s6[n][i]);
+                atomicAdd(&gsum[32 * (2 * v + 1)], (double)types.s12[n][i]);
             }
             else
             {
-                const unsigned wexcl = p.excl[exi].pair[lane];
-                adj_half<kEwald, true>(v, jx, jg, nbfp_s, ttab_lane, xis, gis, acc, p.dnb, cj_lane, im, wexcl, h,
-                                       s.sci, central, ii, jj, k, pbeta, beta2l2, c2b, b2c2b);
+                gsum[32 * (2 * v)] -= (double)types.s6[n][i];
+                gsum[32 * (2 * v + 1)] += (double)types.s12[n][i];
             }
         }
     }
-    // the i-side sums: the 4 lane slots of every i-atom, one vector red per atom
-    __syncwarp();
-    for (int m = lane; m < kSc; m += 32)
-    {
-        const float4 a0 = acc[m * 4], a1 = acc[m * 4 + 1], a2 = acc[m * 4 + 2], a3 = acc[m * 4 + 3];
-        red_add_v4(&p.dnb[s.sci * kSc + m], (a0.x + a1.x) + (a2.x + a3.x), (a0.y + a1.y) + (a2.y + a3.y),
-                   (a0.z + a1.z) + (a2.z + a3.z), (a0.w + a1.w) + (a2.w + a3.w));
-    }
-    // flush the type-pair gradients of this entry into the block's FP64 sums (shared memory;
-    // added to the global sums once per block at the end).  The replicas are summed in float
-    // first: one conversion and one FP64 add per element, where FP64 runs at a small fraction of
-    // the FP32 rate (a conversion and an add per replica kept the FP64 pipe 37 % busy).
-    __syncwarp();
-    for (int m = lane; m < nt1 * nt1; m += 32)
-    {
-        float tx = 0.0f, ty = 0.0f;
-        for (int r = 0; r < reps; r++)
-        {
-            // replica r: dc6 sums at 2 r stride + m, dc12 sums one stride on (planar)
-            float* const t = reinterpret_cast<float*>(ttab) + 2 * r * tstride + m;
-            tx += t[0];
-            ty += t[tstride];
-            t[0]       = 0.0f;
-            t[tstride] = 0.0f;
-        }
-        if (tx != 0.0f || ty != 0.0f)
-        {
-            atomicAdd(&gnbfp[2 * m], (double)tx);
-            atomicAdd(&gnbfp[2 * m + 1], (double)ty);
-        }
-    }
-    __syncwarp();
 }
 
-// Shared set-up of the adjoint kernels: the type table and zeroed per-warp tables.
-__device__ __forceinline__ void adj_setup(const DeviceView& v, float2* nbfp_s, float2* ttab_all, double* gsum_s)
+// Dynamic shared memory: the type table, the warps' FP64 type-pair sums, the warps' slots.
+template<bool kBig>
+constexpr size_t adj_smem()
+{
+    return sizeof(float2) * kAdjRow * kAdjRow + sizeof(double) * adj_sum_copies<kBig>() * 32 * adj_lane_sums<kBig>()
+           + sizeof(AdjWarp) * kAdjWarps;
+}
+
+// Type table in rows of 16, cleared sums.
+template<bool kBig>
+__device__ __forceinline__ void adj_setup(const DeviceView& v, float2* nbfp_s, double* gsum_s)
 {
     const int nt1 = v.ntypes1;
     for (int m = threadIdx.x; m < nt1 * nt1; m += blockDim.x)
     {
-        nbfp_s[m]         = v.nbfp[m];
-        gsum_s[2 * m]     = 0.0;
-        gsum_s[2 * m + 1] = 0.0;
+        nbfp_s[(m / nt1) * kAdjRow + m % nt1] = v.nbfp[m];
     }
-    const int ntab = kAdjWarps * adj_table_replicas(nt1) * adj_table_stride(nt1);
-    for (int m = threadIdx.x; m < ntab; m += blockDim.x)
+    for (int m = threadIdx.x; m < adj_sum_copies<kBig>() * 32 * adj_lane_sums<kBig>(); m += blockDim.x)
     {
-        ttab_all[m] = make_float2(0.0f, 0.0f);
+        gsum_s[m] = 0.0;
     }
     __syncthreads();
 }
 
-// The block's FP64 type-pair gradient sums into the global ones (one atomic per non-zero element
-// and block instead of one per element and list entry).
-__device__ __forceinline__ void adj_flush(const double* gsum_s, double* gnbfp, int n)
+// The block's type-pair sums into the global padded table: thread (value, lane) adds the warps' sums, one
+// FP64 atomic per non-zero element and block.
+template<bool kBig>
+__device__ __forceinline__ void adj_flush(const DeviceView& v, const double* gsum_s, double* gnbfp)
 {
     __syncthreads();
-    for (int m = threadIdx.x; m < n; m += blockDim.x)
+    constexpr int per = 32 * adj_lane_sums<kBig>();
+    for (int m = threadIdx.x; m < per; m += blockDim.x)
     {
-        if (gsum_s[m] != 0.0)
+        double t = 0.0;
+        for (int w = 0; w < adj_sum_copies<kBig>(); w++)
         {
-            atomicAdd(&gnbfp[m], gsum_s[m]);
+            t += gsum_s[w * per + m];
+        }
+        const int val = m >> 5, lane = m & 31, i = (val >> 1) & 3, n = val >> 3;
+        const int a = (lane >> 2) + 8 * (i >> 1), b = 2 * (lane & 3) + (i & 1) + 8 * n;
+        if (t != 0.0 && a < v.ntypes1 && b < v.ntypes1)
+        {
+            atomicAdd(&gnbfp[2 * (a * v.ntypes1 + b) + (val & 1)], t);
         }
     }
 }
 
-template<bool kEwald>
+template<bool kEwald, bool kGE, bool kBig>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         k_backward(DeviceView v, const float4* __restrict__ gnb, float4* dnb, double* gnbfp, int* work_counter,
                    const double* __restrict__ gE)
 {
     pdl_begin();
-    AdjConsts k{ 0.0f, 0.0f };
-    if (gE)
-    {
-        k.gE_lj = (float)gE[0];
-        k.gE_c  = (float)gE[1];
-    }
-    __shared__ float2 nbfp_s[kAdjMaxTypes1 * kAdjMaxTypes1];
-    __shared__ double gsum_s[2 * kAdjMaxTypes1 * kAdjMaxTypes1];
-    // dynamic: per warp the i-side accumulators (64 i-atoms x 4 lane slots), then the type-pair
-    // gradient tables (kAdjWarps x replicas x stride)
     extern __shared__ float4 adj_dyn[];
-    float4* const acc_w  = adj_dyn + (threadIdx.x >> 5) * (kSc * 4);
-    float2* const ttab_s = reinterpret_cast<float2*>(adj_dyn + kAdjWarps * kSc * 4);
-    __shared__ float4 xis_s[kAdjWarps][kSc];
-    __shared__ float4 gis_s[kAdjWarps][kSc];
-    __shared__ float4 jx_s[kAdjWarps][32];
-    __shared__ float4 jg_s[kAdjWarps][32];
-    adj_setup(v, nbfp_s, ttab_s, gsum_s);
-    float2* const ttab_w = ttab_s + (threadIdx.x >> 5) * adj_table_replicas(v.ntypes1) * adj_table_stride(v.ntypes1);
+    float2* const  nbfp_s = reinterpret_cast<float2*>(adj_dyn);
+    double* const  gsum_s = reinterpret_cast<double*>(nbfp_s + kAdjRow * kAdjRow);
+    AdjWarp* const warps  = reinterpret_cast<AdjWarp*>(gsum_s + adj_sum_copies<kBig>() * 32 * adj_lane_sums<kBig>());
+    adj_setup<kBig>(v, nbfp_s, gsum_s);
     if (v.hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
     {
         return;
     }
+    AdjConsts k = adj_consts(v);
+    if (kGE)
+    {
+        k.gE_lj = (float)gE[0];
+        k.gE_c  = (float)gE[1];
+    }
     const int     warp   = threadIdx.x >> 5;
     const int     lane   = threadIdx.x & 31;
     const int     numSci = v.hdr->num_sci;
-    const float   b2c2b  = v.beta * v.beta * v.c2b;
-    const AdjPtrs p      = { v.xq, v.tgrid, v.cj4, v.excl, v.shiftvec, gnb, dnb };
+    const AdjPtrs p      = { v.xq, v.cj4, v.excl, v.shiftvec, gnb, dnb };
     for (;;)
     {
         int e = 0;
@@ -444,57 +616,29 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         {
             break;
         }
-        adj_entry<kEwald>(v, p, v.sci[e], nbfp_s, ttab_w, xis_s[warp], gis_s[warp], jx_s[warp], jg_s[warp],
-                          acc_w, lane, k, v.pbeta,
-                          v.beta2l2, v.c2b, b2c2b, gsum_s);
+        adj_entry<kEwald, kGE, kBig>(k, p, v.sci[e], reinterpret_cast<const char*>(nbfp_s), warps[warp],
+                                     gsum_s + (kBig ? 0 : warp) * 32 * adj_lane_sums<kBig>() + lane, lane);
     }
-    adj_flush(gsum_s, gnbfp, 2 * v.ntypes1 * v.ntypes1);
-}
-
-__device__ __forceinline__ int adj_find_system(const int* prefix, int nsys, int e)
-{
-    int lo = 0, hi = nsys - 1;
-    while (lo < hi)
-    {
-        const int mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= e)
-        {
-            lo = mid;
-        }
-        else
-        {
-            hi = mid - 1;
-        }
-    }
-    return lo;
+    adj_flush<kBig>(v, gsum_s, gnbfp);
 }
 
 // The adjoint over all systems of a batch (shared type table and type-pair
 // gradient sums; per-system upstream energy gradients gE[2 s], gE[2 s + 1]).
-template<bool kEwald>
+template<bool kEwald, bool kGE, bool kBig>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         k_batch_backward(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
                          double* gnbfp, int* work_counter, const double* __restrict__ gE)
 {
     pdl_begin();
-    __shared__ float2 nbfp_s[kAdjMaxTypes1 * kAdjMaxTypes1];
-    __shared__ double gsum_s[2 * kAdjMaxTypes1 * kAdjMaxTypes1];
-    // dynamic: per warp the i-side accumulators (64 i-atoms x 4 lane slots), then the type-pair
-    // gradient tables (kAdjWarps x replicas x stride)
     extern __shared__ float4 adj_dyn[];
-    float4* const acc_w  = adj_dyn + (threadIdx.x >> 5) * (kSc * 4);
-    float2* const ttab_s = reinterpret_cast<float2*>(adj_dyn + kAdjWarps * kSc * 4);
-    __shared__ float4 xis_s[kAdjWarps][kSc];
-    __shared__ float4 gis_s[kAdjWarps][kSc];
-    __shared__ float4 jx_s[kAdjWarps][32];
-    __shared__ float4 jg_s[kAdjWarps][32];
-    adj_setup(cv, nbfp_s, ttab_s, gsum_s);
-    float2* const ttab_w =
-            ttab_s + (threadIdx.x >> 5) * adj_table_replicas(cv.ntypes1) * adj_table_stride(cv.ntypes1);
-    const int   warp  = threadIdx.x >> 5;
-    const int   lane  = threadIdx.x & 31;
-    const int   total = prefix[nsys];
-    const float b2c2b = cv.beta * cv.beta * cv.c2b;
+    float2* const  nbfp_s = reinterpret_cast<float2*>(adj_dyn);
+    double* const  gsum_s = reinterpret_cast<double*>(nbfp_s + kAdjRow * kAdjRow);
+    AdjWarp* const warps  = reinterpret_cast<AdjWarp*>(gsum_s + adj_sum_copies<kBig>() * 32 * adj_lane_sums<kBig>());
+    adj_setup<kBig>(cv, nbfp_s, gsum_s);
+    AdjConsts k     = adj_consts(cv);
+    const int warp  = threadIdx.x >> 5;
+    const int lane  = threadIdx.x & 31;
+    const int total = prefix[nsys];
     for (;;)
     {
         int e = 0;
@@ -507,20 +651,18 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
         {
             break;
         }
-        const int       sidx = adj_find_system(prefix, nsys, e);
+        const int       sidx = find_system(prefix, nsys, e);
         const BatchSys& b    = sys[sidx];
-        AdjConsts       k{ 0.0f, 0.0f };
-        if (gE)
+        if (kGE)
         {
             k.gE_lj = (float)gE[2 * sidx];
             k.gE_c  = (float)gE[2 * sidx + 1];
         }
-        const AdjPtrs p = { b.xq, b.tgrid, b.cj4, b.excl, b.shiftvec, b.gnb, b.dnb };
-        adj_entry<kEwald>(cv, p, b.sci[e - prefix[sidx]], nbfp_s, ttab_w, xis_s[warp], gis_s[warp],
-                          jx_s[warp], jg_s[warp], acc_w, lane, k,
-                          cv.pbeta, cv.beta2l2, cv.c2b, b2c2b, gsum_s);
+        const AdjPtrs p = { b.xq, b.cj4, b.excl, b.shiftvec, b.gnb, b.dnb };
+        adj_entry<kEwald, kGE, kBig>(k, p, b.sci[e - prefix[sidx]], reinterpret_cast<const char*>(nbfp_s), warps[warp],
+                                     gsum_s + (kBig ? 0 : warp) * 32 * adj_lane_sums<kBig>() + lane, lane);
     }
-    adj_flush(gsum_s, gnbfp, 2 * cv.ntypes1 * cv.ntypes1);
+    adj_flush<kBig>(cv, gsum_s, gnbfp);
 }
 
 // Batched upstream gradients to grid order (blockIdx.y = system), outputs cleared.
@@ -548,7 +690,8 @@ __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const floa
     }
     const int     a = b.atom_indices[k];
     const float*  g = gF + 3 * (size_t)(b.atom_base + (a >= 0 ? a : 0));
-    const_cast<float4*>(b.gnb)[k] = (a >= 0) ? make_float4(g[0], g[1], g[2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float   t = __int_as_float(b.tgrid[k]);
+    const_cast<float4*>(b.gnb)[k] = (a >= 0) ? make_float4(g[0], g[1], g[2], t) : make_float4(0.0f, 0.0f, 0.0f, t);
     b.dnb[k]                      = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
@@ -624,7 +767,7 @@ __global__ void k_match_loss(const float* __restrict__ f, const float* __restric
 
 // Upstream force gradients to grid order; clears the output accumulators.
 // Per grid slot: the coordinates of this evaluation into xq (as k_convert_x, with the box shifts of
-// the last search) when x is given, the upstream force gradient in grid order, a cleared dL/dx
+// the last search) when x is given, the upstream force gradient (and the type) in grid order, a cleared dL/dx
 // accumulator; block 0 also clears the work queue and the FP64 type-pair gradient table (in place
 // of separate memsets).
 __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const float* __restrict__ gF, float4* gnb,
@@ -660,7 +803,8 @@ __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const f
         }
         v.xq[k] = make_float4(c[0], c[1], c[2], old.w);
     }
-    gnb[k] = (a >= 0) ? make_float4(gF[3 * a], gF[3 * a + 1], gF[3 * a + 2], 0.0f) : make_float4(0, 0, 0, 0);
+    const float t = __int_as_float(v.tgrid[k]);
+    gnb[k] = (a >= 0) ? make_float4(gF[3 * a], gF[3 * a + 1], gF[3 * a + 2], t) : make_float4(0.0f, 0.0f, 0.0f, t);
     dnb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
@@ -785,24 +929,39 @@ cudaError_t launch_lb_table_backward(const double* sig, const double* eps, int n
 namespace
 {
 
-// Dynamic shared memory of the adjoint kernels: the warps' i-side accumulators and type-pair tables.
-size_t adj_table_bytes(int nt1)
+template<bool kEwald, bool kGE, bool kBig>
+cudaError_t backward_t(const DeviceView& v, const float4* gnb, float4* dnb, double* gnbfp, int* counter,
+                       const double* gE, int num_sms, cudaStream_t s)
 {
-    return sizeof(float4) * (size_t)kAdjWarps * kSc * 4
-           + sizeof(float2) * (size_t)kAdjWarps * adj_table_replicas(nt1) * adj_table_stride(nt1);
+    constexpr size_t smem = adj_smem<kBig>();
+    cudaError_t      e    = smem_optin<k_backward<kEwald, kGE, kBig>>(smem, smem);
+    if (e == cudaSuccess)
+    {
+        e = launch_pdl(k_backward<kEwald, kGE, kBig>, num_sms * kAdjBlocksPerSm, kAdjThreads, smem, s, v, gnb, dnb,
+                       gnbfp, counter, gE);
+    }
+    return e;
 }
 
-// Opts an adjoint kernel in to its static + dynamic shared memory beyond 48 KB.
-template<auto kKernel>
-cudaError_t adj_optin(size_t dynamic_bytes)
+template<bool kEwald, bool kGE, bool kBig>
+cudaError_t batch_backward_t(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys, double* gnbfp,
+                             int* counter, const double* gE, int num_sms, cudaStream_t s)
 {
-    cudaFuncAttributes a{};
-    cudaError_t        e = cudaFuncGetAttributes(&a, kKernel);
-    if (e != cudaSuccess)
+    constexpr size_t smem = adj_smem<kBig>();
+    cudaError_t      e    = smem_optin<k_batch_backward<kEwald, kGE, kBig>>(smem, smem);
+    if (e == cudaSuccess)
     {
-        return e;
+        e = launch_pdl(k_batch_backward<kEwald, kGE, kBig>, num_sms * kAdjBlocksPerSm, kAdjThreads, smem, s, cv, sys,
+                       prefix, nsys, gnbfp, counter, gE);
     }
-    return smem_optin<kKernel>(a.sharedSizeBytes + dynamic_bytes, dynamic_bytes);
+    return e;
+}
+
+// More types than the 8 rows (and columns) of one tensor-core tile, which the filler type does not count
+// toward: its pairs are never in range.
+bool adj_big(const DeviceView& v)
+{
+    return v.ntypes1 - 1 > 8;
 }
 
 } // namespace
@@ -815,20 +974,17 @@ cudaError_t launch_backward(const DeviceView& v, const float* d_x, const float* 
     const int slots = v.g.cells_capacity * kSc;
     launch_pdl(k_adj_prepare, (slots + tb - 1) / tb, tb, 0, s, v, d_x, d_gF, gnb, dnb, counter, d_gnbfp,
                2 * v.ntypes1 * v.ntypes1);
-    const size_t dyn = adj_table_bytes(v.ntypes1);
-    cudaError_t  e   = cudaSuccess;
-    if (v.coulomb == 0)
-    {
-        e = adj_optin<k_backward<true>>(dyn);
-        launch_pdl(k_backward<true>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, v, gnb, dnb, d_gnbfp, counter,
-                   d_gE);
-    }
-    else
-    {
-        e = adj_optin<k_backward<false>>(dyn);
-        launch_pdl(k_backward<false>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, v, gnb, dnb, d_gnbfp, counter,
-                   d_gE);
-    }
+    using Launch = cudaError_t (*)(const DeviceView&, const float4*, float4*, double*, int*, const double*, int,
+                                   cudaStream_t);
+    // [Ewald][energy gradients][more than 8 types]
+    static const Launch table[2][2][2] = {
+        { { backward_t<false, false, false>, backward_t<false, false, true> },
+          { backward_t<false, true, false>, backward_t<false, true, true> } },
+        { { backward_t<true, false, false>, backward_t<true, false, true> },
+          { backward_t<true, true, false>, backward_t<true, true, true> } },
+    };
+    const cudaError_t e = table[v.coulomb == 0][d_gE != nullptr][adj_big(v)](v, gnb, dnb, d_gnbfp, counter, d_gE,
+                                                                              num_sms, s);
     if (e != cudaSuccess)
     {
         return e;
@@ -845,20 +1001,17 @@ cudaError_t launch_batch_backward(const DeviceView& cv, const BatchSys* sys, con
     const int tb = 256;
     launch_pdl(k_batch_adj_prepare, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_gF, counter, d_gnbfp,
                2 * cv.ntypes1 * cv.ntypes1);
-    const size_t dyn = adj_table_bytes(cv.ntypes1);
-    cudaError_t  e   = cudaSuccess;
-    if (cv.coulomb == 0)
-    {
-        e = adj_optin<k_batch_backward<true>>(dyn);
-        launch_pdl(k_batch_backward<true>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, cv, sys, prefix, nsys,
-                   d_gnbfp, counter, d_gE);
-    }
-    else
-    {
-        e = adj_optin<k_batch_backward<false>>(dyn);
-        launch_pdl(k_batch_backward<false>, num_sms * kAdjBlocksPerSm, kAdjThreads, dyn, s, cv, sys, prefix, nsys,
-                   d_gnbfp, counter, d_gE);
-    }
+    using Launch = cudaError_t (*)(const DeviceView&, const BatchSys*, const int*, int, double*, int*, const double*,
+                                   int, cudaStream_t);
+    // [Ewald][energy gradients][more than 8 types]
+    static const Launch table[2][2][2] = {
+        { { batch_backward_t<false, false, false>, batch_backward_t<false, false, true> },
+          { batch_backward_t<false, true, false>, batch_backward_t<false, true, true> } },
+        { { batch_backward_t<true, false, false>, batch_backward_t<true, false, true> },
+          { batch_backward_t<true, true, false>, batch_backward_t<true, true, true> } },
+    };
+    const cudaError_t e = table[cv.coulomb == 0][d_gE != nullptr][adj_big(cv)](cv, sys, prefix, nsys, d_gnbfp, counter,
+                                                                                d_gE, num_sms, s);
     if (e != cudaSuccess)
     {
         return e;
