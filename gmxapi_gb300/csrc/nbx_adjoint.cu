@@ -21,16 +21,17 @@
 // lane's i-side sums beside them (one slot per lane and i-cluster: no conflicts); the j-side sums stay in
 // registers and end in one add per lane.
 //
-// Type-pair gradients.  d6 / d12 of a step are 8x8 matrices G over (i-atom, j-atom), and the table gradient
-// is sum_steps P_i^T G P_j with one-hot type matrices P: a contraction, so it runs on the tensor cores.
-// The lane mapping above is the B fragment of mma.m16n8k8 (k = i-atom, n = j-atom), P_i^T is its A
-// fragment, and the products are exact: a one-hot factor times a float split into three tf32 parts
-// (11 + 11 + 2 bits).  The high parts and the lower ones are summed in accumulators of their own over the
-// at most 8 steps of a j-cluster, then a second product with P_j gives the types (a, b), added in FP32 over
-// the entry and in FP64 beyond it.  (Float atomics on per-warp tables in shared memory, which this
-// replaces, are compare-and-swap loops.)  The kernel is bound by instruction issue and latency.
-// 24,000-atom 8-type liquid: 91.6 us with one pair per lane and table atomics; 16 liquids of 2,000 to
-// 50,000 atoms: 758 us.
+// Type-pair gradients.  The terms d6 and d12 of a step are 8x8 matrices G over (j-atom, i-atom), and the
+// table gradient is sum_steps P_j^T G P_i with one-hot type matrices P: a contraction, so it runs on the
+// tensor cores.  The lane mapping above is the A fragment of mma.m16n8k8 (rows: the j-atoms of d6, then
+// those of d12; k = i-atom) and P_i its B fragment.  A float is split into two tf32 parts of 11 bits; a
+// one-hot factor keeps their products exact, and the two are summed in accumulators of their own over the at
+// most 8 steps of a j-cluster.  The products D = G P_i then turn through shared memory into the B fragment
+// of P_j^T D, which is added in FP32 over the entry and in FP64 beyond it.  (Float atomics on per-warp
+// tables in shared memory, which this replaces, are compare-and-swap loops.)  Against 64 bits the sigma and
+// epsilon gradients are off by 0.1-2e-7 (1 to 15 types), with those tables by 3-5.6e-7.
+// The kernel is bound by instruction issue and latency.  24,000-atom 8-type liquid: 91.5 us with one pair per
+// lane and table atomics, 53.0 us now; a gradient step of 16 liquids of 2,000 to 50,000 atoms 1271 and 958 us.
 #include "nbx_internal.cuh"
 #include "nbx_pair_x2.cuh"
 
@@ -50,7 +51,7 @@ constexpr int kAdjRow         = 16;  // type-pair rows of 16 entries in shared m
 // Constants of the pair loop; gE_*: upstream energy gradients (0 in the flavours without them).
 struct AdjConsts
 {
-    float rc2, pbeta, nbeta2l2, c2b, nb2c2b, sh_ewald, nk_rf2, k_rf, c_rf, epsfac, cpot6, cpot12;
+    float rc2, pbeta, nbeta2l2, c2b, nb2c2b2, sh_ewald, nk_rf2, k_rf, c_rf, epsfac, cpot6, cpot12;
     float gE_lj, gE_c;
     int   filler;  // the type of empty slots
 };
@@ -62,7 +63,7 @@ __device__ __forceinline__ AdjConsts adj_consts(const DeviceView& v)
     k.pbeta    = v.pbeta;
     k.nbeta2l2 = -v.beta2l2;
     k.c2b      = v.c2b;
-    k.nb2c2b   = -v.beta * v.beta * v.c2b;
+    k.nb2c2b2  = -2.0f * v.beta * v.beta * v.c2b;
     k.sh_ewald = v.sh_ewald;
     k.nk_rf2   = -2.0f * v.k_rf;
     k.k_rf     = v.k_rf;
@@ -97,73 +98,34 @@ struct AdjWarp
     // reduction reads eight lanes' sums of two clusters at a time)
     float4 acc[kNcl][2 * 32 + 4];
     float4 jx[32], jg[32];
+    float4 turn[32];  // the type products between the two tensor-core passes
 };
 
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], float b0, float b1)
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], float b0, float b1)
 {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
                  "{%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+                 : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
+                   "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
 
-// The leading 11 significant bits of x (a tf32 value).
-__device__ __forceinline__ float tf32_head(float x)
+// x as two tf32 operands: its leading 11 significant bits, and the rest rounded to 11 bits (the tensor cores
+// read the upper 19 bits of an operand, so half a unit of the last of them is added; cvt.rna takes three
+// instructions for the same).
+__device__ __forceinline__ void tf32_split(float x, float& head, float& rest)
 {
-    return __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+    head = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+    rest = __uint_as_float(__float_as_uint(x - head) + 0x1000u);
 }
 
-// d_hi, d_lo += A {b0, b1} with b split into three tf32 parts, exactly representable each.
-__device__ __forceinline__ void mma_split_b(float (&d_hi)[4], float (&d_lo)[4], const unsigned (&a)[4], float b0,
-                                            float b1)
-{
-    const float h0 = tf32_head(b0), h1 = tf32_head(b1);
-    const float r0 = b0 - h0, r1 = b1 - h1;
-    const float m0 = tf32_head(r0), m1 = tf32_head(r1);
-    mma_tf32(d_hi, a, h0, h1);
-    mma_tf32(d_lo, a, m0, m1);
-    mma_tf32(d_lo, a, r0 - m0, r1 - m1);
-}
-
-// The same with the split factor as A (rows 8.. only with kBig) and a one-hot B; the sum is returned in d.
+// j-side sums of the lane's j-atom over its two i-atoms' slots, and the j-cluster's products D of type tile n
+// (columns 2 ip + {0, 1}): {d6, d6', d12, d12'} of the heads and of the rests.
 template<bool kBig>
-__device__ __forceinline__ void mma_split_a(float (&d)[4], const float (&x)[4], float b0, float b1)
-{
-    float    lo[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
-    unsigned h[4], m[4], l[4];
-    // C fragment (row, 2 l), (row, 2 l + 1), (row + 8, ...) as the A fragment with columns in that order
-    const float c[4] = { x[0], x[2], x[1], x[3] };
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-    {
-        if (!kBig && (i & 1))
-        {
-            h[i] = m[i] = l[i] = 0u;
-            continue;
-        }
-        const float hi = tf32_head(c[i]);
-        const float r  = c[i] - hi;
-        const float mi = tf32_head(r);
-        h[i]           = __float_as_uint(hi);
-        m[i]           = __float_as_uint(mi);
-        l[i]           = __float_as_uint(r - mi);
-    }
-    d[0] = d[1] = d[2] = d[3] = 0.0f;
-    mma_tf32(d, h, b0, b1);
-    mma_tf32(lo, m, b0, b1);
-    mma_tf32(lo, l, b0, b1);
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-    {
-        d[i] += lo[i];
-    }
-}
-
-// j-side sums of the lane's j-atom over its two i-atoms' slots, and the type-pair products of one j-cluster.
 struct AdjJ
 {
     float2 x, y, z, q;
-    float  h6[4], l6[4], h12[4], l12[4];
+    float  hi[kBig ? 2 : 1][4], lo[kBig ? 2 : 1][4];
 };
 
 // One step: i-cluster c against the lane's j-atom.  okA / okB: the pair's mask bit (and, on the diagonal,
@@ -171,7 +133,7 @@ struct AdjJ
 template<bool kEwald, bool kGE, bool kBig, bool kExcl>
 __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w, int c,
                                          int lane, const float4 xj, const float4 gj, float qje, int tjb, bool okA,
-                                         bool okB, float intA, float intB, AdjJ& dj)
+                                         bool okB, float intA, float intB, AdjJ<kBig>& dj)
 {
     const int     ip = lane & 3;
     const float4  i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
@@ -195,11 +157,12 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     {
         rinv6 = mul2(rinv6, make_float2(intA, intB));
     }
-    const float2 vdisp   = make_float2(ljA.x * rinv6.x, ljB.x * rinv6.y);
-    const float2 vrep    = make_float2(ljA.y * rinv6.x * rinv6.x, ljB.y * rinv6.y * rinv6.y);
-    const float2 phi_lj  = mul2(sub2(vrep, vdisp), rinv2);
-    const float2 dphi_lj = mul2(fma2(f2(-7.0f), vrep, mul2(f2(4.0f), vdisp)), mul2(rinv2, rinv2));
-    float2       psi, dpsi, hq = f2(0.0f);  // Coulomb phi / qq, its s-derivative, energy / qq
+    const float2 rinv8  = mul2(rinv6, rinv2);
+    const float2 rinv14 = mul2(rinv6, rinv8);
+    const float2 fdisp  = make_float2(ljA.x * rinv8.x, ljB.x * rinv8.y);
+    const float2 frep   = make_float2(ljA.y * rinv14.x, ljB.y * rinv14.y);
+    const float2 phi_lj = sub2(frep, fdisp);
+    float2       psi, dpsi, hq = f2(0.0f);  // Coulomb phi / qq, 2 r^2 times its s-derivative, energy / qq
     if (kEwald)
     {
         const float2 tt   = fma2(f2(k.pbeta), mul2(r2, rinv), f2(1.0f));
@@ -221,13 +184,13 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
                 hq = add2(hq, ex);
             }
         }
-        dpsi = mul2(fma2(f2(-1.5f), psi, mul2(f2(k.nb2c2b), expm)), rinv2);
+        dpsi = fma2(f2(-3.0f), psi, mul2(f2(k.nb2c2b2), expm));
     }
     else
     {
         const float2 r3 = kExcl ? mul2(mul2(rinv, rinv2), make_float2(intA, intB)) : mul2(rinv, rinv2);
         psi             = add2(r3, make_float2(inA ? k.nk_rf2 : 0.0f, inB ? k.nk_rf2 : 0.0f));
-        dpsi            = mul2(mul2(f2(-1.5f), r3), rinv2);
+        dpsi            = mul2(f2(-3.0f), r3);
         if (kGE)
         {
             const float2 h = fma2(f2(k.k_rf), r2, sub2(mul2(rinv, make_float2(intA, intB)), f2(k.c_rf)));
@@ -237,12 +200,13 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     const float2 qi   = make_float2(i1.z, i1.w);
     const float2 qq   = mul2(qi, f2(qje));
     const float2 phi  = fma2(qq, psi, phi_lj);
-    const float2 dphi = fma2(qq, dpsi, dphi_lj);
     const float2 gx   = sub2(make_float2(i2.x, i2.y), f2(gj.x));
     const float2 gy   = sub2(make_float2(i2.z, i2.w), f2(gj.y));
     const float2 gz   = sub2(make_float2(i3.x, i3.y), f2(gj.z));
     const float2 gr   = fma2(gz, dz, fma2(gy, dy, mul2(gx, dx)));
-    float2       coef = mul2(mul2(f2(2.0f), dphi), gr);
+    // 2 phi' (g.r), phi' = (qq dpsi + 8 fdisp - 14 frep) / (2 r^2)
+    const float2 dphi = fma2(qq, dpsi, fma2(f2(-14.0f), frep, mul2(f2(8.0f), fdisp)));
+    float2       coef = mul2(mul2(dphi, rinv2), gr);
     float2       wq   = mul2(psi, gr);  // dL/d(q_i q_j) / epsfac
     if (kGE)
     {
@@ -263,8 +227,8 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     dj.z   = add2(dj.z, uz);
     dj.q   = fma2(wq, qi, dj.q);
     // dL/d(6C6) and dL/d(12C12) of the pairs, by i type
-    float2 d6  = mul2(gr, mul2(rinv6, rinv2));
-    float2 d12 = mul2(d6, rinv6);
+    float2 d6  = mul2(gr, rinv8);
+    float2 d12 = mul2(gr, rinv14);
     if (kGE)
     {
         const bool   cA = inA && (!kExcl || intA != 0.0f), cB = inB && (!kExcl || intB != 0.0f);
@@ -274,16 +238,23 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
         d6  = fma2(f2(k.gE_lj), e6, d6);
         d12 = fma2(f2(k.gE_lj), e12, d12);
     }
-    const int      row   = lane >> 2;
-    const unsigned one   = 0x3f800000u;
-    const unsigned hot[4] = { tA == row ? one : 0u, kBig && tA == row + 8 ? one : 0u, tB == row ? one : 0u,
-                              kBig && tB == row + 8 ? one : 0u };
-    mma_split_b(dj.h6, dj.l6, hot, d6.x, d6.y);
-    mma_split_b(dj.h12, dj.l12, hot, d12.x, d12.y);
+    const int row = lane >> 2;
+    float     h[4], r[4];
+    tf32_split(d6.x, h[0], r[0]);
+    tf32_split(d12.x, h[1], r[1]);
+    tf32_split(d6.y, h[2], r[2]);
+    tf32_split(d12.y, h[3], r[3]);
+#pragma unroll
+    for (int n = 0; n < (kBig ? 2 : 1); n++)
+    {
+        const float b0 = tA == row + 8 * n ? 1.0f : 0.0f, b1 = tB == row + 8 * n ? 1.0f : 0.0f;
+        mma_tf32(dj.hi[n], h, b0, b1);
+        mma_tf32(dj.lo[n], r, b0, b1);
+    }
 }
 
-// Type-pair sums of an entry: C fragments (type rows lane >> 2 (+ 8), columns 2 (lane & 3) + {0, 1} of
-// column tile n) of dL/d(6C6) (negated) and dL/d(12C12).
+// Type-pair sums of an entry: C fragments of P_j^T D (rows: j types lane >> 2 (+ 8), columns: i types
+// 2 (lane & 3) + {0, 1} of tile n) of dL/d(6C6) (negated) and dL/d(12C12).
 template<bool kBig>
 struct AdjTypes
 {
@@ -316,12 +287,16 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         const unsigned mj   = tj == k.filler ? 0u : m >> (jm * kNcl);
         const unsigned xA   = wA >> (jm * kNcl), xB = wB >> (jm * kNcl);
         const int      diag = kExcl && central ? cj - sci * kNcl : -1;  // the diagonal i-cluster, if in 0 .. 7
-        AdjJ           dj;
+        AdjJ<kBig>     dj;
         dj.x = dj.y = dj.z = dj.q = f2(0.0f);
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int n = 0; n < (kBig ? 2 : 1); n++)
         {
-            dj.h6[i] = dj.l6[i] = dj.h12[i] = dj.l12[i] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+            {
+                dj.hi[n][i] = dj.lo[n][i] = 0.0f;
+            }
         }
         auto step = [&](int c) {
             bool  okA = (mj >> c) & 1u, okB = okA;
@@ -363,31 +338,34 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         keep.y += __shfl_xor_sync(full, send.y, 2);
         float one = (o1 ? keep.y : keep.x) + __shfl_xor_sync(full, o1 ? keep.x : keep.y, 1);
         atomicAdd(reinterpret_cast<float*>(&dnb[cj * kCl + j]) + ip, -one);
-        // type pairs: columns j = 2 ip, 2 ip + 1 of the products times the one-hot j types
-        const int t0 = __shfl_sync(full, tj, 8 * ip), t1 = __shfl_sync(full, tj, 8 * ip + 4);
-        float     c6[4], c12[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-        {
-            c6[i]  = dj.h6[i] + dj.l6[i];
-            c12[i] = dj.h12[i] + dj.l12[i];
-        }
+        // type pairs: D of row j turns into the B fragment (k = j-atoms ip and ip + 4, n = i type lane >> 2)
+        // of the product with the one-hot j types
+        const int   t0 = __shfl_sync(full, tj, 4 * ip), t1 = __shfl_sync(full, tj, 16 + 4 * ip);
+        const float p[4] = { t0 == j ? 1.0f : 0.0f, kBig && t0 == j + 8 ? 1.0f : 0.0f, t1 == j ? 1.0f : 0.0f,
+                             kBig && t1 == j + 8 ? 1.0f : 0.0f };
 #pragma unroll
         for (int n = 0; n < (kBig ? 2 : 1); n++)
         {
-            const float b0 = t0 == j + 8 * n ? 1.0f : 0.0f, b1 = t1 == j + 8 * n ? 1.0f : 0.0f;
-            float       d[4];
-            mma_split_a<kBig>(d, c6, b0, b1);
+            __syncwarp();  // the readers of the last product are done
+            w.turn[lane] = make_float4(dj.hi[n][0] + dj.lo[n][0], dj.hi[n][1] + dj.lo[n][1], dj.hi[n][2] + dj.lo[n][2],
+                                       dj.hi[n][3] + dj.lo[n][3]);
+            __syncwarp();
+            // element (j, type a) of d6 sits in lane 4 j + a / 2, component a & 1 (d12: + 2)
+            const float* d = reinterpret_cast<const float*>(w.turn) + 16 * ip + 4 * (j >> 1) + (j & 1);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int q = 0; q < 2; q++)
             {
-                types.s6[n][i] += d[i];
-            }
-            mma_split_a<kBig>(d, c12, b0, b1);
+                float h0, r0, h1, r1, hs[4] = { 0, 0, 0, 0 }, rs[4] = { 0, 0, 0, 0 };
+                tf32_split(d[2 * q], h0, r0);
+                tf32_split(d[64 + 2 * q], h1, r1);
+                mma_tf32(hs, p, h0, h1);
+                mma_tf32(rs, p, r0, r1);
+                float(&sum)[4] = q == 0 ? types.s6[n] : types.s12[n];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-            {
-                types.s12[n][i] += d[i];
+                for (int i = 0; i < (kBig ? 4 : 2); i++)
+                {
+                    sum[i] += hs[i] + rs[i];
+                }
             }
         }
     }
@@ -571,7 +549,7 @@ __device__ __forceinline__ void adj_flush(const DeviceView& v, const double* gsu
             t += gsum_s[w * per + m];
         }
         const int val = m >> 5, lane = m & 31, i = (val >> 1) & 3, n = val >> 3;
-        const int a = (lane >> 2) + 8 * (i >> 1), b = 2 * (lane & 3) + (i & 1) + 8 * n;
+        const int b = (lane >> 2) + 8 * (i >> 1), a = 2 * (lane & 3) + (i & 1) + 8 * n;  // j type, i type
         if (t != 0.0 && a < v.ntypes1 && b < v.ntypes1)
         {
             atomicAdd(&gnbfp[2 * (a * v.ntypes1 + b) + (val & 1)], t);

@@ -282,3 +282,18 @@ def test_fused_force_matching_loss_matches_the_torch_expression():
     with pytest.raises(TypeError):
         force_matching_loss(f_t.double(), f_t.double())
     eng.close()
+
+
+@pytest.mark.parametrize("coulomb", [COULOMB_EWALD, COULOMB_RF])
+@pytest.mark.parametrize("loss_kind", ["linear", "match"])
+@pytest.mark.parametrize("ntypes", [1, 7, 8, 9, 15])
+def test_adjoint_type_tiles_match_fp64_autograd(ntypes, loss_kind, coulomb):
+    """Type counts at the edges of the tensor-core tiles (8 rows or columns, at most 15 types), with and
+    without energy gradients (the two flavours of the kernel)."""
+    s = systems.lj_liquid(n=700, ntypes=ntypes, seed=40 + ntypes, sigma_range=(0.25, 0.30))
+    rng = np.random.default_rng(ntypes)
+    g_f, g_e = rng.normal(size=(s.n, 3)), np.array([0.3, -0.2])
+    f_target = 100.0 * rng.normal(size=(s.n, 3))
+    g = _gpu(s, coulomb, g_f, g_e, loss_kind, f_target)
+    r = _fp64(s, coulomb, g_f, g_e, loss_kind, f_target)
+    print(ntypes, loss_kind, coulomb, _compare(g, r))
