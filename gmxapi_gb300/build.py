@@ -26,6 +26,7 @@ UNITS = {
     "nbx_prune.cu": ["--fmad=false"],
     "nbx_force.cu": [],
     "nbx_force_x2.cu": [],
+    "nbx_force_x2_lj.cu": [],
     "nbx_batch.cu": [],
     "nbx_batch_x2.cu": [],
     "nbx_adjoint.cu": [],

@@ -34,17 +34,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     WarpSmemX2      w;
     carve_x2<kDepth>(smem_bx2 + nt1 * nt1, threadIdx.x >> 5, js, w);
     stage_init_x2(js, lane);
-    PairConstsX2 k;
-    k.rc2      = cv.rc2;
-    k.pbeta    = cv.pbeta;
-    k.nbeta2l2 = -cv.beta2l2;
-    k.c2b      = cv.c2b;
-    k.k_rf2    = cv.k_rf2;
-    k.nk_rf2   = -cv.k_rf2;
-    k.sh_ewald = cv.sh_ewald;
-    k.k_rf     = cv.k_rf;
-    k.c_rf     = cv.c_rf;
-    k.epsfac   = cv.epsfac;
+    const PairConstsX2 k = pair_consts_x2(cv);
     // per-lane FP64 energies of the system in hand, added to its sums when the warp's entries move on to
     // another system (the queue hands out entries in system order)
     __shared__ double e_acc_s[2][kThreads];
@@ -98,7 +88,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         const Sci       si = s;
         const SysPtrsX2 p  = { b.xq, b.tgrid, b.xqp, b.fnb, b.cj4, b.excl, b.shiftvec,
                                fshift + (size_t)kNShift * 3 * sidx };
-        if (!process_entry_x2<kEnergy, kCoul, kDepth>(k, p, si, reinterpret_cast<const char*>(nbfp_s), js, w, nt1,
+        if (!process_entry_x2<kEnergy, kCoul, kDepth, 0>(k, p, si, reinterpret_cast<const char*>(nbfp_s), js, w, nt1,
                                                        lane, cv.wait_test_bytes, e_lj_acc, e_el_acc, claim, fetch))
         {
             stage_timeout_x2(js, const_cast<unsigned*>(&b.hdr->status), lane);

@@ -9,10 +9,8 @@
 //   RF      qq*(1/r + k_rf r^2 - c_rf),
 // and the forces on j are the negated forces on i (half list).
 //
-// This file holds the one-pair-per-lane kernel (k_force: the switch modifiers, LJ-PME and the
-// autotuner's tile 0), the force reduction, the allocation-free entry and the launch dispatch; the
-// default kernel for potential-shift and plain cut-off LJ is the packed two-pairs-per-lane core of
-// nbx_force_x2.cu / nbx_pair_x2.cuh, which shares the work queue, the exclusion work items and the
+// This file holds the one-pair-per-lane kernel (k_force: the autotuner's tile 0), the force reduction, the allocation-free entry and the launch dispatch; the
+// default kernel is the packed two-pairs-per-lane core of nbx_force_x2.cuh / nbx_pair_x2.cuh, which shares the work queue, the exclusion work items and the
 // reduction below.
 //
 // GB300 design (not the reference's 8x8-thread blocks):
@@ -585,10 +583,17 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
                    : (v.vdw_mod == NBX_VDW_POTSWITCH) ? 2
                    : (v.vdw_mod == NBX_VDW_LJPME)     ? 3
                                                        : 0;
-    if (lj == 0 && v.pair_core == 1)
+    if (v.pair_core == 1)
     {
-        // the packed core (potential shift or plain cut-off)
-        launch_force_x2(kv, energy, s, num_sms, counter);
+        // the packed core; the modifiers have its default shape only
+        if (lj == 0)
+        {
+            launch_force_x2(kv, energy, s, num_sms, counter);
+        }
+        else
+        {
+            launch_force_x2_lj(kv, lj, energy, s, num_sms, counter);
+        }
         if (ev1)
         {
             cudaEventRecord(ev1, s);

@@ -256,8 +256,8 @@ struct DeviceView
     // this many work items of excl_atoms atoms interleaved with the list entries
     int excl_chunks;
     int excl_atoms;
-    // force kernel tile: 1 = packed core (two pairs per lane, FP32x2 arithmetic; potential-shift
-    // or plain cut-off LJ), 0 = scalar core (one pair per lane); j-stage buffers per warp (2, 3)
+    // force kernel tile: 1 = packed core (two pairs per lane, FP32x2 arithmetic), 0 = scalar core (one
+    // pair per lane); j-stage buffers per warp (2, 3)
     int pair_core;
     int stage_depth;
     int force_blocks;  // resident blocks of 256 threads per SM for the packed kernel (2, 3)
@@ -444,6 +444,8 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
 // the packed-core force kernel (v.pair_core 1; potential-shift or plain cut-off LJ), with the
 // v.stage_depth j-stage buffers and v.force_blocks blocks per SM
 cudaError_t launch_force_x2(const DeviceView& v, bool energy, cudaStream_t s, int num_sms, int* counter);
+// the same with lj 1 force switch, 2 potential switch, 3 LJ-PME
+cudaError_t launch_force_x2_lj(const DeviceView& v, int lj, bool energy, cudaStream_t s, int num_sms, int* counter);
 // forces to atom order (+ virial); with d_e / d_vir the last block also finishes the energies
 // and virial (the accumulators must have been cleared by launch_convert_x(clear))
 // (stage: write the forces through shared memory as contiguous floats, for f in host memory)

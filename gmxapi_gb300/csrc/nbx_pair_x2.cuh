@@ -206,8 +206,39 @@ struct EnergySumsX2
 // Constants of the pair loop, read once per entry.
 struct PairConstsX2
 {
-    float rc2, pbeta, nbeta2l2, c2b, k_rf2, nk_rf2, sh_ewald, k_rf, c_rf, epsfac;
+    float rc2, pbeta, nbeta2l2, c2b, nk_rf2, sh_ewald, k_rf, c_rf, epsfac;
+    // LJ modifiers (kLj): switching distance and the coefficients of DeviceView
+    float rvdw_switch, fsw_disp_c2, fsw_disp_c3, fsw_rep_c2, fsw_rep_c3, psw_c3, psw_c4, psw_c5;
+    float nlje_l2, lje_coeff6_6, sh_lj_ewald;  // LJ-PME: -beta_lj^2 log2(e), beta_lj^6 / 6, shift
+    float lje_coeff2;
 };
+
+__device__ __forceinline__ PairConstsX2 pair_consts_x2(const DeviceView& v)
+{
+    PairConstsX2 k;
+    k.rc2          = v.rc2;
+    k.pbeta        = v.pbeta;
+    k.nbeta2l2     = -v.beta2l2;
+    k.c2b          = v.c2b;
+    k.nk_rf2       = -v.k_rf2;
+    k.sh_ewald     = v.sh_ewald;
+    k.k_rf         = v.k_rf;
+    k.c_rf         = v.c_rf;
+    k.epsfac       = v.epsfac;
+    k.rvdw_switch  = v.rvdw_switch;
+    k.fsw_disp_c2  = v.fsw_disp_c2;
+    k.fsw_disp_c3  = v.fsw_disp_c3;
+    k.fsw_rep_c2   = v.fsw_rep_c2;
+    k.fsw_rep_c3   = v.fsw_rep_c3;
+    k.psw_c3       = v.psw_c3;
+    k.psw_c4       = v.psw_c4;
+    k.psw_c5       = v.psw_c5;
+    k.nlje_l2      = -1.4426950408889634f * v.lje_coeff2;
+    k.lje_coeff2   = v.lje_coeff2;
+    k.lje_coeff6_6 = v.lje_coeff6_6;
+    k.sh_lj_ewald  = v.sh_lj_ewald;
+    return k;
+}
 
 // The geometry of one packed step: i-cluster c's atom ii (record rec in shared memory) against
 // the lane's two j-atoms.  in: the pair is inside the cut-off and its half's mask bit is set (and,
@@ -241,7 +272,8 @@ __device__ __forceinline__ void pair_geom_x2(const PairConstsX2& k, float4* __re
 
 // The forces and energies of one packed step whose geometry is g; the lane's i-force partial for
 // atom (c, ii) is read, updated and written back in shared memory.
-template<bool kEnergy, int kCoul, bool kExcl>
+// kLj: 0 potential shift or plain cut-off, 1 force switch, 2 potential switch, 3 LJ-PME (grid part).
+template<bool kEnergy, int kCoul, bool kExcl, int kLj>
 __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* __restrict__ nbfp_b, const GeomX2& g,
                                              int jj, const float2 qje, const int2 tjb, float2& fjx, float2& fjy,
                                              float2& fjz, float2& ejel, float2& ejlj)
@@ -269,14 +301,80 @@ __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* 
     // come from two table rows)
     const float4 lA    = *reinterpret_cast<const float4*>(nbfp_b + ti + tjb.x);
     const float4 lB    = *reinterpret_cast<const float4*>(nbfp_b + ti + tjb.y);
-    float2       rinv6 = mul2(mul2(rinv2, rinv2), rinv2);
+    float2       rinv6    = mul2(mul2(rinv2, rinv2), rinv2);
+    const float2 rinv6_nm = rinv6;  // LJ-PME: the grid part also acts on excluded pairs
     if (kExcl)
     {
         rinv6 = mul2(rinv6, make_float2(intA, intB));
     }
     const float2 nvdisp = make_float2(lA.x * rinv6.x, lB.x * rinv6.y);
-    const float2 flj    = make_float2(fmaf(lA.y * rinv6.x, rinv6.x, nvdisp.x),
+    float2       flj    = make_float2(fmaf(lA.y * rinv6.x, rinv6.x, nvdisp.x),
                                       fmaf(lB.y * rinv6.y, rinv6.y, nvdisp.y));  // F r^2: vrep - vdisp
+    // Only pairs inside the cut-off that are not excluded count in the energies.  Outside the cut-off 1/r = 0
+    // already zeroes every r-dependent term, so only the constant shifts need the mask; an excluded pair
+    // inside the cut-off (int 0) has 1/r^6 = 0 (LJ) but its Ewald and switched terms must go.
+    const bool cA = kExcl ? (inA && intA != 0.0f) : inA;
+    const bool cB = kExcl ? (inB && intB != 0.0f) : inB;
+    // LJ energy: vrep/12 - vdisp/6 + shift = (flj - vdisp)/12 + shift
+    float2 vlj = f2(0.0f);
+    if (kEnergy || kLj == 2)
+    {
+        vlj = fma2(add2(flj, nvdisp), f2(1.0f / 12.0f), make_float2(cA ? lA.z : 0.0f, cB ? lB.z : 0.0f));
+    }
+    if (kLj == 1 || kLj == 2)
+    {
+        // force / potential switch from rvdw_switch to rc (kernel_ref_inner.h:168-200); r = 0 for pairs out of
+        // range
+        const float2 r   = mul2(r2, rinv);
+        const float2 rsw = make_float2(fmaxf(r.x - k.rvdw_switch, 0.0f), fmaxf(r.y - k.rvdw_switch, 0.0f));
+        const float2 rs2 = mul2(rsw, rsw);
+        if (kLj == 1)
+        {
+            // F r^2 += (12C12 (c2' + c3' rsw) - 6C6 (c2 + c3 rsw)) rsw^2 r; the energy gains the integral terms
+            // (-c2/3 - c3/4 rsw) rsw^3 of each
+            const float2 rep  = fma2(f2(k.fsw_rep_c3), rsw, f2(k.fsw_rep_c2));
+            const float2 disp = fma2(f2(k.fsw_disp_c3), rsw, f2(k.fsw_disp_c2));
+            const float2 sum  = make_float2(fmaf(lA.y, rep.x, lA.x * disp.x), fmaf(lB.y, rep.y, lB.x * disp.y));
+            flj               = fma2(mul2(sum, rs2), r, flj);
+            if (kEnergy)
+            {
+                const float2 erep  = fma2(f2(k.fsw_rep_c3 * -0.25f), rsw, f2(k.fsw_rep_c2 * (-1.0f / 3.0f)));
+                const float2 edisp = fma2(f2(k.fsw_disp_c3 * -0.25f), rsw, f2(k.fsw_disp_c2 * (-1.0f / 3.0f)));
+                const float2 esum  = make_float2(fmaf(lA.y, erep.x, lA.x * edisp.x),
+                                                 fmaf(lB.y, erep.y, lB.x * edisp.y));
+                vlj                = fma2(esum, mul2(rs2, rsw), vlj);
+            }
+        }
+        else
+        {
+            // sw = 1 + c3 rsw^3 + c4 rsw^4 + c5 rsw^5; F r^2 = F r^2 sw - r V dsw, V *= sw
+            const float2 p   = fma2(fma2(f2(k.psw_c5), rsw, f2(k.psw_c4)), rsw, f2(k.psw_c3));
+            const float2 sw  = fma2(p, mul2(rs2, rsw), f2(1.0f));
+            const float2 dp  = fma2(fma2(f2(5.0f * k.psw_c5), rsw, f2(4.0f * k.psw_c4)), rsw, f2(3.0f * k.psw_c3));
+            const float2 rvd = mul2(mul2(r, vlj), mul2(dp, rs2));
+            flj              = sub2(mul2(flj, sw), rvd);
+            vlj              = mul2(vlj, sw);
+        }
+    }
+    if (kLj == 3)
+    {
+        // LJ-PME, geometric grid c6grid = l.w (kernel_ref_inner.h:204-252): subtract the grid part
+        // c6grid (1 - e^-b (1 + b + b^2/2)) / r^6, b = beta_lj^2 r^2, from F r^2 and V
+        const float2 earg = mul2(f2(k.nlje_l2), r2);
+        const float2 ex   = make_float2(fast_ex2(earg.x), fast_ex2(earg.y));
+        const float2 cr2  = mul2(f2(k.lje_coeff2), r2);
+        const float2 poly = fma2(mul2(f2(0.5f), cr2), cr2, add2(f2(1.0f), cr2));
+        const float2 part = sub2(rinv6_nm, mul2(ex, fma2(rinv6_nm, poly, f2(k.lje_coeff6_6))));
+        flj               = make_float2(fmaf(lA.w, part.x, flj.x), fmaf(lB.w, part.y, flj.y));
+        if (kEnergy)
+        {
+            // the grid potential's shift only for pairs that interact
+            const float2 ep = mul2(ex, poly);
+            const float2 v  = make_float2(fmaf(rinv6_nm.x, 1.0f - ep.x, k.sh_lj_ewald),
+                                          fmaf(rinv6_nm.y, 1.0f - ep.y, k.sh_lj_ewald));
+            vlj             = make_float2(fmaf(lA.w * (1.0f / 6.0f), v.x, vlj.x), fmaf(lB.w * (1.0f / 6.0f), v.y, vlj.y));
+        }
+    }
     const float2 qq     = mul2(g.qi, qje);
     float2       fcr2;  // Coulomb F r^2 / (q_i q_j)
     float2       hel;   // Coulomb energy / (q_i q_j epsfac), before masking
@@ -317,14 +415,11 @@ __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* 
     const float2 fscal = mul2(fma2(qq, fcr2, flj), rinv2);
     if (kEnergy)
     {
-        // Only pairs inside the cut-off that are not excluded count.  Outside the cut-off 1/r = 0
-        // already zeroes every r-dependent term, so only the constant shifts need the mask; an
-        // excluded pair inside the cut-off (int 0) has 1/r^6 = 0 (LJ) but its Ewald term must go.
-        const bool cA = kExcl ? (inA && intA != 0.0f) : inA;
-        const bool cB = kExcl ? (inB && intB != 0.0f) : inB;
-        // LJ energy: vrep/12 - vdisp/6 + shift = (flj - vdisp)/12 + shift
-        const float2 vlj = fma2(add2(flj, nvdisp), f2(1.0f / 12.0f), make_float2(cA ? lA.z : 0.0f, cB ? lB.z : 0.0f));
-        ejlj             = add2(ejlj, vlj);
+        if ((kLj == 1 && kExcl) || kLj == 3)
+        {
+            vlj = make_float2(cA ? vlj.x : 0.0f, cB ? vlj.y : 0.0f);
+        }
+        ejlj = add2(ejlj, vlj);
         if (kExcl)
         {
             hel = make_float2(cA ? hel.x : 0.0f, cB ? hel.y : 0.0f);
@@ -397,7 +492,7 @@ __device__ __forceinline__ bool next_step_x2(const PairConstsX2& k, float4* __re
 
 // The set i-clusters `rem` of one j-cluster, the ones with pairs inside the cut-off visited two at
 // a time so that two independent pair computations share a basic block.
-template<bool kEnergy, int kCoul, bool kExcl, bool kSame>
+template<bool kEnergy, int kCoul, bool kExcl, bool kSame, int kLj>
 __device__ __forceinline__ void jcluster_x2(const PairConstsX2& k, const char* __restrict__ nbfp_b,
                                             float4* __restrict__ lane_rec, unsigned rem, unsigned mA, unsigned mB,
                                             unsigned xA, unsigned xB, bool central, int sci, int cj, int ii, int jj,
@@ -416,17 +511,17 @@ __device__ __forceinline__ void jcluster_x2(const PairConstsX2& k, const char* _
         GeomX2 gb;
         if (!next_step_x2<kExcl, kSame>(k, lane_rec, rem, mA, mB, xA, xB, central, sci, cj, ii, jj, xj, yj, zj, gb))
         {
-            pair_phys_x2<kEnergy, kCoul, kExcl>(k, nbfp_b, ga, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
+            pair_phys_x2<kEnergy, kCoul, kExcl, kLj>(k, nbfp_b, ga, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
             break;
         }
-        pair_phys_x2<kEnergy, kCoul, kExcl>(k, nbfp_b, ga, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
-        pair_phys_x2<kEnergy, kCoul, kExcl>(k, nbfp_b, gb, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
+        pair_phys_x2<kEnergy, kCoul, kExcl, kLj>(k, nbfp_b, ga, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
+        pair_phys_x2<kEnergy, kCoul, kExcl, kLj>(k, nbfp_b, gb, jj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
     }
 }
 
 // All set cluster pairs of one cj4 group.  m0 / m1: the group's half masks; wA / wB: the
 // lane's exclusion words of the two halves (all ones without exclusions).
-template<bool kEnergy, int kCoul, bool kExcl>
+template<bool kEnergy, int kCoul, bool kExcl, int kLj>
 __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2& p, const char* __restrict__ nbfp_b,
                                          const float* __restrict__ jx,
                                          float4* __restrict__ lane_rec, int cj_lane, unsigned m0, unsigned m1,
@@ -458,12 +553,12 @@ __device__ __forceinline__ void group_x2(const PairConstsX2& k, const SysPtrsX2&
         if (!kExcl && ((mA ^ mB) & 0xffu) == 0)
         {
             // both halves set for every i-cluster of this j-cluster (the common case)
-            jcluster_x2<kEnergy, kCoul, false, true>(k, nbfp_b, lane_rec, rem, mA, mB, xA, xB, central, sci, cj, ii,
+            jcluster_x2<kEnergy, kCoul, false, true, kLj>(k, nbfp_b, lane_rec, rem, mA, mB, xA, xB, central, sci, cj, ii,
                                                      jj, xj, yj, zj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
         }
         else
         {
-            jcluster_x2<kEnergy, kCoul, kExcl, false>(k, nbfp_b, lane_rec, rem, mA, mB, xA, xB, central, sci, cj, ii,
+            jcluster_x2<kEnergy, kCoul, kExcl, false, kLj>(k, nbfp_b, lane_rec, rem, mA, mB, xA, xB, central, sci, cj, ii,
                                                       jj, xj, yj, zj, qje, tjb, fjx, fjy, fjz, ejel, ejlj);
         }
         if (kEnergy)
@@ -509,7 +604,7 @@ __device__ __forceinline__ uint2 excl_words(const SysPtrsX2& p, const int4 ime, 
 // claim() is called before the entry's force reduction and fetch() after it: the warp's next work item is
 // taken from the queue and its record loaded under this entry's last work (taken a group earlier, items
 // wait in busy warps' hands at the end of the launch: md steps of 32k atoms 98.7 instead of 96.3 us).
-template<bool kEnergy, int kCoul, int kDepth, class Claim, class Fetch>
+template<bool kEnergy, int kCoul, int kDepth, int kLj, class Claim, class Fetch>
 __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const SysPtrsX2& p, const Sci& s,
                                                  const char* __restrict__ nbfp_b, JStageP<kDepth>& js,
                                                  const WarpSmemX2& w, int nt1, int lane, unsigned wait_test_bytes,
@@ -604,12 +699,12 @@ __device__ __forceinline__ bool process_entry_x2(const PairConstsX2& k, const Sy
         const float* jx = js.x + b * kJg * kPackWords;
         if ((ime.y | ime.w) == 0)
         {
-            group_x2<kEnergy, kCoul, false>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, ~0u, ~0u, s.sci, central,
+            group_x2<kEnergy, kCoul, false, kLj>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, ~0u, ~0u, s.sci, central,
                                              ii, jj, es);
         }
         else
         {
-            group_x2<kEnergy, kCoul, true>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, wAB.x, wAB.y, s.sci,
+            group_x2<kEnergy, kCoul, true, kLj>(k, p, nbfp_b, jx, lane_rec, cj_lane, m0, m1, wAB.x, wAB.y, s.sci,
                                             central, ii, jj, es);
         }
     }

@@ -170,8 +170,8 @@ int nbx_get_phase_timings(nbx_handle* h, double* ms, long long* counts, int rese
 /* Force-kernel shape (no counterpart in the reference; the autotuner's tile and staging
  * axes).  tile 0: one atom pair per lane, a warp instruction covers 8 i-atoms x 4 j-atoms
  * (scalar FP32); tile 1 (default): two pairs per lane, 8 x 8 atoms per warp instruction
- * (packed FP32x2 arithmetic; potential-shift or plain cut-off LJ -- the switch modifiers and
- * LJ-PME always run tile 0).  stage_depth: j-cluster stage buffers per warp of tile 1, 2
+ * (packed FP32x2 arithmetic; the switch modifiers and LJ-PME run it with stage_depth 2 and
+ * blocks_per_sm 2 whatever is set).  stage_depth: j-cluster stage buffers per warp of tile 1, 2
  * (default) or 3 (two groups' copies in flight).  blocks_per_sm: resident 256-thread blocks per
  * SM of tile 1, 2 (default; up to 128 registers a thread) or 3 (80 registers).  Results agree
  * to rounding between shapes. */

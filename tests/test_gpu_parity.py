@@ -359,6 +359,34 @@ def test_lj_modifiers_vs_oracle(name, mod):
     assert rel_rms(f, f64) <= FORCE_RTOL
 
 
+@pytest.mark.parametrize("coulomb,shift", [(nblib.CoulombType.Pme, False), (nblib.CoulombType.Pme, True),
+                                           (nblib.CoulombType.ReactionField, False)])
+@pytest.mark.parametrize("mod", [nblib.VdwModifier.ForceSwitch, nblib.VdwModifier.PotSwitch, nblib.VdwModifier.LjPme])
+@pytest.mark.parametrize("name", ["water_small_box", "water_tiny", "lj_liquid"])
+def test_lj_modifiers_same_from_both_tiles(name, mod, coulomb, shift):
+    """The packed kernel (tile 1, the default) and the one-pair-per-lane kernel (tile 0) agree for every
+    modifier and Coulomb flavour, with and without energies: each is held to the force and energy bars
+    against the oracle elsewhere, so they are held to twice the bars against each other."""
+    s = SYSTEMS[name]()
+    calc = nblib.ForceCalculator(s, nblib.NBKernelOptions(
+        coulomb_type=coulomb, pairlist_cutoff=1.0, rcoulomb=0.9, vdw_modifier=mod, epsilon_rf=78.0,
+        rvdw_switch=0.7 if mod != nblib.VdwModifier.LjPme else 0.0, use_ewald_shift=shift,
+        compute_virial_and_energy=True))
+    got = []
+    for tile in (0, 1):
+        calc.set_force_kernel(tile, 2, 2)
+        f = calc.compute(s.x).copy()
+        f_only = calc.compute(s.x, energies=False)
+        assert rel_rms(f_only, f) <= FORCE_RTOL
+        got.append((f, calc.energies.copy(), calc.virial.copy()))
+    (f0, e0, v0), (f1, e1, v1) = got
+    assert rel_rms(f1, f0) <= 2 * FORCE_RTOL
+    etol = ENERGY_RTOL if coulomb == nblib.CoulombType.Pme else ENERGY_RTOL_RF
+    assert np.all(np.abs(e1 - e0) <= 2 * etol * np.abs(e0) + 1e-9), (e0, e1)
+    assert np.abs(v1 - v0).max() <= 2 * FORCE_RTOL * np.abs(v0).max()
+    calc.close()
+
+
 def test_switch_modifiers_rejected_where_unsupported():
     s = systems.lj_liquid(n=600, ntypes=4, seed=3)
     with pytest.raises(nblib.InputException):
