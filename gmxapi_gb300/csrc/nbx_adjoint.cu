@@ -643,13 +643,14 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
     adj_flush<kBig>(cv, gsum_s, gnbfp);
 }
 
-// Batched upstream gradients to grid order (blockIdx.y = system), outputs cleared.
-__global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const float* __restrict__ gF, int* counter,
+// Batched upstream gradients to grid order, outputs cleared.
+__global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, BatchMap map, const float* __restrict__ gF,
+                                    int* counter,
                                     double* gnbfp, int n_gnbfp)
 {
     pdl_begin();
-    // block (0, 0) also clears the work queue and the FP64 type-pair gradient table
-    if (blockIdx.x == 0 && blockIdx.y == 0)
+    // block 0 also clears the work queue and the FP64 type-pair gradient table
+    if (blockIdx.x == 0)
     {
         for (int i = threadIdx.x; i < n_gnbfp; i += blockDim.x)
         {
@@ -660,8 +661,9 @@ __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const floa
             *counter = 0;
         }
     }
-    const BatchSys& b = sys[blockIdx.y];
-    const int       k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int2      part = map.slots[blockIdx.x];
+    const BatchSys& b    = sys[part.x];
+    const int       k    = part.y + threadIdx.x;
     if (k >= b.hdr->num_cells * kSc)
     {
         return;
@@ -673,13 +675,15 @@ __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, const floa
     b.dnb[k]                      = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
-// Batched atom-order outputs (blockIdx.y = system), dL/dq with the self-energy term.
-__global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ sys, const double* __restrict__ gE,
+// Batched atom-order outputs, dL/dq with the self-energy term.
+__global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ sys, BatchMap map,
+                                   const double* __restrict__ gE,
                                    float* gx, float* gq)
 {
     pdl_begin();
-    const BatchSys& b = sys[blockIdx.y];
-    const int       a = blockIdx.x * blockDim.x + threadIdx.x;
+    const int2      part = map.atoms[blockIdx.x];
+    const BatchSys& b    = sys[part.x];
+    const int       a    = part.y + threadIdx.x;
     if (a >= b.n)
     {
         return;
@@ -698,16 +702,17 @@ __global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ s
         const float q    = b.xq[k].w;
         const float self = (cv.coulomb == 0) ? -2.0f * cv.epsfac * cv.beta * 0.5641895835477563f * q
                                              : -cv.epsfac * cv.c_rf * q;
-        gq[o]            = gE ? d.w + (float)gE[2 * blockIdx.y + 1] * self : d.w;
+        gq[o]            = gE ? d.w + (float)gE[2 * part.x + 1] * self : d.w;
     }
 }
 
 // Charges of all systems (concatenated atom order) into xq.w and each system's q.
-__global__ void k_batch_set_q(const BatchSys* __restrict__ sys, const float* __restrict__ q)
+__global__ void k_batch_set_q(const BatchSys* __restrict__ sys, BatchMap map, const float* __restrict__ q)
 {
     pdl_begin();
-    const BatchSys& b = sys[blockIdx.y];
-    const int       k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int2      part = map.slots[blockIdx.x];
+    const BatchSys& b    = sys[part.x];
+    const int       k    = part.y + threadIdx.x;
     if (k >= b.hdr->num_cells * kSc)
     {
         return;
@@ -973,11 +978,10 @@ cudaError_t launch_backward(const DeviceView& v, const float* d_x, const float* 
 }
 
 cudaError_t launch_batch_backward(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys,
-                                  int max_slots, int max_atoms, const float* d_gF, const double* d_gE,
+                                  const BatchMap& map, const float* d_gF, const double* d_gE,
                                   double* d_gnbfp, int* counter, float* d_gx, float* d_gq, int num_sms, cudaStream_t s)
 {
-    const int tb = 256;
-    launch_pdl(k_batch_adj_prepare, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_gF, counter, d_gnbfp,
+    launch_pdl(k_batch_adj_prepare, map.nslots, kBatchPart, 0, s, sys, map, d_gF, counter, d_gnbfp,
                2 * cv.ntypes1 * cv.ntypes1);
     using Launch = cudaError_t (*)(const DeviceView&, const BatchSys*, const int*, int, double*, int*, const double*,
                                    int, cudaStream_t);
@@ -994,14 +998,13 @@ cudaError_t launch_batch_backward(const DeviceView& cv, const BatchSys* sys, con
     {
         return e;
     }
-    launch_pdl(k_batch_adj_finish, dim3((max_atoms + tb - 1) / tb, nsys), tb, 0, s, cv, sys, d_gE, d_gx, d_gq);
+    launch_pdl(k_batch_adj_finish, map.natoms, kBatchPart, 0, s, cv, sys, map, d_gE, d_gx, d_gq);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_set_q(const BatchSys* sys, int nsys, int max_slots, const float* d_q, cudaStream_t s)
+cudaError_t launch_batch_set_q(const BatchSys* sys, const BatchMap& map, const float* d_q, cudaStream_t s)
 {
-    const int tb = 256;
-    launch_pdl(k_batch_set_q, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_q);
+    launch_pdl(k_batch_set_q, map.nslots, kBatchPart, 0, s, sys, map, d_q);
     return cudaGetLastError();
 }
 

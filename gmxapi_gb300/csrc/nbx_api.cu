@@ -1778,8 +1778,8 @@ struct nbx_batch
     double*                  d_sums   = nullptr;
     size_t                   sums_bytes = 0;
     int*                     d_counter  = nullptr;
-    int                      max_slots  = 0;
-    int                      max_atoms  = 0;
+    BatchMap                 map{};    // parts of systems per block (d_map)
+    int2*                    d_map      = nullptr;
     bool                     have_list  = false;
     long long                list_step  = 0;
     int                      prune_part = 0;
@@ -1995,7 +1995,7 @@ int batch_compute(nbx_batch* b, const float* d_x, float* d_f, double* d_e, doubl
 {
     const int nsys = (int)b->sys.size();
     auto      run  = [&](cudaStream_t s) {
-        return launch_batch_compute(b->cv, b->d_table, b->d_prefix, nsys, b->max_slots, b->max_atoms, d_x, d_f,
+        return launch_batch_compute(b->cv, b->d_table, b->d_prefix, nsys, b->map, d_x, d_f,
                                     b->d_sums, b->sums_bytes, b->d_counter, d_e, d_vir, batch_variant_code(b), b->num_sms, s);
     };
     if (!b->use_graph)
@@ -2094,7 +2094,7 @@ cudaError_t batch_backward_launch(nbx_batch* b, const float* d_gF, const double*
                                   double* d_gnbfp, cudaStream_t s)
 {
     const int   nsys = (int)b->sys.size();
-    cudaError_t e    = launch_batch_backward(b->cv, b->d_table, b->d_prefix, nsys, b->max_slots, b->max_atoms, d_gF,
+    cudaError_t e    = launch_batch_backward(b->cv, b->d_table, b->d_prefix, nsys, b->map, d_gF,
                                              d_gE, b->d_gnbfp_pad, b->d_adj_counter, d_gx, d_gq, b->num_sms, s);
     if (e == cudaSuccess && d_gnbfp)
     {
@@ -2130,7 +2130,7 @@ int nbx_batch_set_parameters_device(nbx_batch* b, const float* d_q, const float*
     }
     if (e == cudaSuccess && d_q)
     {
-        e = launch_batch_set_q(b->d_table, (int)b->sys.size(), b->max_slots, d_q, b->stream);
+        e = launch_batch_set_q(b->d_table, b->map, d_q, b->stream);
     }
     return e == cudaSuccess ? NBX_OK : batch_error(b, NBX_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -2153,7 +2153,7 @@ int nbx_batch_backward_device(nbx_batch* b, const float* d_x, const float* d_gF,
         return rc;
     }
     // coordinates into the grid layout (the kernel also clears the force buffers)
-    cudaError_t e = launch_batch_convert(b->d_table, (int)b->sys.size(), b->max_slots, d_x, b->stream);
+    cudaError_t e = launch_batch_convert(b->d_table, b->map, d_x, b->stream);
     if (e == cudaSuccess) e = batch_backward_launch(b, d_gF, d_gE, d_gx, d_gq, d_gnbfp, b->stream);
     return e == cudaSuccess ? NBX_OK : batch_error(b, NBX_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -2181,9 +2181,9 @@ int nbx_batch_force_match_device(nbx_batch* b, const float* d_x, const float* d_
     const size_t n3   = 3 * (size_t)b->offsets.back();
     auto         run  = [&](cudaStream_t s) {
         cudaError_t e = launch_set_parameters(b->sys[0]->v, nullptr, d_nbfp, s);
-        if (e == cudaSuccess) e = launch_batch_set_q(b->d_table, nsys, b->max_slots, d_q, s);
+        if (e == cudaSuccess) e = launch_batch_set_q(b->d_table, b->map, d_q, s);
         if (e == cudaSuccess)
-            e = launch_batch_compute(b->cv, b->d_table, b->d_prefix, nsys, b->max_slots, b->max_atoms, d_x,
+            e = launch_batch_compute(b->cv, b->d_table, b->d_prefix, nsys, b->map, d_x,
                                      b->d_fm_f, b->d_sums, b->sums_bytes, b->d_counter, d_e, d_vir, batch_variant_code(b),
                                      b->num_sms, s);
         if (e == cudaSuccess) e = launch_match_loss(b->d_fm_f, d_ftarget, n3, b->d_fm_g, d_loss, b->num_sms, s);
@@ -2293,8 +2293,6 @@ int nbx_batch_create(int num_systems, const nbx_system_desc* systems, const nbx_
         nbx_set_stream(h, b->stream);
         b->sys.push_back(h);
         b->offsets.push_back(b->offsets.back() + systems[i].num_atoms);
-        b->max_slots = std::max(b->max_slots, h->v.g.cells_capacity * kSc);
-        b->max_atoms = std::max(b->max_atoms, h->n);
     }
     b->cv        = b->sys[0]->v;
     b->use_prune = b->opts.nstlist_prune > 0;
@@ -2303,10 +2301,34 @@ int nbx_batch_create(int num_systems, const nbx_system_desc* systems, const nbx_
     b->sums_bytes     = sizeof(double) * (2 + kNShift * 3 + 9) * nsys + 64;
     if (e == cudaSuccess) e = cudaMalloc(&b->d_table, sizeof(BatchSys) * nsys);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_table, sizeof(BatchSys) * nsys);
-    // entry prefix sums, then the exclusion work items' prefix sums (k_batch_prefix)
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_prefix, sizeof(int) * 2 * (nsys + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_prefix, sizeof(int) * (nsys + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_status, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_sums, b->sums_bytes);
+    if (e == cudaSuccess)
+    {
+        std::vector<int2> parts[3];
+        for (int i = 0; i < num_systems; i++)
+        {
+            const nbx_handle* h   = b->sys[i];
+            const int         n[] = { h->v.g.cells_capacity * kSc, h->n, h->n };
+            for (int m = 0; m < 3; m++)
+            {
+                for (int k = 0; k < n[m]; k += m == 2 ? 4 * kBatchPart : kBatchPart)
+                {
+                    parts[m].push_back(make_int2(i, k));
+                }
+            }
+        }
+        e = cudaMalloc(&b->d_map, sizeof(int2) * (parts[0].size() + parts[1].size() + parts[2].size()));
+        int2* at = b->d_map;
+        for (int m = 0; m < 3 && e == cudaSuccess; m++)
+        {
+            e = cudaMemcpy(at, parts[m].data(), sizeof(int2) * parts[m].size(), cudaMemcpyHostToDevice);
+            (m == 0 ? b->map.slots : m == 1 ? b->map.atoms : b->map.atoms4)     = at;
+            (m == 0 ? b->map.nslots : m == 1 ? b->map.natoms : b->map.natoms4) = (int)parts[m].size();
+            at += parts[m].size();
+        }
+    }
     if (e != cudaSuccess)
     {
         nbx_batch_destroy(b);
@@ -2360,6 +2382,7 @@ int nbx_batch_destroy(nbx_batch* b)
     cudaFree(b->d_prefix);
     cudaFree(b->d_status);
     cudaFree(b->d_sums);
+    cudaFree(b->d_map);
     if (b->own_stream && b->stream)
     {
         cudaStreamDestroy(b->stream);

@@ -1,9 +1,9 @@
 // Batched evaluation of many independent systems of uneven size.
 //
 // Each system keeps its own grid and pair list (built by the single-system
-// search); one step for the whole batch is six launches, independent of the
-// number of systems: clearing the sums, coordinate conversion, FP64 exclusion
-// energies (one wave of warps over 128-atom items of all systems), one
+// search); one step for the whole batch is five launches, independent of the
+// number of systems: coordinate conversion (which clears the sums), FP64 exclusion
+// energies, one
 // persistent force kernel over the concatenated entry space of all systems
 // (an entry finds its system by searching the entry prefix sums), the force
 // gather + virial, and the per-system energy / virial finish.  The sequence
@@ -17,10 +17,8 @@ namespace nbx
 namespace
 {
 
-// Entry prefix sums over the systems' lists (after every search), prefix[0..nsys], and the
-// prefix sums of their exclusion work items (kExclChunkAtoms atoms each),
-// prefix[nsys + 1 .. 2 nsys + 1]; systems whose list or grid overflowed contribute neither
-// and are flagged.
+// Entry prefix sums over the systems' lists (after every search), prefix[0..nsys]; systems whose list or
+// grid overflowed contribute nothing and are flagged.
 __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsigned* status)
 {
     pdl_begin();
@@ -28,13 +26,11 @@ __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsig
     {
         return;
     }
-    int*     chunk_prefix = prefix + nsys + 1;
-    int      run = 0, run_c = 0;
+    int      run = 0;
     unsigned st  = 0;
     for (int s = 0; s < nsys; s++)
     {
-        prefix[s]          = run;
-        chunk_prefix[s]    = run_c;
+        prefix[s]           = run;
         const ListHeader* h = sys[s].hdr;
         if (h->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
         {
@@ -42,20 +38,24 @@ __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsig
             continue;
         }
         run += h->num_sci;
-        run_c += (sys[s].n + kExclChunkAtoms - 1) / kExclChunkAtoms;
     }
-    prefix[nsys]       = run;
-    chunk_prefix[nsys] = run_c;
-    *status            = st;
+    prefix[nsys] = run;
+    *status      = st;
 }
 
-// nbnxn_atomdata_copy_x_to_nbat_x for all systems (blockIdx.y = system); also
-// clears the grid-order force accumulators, so no per-system memset is needed.
-__global__ void k_batch_convert(const BatchSys* __restrict__ sys, const float* __restrict__ x)
+// nbnxn_atomdata_copy_x_to_nbat_x for all systems; also clears the grid-order force accumulators and, with
+// sums, the evaluation's FP64 sums and work counter (n8 8-byte words), so no memset is needed.
+__global__ void __launch_bounds__(kBatchPart) k_batch_convert(const BatchSys* __restrict__ sys, BatchMap map,
+                                                              const float* __restrict__ x, double* sums, int n8)
 {
     pdl_begin();
-    const BatchSys& b = sys[blockIdx.y];
-    const int       k = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x)
+    {
+        sums[i] = 0.0;
+    }
+    const int2      part = map.slots[blockIdx.x];
+    const BatchSys& b    = sys[part.x];
+    const int       k    = part.y + threadIdx.x;
     if (k >= b.hdr->num_cells * kSc)
     {
         return;
@@ -78,38 +78,43 @@ __global__ void k_batch_convert(const BatchSys* __restrict__ sys, const float* _
     }
 }
 
-
-// Excluded-pair Coulomb energies and self terms in FP64 for all systems: one warp per work
-// item of kExclChunkAtoms atoms (the item prefix sums of k_batch_prefix), one wave of blocks,
-// one FP64 atomic per item into its system's energy.
-__global__ void __launch_bounds__(256) k_batch_excl_energy(DeviceView cv, const BatchSys* __restrict__ sys,
-                                                           const int* __restrict__ prefix, int nsys,
-                                                           double* energies)
+// Excluded-pair Coulomb energies and self terms in FP64 for all systems: one atom per thread (an atom's
+// exclusions are a chain of dependent loads; with four atoms a lane 64 boxes took 43 us), one FP64 atomic
+// per block into its system's energy.
+__global__ void __launch_bounds__(kBatchPart) k_batch_excl_energy(DeviceView cv, const BatchSys* __restrict__ sys,
+                                                                  BatchMap map, double* energies)
 {
     pdl_begin();
-    const int* chunk_prefix = prefix + nsys + 1;
-    const int  total        = chunk_prefix[nsys];
-    const int  lane         = threadIdx.x & 31;
-    const int  nwarps       = (gridDim.x * blockDim.x) >> 5;
-    const double beta2      = (double)cv.beta * (double)cv.beta;
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total; c += nwarps)
+    const int2      part  = map.atoms[blockIdx.x];
+    const BatchSys& b     = sys[part.x];
+    const int       i     = part.y + threadIdx.x;
+    const double    beta2 = (double)cv.beta * (double)cv.beta;
+    double          acc = 0.0, acc_s = 0.0, acc_lj = 0.0;
+    if (i < b.n)
     {
-        const int       cs = find_system(chunk_prefix, nsys, c);
-        const BatchSys& b  = sys[cs];
-        const int       a0 = (c - chunk_prefix[cs]) * kExclChunkAtoms;
-        double          acc = 0.0, acc_s = 0.0, acc_lj = 0.0;
-        for (int i = a0 + lane; i < min(b.n, a0 + kExclChunkAtoms); i += 32)
+        excl_atom(cv, b, i, false, beta2, acc, acc_s, acc_lj);
+    }
+    acc += acc_s * (-(double)cv.beta * 1.1283791670955125739);
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    }
+    __shared__ double sum[kBatchPart / 32];
+    if ((threadIdx.x & 31) == 0)
+    {
+        sum[threadIdx.x >> 5] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        double t = 0.0;
+        for (double w : sum)
         {
-            excl_atom(cv, b, i, false, beta2, acc, acc_s, acc_lj);
+            t += w;
         }
-        acc += acc_s * (-(double)cv.beta * 1.1283791670955125739);
-        for (int o = 16; o > 0; o >>= 1)
+        if (t != 0.0)
         {
-            acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        }
-        if (lane == 0 && acc != 0.0)
-        {
-            atomicAdd(&energies[2 * cs + 1], acc * cv.epsfac_d);
+            atomicAdd(&energies[2 * part.x + 1], t * cv.epsfac_d);
         }
     }
 }
@@ -184,46 +189,65 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     }
 }
 
-constexpr int kBatchReduceAtoms = 8;
+constexpr int kBatchReduceAtoms = 4;
 
 // f (concatenated, atom order) and per-system sum x (x) f, float partials reduced in FP64.
-__global__ void k_batch_reduce(const BatchSys* __restrict__ sys, float* __restrict__ f, double* virial,
-                               int do_virial)
+__global__ void __launch_bounds__(kBatchPart) k_batch_reduce(const BatchSys* __restrict__ sys, BatchMap map,
+                                                             float* __restrict__ f, double* virial, int do_virial)
 {
     pdl_begin();
-    const BatchSys& b = sys[blockIdx.y];
+    const int2      part = map.atoms4[blockIdx.x];
+    const BatchSys& b    = sys[part.x];
     float           w[9];
 #pragma unroll
     for (int k = 0; k < 9; k++)
     {
         w[k] = 0.0f;
     }
-    const int a0 = blockIdx.x * blockDim.x * kBatchReduceAtoms + threadIdx.x;
+    // all gathers first, then the stores (loads written after a store would wait for it)
+    const int a0 = part.y + threadIdx.x;
+    int       ks[kBatchReduceAtoms];
 #pragma unroll
     for (int r = 0; r < kBatchReduceAtoms; r++)
     {
-        const int a = a0 + r * blockDim.x;
-        if (a < b.n)
+        const int a = a0 + r * kBatchPart;
+        ks[r]       = a < b.n ? b.cells[a] : -1;
+    }
+    float4 fa[kBatchReduceAtoms], xa[kBatchReduceAtoms];
+#pragma unroll
+    for (int r = 0; r < kBatchReduceAtoms; r++)
+    {
+        fa[r] = xa[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (ks[r] >= 0)
         {
-            const int    k  = b.cells[a];
-            const float4 fa = b.fnb[k];
-            float*       fo = f + 3 * (size_t)(b.atom_base + a);
-            fo[0]           = fa.x;
-            fo[1]           = fa.y;
-            fo[2]           = fa.z;
+            fa[r] = b.fnb[ks[r]];
             if (do_virial)
             {
-                const float4 xa    = b.xq[k];
-                const float  xv[3] = { xa.x, xa.y, xa.z };
-                const float  fv[3] = { fa.x, fa.y, fa.z };
+                xa[r] = b.xq[ks[r]];
+            }
+        }
+    }
 #pragma unroll
-                for (int p = 0; p < 3; p++)
+    for (int r = 0; r < kBatchReduceAtoms; r++)
+    {
+        if (ks[r] >= 0)
+        {
+            float* fo = f + 3 * (size_t)(b.atom_base + a0 + r * kBatchPart);
+            fo[0]     = fa[r].x;
+            fo[1]     = fa[r].y;
+            fo[2]     = fa[r].z;
+        }
+        if (do_virial)
+        {
+            const float xv[3] = { xa[r].x, xa[r].y, xa[r].z };
+            const float fv[3] = { fa[r].x, fa[r].y, fa[r].z };
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+            {
+#pragma unroll
+                for (int q = 0; q < 3; q++)
                 {
-#pragma unroll
-                    for (int q = 0; q < 3; q++)
-                    {
-                        w[p * 3 + q] = fmaf(xv[p], fv[q], w[p * 3 + q]);
-                    }
+                    w[p * 3 + q] = fmaf(xv[p], fv[q], w[p * 3 + q]);
                 }
             }
         }
@@ -260,7 +284,7 @@ __global__ void k_batch_reduce(const BatchSys* __restrict__ sys, float* __restri
         }
         if (t != 0.0)
         {
-            atomicAdd(&virial[9 * blockIdx.y + threadIdx.x], t);
+            atomicAdd(&virial[9 * part.x + threadIdx.x], t);
         }
     }
 }
@@ -280,15 +304,40 @@ __global__ void k_batch_finish(const BatchSys* __restrict__ sys, int nsys, const
     {
         d_e[2 * s + t] = energies[2 * s + t] + (t == 1 ? sys[s].self_energy : 0.0);
     }
-    if (d_vir && t < 9)
+    if (d_vir)
     {
-        const int p = t / 3, q = t % 3;
-        double    acc = virial[9 * s + t];
-        for (int sh = 0; sh < kNShift; sh++)
+        // the 45 shifts over the lanes
+        double acc[9];
+#pragma unroll
+        for (int c = 0; c < 9; c++)
         {
-            acc += (double)sys[s].shiftvec[3 * sh + p] * fshift[(size_t)kNShift * 3 * s + 3 * sh + q];
+            acc[c] = 0.0;
         }
-        d_vir[9 * s + t] = -0.5 * acc;
+        for (int sh = t; sh < kNShift; sh += 32)
+        {
+            const double* fsh = fshift + (size_t)kNShift * 3 * s + 3 * sh;
+            const double  fx = fsh[0], fy = fsh[1], fz = fsh[2];
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+            {
+                const double v = (double)sys[s].shiftvec[3 * sh + p];
+                acc[3 * p] += v * fx;
+                acc[3 * p + 1] += v * fy;
+                acc[3 * p + 2] += v * fz;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 9; c++)
+        {
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+            }
+            if (t == c)
+            {
+                d_vir[9 * s + c] = -0.5 * (virial[9 * s + c] + acc[c]);
+            }
+        }
     }
 }
 
@@ -339,31 +388,26 @@ cudaError_t launch_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsi
     return cudaGetLastError();
 }
 
-// One batched step: sums (energies | fshift | virial partials | work counter)
-cudaError_t launch_batch_convert(const BatchSys* sys, int nsys, int max_slots, const float* d_x, cudaStream_t s)
+cudaError_t launch_batch_convert(const BatchSys* sys, const BatchMap& map, const float* d_x, cudaStream_t s)
 {
-    const int tb = 256;
-    launch_pdl(k_batch_convert, dim3((max_slots + tb - 1) / tb, nsys), tb, 0, s, sys, d_x);
-    return cudaGetLastError();
+    return launch_pdl(k_batch_convert, map.nslots, kBatchPart, 0, s, sys, map, d_x, nullptr, 0);
 }
 
-// cleared with one memset, then the five kernels.
+// One batched step.  sums: energies | fshift | virial partials | work counter, cleared by the conversion.
 cudaError_t launch_batch_compute(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys,
-                                 int max_slots, int max_atoms, const float* d_x, float* d_f, double* sums,
+                                 const BatchMap& map, const float* d_x, float* d_f, double* sums,
                                  size_t sums_bytes, int* counter, double* d_e, double* d_vir, int variant,
                                  int num_sms, cudaStream_t s)
 {
-    const bool energy  = (d_e != nullptr) || (d_vir != nullptr);
-    double*    en      = sums;
-    double*    fs      = sums + 2 * (size_t)nsys;
-    double*    vir     = fs + (size_t)kNShift * 3 * nsys;
-    cudaError_t e      = cudaMemsetAsync(sums, 0, sums_bytes, s);
-    const int  tb      = 256;
-    dim3       gconv((max_slots + tb - 1) / tb, nsys);
-    launch_pdl(k_batch_convert, gconv, tb, 0, s, sys, d_x);
+    const bool  energy = (d_e != nullptr) || (d_vir != nullptr);
+    double*     en     = sums;
+    double*     fs     = sums + 2 * (size_t)nsys;
+    double*     vir    = fs + (size_t)kNShift * 3 * nsys;
+    cudaError_t e      = launch_pdl(k_batch_convert, map.nslots, kBatchPart, 0, s, sys, map, d_x, sums,
+                                    (int)(sums_bytes / sizeof(double)));
     if (energy)
     {
-        launch_pdl(k_batch_excl_energy, num_sms * 8, 256, 0, s, cv, sys, prefix, nsys, en);
+        launch_pdl(k_batch_excl_energy, map.natoms, kBatchPart, 0, s, cv, sys, map, en);
     }
     const bool ewald = (cv.coulomb == 0);
     if (variant & 4)
@@ -390,8 +434,7 @@ cudaError_t launch_batch_compute(const DeviceView& cv, const BatchSys* sys, cons
         else
             launch_batch_force_variant<false, false>(variant, cv, sys, prefix, nsys, counter, en, fs, num_sms, s);
     }
-    dim3 gred((max_atoms + tb * kBatchReduceAtoms - 1) / (tb * kBatchReduceAtoms), nsys);
-    launch_pdl(k_batch_reduce, gred, tb, 0, s, sys, d_f, vir, d_vir ? 1 : 0);
+    launch_pdl(k_batch_reduce, map.natoms4, kBatchPart, 0, s, sys, map, d_f, vir, d_vir ? 1 : 0);
     if (energy)
     {
         launch_pdl(k_batch_finish, nsys, 32, 0, s, sys, nsys, en, fs, vir, d_e, d_vir);

@@ -376,6 +376,18 @@ struct BatchSys
     float             shiftvec[kNShift * 3];
 };
 
+// Which part of which system a block of a batched kernel takes, {system, first slot or atom}: a grid of
+// (largest system x systems) blocks, most of them without work, took 43 us to convert 64 boxes of 500 to
+// 20,000 atoms.  Built once: a handle's sizes do not change.
+struct BatchMap
+{
+    const int2* slots;   // parts of 256 grid slots (up to the grid's capacity)
+    const int2* atoms;   // parts of 256 atoms
+    const int2* atoms4;  // parts of 1024 atoms
+    int         nslots, natoms, natoms4;
+};
+constexpr int kBatchPart = 256;
+
 // Dynamic shared memory beyond the 48 KB default needs a per-kernel opt-in; the attribute is a
 // property of the kernel in the current device's context.  total_bytes (dynamic + static) decides
 // whether the opt-in is needed; the largest dynamic size set so far is remembered per kernel and
@@ -467,10 +479,10 @@ cudaError_t launch_lb_table_backward(const double* sig, const double* eps, int n
                                      double* gsig, double* geps, cudaStream_t s);
 cudaError_t launch_compact_gnbfp(const double* padded, double* out, int nt, cudaStream_t s);
 cudaError_t launch_batch_backward(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys,
-                                  int max_slots, int max_atoms, const float* d_gF, const double* d_gE,
+                                  const BatchMap& map, const float* d_gF, const double* d_gE,
                                   double* d_gnbfp, int* counter, float* d_gx, float* d_gq, int num_sms, cudaStream_t s);
-cudaError_t launch_batch_convert(const BatchSys* sys, int nsys, int max_slots, const float* d_x, cudaStream_t s);
-cudaError_t launch_batch_set_q(const BatchSys* sys, int nsys, int max_slots, const float* d_q, cudaStream_t s);
+cudaError_t launch_batch_convert(const BatchSys* sys, const BatchMap& map, const float* d_x, cudaStream_t s);
+cudaError_t launch_batch_set_q(const BatchSys* sys, const BatchMap& map, const float* d_q, cudaStream_t s);
 cudaError_t launch_match_loss(const float* d_f, const float* d_ft, size_t n3, float* d_gF, double* d_loss,
                               int num_sms, cudaStream_t s);
 cudaError_t launch_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsigned* status, cudaStream_t s);
@@ -481,7 +493,7 @@ cudaError_t launch_batch_force_x2(const DeviceView& cv, const BatchSys* sys, con
                                   int num_sms, cudaStream_t s);
 cudaError_t optin_batch_force_x2_smem();
 cudaError_t launch_batch_compute(const DeviceView& cv, const BatchSys* sys, const int* prefix, int nsys,
-                                 int max_slots, int max_atoms, const float* d_x, float* d_f, double* sums,
+                                 const BatchMap& map, const float* d_x, float* d_f, double* sums,
                                  size_t sums_bytes, int* counter, double* d_e, double* d_vir, int variant,
                                  int num_sms, cudaStream_t s);
 
