@@ -368,6 +368,10 @@ void fft_plan_destroy(FftPlan3* p)
 
 cudaError_t fft_r2c_zy(const FftPlan3& p, const float* real, float2* cplx, cudaStream_t s)
 {
+    if (p.n[1] == p.n[2] && p.len[2] && p.len[2]->plane_r2c)
+    {
+        return p.len[2]->plane_r2c(p.ax[2].roots, real, cplx, p.n[0], s);
+    }
     cudaError_t e = z_pass(false, p, real, nullptr, cplx, s);
     if (e == cudaSuccess && p.n[1] > 1)
     {
@@ -388,6 +392,10 @@ cudaError_t fft_r2c(const FftPlan3& p, const float* real, float2* cplx, cudaStre
 
 cudaError_t fft_c2r_yz(const FftPlan3& p, float2* cplx, float* real, cudaStream_t s)
 {
+    if (p.n[1] == p.n[2] && p.len[2] && p.len[2]->plane_c2r)
+    {
+        return p.len[2]->plane_c2r(p.ax[2].roots, cplx, real, p.n[0], s);
+    }
     cudaError_t e = cudaSuccess;
     if (p.n[1] > 1)
     {

@@ -243,6 +243,9 @@ struct FftLen
     void (*strided)(bool inv, const float2* roots, float2* data, int nouter, int elem_stride, int outer_stride,
                     int nzc, cudaStream_t s);
     void (*x_solve)(const float2* roots, float2* cgrid, const PmeSolve& ps, cudaStream_t s);
+    // z and y of all nx planes of a grid with ny = nz = n; nullptr where a plane does not fit a block
+    cudaError_t (*plane_r2c)(const float2* roots, const float* real, float2* cplx, int nx, cudaStream_t s);
+    cudaError_t (*plane_c2r)(const float2* roots, const float2* cplx, float* real, int nx, cudaStream_t s);
 };
 
 // The passes of length n, or nullptr: then the runtime-length path above runs.

@@ -6,7 +6,8 @@
 // points q + R1 s in natural order.  One trip through shared memory per line instead of one per
 // radix-4/2/3/5 stage: the passes are bound by latency (the grids sit in L2), and a thread has all
 // its loads in flight at once.  96^3 / 120^3 grids, per pass: 7.5 / 8.4 us with a warp per line and
-// four or five Stockham stages, see the table in nbx_fft.cu for the passes now.
+// four or five Stockham stages, 4.6-5.0 / 5.7-6.8 us now (the x pass with the solve 7.6, with energies
+// 15.9 us at 120^3).
 //
 // The strided passes (y and x) take kCols consecutive z-frequencies of a line per block, thread
 // (j, c) with c fastest, so global rows of 64 bytes are read and written whole, without staging.
@@ -480,6 +481,251 @@ __global__ void __launch_bounds__(round32(kCols* Shape<R1, R2>::threads))
     }
 }
 
+// ---- z and y in one kernel: a block per x plane of a grid with ny = nz ----
+// The planes are small (96^2: 37 KB) and the passes bound by latency, so a plane stays in shared memory
+// between the z and the y transforms: one kernel and one trip through L2 instead of two.  Thread (p, j)
+// takes a line pair in the z part, thread (c, j) a column in the y part.  A convolution of 3 000 atoms
+// went from 24.1 to 20.5 us, of 288 000 atoms (120^3) from 86.6 to 82.6 us, 20 steps of dynamics of
+// 32 000 atoms from 1925 to 1836 us.  Taken up to 768 threads (n <= 120 but 112); longer lines need more
+// threads than a block has or leave it fewer than 80 registers a thread, and keep a pass per axis.
+template<int R1, int R2>
+struct Plane
+{
+    using S                      = Shape<R1, R2>;
+    static constexpr int n       = S::n;
+    static constexpr int nzc     = n / 2 + 1;
+    static constexpr int pairs   = (n + 1) / 2;
+    static constexpr int line    = R1 * S::row;  // exchange words of one line
+    static constexpr int threads = round32(nzc * S::threads);
+    static constexpr int words   = nzc * line > n * nzc ? nzc * line : n * nzc;  // pairs <= nzc
+    static constexpr bool fits   = threads <= 768;
+};
+
+template<int R1, int R2>
+__global__ void __launch_bounds__(Plane<R1, R2>::threads)
+        k_plane_r2c(const float2* __restrict__ roots, const float* __restrict__ real, float2* __restrict__ cplx)
+{
+    pdl_begin();
+    using S = Shape<R1, R2>;
+    using P = Plane<R1, R2>;
+    constexpr int n = P::n, nzc = P::nzc;
+    extern __shared__ float2 psm[];
+    {
+        const int     p  = threadIdx.x / S::threads, j = threadIdx.x - p * S::threads;
+        const bool    on = p < P::pairs, hb = 2 * p + 1 < n;
+        float2* const ln = psm + p * P::line;
+        if (on && j < R2)
+        {
+            const float* a = real + ((size_t)blockIdx.x * n + 2 * p) * n;
+            float2       v[R1];
+#pragma unroll
+            for (int r = 0; r < R1; r++)
+            {
+                v[r] = make_float2(a[j + R2 * r], hb ? a[n + j + R2 * r] : 0.0f);
+            }
+            dft<R1, false>(v);
+            twiddle<R1, false>(v, roots, j);
+#pragma unroll
+            for (int q = 0; q < R1; q++)
+            {
+                ln[q * S::row + j] = v[q];
+            }
+        }
+        __syncthreads();
+        float2 w[R2];
+        if (on && j < R1)
+        {
+#pragma unroll
+            for (int b = 0; b < R2; b++)
+            {
+                w[b] = ln[j * S::row + b];
+            }
+            dft<R2, false>(w);
+        }
+        __syncthreads();
+        if (on && j < R1)
+        {
+#pragma unroll
+            for (int s = 0; s < R2; s++)
+            {
+                ln[j + R1 * s] = w[s];
+            }
+        }
+        __syncthreads();
+    }
+    // column c (z-frequency) along y: the value of line y comes from the pair y / 2 (see k_z_r2c)
+    const int  j = threadIdx.x / nzc, c = threadIdx.x - j * nzc;
+    const bool in = j < R2, out = j < R1;
+    float2     v[R1];
+    if (in)
+    {
+#pragma unroll
+        for (int r = 0; r < R1; r++)
+        {
+            const int     y  = j + R2 * r;
+            const float2* z  = psm + (y >> 1) * P::line;
+            const float2  zk = z[c], zn = z[c == 0 ? 0 : n - c];
+            v[r] = (y & 1) ? make_float2(0.5f * (zk.y + zn.y), 0.5f * (zn.x - zk.x))
+                           : make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y));
+        }
+        dft<R1, false>(v);
+        twiddle<R1, false>(v, roots, j);
+    }
+    __syncthreads();
+    if (in)
+    {
+#pragma unroll
+        for (int q = 0; q < R1; q++)
+        {
+            psm[(q * S::row + j) * nzc + c] = v[q];
+        }
+    }
+    __syncthreads();
+    if (out)
+    {
+        float2 w[R2];
+#pragma unroll
+        for (int b = 0; b < R2; b++)
+        {
+            w[b] = psm[(j * S::row + b) * nzc + c];
+        }
+        dft<R2, false>(w);
+        float2* o = cplx + (size_t)blockIdx.x * n * nzc + c;
+#pragma unroll
+        for (int s = 0; s < R2; s++)
+        {
+            o[(j + R1 * s) * nzc] = w[s];
+        }
+    }
+}
+
+template<int R1, int R2>
+__global__ void __launch_bounds__(Plane<R1, R2>::threads)
+        k_plane_c2r(const float2* __restrict__ roots, const float2* __restrict__ cplx, float* __restrict__ real)
+{
+    pdl_begin();
+    using S = Shape<R1, R2>;
+    using P = Plane<R1, R2>;
+    constexpr int n = P::n, nzc = P::nzc;
+    extern __shared__ float2 psm[];
+    {
+        const int  j = threadIdx.x / nzc, c = threadIdx.x - j * nzc;
+        const bool in = j < R2, out = j < R1;
+        if (in)
+        {
+            const float2* a = cplx + (size_t)blockIdx.x * n * nzc + c;
+            float2        v[R1];
+#pragma unroll
+            for (int r = 0; r < R1; r++)
+            {
+                v[r] = a[(j + R2 * r) * nzc];
+            }
+            dft<R1, true>(v);
+            twiddle<R1, true>(v, roots, j);
+#pragma unroll
+            for (int q = 0; q < R1; q++)
+            {
+                psm[(q * S::row + j) * nzc + c] = v[q];
+            }
+        }
+        __syncthreads();
+        float2 w[R2];
+        if (out)
+        {
+#pragma unroll
+            for (int b = 0; b < R2; b++)
+            {
+                w[b] = psm[(j * S::row + b) * nzc + c];
+            }
+            dft<R2, true>(w);
+        }
+        __syncthreads();
+        if (out)
+        {
+#pragma unroll
+            for (int s = 0; s < R2; s++)
+            {
+                psm[(j + R1 * s) * nzc + c] = w[s];
+            }
+        }
+        __syncthreads();
+    }
+    // lines 2p and 2p + 1 along z (see k_z_c2r)
+    const int  p  = threadIdx.x / S::threads, j = threadIdx.x - p * S::threads;
+    const bool on = p < P::pairs, hb = 2 * p + 1 < n;
+    float2     v[R1];
+    if (on && j < R2)
+    {
+        const float2* a = psm + 2 * p * nzc;
+#pragma unroll
+        for (int r = 0; r < R1; r++)
+        {
+            const int    k  = j + R2 * r;
+            const int    kk = k < nzc ? k : n - k;
+            const float  sg = k >= nzc ? -1.0f : (k == 0 || 2 * k == n) ? 0.0f : 1.0f;
+            const float2 A  = a[kk], B = hb ? a[nzc + kk] : make_float2(0.0f, 0.0f);
+            v[r]            = make_float2(A.x - sg * B.y, fmaf(sg, A.y, B.x));
+        }
+        dft<R1, true>(v);
+        twiddle<R1, true>(v, roots, j);
+    }
+    __syncthreads();
+    float2* const ln = psm + p * P::line;
+    if (on && j < R2)
+    {
+#pragma unroll
+        for (int q = 0; q < R1; q++)
+        {
+            ln[q * S::row + j] = v[q];
+        }
+    }
+    __syncthreads();
+    if (on && j < R1)
+    {
+        float2 w[R2];
+#pragma unroll
+        for (int b = 0; b < R2; b++)
+        {
+            w[b] = ln[j * S::row + b];
+        }
+        dft<R2, true>(w);
+        float* a = real + ((size_t)blockIdx.x * n + 2 * p) * n;
+#pragma unroll
+        for (int s = 0; s < R2; s++)
+        {
+            a[j + R1 * s] = w[s].x;
+            if (hb)
+            {
+                a[n + j + R1 * s] = w[s].y;
+            }
+        }
+    }
+}
+
+template<int R1, int R2>
+cudaError_t launch_plane_r2c(const float2* roots, const float* real, float2* cplx, int nx, cudaStream_t s)
+{
+    constexpr size_t smem = sizeof(float2) * Plane<R1, R2>::words;
+    cudaError_t      e    = smem_optin<k_plane_r2c<R1, R2>>(smem, smem);
+    if (e == cudaSuccess)
+    {
+        e = launch_pdl(k_plane_r2c<R1, R2>, nx, Plane<R1, R2>::threads, smem, s, roots, real, cplx);
+    }
+    return e;
+}
+
+template<int R1, int R2>
+cudaError_t launch_plane_c2r(const float2* roots, const float2* cplx, float* real, int nx, cudaStream_t s)
+{
+    constexpr size_t smem = sizeof(float2) * Plane<R1, R2>::words;
+    cudaError_t      e    = smem_optin<k_plane_c2r<R1, R2>>(smem, smem);
+    if (e == cudaSuccess)
+    {
+        e = launch_pdl(k_plane_c2r<R1, R2>, nx, Plane<R1, R2>::threads, smem, s, roots, cplx, real);
+    }
+    return e;
+}
+
 template<int R1, int R2>
 void launch_z_r2c(const float2* roots, const float* real, float2* cplx, int nlines, cudaStream_t s)
 {
@@ -526,7 +772,14 @@ void launch_x_solve(const float2* roots, float2* cgrid, const PmeSolve& ps, cuda
 template<int R1, int R2>
 constexpr FftLen make_len()
 {
-    return { R1 * R2, launch_z_r2c<R1, R2>, launch_z_c2r<R1, R2>, launch_strided<R1, R2>, launch_x_solve<R1, R2> };
+    FftLen l = { R1 * R2, launch_z_r2c<R1, R2>, launch_z_c2r<R1, R2>, launch_strided<R1, R2>, launch_x_solve<R1, R2>,
+                 nullptr, nullptr };
+    if constexpr (Plane<R1, R2>::fits)
+    {
+        l.plane_r2c = launch_plane_r2c<R1, R2>;
+        l.plane_c2r = launch_plane_c2r<R1, R2>;
+    }
+    return l;
 }
 
 } // namespace fftr

@@ -10,6 +10,6 @@ extern const FftLen kFftLen0[] = {
     fftr::make_len<10, 16>(),
     fftr::make_len<12, 14>(),
     fftr::make_len<5, 5>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

@@ -9,6 +9,6 @@ extern const FftLen kFftLen1[] = {
     fftr::make_len<10, 10>(),
     fftr::make_len<12, 12>(),
     fftr::make_len<14, 16>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

@@ -10,6 +10,6 @@ extern const FftLen kFftLen2[] = {
     fftr::make_len<12, 16>(),
     fftr::make_len<6, 6>(),
     fftr::make_len<4, 11>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

@@ -10,6 +10,6 @@ extern const FftLen kFftLen3[] = {
     fftr::make_len<15, 16>(),
     fftr::make_len<5, 8>(),
     fftr::make_len<6, 7>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

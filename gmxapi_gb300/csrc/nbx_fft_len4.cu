@@ -9,6 +9,6 @@ extern const FftLen kFftLen4[] = {
     fftr::make_len<8, 14>(),
     fftr::make_len<16, 16>(),
     fftr::make_len<4, 13>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

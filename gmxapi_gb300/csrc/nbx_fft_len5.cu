@@ -8,6 +8,6 @@ extern const FftLen kFftLen5[] = {
     fftr::make_len<9, 10>(),
     fftr::make_len<10, 12>(),
     fftr::make_len<8, 16>(),
-    { 0, nullptr, nullptr, nullptr, nullptr },
+    { 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr },
 };
 } // namespace nbx

@@ -117,3 +117,17 @@ def test_unsupported_grid_is_an_input_error():
     for grid in ((257, 16, 16), (16, 1031, 16), (0, 8, 8)):
         with pytest.raises(Exception, match="prime factors|null"):
             pme.Fft3d(grid)
+
+
+# square planes take z and y in one kernel: every length that has one, odd ones and uneven x among them
+@pytest.mark.parametrize("n", [20, 24, 25, 28, 32, 36, 40, 42, 44, 48, 52, 56, 60, 64, 72, 80, 84, 90, 96, 100, 104,
+                               108, 112, 120, 128])
+def test_square_planes_match_fp64_numpy(n):
+    grid = (3, n, n)
+    rng = np.random.default_rng(n)
+    p = _fft(grid)
+    x = rng.standard_normal(grid).astype(np.float32)
+    _check(_forward(p, grid, x), np.fft.rfftn(x.astype(np.float64)))
+    c = np.fft.rfftn(rng.standard_normal(grid))
+    _check(_backward(p, grid, c), np.fft.irfftn(c, s=grid, axes=(0, 1, 2)) * np.prod(grid))
+    p.close()
