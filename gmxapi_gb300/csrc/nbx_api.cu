@@ -1089,10 +1089,31 @@ int nbx_md_step_device(nbx_handle* h, long long step, const float* d_x, float* d
     {
         return NBX_ERR_INVALID_INPUT;
     }
+    bool      searched = false;
+    const int rc       = nbx::md_lists(h, step, d_x, &searched);
+    return rc == NBX_OK ? compute_async(h, d_x, d_f, d_e, d_vir) : rc;
+}
+
+} // extern "C"
+
+namespace nbx
+{
+
+int md_forces(nbx_handle* h, const float* d_x, float* d_f, double* d_e, int force_grid)
+{
+    h->v.force_grid = force_grid;
+    const int rc    = compute_async(h, d_x, d_f, d_e, nullptr);
+    h->v.force_grid = 0;
+    return rc;
+}
+
+int md_lists(nbx_handle* h, long long step, const float* d_x, bool* searched)
+{
     cudaSetDevice(h->device);
     const int nstlist = std::max(1, h->opts.nstlist);
     int       rc      = NBX_OK;
-    if (!h->have_list || step % nstlist == 0)
+    *searched         = !h->have_list || step % nstlist == 0;
+    if (*searched)
     {
         // the search grids the atoms put in the box (mdlib/sim_util.cpp:1316); their
         // box shifts are kept for the coordinate conversion until the next search
@@ -1120,8 +1141,12 @@ int nbx_md_step_device(nbx_handle* h, long long step, const float* d_x, float* d
             }
         }
     }
-    return compute_async(h, d_x, d_f, d_e, d_vir);
+    return NBX_OK;
 }
+
+} // namespace nbx
+
+extern "C" {
 
 int nbx_md_step(nbx_handle* h, long long step, const float* x, float* f, double* energies, double* virial)
 {

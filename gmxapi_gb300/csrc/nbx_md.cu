@@ -156,6 +156,9 @@ struct nbx_leapfrog
     int          num_sms    = 1;
     cudaStream_t stream     = nullptr;
     bool         own_stream = false;
+    cudaStream_t side       = nullptr;  // mesh part of a step, beside the short-range forces
+    cudaEvent_t  x_ready    = nullptr;  // coordinates of the step
+    cudaEvent_t  potential  = nullptr;  // mesh potential of the step
     float        box[3]     = { 0, 0, 0 };
     float*       inv_mass   = nullptr;  // [N]
     double*      partials   = nullptr;  // [blocks]
@@ -251,6 +254,9 @@ int nbx_leapfrog_create(int num_atoms, const float* inv_mass, const float* box, 
     cudaError_t e = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     p->own_stream = e == cudaSuccess;
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->x_ready, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->potential, cudaEventDisableTiming);
     const size_t bytes = sizeof(float) * std::max(1, num_atoms);
     if (e == cudaSuccess) e = cudaMalloc(&p->inv_mass, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&p->partials, sizeof(double) * kLfBlocksPerSm * p->num_sms);
@@ -287,6 +293,18 @@ int nbx_leapfrog_destroy(nbx_leapfrog* p)
     if (p->own_stream)
     {
         cudaStreamDestroy(p->stream);
+    }
+    if (p->side)
+    {
+        cudaStreamDestroy(p->side);
+    }
+    if (p->x_ready)
+    {
+        cudaEventDestroy(p->x_ready);
+    }
+    if (p->potential)
+    {
+        cudaEventDestroy(p->potential);
     }
     delete p;
     return NBX_OK;
@@ -372,7 +390,7 @@ int nbx_md_run_device(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long f
     {
         return md_error(lf, NBX_ERR_INVALID_INPUT, "null argument, negative step count or bad nstcalcenergy");
     }
-    // one stream for the whole step: the nonbonded handle's
+    // the nonbonded handle's stream for the whole step; step_with_mesh branches off it and joins again
     void* s  = nbx_get_stream(h);
     int   rc = nbx_leapfrog_set_stream(lf, s);
     if (rc == NBX_OK && pme)
@@ -417,26 +435,71 @@ int nbx_md_run_device(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long f
 namespace
 {
 
+// Up to this many atoms the force kernel beside a mesh part leaves a quarter of its block slots free: the mesh
+// kernels are as long as it and bound by latency.  20 steps of 10 976 / 32 000 / 55 296 / 87 808 / 364 500 atoms:
+// 1142 / 1601 / 2017 / 2750 / 10097 us so, 1139 / 1663 / 2116 / 2665 / 9672 us with all of its blocks.
+constexpr int kSharedSmAtoms = 65536;
+
+// Forces of one step with PME: the mesh potential (spread, transforms, solve) on the side stream beside the
+// short-range forces, then the mesh forces added to them.  One after the other, 20 steps took 1496 / 1865 / 2335 us
+// at 10 976 / 32 000 / 55 296 atoms and 10034 us at 364 500 atoms.
+int step_with_mesh(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long step, float* d_x, float* d_f,
+                   const float* d_q, double* row, int natoms, cudaStream_t main)
+{
+    double*     e_rec    = row ? row + 2 : nullptr;
+    bool        searched = false;
+    cudaError_t e        = cudaEventRecord(lf->x_ready, main);
+    int         rc       = nbx::md_lists(h, step, d_x, &searched);
+    if (rc != NBX_OK)
+    {
+        return rc;
+    }
+    // a search puts the atoms in the box: the mesh part starts after it
+    if (e == cudaSuccess && searched) e = cudaEventRecord(lf->x_ready, main);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(lf->side, lf->x_ready, 0);
+    if (e == cudaSuccess)
+    {
+        rc = nbx::pme_potential(pme, natoms, d_x, d_q, e_rec, nullptr, lf->side);
+        e  = cudaEventRecord(lf->potential, lf->side);
+    }
+    if (e == cudaSuccess && rc == NBX_OK)
+    {
+        rc = nbx::md_forces(h, d_x, d_f, row, natoms <= kSharedSmAtoms ? lf->num_sms * 3 / 2 : 0);
+    }
+    // the side stream joins also when something failed
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(main, lf->potential, 0);
+    if (e != cudaSuccess)
+    {
+        return md_error(lf, NBX_ERR_CUDA, cudaGetErrorString(e));
+    }
+    return rc == NBX_OK ? nbx::pme_forces(pme, natoms, d_x, d_q, d_f, e_rec, nullptr) : rc;
+}
+
 int run_steps(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long first_step, int num_steps, float dt,
               float* d_x, float* d_v, float* d_f, const float* d_q, int nstcalcenergy, double* d_energies,
               int nstlist, int natoms, void* s)
 {
-    int rc = NBX_OK;
+    int                rc   = NBX_OK;
+    const cudaStream_t main = static_cast<cudaStream_t>(s);
     for (int k = 0; k < num_steps; k++)
     {
         const long long step   = first_step + k;
         const bool      energy = d_energies && (step - first_step) % nstcalcenergy == 0;
         double*         row    = energy ? d_energies + 4 * ((step - first_step) / nstcalcenergy) : nullptr;
         // row: {E_LJ, E_Coulomb real space (incl. self and exclusion corrections), E_Coulomb reciprocal, E_kin}
-        if ((rc = nbx_md_step_device(h, step, d_x, d_f, row, nullptr)) != NBX_OK)
+        if (!pme)
+        {
+            rc = nbx_md_step_device(h, step, d_x, d_f, row, nullptr);
+        }
+        else
+        {
+            rc = step_with_mesh(h, pme, lf, step, d_x, d_f, d_q, row, natoms, main);
+        }
+        if (rc != NBX_OK)
         {
             return rc;
         }
-        if (pme && (rc = nbx_pme_compute_device(pme, natoms, d_x, d_q, d_f, row ? row + 2 : nullptr, nullptr)) != NBX_OK)
-        {
-            return rc;
-        }
-        if (row && !pme && cudaMemsetAsync(row + 2, 0, sizeof(double), static_cast<cudaStream_t>(s)) != cudaSuccess)
+        if (row && !pme && cudaMemsetAsync(row + 2, 0, sizeof(double), main) != cudaSuccess)
         {
             return md_error(lf, NBX_ERR_CUDA, "energy row");
         }

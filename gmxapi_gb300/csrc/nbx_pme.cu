@@ -858,6 +858,7 @@ struct nbx_pme
     Bricks bricks{};
     int    brick_atoms = 0;      // atoms the filing arrays are sized for
     bool   filed       = false;  // atoms are filed and the counts not yet cleared by a gather
+    bool   by_bricks   = false;  // the last pme_potential went by bricks, and so does its gather
     std::string  err;
 };
 
@@ -1454,17 +1455,27 @@ int nbx_pme_compute_device(nbx_pme* p, int natoms, const float* d_x, const float
     {
         return pme_error(p, NBX_ERR_INVALID_INPUT, "null argument or negative atom count");
     }
+    const int rc = nbx::pme_potential(p, natoms, d_x, d_q, d_energy, d_virial, p->stream);
+    return rc == NBX_OK ? nbx::pme_forces(p, natoms, d_x, d_q, d_f, d_energy, d_virial) : rc;
+}
+
+} // extern "C"
+
+namespace nbx
+{
+
+int pme_potential(nbx_pme* p, int natoms, const float* d_x, const float* d_q, double* d_energy, double* d_virial,
+                  cudaStream_t s)
+{
     cudaSetDevice(p->device);
-    const bool  bricks = use_bricks(p, natoms) && ensure_bricks(p, natoms);
-    cudaError_t e      = bricks ? launch_spread_bricks(p, natoms, d_x, d_q, p->grid)
-                                : launch_spread(p, natoms, d_x, d_q, p->grid);
-    PmeTotals tot = { nullptr, nullptr, nullptr };
+    const cudaStream_t keep = p->stream;
+    p->stream               = s;
+    const bool  bricks      = use_bricks(p, natoms) && ensure_bricks(p, natoms);
+    cudaError_t e           = bricks ? launch_spread_bricks(p, natoms, d_x, d_q, p->grid)
+                                     : launch_spread(p, natoms, d_x, d_q, p->grid);
+    p->by_bricks            = bricks;
     if (fused_x_solve(p))
     {
-        if (d_energy || d_virial)
-        {
-            tot = { p->sums, d_energy, d_virial };
-        }
         // z and y forward, then x forward + solve + x backward in one pass, then y and z backward
         if (e == cudaSuccess) e = nbx::fft_r2c_zy(p->fft, p->grid, p->cgrid, p->stream);
         if (e == cudaSuccess) e = launch_x_solve(p, d_energy, d_virial);
@@ -1476,13 +1487,25 @@ int nbx_pme_compute_device(nbx_pme* p, int natoms, const float* d_x, const float
         if (e == cudaSuccess) e = launch_solve(p, p->cgrid, d_energy, d_virial);
         if (e == cudaSuccess) e = nbx::fft_c2r(p->fft, p->cgrid, p->grid, p->stream);
     }
-    if (e == cudaSuccess)
-    {
-        e = bricks ? launch_gather_bricks(p, d_x, d_q, p->grid, d_f, tot)
-                   : launch_gather(p, natoms, d_x, d_q, p->grid, d_f, tot);
-    }
+    p->stream = keep;
     return cuda_status(p, e);
 }
+
+int pme_forces(nbx_pme* p, int natoms, const float* d_x, const float* d_q, float* d_f, double* d_energy,
+               double* d_virial)
+{
+    PmeTotals tot = { nullptr, nullptr, nullptr };
+    if (fused_x_solve(p) && (d_energy || d_virial))
+    {
+        tot = { p->sums, d_energy, d_virial };
+    }
+    return cuda_status(p, p->by_bricks ? launch_gather_bricks(p, d_x, d_q, p->grid, d_f, tot)
+                                       : launch_gather(p, natoms, d_x, d_q, p->grid, d_f, tot));
+}
+
+} // namespace nbx
+
+extern "C" {
 
 int nbx_pme_synchronize(nbx_pme* p)
 {

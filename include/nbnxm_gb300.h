@@ -467,7 +467,9 @@ int nbx_leapfrog_integrate_device(nbx_leapfrog* p, float dt, float* d_x, float* 
  * nonbonded forces with the handle's search / rolling-prune schedule (nbx_md_step_device)
  * written to d_f (overwriting, whatever nbx_set_force_accumulate says), PME forces added when
  * pme is not NULL (charges d_q[N]), leap-frog update of d_x / d_v;
- * atoms are put in the box only on the update before a search step.  All on h's stream.
+ * atoms are put in the box only on the update before a search step.  All on h's stream, but the
+ * grid part of PME: it runs beside the nonbonded forces on a stream of lf's that leaves h's stream and
+ * joins it again within each step.
  * Every nstcalcenergy steps (counted from first_step) a row of d_energies receives
  * {E_LJ, E_Coulomb real space, E_Coulomb reciprocal, E_kin} (FP64; E_kin as in
  * nbx_leapfrog_integrate_device); d_energies may be NULL. */

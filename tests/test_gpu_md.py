@@ -146,6 +146,38 @@ def test_md_run_matches_oracle(md, with_pme, prune):
     run.close()
 
 
+@pytest.mark.parametrize("cells", [6, 9, 26])
+def test_md_run_forces_match_separate_calls(md, cells):
+    """Steps of length zero with the mesh part beside the short-range forces (fewer force blocks up to 65,536 atoms,
+    all of them beyond) leave the forces and energies that the two parts give on their own, on one stream.  The
+    forces are the same sums with float atomics in another order (1e-6 as for the accumulated forces above)."""
+    import torch
+
+    from gmxapi_gb300 import nblib, systems
+
+    s = systems.lj_fcc(cells=cells, lattice=0.5256, charge=0.3, seed=21)
+    rng = np.random.default_rng(4)
+    s.x = (s.x + rng.uniform(-0.02, 0.02, s.x.shape)).astype(np.float32) % np.asarray(s.box, np.float32)
+    masses = np.full(s.n, systems.ARGON_MASS, np.float32)
+    opts = nblib.NBKernelOptions(pairlist_cutoff=1.0, rcoulomb=0.9, nstlist=10, compute_virial_and_energy=True,
+                                 rlist_inner=0.92, nstlist_prune=4)
+    run = md.MdRunner(s, masses, opts, dt=0.0)
+    rows = run.run(13, nstcalcenergy=6)
+    f = run.f.cpu().numpy()
+    ref = md.MdRunner(s, masses, opts, dt=0.0)
+    e = torch.zeros(3, dtype=torch.float64, device="cuda")
+    ref.pme.set_stream(ref.stream.cuda_stream)
+    ref.calc.md_step_device(0, ref.x.data_ptr(), ref.f.data_ptr(), e.data_ptr(), None)
+    ref.pme.compute_device(s.n, ref.x.data_ptr(), ref.q.data_ptr(), ref.f.data_ptr(), e[2:].data_ptr(), None)
+    torch.cuda.synchronize()
+    assert rel_rms(f, ref.f.cpu().numpy()) <= 1e-6
+    assert rows.shape == (3, 4)
+    for row in rows:
+        np.testing.assert_allclose(row[:3], e.cpu().numpy(), rtol=1e-6)
+    run.close()
+    ref.close()
+
+
 def test_md_nve_energy_drift(md):
     """2,000 steps (4 ps) of NVE argon-like atoms with charges (LJ + Ewald + PME), started from
     the lattice at 120 K: total-energy drift bounded."""
