@@ -6,17 +6,16 @@
 // boundingbox_only_distance2 (:2841-2878), setSelfAndNewtonExclusionsGpu
 // (:880-904) and setExclusionsForIEntry for GPU lists (:1874-1972).
 //
-// Count pass: one warp per i-cell (super-cluster) walks the shifts in the
-// reference's order with the same single-precision arithmetic (this file is
-// compiled with --fmad=false).  For each shift the lanes find the z-ranges of
-// cells of up to 32 candidate j-columns at once; the warp then takes the flat,
-// increasing sequence of j-cells four at a time, lane (cell, j-cluster)
-// testing its j-cluster's bounding box against the 8 i-clusters.  The j-clusters
-// found are stored as per-cell records (index, 8-bit i-cluster mask) with one
-// code per entry, and the cell's entry / cj4 counts are written.  After a
-// prefix sum of the counts, the emit pass (one warp per list entry) turns the
-// records into sci / cj4 entries at fixed offsets, with the outer masks and
-// per-group pair counts, and sets the diagonal and topology exclusion masks.
+// Count pass: one block per i-cell (super-cluster), with the reference's single-precision
+// arithmetic (this file is compiled with --fmad=false).  Its shifts, a lane each, give the
+// candidate columns; a thread per column finds its z-range of j-cells; the flat sequence of
+// j-cells, in the reference's order, goes through shared memory a window at a time: a warp
+// tests four of them at once, lane (cell, j-cluster) its j-cluster's bounding box against the
+// 8 i-clusters.  The j-clusters found are stored as per-cell records (index, 8-bit i-cluster
+// mask) in order, with one code per entry, and the cell's entry / cj4 counts are written.  After
+// a prefix sum of the counts, the emit pass (one warp per list entry) turns the records into
+// sci / cj4 entries at fixed offsets, with the outer masks and per-group pair counts, and sets
+// the diagonal and topology exclusion masks.
 #include "nbx_internal.cuh"
 
 #include <cstddef>
@@ -39,11 +38,6 @@ __device__ __forceinline__ float sq(float x)
     return x * x;
 }
 
-__device__ __forceinline__ int xyz2is(int x, int y, int z)
-{
-    return 5 * (3 * (z + 1) + y + 1) + x + 2;
-}
-
 // get_cell_range (pairlist.cpp:286-309), lower corner 0.
 __device__ void get_cell_range(float b0, float b1, int numCells, float cellSize, float invCellSize, float d2,
                                float rlist, int* cf, int* cl)
@@ -64,92 +58,129 @@ __device__ void get_cell_range(float b0, float b1, int numCells, float cellSize,
     *cl = l;
 }
 
-// clusterBoundingBoxDistance2 (pairlist.cpp:351-372)
-__device__ __forceinline__ float bb_dist2(const float4 ilo, const float4 ihi, const float4 jlo, const float4 jhi)
+__device__ __forceinline__ float max3(float a, float b, float c)
 {
-    float dl  = ilo.x - jhi.x;
-    float dh  = jlo.x - ihi.x;
-    float dm  = fmaxf(dl, dh);
-    float dm0 = fmaxf(dm, 0.0f);
-    float d2  = dm0 * dm0;
-    dl        = ilo.y - jhi.y;
-    dh        = jlo.y - ihi.y;
-    dm        = fmaxf(dl, dh);
-    dm0       = fmaxf(dm, 0.0f);
-    d2        = d2 + dm0 * dm0;
-    dl        = ilo.z - jhi.z;
-    dh        = jlo.z - ihi.z;
-    dm        = fmaxf(dl, dh);
-    dm0       = fmaxf(dm, 0.0f);
-    d2        = d2 + dm0 * dm0;
-    return d2;
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Every operation rounded: packed products and sums would be contracted into fused multiply-adds
+// whatever the compiler is told, so these are scalar.
+__device__ __forceinline__ float norm2(float dx, float dy, float dz)
+{
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+
+// clusterBoundingBoxDistance2 (pairlist.cpp:351-372) of i-clusters i and i + 1 to one j-cluster, both
+// differences of a dimension in packed arithmetic (the same roundings).
+// x, y: {lower x, -upper x, lower y, -upper y}, z: {lower z, -upper z} of both; jx, jy, jz: {-upper, lower}.
+__device__ __forceinline__ float2 bb_dist2(const float4 xy0, const float4 xy1, const float4 z, const float2 jx,
+                                           const float2 jy, const float2 jz)
+{
+    const float2 x0 = __fadd2_rn(make_float2(xy0.x, xy0.y), jx), x1 = __fadd2_rn(make_float2(xy1.x, xy1.y), jx);
+    const float2 y0 = __fadd2_rn(make_float2(xy0.z, xy0.w), jy), y1 = __fadd2_rn(make_float2(xy1.z, xy1.w), jy);
+    const float2 z0 = __fadd2_rn(make_float2(z.x, z.y), jz), z1 = __fadd2_rn(make_float2(z.z, z.w), jz);
+    return make_float2(norm2(max3(x0.x, x0.y, 0.0f), max3(y0.x, y0.y, 0.0f), max3(z0.x, z0.y, 0.0f)),
+                       norm2(max3(x1.x, x1.y, 0.0f), max3(y1.x, y1.y, 0.0f), max3(z1.x, z1.y, 0.0f)));
 }
 
 constexpr int kEmitStage = 512;  // j-lists up to this length are staged in shared memory for the
                                  // exclusion lookups
 
-struct CountSmem
+constexpr int kShiftSlots   = kCentral + 1;  // shifts 0 .. central, the visiting order
+constexpr int kManyCells    = 4096;          // i-cells from which a cell takes two warps
+constexpr int kCellWindow   = 128;           // candidate j-cells in shared memory at a time
+static_assert(kShiftSlots <= kMaxEntriesPerCell && kShiftSlots <= 32, "one lane and one entry code per shift");
+
+// The i-cell under one shift: its bounds, the candidate columns (cx major) and their first number
+// among the columns of all shifts.
+struct ShiftRange
 {
-    float4 bbc_lo[kNcl], bbc_hi[kNcl];  // the i-cell's cluster bounding boxes
-    float4 bbi_lo[kNcl], bbi_hi[kNcl];  // and shifted for the current entry
+    float bx0, bx1, by0, by1, bz0, bz1;
+    float d2z, bz1_frac;
+    float shx, shy, shz;
+    int   cxf, cyf, ny;
 };
 
-__global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) k_search_count(DeviceView v)
+struct CountSmem
 {
-    pdl_begin();
-    __shared__ CountSmem wsm[kWarpsPerBlock];
-    const int           lane = threadIdx.x & 31;
-    const int           wib  = threadIdx.x >> 5;
-    CountSmem&          sm   = wsm[wib];
-    const int           ci   = blockIdx.x * kWarpsPerBlock + wib;
-    const int           numCells = v.hdr->num_cells;
-    if (ci >= numCells)
+    float4        bbi_xy[kShiftSlots][kNcl];  // shifted cluster bounding boxes: {lower, -upper} of x and y
+    float2        bbi_z[kShiftSlots][kNcl];   // and of z
+    uint2         masks[kCellWindow];                                    // i-cluster masks of the 8 j-clusters
+    int           cell[kCellWindow];                                     // candidate j-cells
+    unsigned char cell_shift[kCellWindow];
+    ShiftRange    sr[kShiftSlots];
+    int           col0[32];  // first column of each shift
+    int           nj[32];    // j-clusters found per shift
+    int           warp_sum[2][4];
+    int           ncols, ci_x, ci_y, pairs;
+    unsigned      active;  // shifts with candidate columns
+    int2          flag[4][32];  // per warp: {j-cluster, shift * 8 + i-cluster} to check by atoms
+};
+
+// Inclusive prefix sum over the block; *total receives the sum of all threads.
+template<int kWarps>
+__device__ __forceinline__ int block_scan(int x, int* warp_sum, int* total)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int       incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
     {
-        return;
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+        {
+            incl += t;
+        }
     }
+    if (lane == 31)
+    {
+        warp_sum[warp] = incl;
+    }
+    __syncthreads();
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++)
+    {
+        incl += w < warp ? warp_sum[w] : 0;
+        sum += warp_sum[w];
+    }
+    *total = sum;
+    return incl;
+}
+
+// The shifts of i-cell ci, lane = shift (one warp): their ranges of candidate columns.
+__device__ __forceinline__ void shift_ranges(const DeviceView& v, int ci, CountSmem& sm)
+{
     const unsigned full = 0xffffffffu;
-    // column of this cell (next_ci, pairlist.cpp:2808-2836)
-    int lo = 0, hi = v.g.ncol - 1;
-    while (lo < hi)
+    const int      lane = threadIdx.x & 31;
+    const float*   box  = v.g.box;
+    const float    rlist = v.rlist, rlist2 = v.rlist2;
+    const float2   bbcz_i = v.bbcz[ci];
+    // column of this cell (next_ci, pairlist.cpp:2808-2836): the last that starts at or before it; the
+    // window shrinks 32-fold per step
+    int ci_xy = 0;
+    for (int len = v.g.ncol; len > 1;)
     {
-        const int mid = (lo + hi + 1) >> 1;
-        if (v.cxy_ind[mid] <= ci)
-        {
-            lo = mid;
-        }
-        else
-        {
-            hi = mid - 1;
-        }
+        const int  step = (len + 31) / 32;
+        const int  c    = ci_xy + lane * step;
+        const bool le   = c < ci_xy + len && v.cxy_ind[c] <= ci;
+        const int  lo   = ci_xy + (__popc(__ballot_sync(full, le)) - 1) * step;
+        len             = min(step, ci_xy + len - lo);
+        ci_xy           = lo;
     }
-    const int   ci_xy = lo;
-    const int   ci_x  = ci_xy / v.g.ncy;
-    const int   ci_y  = ci_xy - ci_x * v.g.ncy;
-    const float rlist = v.rlist, rlist2 = v.rlist2, rbb2 = v.rbb2;
-    const float listRangeBBToJCell2 = rlist * rlist;
-    const float* box  = v.g.box;
-    const float2 bbcz_i = v.bbcz[ci];
-    const int    ncl_i  = v.nclusters[ci];
-    // the cell's i-cluster bounding boxes, shifted per entry below
-    if (lane < kNcl)
+    const int ci_x = ci_xy / v.g.ncy;
+    const int ci_y = ci_xy - ci_x * v.g.ncy;
+    const int shp_x = (box[0] < rlist) ? 2 : 1;
+    const int tz = lane / 15 - 1, ty = lane / 5 % 3 - 1, tx = lane % 5 - 2;
+    int       ncol = 0;
+    if (lane < kShiftSlots && abs(tx) <= shp_x)
     {
-        sm.bbc_lo[lane] = v.bb[2 * (ci * kNcl + lane)];
-        sm.bbc_hi[lane] = v.bb[2 * (ci * kNcl + lane) + 1];
-    }
-    int          shp_x  = (box[0] < rlist) ? 2 : 1;
-
-    int            num_entries = 0, num_cj4 = 0;
-    int            rec_n = 0;   // records of this cell so far
-    unsigned       pairs = 0u;  // cluster pairs found by this lane
-    int* const           rec_cj = v.rec_cj + (size_t)ci * v.rec_cap;
-    unsigned char* const rec_m  = v.rec_m + (size_t)ci * v.rec_cap;
-
-    const float d2cx = 0.0f;
-    for (int tz = -1; tz <= 1; tz++)
-    {
-        const float shz = (float)tz * box[2];
-        const float bz0 = bbcz_i.x + shz;
-        const float bz1 = bbcz_i.y + shz;
+        const float d2cx = 0.0f;
+        const float shz  = (float)tz * box[2];
+        const float bz0  = bbcz_i.x + shz;
+        const float bz1  = bbcz_i.y + shz;
         float       d2z;
         if (tz == 0)
         {
@@ -164,26 +195,18 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) k_search_count(DeviceV
             d2z = sq(bz0 - box[2]);
         }
         const float d2z_cx = d2z + d2cx;
-        if (d2z_cx >= rlist2)
+        if (!(d2z_cx >= rlist2))
         {
-            continue;
-        }
-        float bz1_frac = bz1 / (float)(v.cxy_ind[ci_xy + 1] - v.cxy_ind[ci_xy]);
-        if (bz1_frac < 0.0f)
-        {
-            bz1_frac = 0.0f;
-        }
-        for (int ty = -1; ty <= 1; ty++)
-        {
+            float bz1_frac = bz1 / (float)(v.cxy_ind[ci_xy + 1] - v.cxy_ind[ci_xy]);
+            if (bz1_frac < 0.0f)
+            {
+                bz1_frac = 0.0f;
+            }
             const float shy = (float)ty * box[1] + (float)tz * 0.0f;
             const float by0 = 0.0f + (float)ci_y * v.g.cs[1] + shy;
             const float by1 = 0.0f + ((float)ci_y + 1.0f) * v.g.cs[1] + shy;
             int         cyf, cyl;
             get_cell_range(by0, by1, v.g.ncy, v.g.cs[1], v.g.ics[1], d2z_cx, rlist, &cyf, &cyl);
-            if (cyf > cyl)
-            {
-                continue;
-            }
             float d2z_cy = d2z;
             if (by1 < 0.0f)
             {
@@ -193,271 +216,392 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) k_search_count(DeviceV
             {
                 d2z_cy = d2z_cy + sq(by0 - box[1]);
             }
-            for (int tx = -shp_x; tx <= shp_x; tx++)
+            const float shx = (float)tx * box[0] + (float)ty * 0.0f + (float)tz * 0.0f;
+            const float bx0 = 0.0f + (float)ci_x * v.g.cs[0] + shx;
+            const float bx1 = 0.0f + ((float)ci_x + 1.0f) * v.g.cs[0] + shx;
+            int         cxf = 0, cxl = -1;
+            if (cyf <= cyl)
             {
-                const int shift = xyz2is(tx, ty, tz);
-                if (shift > kCentral)
-                {
-                    continue;  // c_pbcShiftBackward (pairlist.cpp:94)
-                }
-                const bool  excludeSubDiagonal = (shift == kCentral);
-                const float shx = (float)tx * box[0] + (float)ty * 0.0f + (float)tz * 0.0f;
-                const float bx0 = 0.0f + (float)ci_x * v.g.cs[0] + shx;
-                const float bx1 = 0.0f + ((float)ci_x + 1.0f) * v.g.cs[0] + shx;
-                int         cxf, cxl;
                 get_cell_range(bx0, bx1, v.g.ncx, v.g.cs[0], v.g.ics[0], d2z_cy, rlist, &cxf, &cxl);
-                if (cxf > cxl)
-                {
-                    continue;
-                }
-                if (excludeSubDiagonal && cxf < ci_x)
+            }
+            if (cxf <= cxl)
+            {
+                if (lane == kCentral && cxf < ci_x)
                 {
                     cxf = ci_x;
                 }
-                // shifted i-cluster bounding boxes (set_icell_bb, pairlist.cpp:2260-2303)
-                __syncwarp();
-                if (lane < kNcl)
-                {
-                    const float4 l  = sm.bbc_lo[lane];
-                    const float4 h  = sm.bbc_hi[lane];
-                    sm.bbi_lo[lane] = make_float4(l.x + shx, l.y + shy, l.z + shz, 0.0f);
-                    sm.bbi_hi[lane] = make_float4(h.x + shx, h.y + shy, h.z + shz, 0.0f);
-                }
-                __syncwarp();
-                int nj = 0;  // j-clusters in this entry
-                // The candidate j-columns (cx major, cy minor, the reference's visiting order), 32
-                // at a time: each lane finds the z-range of cells of one column, a warp scan turns
-                // the cell counts into offsets of one flat, increasing sequence of j-cells.
-                const int ny   = cyl - cyf + 1;
-                const int ncol = (cxl - cxf + 1) * ny;
-                for (int c0 = 0; c0 < ncol; c0 += 32)
-                {
-                    int       first = 0, count = 0;
-                    const int c     = c0 + lane;
-                    if (c < ncol)
-                    {
-                        const int   cx      = cxf + c / ny;
-                        const int   cy      = cyf + c % ny;
-                        const float cx_real = (float)cx;
-                        float       d2zx    = d2z;
-                        if (0.0f + cx_real * v.g.cs[0] > bx1)
-                        {
-                            d2zx = d2zx + sq(0.0f + cx_real * v.g.cs[0] - bx1);
-                        }
-                        else if (0.0f + (cx_real + 1.0f) * v.g.cs[0] < bx0)
-                        {
-                            d2zx = d2zx + sq(0.0f + (cx_real + 1.0f) * v.g.cs[0] - bx0);
-                        }
-                        const int cyf_x = (cx == 0 && shift == kCentral && cyf < ci_y) ? ci_y : cyf;
-                        const int columnStart = v.cxy_ind[cx * v.g.ncy + cy];
-                        const int columnEnd   = v.cxy_ind[cx * v.g.ncy + cy + 1];
-                        // the column's cell z-bounds into L1 ahead of the walks below
-                        for (int c = columnStart; c < columnEnd; c += 16)
-                        {
-                            asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(v.bbcz + c)));
-                        }
-                        const float cy_real   = (float)cy;
-                        float       d2zxy     = d2zx;
-                        if (0.0f + cy_real * v.g.cs[1] > by1)
-                        {
-                            d2zxy = d2zxy + sq(0.0f + cy_real * v.g.cs[1] - by1);
-                        }
-                        else if (0.0f + (cy_real + 1.0f) * v.g.cs[1] < by0)
-                        {
-                            d2zxy = d2zxy + sq(0.0f + (cy_real + 1.0f) * v.g.cs[1] - by0);
-                        }
-                        if (cy >= cyf_x && columnStart < columnEnd && d2zxy < listRangeBBToJCell2)
-                        {
-                            int midCell = columnStart + (int)(bz1_frac * (float)(columnEnd - columnStart));
-                            if (midCell >= columnEnd)
-                            {
-                                midCell = columnEnd - 1;
-                            }
-                            const float d2xy = d2zxy - d2z;
-                            int         down = midCell;
-                            while (down >= columnStart)
-                            {
-                                const float u = v.bbcz[down].y;
-                                if (!(u >= bz0 || d2xy + sq(u - bz0) < rlist2))
-                                {
-                                    break;
-                                }
-                                down--;
-                            }
-                            int firstCell = down + 1;
-                            int up        = midCell + 1;
-                            while (up < columnEnd)
-                            {
-                                const float l = v.bbcz[up].x;
-                                if (!(l <= bz1 || d2xy + sq(l - bz1) < rlist2))
-                                {
-                                    break;
-                                }
-                                up++;
-                            }
-                            const int lastCell = up - 1;
-                            if (shift == kCentral && firstCell < ci)
-                            {
-                                firstCell = ci;
-                            }
-                            if (lastCell >= firstCell)
-                            {
-                                first = firstCell;
-                                count = lastCell - firstCell + 1;
-                            }
-                        }
-                    }
-                    int incl = count;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1)
-                    {
-                        const int t = __shfl_up_sync(full, incl, o);
-                        if (lane >= o)
-                        {
-                            incl += t;
-                        }
-                    }
-                    const int total = __shfl_sync(full, incl, 31);
-                    // four j-cells per step: lane (kk, jc) tests j-cluster jc of j-cell k0 + kk
-                    // against the 8 i-clusters (make_cluster_list_supersub for (ci, scj))
-                    const int kk = lane >> 3;
-                    const int jc = lane & 7;
-                    // j-cell of this lane at flat index k0 + kk
-                    auto locate = [&](int k0) {
-                        int col = 0;
-#pragma unroll
-                        for (int q = 0; q < 4; q++)
-                        {
-                            // columns that end at or before flat index k0 + q
-                            const int before = __popc(__ballot_sync(full, incl <= k0 + q));
-                            col              = (kk == q) ? before : col;
-                        }
-                        col                = min(col, 31);
-                        const int colFirst = __shfl_sync(full, first, col);
-                        const int colIncl  = __shfl_sync(full, incl, col);
-                        const int colCount = __shfl_sync(full, count, col);
-                        return colFirst + (k0 + kk - (colIncl - colCount));
-                    };
-                    // the j-cluster's bounding box is read with the cell's cluster count (empty
-                    // cluster slots hold far-away boxes, their results are discarded); the next
-                    // four j-cells' boxes are loaded while the current ones are tested
-                    int    scj_n  = locate(0);
-                    int    ncl_n  = 0;
-                    float4 jlo_n{}, jhi_n{};
-                    if (kk < total)
-                    {
-                        ncl_n = v.nclusters[scj_n];
-                        jlo_n = v.bb[2 * (scj_n * kNcl + jc)];
-                        jhi_n = v.bb[2 * (scj_n * kNcl + jc) + 1];
-                    }
-                    for (int k0 = 0; k0 < total; k0 += 4)
-                    {
-                        const int    scj      = scj_n;
-                        const bool   has_cell = k0 + kk < total;
-                        const int    ncl_j    = ncl_n;
-                        const float4 jlo = jlo_n, jhi = jhi_n;
-                        if (k0 + 4 < total)
-                        {
-                            scj_n = locate(k0 + 4);
-                            if (k0 + 4 + kk < total)
-                            {
-                                ncl_n = v.nclusters[scj_n];
-                                jlo_n = v.bb[2 * (scj_n * kNcl + jc)];
-                                jhi_n = v.bb[2 * (scj_n * kNcl + jc) + 1];
-                            }
-                            else
-                            {
-                                ncl_n = 0;
-                            }
-                        }
-                        const bool diag  = has_cell && excludeSubDiagonal && (scj == ci);
-                        const int  ci1   = diag ? jc + 1 : ncl_i;
-                        unsigned   im8   = 0u;
-                        float      d2one = 0.0f;
-                        if (jc < ncl_j)
-                        {
-#pragma unroll
-                            for (int i = 0; i < kNcl; i++)
-                            {
-                                const float d2 = bb_dist2(sm.bbi_lo[i], sm.bbi_hi[i], jlo, jhi);
-                                if (i < ci1 && d2 < rlist2)
-                                {
-                                    im8 |= 1u << i;
-                                    d2one = d2;
-                                }
-                            }
-                        }
-                        // a single cluster pair in range beyond the bounding-box-only distance:
-                        // check its atom pairs (PRUNE_LIST_CPU_ONE), one flagged j-cluster at a time
-                        unsigned flagged = __ballot_sync(full, __popc(im8) == 1 && d2one >= rbb2);
-                        while (flagged)
-                        {
-                            const int src = __ffs(flagged) - 1;
-                            flagged &= flagged - 1;
-                            const int    s_scj = __shfl_sync(full, scj, src);
-                            const int    s_cl  = __ffs(__shfl_sync(full, im8, src)) - 1;
-                            const float4 xi    = v.xq[ci * kSc + s_cl * kCl + (lane & 7)];
-                            const float  ix = xi.x + shx, iy = xi.y + shy, iz = xi.z + shz;
-                            const int    csj = s_scj * kNcl + (src & 7);
-                            bool         in  = false;
-#pragma unroll
-                            for (int h = 0; h < 2; h++)
-                            {
-                                const float4 xj = v.xq[csj * kCl + (lane >> 3) + 4 * h];
-                                const float  dx = ix - xj.x, dy = iy - xj.y, dz = iz - xj.z;
-                                const float  r2 = dx * dx + dy * dy + dz * dz;
-                                in              = in || (r2 < rlist2);
-                            }
-                            if (!__any_sync(full, in) && lane == src)
-                            {
-                                im8 = 0u;
-                            }
-                        }
-                        const unsigned nz = __ballot_sync(full, im8 != 0u);
-                        if (im8 != 0u)
-                        {
-                            const int r = rec_n + nj + __popc(nz & ((1u << lane) - 1u));
-                            if (r < v.rec_cap)
-                            {
-                                rec_cj[r] = scj * kNcl + jc;
-                                rec_m[r]  = (unsigned char)im8;
-                            }
-                            pairs += __popc(im8);
-                        }
-                        nj += __popc(nz);
-                    }
-                }
-                if (nj == 0)
-                {
-                    continue;  // closeIEntry drops empty entries
-                }
-                const int ncj4 = (nj + kJg - 1) / kJg;
-                if (ncj4 > kMaxCj4PerEntry && lane == 0)
-                {
-                    set_status(v.hdr, kStatusEntryOverflow);
-                }
-                if (lane == 0)
-                {
-                    v.rec_ent[ci * kMaxEntriesPerCell + num_entries] = shift | (nj << 8);
-                }
-                num_entries++;
-                num_cj4 += ncj4;
-                rec_n += nj;
+                const int ny = cyl - cyf + 1;
+                ncol         = max(cxl - cxf + 1, 0) * ny;
+                sm.sr[lane]  = { bx0, bx1, by0, by1, bz0, bz1, d2z, bz1_frac, shx, shy, shz, cxf, cyf, ny };
             }
         }
+    }
+    int incl = ncol;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int t = __shfl_up_sync(full, incl, o);
+        if (lane >= o)
+        {
+            incl += t;
+        }
+    }
+    sm.col0[lane]         = incl - ncol;
+    sm.nj[lane]           = 0;
+    const unsigned active = __ballot_sync(full, ncol > 0);
+    if (lane == 31)
+    {
+        sm.active = active;
+        sm.ncols = incl;
+        sm.ci_x  = ci_x;
+        sm.ci_y  = ci_y;
+        sm.pairs = 0;
+    }
+}
+
+// The z-range of j-cells of candidate column c (numbered over all shifts); *count 0 when none.
+__device__ __forceinline__ void column_cells(const DeviceView& v, int ci, const CountSmem& sm, int c, int* shift,
+                                             int* first, int* count)
+{
+    int s = 0;
+    for (unsigned m = sm.active; m; m &= m - 1u)
+    {
+        const int q = __ffs(m) - 1;
+        s           = sm.col0[q] <= c ? q : s;
+    }
+    const ShiftRange& r = sm.sr[s];
+    *shift              = s;
+    const float rlist2  = v.rlist2;
+    const float listRangeBBToJCell2 = v.rlist * v.rlist;
+    const float d2z = r.d2z, bz0 = r.bz0, bz1 = r.bz1;
+    const int   k  = c - sm.col0[s];
+    const int   cx = r.cxf + k / r.ny;
+    const int   cy = r.cyf + k % r.ny;
+    const int   columnStart = v.cxy_ind[cx * v.g.ncy + cy];
+    const int   columnEnd   = v.cxy_ind[cx * v.g.ncy + cy + 1];
+    const float cx_real = (float)cx;
+    float       d2zx    = d2z;
+    if (0.0f + cx_real * v.g.cs[0] > r.bx1)
+    {
+        d2zx = d2zx + sq(0.0f + cx_real * v.g.cs[0] - r.bx1);
+    }
+    else if (0.0f + (cx_real + 1.0f) * v.g.cs[0] < r.bx0)
+    {
+        d2zx = d2zx + sq(0.0f + (cx_real + 1.0f) * v.g.cs[0] - r.bx0);
+    }
+    const int   cyf_x   = (cx == 0 && s == kCentral && r.cyf < sm.ci_y) ? sm.ci_y : r.cyf;
+    const float cy_real = (float)cy;
+    float       d2zxy   = d2zx;
+    if (0.0f + cy_real * v.g.cs[1] > r.by1)
+    {
+        d2zxy = d2zxy + sq(0.0f + cy_real * v.g.cs[1] - r.by1);
+    }
+    else if (0.0f + (cy_real + 1.0f) * v.g.cs[1] < r.by0)
+    {
+        d2zxy = d2zxy + sq(0.0f + (cy_real + 1.0f) * v.g.cs[1] - r.by0);
+    }
+    if (!(cy >= cyf_x && columnStart < columnEnd && d2zxy < listRangeBBToJCell2))
+    {
+        return;
+    }
+    int midCell = columnStart + (int)(r.bz1_frac * (float)(columnEnd - columnStart));
+    if (midCell >= columnEnd)
+    {
+        midCell = columnEnd - 1;
+    }
+    const float d2xy = d2zxy - d2z;
+    // the walks up and down from the middle cell read four cells' bounds at a time
+    int  down = midCell;
+    bool more = true;
+    while (more && down >= columnStart)
+    {
+        float u[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            u[q] = v.bbcz[max(down - q, columnStart)].y;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            more = more && down >= columnStart && (u[q] >= bz0 || d2xy + sq(u[q] - bz0) < rlist2);
+            down -= more ? 1 : 0;
+        }
+    }
+    int firstCell = down + 1;
+    int up        = midCell + 1;
+    more          = true;
+    while (more && up < columnEnd)
+    {
+        float l[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            l[q] = v.bbcz[min(up + q, columnEnd - 1)].x;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+        {
+            more = more && up < columnEnd && (l[q] <= bz1 || d2xy + sq(l[q] - bz1) < rlist2);
+            up += more ? 1 : 0;
+        }
+    }
+    const int lastCell = up - 1;
+    if (s == kCentral && firstCell < ci)
+    {
+        firstCell = ci;
+    }
+    if (lastCell >= firstCell)
+    {
+        *first = firstCell;
+        *count = lastCell - firstCell + 1;
+    }
+}
+
+// Bound by latency: a cell at a corner of the box has eight shifts with columns of their own.  With one warp a
+// cell, which took shift after shift, 45k atoms needed 47.4 us, now 19.6 us; 960k atoms fill the GPU and
+// stay at 126 us (windows of 512 j-cells, 14 KB a block, leave less L1: 149 us).
+template<int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_search_count(DeviceView v)
+{
+    constexpr int kThreads = 32 * kWarps;
+    pdl_begin();
+    __shared__ CountSmem sm;
+    const int            ci = blockIdx.x;
+    if (ci >= v.hdr->num_cells)
+    {
+        return;
+    }
+    const unsigned full  = 0xffffffffu;
+    const int      tid   = threadIdx.x;
+    const int      lane  = tid & 31;
+    const int      warp  = tid >> 5;
+    const float    rlist2 = v.rlist2, rbb2 = v.rbb2;
+    if (warp == 0)
+    {
+        shift_ranges(v, ci, sm);
+    }
+    __syncthreads();
+    // shifted i-cluster bounding boxes (set_icell_bb, pairlist.cpp:2260-2303)
+    if (lane < kNcl)
+    {
+        const float4 l = v.bb[2 * (ci * kNcl + lane)];
+        const float4 h = v.bb[2 * (ci * kNcl + lane) + 1];
+        int          w = 0;
+        for (unsigned m = sm.active; m; m &= m - 1u)
+        {
+            if (w == warp)
+            {
+                const int         s = __ffs(m) - 1;
+                const ShiftRange& r = sm.sr[s];
+                sm.bbi_xy[s][lane]  = make_float4(l.x + r.shx, -(h.x + r.shx), l.y + r.shy, -(h.y + r.shy));
+                sm.bbi_z[s][lane]   = make_float2(l.z + r.shz, -(h.z + r.shz));
+            }
+            w = w + 1 == kWarps ? 0 : w + 1;
+        }
+    }
+    int* const           rec_cj = v.rec_cj + (size_t)ci * v.rec_cap;
+    unsigned char* const rec_m  = v.rec_m + (size_t)ci * v.rec_cap;
+    int                  rec_n  = 0;  // records of this cell so far
+    unsigned             pairs  = 0u;  // cluster pairs found by this lane
+    const int            ncols  = sm.ncols;
+    // The candidate columns of all shifts (the reference's visiting order), a thread each; a block scan turns
+    // their cell counts into offsets of one flat sequence of j-cells, increasing within a shift.
+    for (int c0 = 0; c0 < ncols; c0 += kThreads)
+    {
+        int shift = 0, first = 0, count = 0, total = 0;
+        if (c0 + tid < ncols)
+        {
+            column_cells(v, ci, sm, c0 + tid, &shift, &first, &count);
+        }
+        const int start = block_scan<kWarps>(count, sm.warp_sum[0], &total) - count;
+        for (int w0 = 0; w0 < total; w0 += kCellWindow)
+        {
+            const int wn = min(total - w0, kCellWindow);
+            for (int q = max(w0 - start, 0); q < min(count, w0 + wn - start); q++)
+            {
+                sm.cell[start + q - w0]       = first + q;
+                sm.cell_shift[start + q - w0] = (unsigned char)shift;
+            }
+            __syncthreads();
+            // four j-cells per step: lane (kk, jc) tests j-cluster jc of its j-cell against the 8 i-clusters
+            // (make_cluster_list_supersub for (ci, scj)); the j-cluster's bounding box is read with the cell's
+            // cluster count (empty cluster slots hold far-away boxes, their results are discarded), the next
+            // step's while the current one is tested
+            const int kk = lane >> 3;
+            const int jc = lane & 7;
+            int       k0    = 4 * warp;
+            int       scj_n = 0, ncl_n = 0;
+            float4    jlo{}, jhi{};
+            auto      load = [&](int k) {
+                ncl_n = 0;
+                if (k < wn)
+                {
+                    scj_n = sm.cell[k];
+                    ncl_n = v.nclusters[scj_n];
+                    jlo   = v.bb[2 * (scj_n * kNcl + jc)];
+                    jhi   = v.bb[2 * (scj_n * kNcl + jc) + 1];
+                }
+            };
+            load(k0 + kk);
+            for (; k0 < wn; k0 += 4 * kWarps)
+            {
+                const int    k     = k0 + kk;
+                const int    scj   = scj_n;
+                const int    ncl_j = ncl_n;
+                const float2 jx = make_float2(-jhi.x, jlo.x), jy = make_float2(-jhi.y, jlo.y),
+                             jz = make_float2(-jhi.z, jlo.z);
+                load(k + 4 * kWarps);
+                const int s     = k < wn ? sm.cell_shift[k] : 0;
+                unsigned  im8   = 0u;
+                float     d2one = 0.0f;
+                if (jc < ncl_j)
+                {
+#pragma unroll
+                    for (int i = 0; i < kNcl; i += 2)
+                    {
+                        const float2 d2 = bb_dist2(sm.bbi_xy[s][i], sm.bbi_xy[s][i + 1],
+                                                   *reinterpret_cast<const float4*>(&sm.bbi_z[s][i]), jx, jy, jz);
+                        if (d2.x < rlist2)
+                        {
+                            im8 |= 1u << i;
+                            d2one = d2.x;
+                        }
+                        if (d2.y < rlist2)
+                        {
+                            im8 |= 2u << i;
+                            d2one = d2.y;
+                        }
+                    }
+                    // empty i-clusters are far away; of the cell's own clusters only i <= j (a single one is
+                    // i = j, at distance 0)
+                    if (s == kCentral && scj == ci)
+                    {
+                        im8 &= (2u << jc) - 1u;
+                        d2one = 0.0f;
+                    }
+                }
+                // a single cluster pair in range beyond the bounding-box-only distance: check its atom pairs
+                // (PRUNE_LIST_CPU_ONE), four flagged j-clusters at a time, eight lanes each (lane jc an i-atom)
+                const bool     mine    = __popc(im8) == 1 && d2one >= rbb2;
+                const unsigned flagged = __ballot_sync(full, mine);
+                if (flagged)
+                {
+                    const int rank = __popc(flagged & ((1u << lane) - 1u));
+                    if (mine)
+                    {
+                        sm.flag[warp][rank] = make_int2(scj * kNcl + jc, s * kNcl + __ffs(im8) - 1);
+                    }
+                    __syncwarp();
+                    const int nf = __popc(flagged);
+                    for (int f0 = 0; f0 < nf; f0 += 4)
+                    {
+                        bool in = false;
+                        if (f0 + kk < nf)
+                        {
+                            const int2   fl = sm.flag[warp][f0 + kk];
+                            const auto&  r  = sm.sr[fl.y >> 3];
+                            const float4 xi = v.xq[ci * kSc + (fl.y & 7) * kCl + jc];
+                            const float  ix = xi.x + r.shx, iy = xi.y + r.shy, iz = xi.z + r.shz;
+                            float        least = 3.0e38f;
+#pragma unroll 4
+                            for (int h = 0; h < kCl; h++)
+                            {
+                                const float4 xj = v.xq[fl.x * kCl + h];
+                                least           = fminf(least, norm2(ix - xj.x, iy - xj.y, iz - xj.z));
+                            }
+                            in = least < rlist2;
+                        }
+                        const unsigned found = __ballot_sync(full, in);
+                        if (mine && (rank >> 2) == (f0 >> 2) && ((found >> (8 * (rank & 3))) & 0xffu) == 0u)
+                        {
+                            im8 = 0u;
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (k < wn)
+                {
+                    reinterpret_cast<unsigned char*>(sm.masks)[8 * k + jc] = (unsigned char)im8;
+                }
+                pairs += __popc(im8);
+            }
+            __syncthreads();
+            // the records of the window in order, a j-cell per thread
+            for (int b = 0; b < wn; b += kThreads)
+            {
+                const int   k = b + tid;
+                const uint2 m = k < wn ? sm.masks[k] : make_uint2(0u, 0u);
+                int         found = 0, sum = 0;
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                {
+                    found += (((q < 4 ? m.x : m.y) >> (8 * (q & 3))) & 0xffu) != 0u ? 1 : 0;
+                }
+                int r = rec_n + block_scan<kWarps>(found, sm.warp_sum[1], &sum) - found;
+                if (found > 0)
+                {
+                    atomicAdd(&sm.nj[sm.cell_shift[k]], found);
+                    const int cj = sm.cell[k] * kNcl;
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                    {
+                        const unsigned im = ((q < 4 ? m.x : m.y) >> (8 * (q & 3))) & 0xffu;
+                        if (im != 0u)
+                        {
+                            if (r < v.rec_cap)
+                            {
+                                rec_cj[r] = cj + q;
+                                rec_m[r]  = (unsigned char)im;
+                            }
+                            r++;
+                        }
+                    }
+                }
+                rec_n += sum;
+                __syncthreads();  // the window and the scan's sums are free again
+            }
+        }
+        __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1)
     {
         pairs += __shfl_xor_sync(full, pairs, o);
     }
+    if (lane == 0 && pairs > 0u)
+    {
+        atomicAdd(&sm.pairs, (int)pairs);
+    }
+    __syncthreads();
+    if (warp > 0)
+    {
+        return;
+    }
+    // the entries, lane = shift: closeIEntry drops empty ones
+    const int      nj   = lane < kShiftSlots ? sm.nj[lane] : 0;
+    const unsigned has  = __ballot_sync(full, nj > 0);
+    const int      ncj4 = (nj + kJg - 1) / kJg;
+    if (nj > 0)
+    {
+        v.rec_ent[ci * kMaxEntriesPerCell + __popc(has & ((1u << lane) - 1u))] = lane | (nj << 8);
+        if (ncj4 > kMaxCj4PerEntry)
+        {
+            set_status(v.hdr, kStatusEntryOverflow);
+        }
+    }
+    int num_cj4 = ncj4;
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        num_cj4 += __shfl_xor_sync(full, num_cj4, o);
+    }
     if (lane == 0)
     {
-        v.sci_count[ci] = num_entries;
+        v.sci_count[ci] = __popc(has);
         v.cj4_count[ci] = num_cj4;
         // cluster pairs of the list, the count that list balancing splits by
-        if (pairs > 0u)
+        if (sm.pairs > 0)
         {
-            atomicAdd(&v.hdr->num_subpairs, (int)pairs);
+            atomicAdd(&v.hdr->num_subpairs, sm.pairs);
         }
         if (rec_n > v.rec_cap)
         {
@@ -956,11 +1100,19 @@ __global__ void k_scan_counts(DeviceView v)
 cudaError_t launch_search_count(const DeviceView& v, cudaStream_t s)
 {
     const int cap    = v.g.cells_capacity;
-    const int blocks = (cap + kWarpsPerBlock - 1) / kWarpsPerBlock;
     // num_subpairs .. rec_need: accumulated by the count pass or set by balancing
     cudaMemsetAsync(&v.hdr->num_subpairs, 0,
                     offsetof(ListHeader, rec_need) + sizeof(int) - offsetof(ListHeader, num_subpairs), s);
-    launch_pdl(k_search_count, blocks, 32 * kWarpsPerBlock, 0, s, v);
+    // two warps a cell once the cells alone fill the GPU (960k atoms, 15.6k cells: the search step 1671 us, with
+    // four 1686 us), four while a cell's latency counts (45k atoms: 235 us, with two 240 us)
+    if (cap > kManyCells)
+    {
+        launch_pdl(k_search_count<2>, cap, 64, 0, s, v);
+    }
+    else
+    {
+        launch_pdl(k_search_count<4>, cap, 128, 0, s, v);
+    }
     launch_pdl(k_scan_counts, 1, 1024, 0, s, v);
     return cudaGetLastError();
 }

@@ -123,6 +123,20 @@ def test_search_records_grow_for_long_lists():
     calc.close()
 
 
+@pytest.mark.parametrize("molecules,edge,rlist", [(40, 1.1, 1.05), (1000, 3.11, 1.5), (2700, 4.33, 2.1), (9, 12.0, 1.0)])
+def test_search_windows_match_oracle(molecules, edge, rlist):
+    """Boxes shorter than one list radius (five shifts in x), cells with more than 128 candidate columns and
+    several windows of 128 candidate j-cells, and cells as wide as the box: the same entries in the same order
+    with the same pairs."""
+    s = systems.spc_water(molecules, edge, seed=13)
+    calc, o = _pair(s, rc=min(0.9, 0.49 * edge), rlist=rlist)
+    pg, po = calc.pairlist(), o.pairlist()
+    np.testing.assert_array_equal(pg["sci"], po["sci"])
+    assert np.array_equal(canonical_pairs(pg["sci"], pg["cj4"], pg["excl"]),
+                          canonical_pairs(po["sci"], po["cj4"], po["excl"]))
+    calc.close()
+
+
 def test_balancing_leaves_forces_unchanged():
     s = systems.water_small()
     calc, _o = _pair(s)
