@@ -246,7 +246,7 @@ int ensure_list_capacity(nbx_handle* h, int num_sci, int num_cj4)
     v.excl_cap = 2 * need_cj4 + 1;  // at most one mask per cj4 half
     cudaError_t e = dalloc(h, &v.sci, v.sci_cap);
     if (e == cudaSuccess) e = dalloc(h, &v.sci_tmp, v.sci_cap);
-    if (e == cudaSuccess) e = dalloc(h, &v.sci_pieces, (size_t)v.sci_cap + 1);
+    if (e == cudaSuccess) e = dalloc(h, &v.sci_pieces, (size_t)v.sci_cap + 1 + kSortChunks * kSizeClasses);
     if (e == cudaSuccess) e = dalloc(h, &v.cj4, v.cj4_cap);
     if (e == cudaSuccess) e = dalloc(h, &v.excl, v.excl_cap);
     if (e == cudaSuccess) e = dalloc(h, &v.imask_outer, 2 * (size_t)v.cj4_cap);

@@ -27,10 +27,10 @@ namespace
 {
 
 constexpr int kMinTarget    = 36;   // nsubpair_target_min, pairlist.cpp:2495
-constexpr int kMaxSizeClass = 255;
-constexpr int kSortThreads  = 1024;
+constexpr int kMaxSizeClass = kSizeClasses - 1;
+constexpr int kSortThreads  = kSizeClasses;  // a thread per class in the offsets
 constexpr int kSortWarps    = kSortThreads / 32;
-constexpr int kSortBatch    = 8;  // entries per lane loaded at a time by the sort
+constexpr int kSortBatch    = 2;  // entries per lane loaded at a time by the sort
 constexpr int kScanBatch    = 8;  // piece counts per thread loaded at a time by the scan
 
 __device__ __forceinline__ int balance_target(const ListHeader* hdr, int min_ci_balanced)
@@ -103,6 +103,24 @@ __device__ int split_entry(const unsigned char* __restrict__ grp_pairs, Sci e, i
     return n;
 }
 
+// Entries per chunk and class (see sci_pieces).
+__device__ __forceinline__ int* sort_hist(const DeviceView& v)
+{
+    return v.sci_pieces + v.sci_cap + 1;
+}
+
+// The largest size class of a list of n entries: sizes above twice the average share it; 0: one class, order kept.
+__device__ __forceinline__ int largest_class(const ListHeader* hdr, int n)
+{
+    const int m = hdr->num_cj4 > n ? (int)((2LL * hdr->num_cj4) / n) : 0;
+    return m > kMaxSizeClass ? kMaxSizeClass : m;
+}
+
+__device__ __forceinline__ int sort_chunk(int n)
+{
+    return (n + kSortChunks - 1) / kSortChunks;
+}
+
 __global__ void k_balance_count(DeviceView v, int min_ci_balanced)
 {
     pdl_begin();
@@ -119,7 +137,12 @@ __global__ void k_balance_count(DeviceView v, int min_ci_balanced)
         v.hdr->nsp_max         = nsp_max;
         v.hdr->num_sci_unsplit = nsci;
     }
-    if (e < nsci)
+    for (int k = e; k < kSortChunks * kSizeClasses; k += gridDim.x * blockDim.x)
+    {
+        sort_hist(v)[k] = 0;
+    }
+    // nothing is split: every entry is one piece, at its own place
+    if (nsp_max > 0 && e < nsci)
     {
         v.sci_pieces[e] = split_entry<false>(v.grp_pairs, v.sci[e], nsp_max, nullptr);
     }
@@ -138,6 +161,14 @@ __global__ void __launch_bounds__(1024) k_balance_scan(DeviceView v)
     }
     const int n    = hdr->num_sci_unsplit;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (hdr->nsp_max == 0)
+    {
+        if (threadIdx.x == 0)
+        {
+            v.hdr->num_sci_split = n;
+        }
+        return;
+    }
     const int per  = (n + blockDim.x - 1) / blockDim.x;
     const int i0   = min(n, (int)threadIdx.x * per);
     const int i1   = min(n, i0 + per);
@@ -222,100 +253,101 @@ __global__ void k_balance_write(DeviceView v)
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e < hdr->num_sci_unsplit)
     {
-        split_entry<true>(v.grp_pairs, v.sci[e], hdr->nsp_max, v.sci_tmp + v.sci_pieces[e]);
+        const int first = hdr->nsp_max > 0 ? v.sci_pieces[e] : e;
+        const int count = split_entry<true>(v.grp_pairs, v.sci[e], hdr->nsp_max, v.sci_tmp + first);
+        // entries per chunk and class for the sort
+        const int m     = largest_class(hdr, hdr->num_sci_split);
+        const int chunk = sort_chunk(hdr->num_sci_split);
+        for (int p = first; p < first + count; p++)
+        {
+            const int len = v.sci_tmp[p].cj4_end - v.sci_tmp[p].cj4_start;
+            atomicAdd(&sort_hist(v)[p / chunk * kSizeClasses + (len < m ? len : m)], 1);
+        }
     }
 }
 
-// Stable counting sort of sci_tmp into sci, size classes descending (one block).  Warp w owns the
-// w-th contiguous chunk of the entries: a per-warp class histogram, then per class the offsets of
-// the warps' runs (warps in order, classes descending), then each warp places its chunk in order,
-// the rank among equal classes of a batch of 32 from __match_any_sync.
+// Stable counting sort of sci_tmp into sci, size classes descending; a block per chunk of the entries.  From the
+// chunks' class counts (k_balance_write) thread c gets the class's place in the list and the chunk's place in the
+// class; warp w owns the w-th run of the chunk: per-warp class counts, then each warp places its run in order, the
+// rank among equal classes of 32 entries from __match_any_sync.  One block of 1024 threads for the whole list took
+// 13.6 us for 7k entries and 36 us for 18k.
 __global__ void __launch_bounds__(kSortThreads) k_sort_entries(DeviceView v)
 {
     pdl_begin();
-    __shared__ int hist[kSortWarps][kMaxSizeClass + 1];  // counts, then each warp's first position
+    __shared__ int hist[kSortWarps][kSizeClasses];  // counts, then each warp's next position
+    __shared__ int warp_sums[kSortWarps];
     ListHeader*    hdr = v.hdr;
     if (hdr->status & (kStatusListOverflow | kStatusExclOverflow | kStatusGridOverflow))
     {
         return;
     }
     const int n    = hdr->num_sci_split;
-    const int ncj4 = hdr->num_cj4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        hdr->num_sci = n;
+    }
     if (n == 0)
     {
-        if (threadIdx.x == 0)
-        {
-            hdr->num_sci = 0;
-        }
         return;
     }
-    int m = (ncj4 > n) ? (int)((2LL * ncj4) / n) : 0;  // m = 0: one class, order kept
-    m     = m > kMaxSizeClass ? kMaxSizeClass : m;
-    for (int k = threadIdx.x; k < kSortWarps * (kMaxSizeClass + 1); k += blockDim.x)
+    const int m     = largest_class(hdr, n);
+    const int chunk = sort_chunk(n);
+    const int c0    = blockIdx.x * chunk;
+    const int run   = (chunk + kSortWarps - 1) / kSortWarps;
+    const int e0    = min(n, c0 + min(chunk, warp * run));
+    const int e1    = min(n, c0 + min(chunk, (warp + 1) * run));
+    // the class of this thread: its entries in the chunks before this one and in all
+    const int cls0   = m - (int)threadIdx.x;
+    int       before = 0, total = 0;
+    if (cls0 >= 0)
+    {
+#pragma unroll 16
+        for (int b = 0; b < kSortChunks; b++)
+        {
+            const int h = sort_hist(v)[b * kSizeClasses + cls0];
+            before += b < (int)blockIdx.x ? h : 0;
+            total += h;
+        }
+    }
+    for (int k = threadIdx.x; k < kSortWarps * kSizeClasses; k += kSortThreads)
     {
         (&hist[0][0])[k] = 0;
     }
-    __syncthreads();
-    const int chunk = (n + kSortWarps - 1) / kSortWarps;
-    const int e0    = min(n, warp * chunk);
-    const int e1    = min(n, e0 + chunk);
-    // kSortBatch entries per lane loaded before any is counted or placed
-    for (int b = e0; b < e1; b += 32 * kSortBatch)
+    int incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
     {
-        int len[kSortBatch];
-#pragma unroll
-        for (int u = 0; u < kSortBatch; u++)
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
         {
-            const int e = b + u * 32 + lane;
-            len[u]      = e < e1 ? v.sci_tmp[e].cj4_end - v.sci_tmp[e].cj4_start : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < kSortBatch; u++)
-        {
-            if (len[u] >= 0)
-            {
-                atomicAdd(&hist[warp][len[u] < m ? len[u] : m], 1);
-            }
+            incl += t;
         }
     }
-    __syncthreads();
-    if (warp == 0)
+    if (lane == 31)
     {
-        // per class: the warps' runs in warp order; classes from m down to 0
-        int base = 0;
-        for (int c0 = m; c0 >= 0; c0 -= 32)
+        warp_sums[warp] = incl;
+    }
+    __syncthreads();
+    for (int e = e0 + lane; e < e1; e += 32)
+    {
+        const int len = v.sci_tmp[e].cj4_end - v.sci_tmp[e].cj4_start;
+        atomicAdd(&hist[warp][len < m ? len : m], 1);
+    }
+    __syncthreads();
+    if (cls0 >= 0)
+    {
+        int pos = incl - total + before;
+        for (int w = 0; w < warp; w++)
         {
-            const int c     = c0 - lane;
-            int       total = 0;
-            if (c >= 0)
-            {
-                for (int w = 0; w < kSortWarps; w++)
-                {
-                    const int h = hist[w][c];
-                    hist[w][c]  = total;
-                    total += h;
-                }
-            }
-            int incl = total;
+            pos += warp_sums[w];
+        }
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o)
-                {
-                    incl += t;
-                }
-            }
-            const int start = base + incl - total;
-            if (c >= 0)
-            {
-                for (int w = 0; w < kSortWarps; w++)
-                {
-                    hist[w][c] += start;
-                }
-            }
-            base += __shfl_sync(0xffffffffu, incl, 31);
+        for (int w = 0; w < kSortWarps; w++)
+        {
+            const int h   = hist[w][cls0];
+            hist[w][cls0] = pos;
+            pos += h;
         }
     }
     __syncthreads();
@@ -347,10 +379,6 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_entries(DeviceView v)
             __syncwarp();
         }
     }
-    if (threadIdx.x == 0)
-    {
-        hdr->num_sci = n;
-    }
 }
 
 } // namespace
@@ -362,7 +390,7 @@ cudaError_t launch_balance(const DeviceView& v, int min_ci_balanced, cudaStream_
     launch_pdl(k_balance_count, blocks, tb, 0, s, v, min_ci_balanced);
     launch_pdl(k_balance_scan, 1, 1024, 0, s, v);
     launch_pdl(k_balance_write, blocks, tb, 0, s, v);
-    launch_pdl(k_sort_entries, 1, kSortThreads, 0, s, v);
+    launch_pdl(k_sort_entries, kSortChunks, kSortThreads, 0, s, v);
     return cudaGetLastError();
 }
 

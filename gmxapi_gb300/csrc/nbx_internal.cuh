@@ -115,6 +115,9 @@ enum StatusBits : unsigned
 // Entries one i-cell can have: one per shift of the half shell, at most 23 (5 x 3 x 3 shifts when the
 // box is shorter than rlist along x, of which 22 backward and the central one).
 constexpr int kMaxEntriesPerCell = 24;
+// the size sort of the list entries: chunks (a block each) and size classes
+constexpr int kSortChunks  = 64;
+constexpr int kSizeClasses = 256;
 
 struct Sci
 {
@@ -201,7 +204,9 @@ struct DeviceView
     // list
     Sci*      sci;
     Sci*      sci_tmp;      // [sci_cap] split entries before the size sort
-    int*      sci_pieces;   // [sci_cap + 1] pieces per searched entry, then their offsets
+    // [sci_cap + 1] pieces per searched entry, then their offsets; [kSortChunks * kSizeClasses] entries per
+    // chunk and size class
+    int*      sci_pieces;
     Cj4*      cj4;
     Excl*     excl;
     unsigned* imask_outer;  // [2*cj4_cap]

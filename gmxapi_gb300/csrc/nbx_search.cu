@@ -611,7 +611,6 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_search_count(Devic
     }
 }
 
-constexpr int kScanBatch = 8;    // cell counts per thread loaded at a time by the prefix sum
 constexpr int kExclStage = 256;  // topology exclusions of a cell's i-atoms staged in shared memory
 
 struct EmitSmem
@@ -992,56 +991,67 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView 
     }
 }
 
-// Exclusive prefix sums of the per-cell entry and cj4 counts, one block.
-__global__ void k_scan_counts(DeviceView v)
+// four values from index i, those at n and beyond as 0
+__device__ __forceinline__ int4 load4(const int* p, int i, int n)
+{
+    if (i + 4 <= n)
+    {
+        return *reinterpret_cast<const int4*>(p + i);
+    }
+    return make_int4(i < n ? p[i] : 0, i + 1 < n ? p[i + 1] : 0, i + 2 < n ? p[i + 2] : 0, 0);
+}
+
+__device__ __forceinline__ void store4(int* p, int i, int n, int4 x)
+{
+    if (i + 4 <= n)
+    {
+        *reinterpret_cast<int4*>(p + i) = x;
+        return;
+    }
+    if (i < n) p[i] = x.x;
+    if (i + 1 < n) p[i + 1] = x.y;
+    if (i + 2 < n) p[i + 2] = x.z;
+}
+
+// Exclusive prefix sums of the per-cell entry and cj4 counts, one block, four cells a thread: rows of 4096 cells
+// with the next one loaded ahead.  15.6k cells took 21 us with a contiguous run of cells per thread.
+__global__ void __launch_bounds__(1024) k_scan_counts(DeviceView v)
 {
     pdl_begin();
     __shared__ int ws[2][32];
-    const int      n        = v.hdr->num_cells;
-    const int      nthreads = blockDim.x;
-    const int      per      = (n + nthreads - 1) / nthreads;
-    const int      c0       = threadIdx.x * per;
-    const int      c1       = min(n, c0 + per);
-    int            ls = 0, lc = 0;
-    // kScanBatch cells per thread loaded at a time
-    for (int b = c0; b < c1; b += kScanBatch)
+    const int      n    = v.hdr->num_cells;
+    const int      lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int            base_s = 0, base_c = 0;
+    int            i  = 4 * threadIdx.x;
+    int4           sn = load4(v.sci_count, i, n), cn = load4(v.cj4_count, i, n);
+    for (int row = 0; row < n; row += 4096, i += 4096)
     {
-        int cs[kScanBatch], cc[kScanBatch];
+        const int4 s = sn, c = cn;
+        sn           = load4(v.sci_count, i + 4096, n);
+        cn           = load4(v.cj4_count, i + 4096, n);
+        const int ls = s.x + s.y + s.z + s.w, lc = c.x + c.y + c.z + c.w;
+        int       is = ls, ic = lc;
 #pragma unroll
-        for (int u = 0; u < kScanBatch; u++)
+        for (int o = 1; o < 32; o <<= 1)
         {
-            cs[u] = b + u < c1 ? v.sci_count[b + u] : 0;
-            cc[u] = b + u < c1 ? v.cj4_count[b + u] : 0;
+            const int ts = __shfl_up_sync(0xffffffffu, is, o);
+            const int tc = __shfl_up_sync(0xffffffffu, ic, o);
+            if (lane >= o)
+            {
+                is += ts;
+                ic += tc;
+            }
         }
+        __syncthreads();  // the row before has been read
+        if (lane == 31)
+        {
+            ws[0][warp] = is;
+            ws[1][warp] = ic;
+        }
+        __syncthreads();
+        // every warp scans the 32 warps' sums
+        int a = ws[0][lane], b = ws[1][lane];
 #pragma unroll
-        for (int u = 0; u < kScanBatch; u++)
-        {
-            ls += cs[u];
-            lc += cc[u];
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int       is = ls, ic = lc;
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const int ts = __shfl_up_sync(0xffffffffu, is, o);
-        const int tc = __shfl_up_sync(0xffffffffu, ic, o);
-        if (lane >= o)
-        {
-            is += ts;
-            ic += tc;
-        }
-    }
-    if (lane == 31)
-    {
-        ws[0][warp] = is;
-        ws[1][warp] = ic;
-    }
-    __syncthreads();
-    if (warp == 0)
-    {
-        int a = (lane < (nthreads >> 5)) ? ws[0][lane] : 0;
-        int b = (lane < (nthreads >> 5)) ? ws[1][lane] : 0;
         for (int o = 1; o < 32; o <<= 1)
         {
             const int ta = __shfl_up_sync(0xffffffffu, a, o);
@@ -1052,41 +1062,22 @@ __global__ void k_scan_counts(DeviceView v)
                 b += tb;
             }
         }
-        ws[0][lane] = a;
-        ws[1][lane] = b;
+        const int wa = __shfl_sync(0xffffffffu, a, max(warp - 1, 0)), wb = __shfl_sync(0xffffffffu, b, max(warp - 1, 0));
+        const int rs = base_s + is - ls + (warp > 0 ? wa : 0);
+        const int rc = base_c + ic - lc + (warp > 0 ? wb : 0);
+        store4(v.sci_offset, i, n, make_int4(rs, rs + s.x, rs + s.x + s.y, rs + s.x + s.y + s.z));
+        store4(v.cj4_offset, i, n, make_int4(rc, rc + c.x, rc + c.x + c.y, rc + c.x + c.y + c.z));
+        base_s += __shfl_sync(0xffffffffu, a, 31);
+        base_c += __shfl_sync(0xffffffffu, b, 31);
     }
-    __syncthreads();
-    int rs = is - ls + (warp > 0 ? ws[0][warp - 1] : 0);
-    int rc = ic - lc + (warp > 0 ? ws[1][warp - 1] : 0);
-    for (int b = c0; b < c1; b += kScanBatch)
+    if (threadIdx.x == 0)
     {
-        int cs[kScanBatch], cc[kScanBatch];
-#pragma unroll
-        for (int u = 0; u < kScanBatch; u++)
-        {
-            cs[u] = b + u < c1 ? v.sci_count[b + u] : 0;
-            cc[u] = b + u < c1 ? v.cj4_count[b + u] : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < kScanBatch; u++)
-        {
-            if (b + u < c1)
-            {
-                v.sci_offset[b + u] = rs;
-                v.cj4_offset[b + u] = rc;
-                rs += cs[u];
-                rc += cc[u];
-            }
-        }
-    }
-    if (threadIdx.x == nthreads - 1)
-    {
-        v.sci_offset[n] = rs;
-        v.cj4_offset[n] = rc;
-        v.hdr->num_sci  = rs;
-        v.hdr->num_cj4  = rc;
+        v.sci_offset[n] = base_s;
+        v.cj4_offset[n] = base_c;
+        v.hdr->num_sci  = base_s;
+        v.hdr->num_cj4  = base_c;
         v.hdr->num_excl = 1;
-        if (rs > v.hdr->sci_capacity || rc > v.hdr->cj4_capacity)
+        if (base_s > v.hdr->sci_capacity || base_c > v.hdr->cj4_capacity)
         {
             set_status(v.hdr, kStatusListOverflow);
         }
