@@ -13,7 +13,7 @@
 // tests four of them at once, lane (cell, j-cluster) its j-cluster's bounding box against the
 // 8 i-clusters.  The j-clusters found are stored as per-cell records (index, 8-bit i-cluster
 // mask) in order, with one code per entry, and the cell's entry / cj4 counts are written.  After
-// a prefix sum of the counts, the emit pass (one warp per list entry) turns the records into
+// a prefix sum of the counts, the emit pass (one block per list entry) turns the records into
 // sci / cj4 entries at fixed offsets, with the outer masks and per-group pair counts, and sets
 // the diagonal and topology exclusion masks.
 #include "nbx_internal.cuh"
@@ -25,7 +25,6 @@ namespace nbx
 namespace
 {
 
-constexpr int kWarpsPerBlock  = 4;
 constexpr int kMaxCj4PerEntry = 1024;  // per (i-cell, shift) entry; beyond it the list overflows
 
 __device__ __forceinline__ void set_status(ListHeader* hdr, unsigned bits)
@@ -611,36 +610,43 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps) k_search_count(Devic
     }
 }
 
+constexpr int kEmitWarps = 2;    // at least 2: a warp per half of the i-atoms' exclusions
 constexpr int kExclStage = 256;  // topology exclusions of a cell's i-atoms staged in shared memory
 
 struct EmitSmem
 {
     unsigned      need[2 * kMaxCj4PerEntry / 32];  // per (cj4, half): exclusion mask needed
+    int           first[2 * kMaxCj4PerEntry / 32];  // masks needed before the word
     int           diag_pos[kNcl];                   // list positions of the diagonal j-clusters
     int           jl[kEmitStage];                   // the entry's j-clusters (short entries)
     unsigned char jm[kEmitStage];                   // and their i-cluster masks
     int           ex_j[kExclStage];                 // excluded partner's grid slot (-1: itself)
     unsigned char ex_i[kExclStage];                 // the i-atom's slot within the cell
+    int           ex_count[2];                      // exclusions of the two halves of the i-atoms
+    int           base, masks;                      // first exclusion mask of the entry and their number
 };
 
-// Emit pass: one warp per list entry (the entries numbered by the prefix sum of the per-cell
-// counts) turns its search records into the entry's sci record and cj4 groups.  The warp finds its
+// Emit pass: one block per list entry (the entries numbered by the prefix sum of the per-cell
+// counts) turns its search records into the entry's sci record and cj4 groups.  Each warp finds the
 // cell by a 32-way search of the entry offsets and the entry's first record and group from the
-// codes of the cell's earlier entries, then writes the cj4 groups (one per lane: four j-clusters,
-// the i-cluster masks of both warp halves, exclusion index 0 = all interacting), the outer masks
-// (the fresh list's masks until a prune refines them) and the group's cluster-pair count for
-// balancing; then the exclusions: flag the (cj4, half) pairs that need a mask (self/Newton pairs of
-// the diagonal j-clusters and topology exclusions), allocate the flagged masks all interacting,
+// codes of the cell's earlier entries; then the block writes the cj4 groups (one per thread: four
+// j-clusters, the i-cluster masks of both warp halves, exclusion index 0 = all interacting), the
+// outer masks (the fresh list's masks until a prune refines them) and the group's cluster-pair count
+// for balancing; then the exclusions: flag the (cj4, half) pairs that need a mask (self/Newton pairs
+// of the diagonal j-clusters and topology exclusions), allocate the flagged masks all interacting,
 // clear j <= i on the diagonal (setSelfAndNewtonExclusionsGpu) and the excluded atom pairs
-// (setExclusionsForIEntry).
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView v)
+// (setExclusionsForIEntry).  A chain of dependent loads and short loops: with one warp an entry 27.8 us at 45k
+// and 90 us at 960k atoms, with two 12.6 and 76 us (with four 12.6 and 82 us).
+__global__ void __launch_bounds__(32 * kEmitWarps) k_search_emit(DeviceView v)
 {
     pdl_begin();
-    __shared__ EmitSmem wsm[kWarpsPerBlock];
-    const int           lane = threadIdx.x & 31;
-    const int           wib  = threadIdx.x >> 5;
-    EmitSmem&           sm   = wsm[wib];
-    const int           e    = blockIdx.x * kWarpsPerBlock + wib;
+    constexpr int       kThreads = 32 * kEmitWarps;
+    constexpr int       kWords   = 2 * kMaxCj4PerEntry / 32;
+    __shared__ EmitSmem sm;
+    const int           tid  = threadIdx.x;
+    const int           lane = tid & 31;
+    const int           warp = tid >> 5;
+    const int           e    = blockIdx.x;
     const unsigned      full = 0xffffffffu;
     if (e >= v.hdr->num_sci
         || (v.hdr->status & (kStatusListOverflow | kStatusRecordOverflow | kStatusEntryOverflow)))
@@ -663,6 +669,17 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView 
             ci              = lo;
         }
     }
+    // the topology exclusions of the cell's i-atoms, half of them per warp: how many
+    int iAtom = -1, x0 = 0, x1 = 0;
+    if (warp < 2)
+    {
+        iAtom = v.atom_indices[ci * kSc + warp * 32 + lane];
+        if (iAtom >= 0)
+        {
+            x0 = v.excl_index[iAtom];
+            x1 = v.excl_index[iAtom + 1];
+        }
+    }
     const int kent = e - v.sci_offset[ci];
     // this entry's code; the records and groups of the cell's earlier entries
     const int cl   = lane <= kent ? v.rec_ent[ci * kMaxEntriesPerCell + lane] : 0;
@@ -675,319 +692,315 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_search_emit(DeviceView 
         grp0 += __shfl_xor_sync(full, grp0, o);
     }
     const int            code    = __shfl_sync(full, cl, kent);
-    const int            sci_out = e;
     const int            cj4_out = v.cj4_offset[ci] + grp0;
     const int*           rec_cj  = v.rec_cj + (size_t)ci * v.rec_cap + rec0;
     const unsigned char* rec_m   = v.rec_m + (size_t)ci * v.rec_cap + rec0;
-    // the topology exclusions of the cell's i-atoms as (i-slot, partner grid slot) pairs (when they
-    // fit; else the entry walks the exclusion lists); both halves of the 64 i-atoms load together
-    int nex = 0;
+    const int            shift   = code & 0xff;
+    const int            nj      = code >> 8;
+    const int            ncj4    = (nj + kJg - 1) / kJg;
+    const bool           excludeSubDiagonal = (shift == kCentral);
+    if (tid < kNcl)
     {
-        int iAtom[2], x0[2] = { 0, 0 }, x1[2] = { 0, 0 };
-#pragma unroll
-        for (int h = 0; h < 2; h++)
+        sm.diag_pos[tid] = -1;
+    }
+    for (int w = tid; w < kWords; w += kThreads)
+    {
+        sm.need[w] = 0u;
+    }
+    // the j-list is sorted on cluster index; short lists go to shared memory for the group writes and the
+    // exclusion lookups
+    const bool staged = nj <= kEmitStage;
+    if (staged)
+    {
+#pragma unroll 4
+        for (int p = tid; p < nj; p += kThreads)
         {
-            iAtom[h] = v.atom_indices[ci * kSc + h * 32 + lane];
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-        {
-            if (iAtom[h] >= 0)
-            {
-                x0[h] = v.excl_index[iAtom[h]];
-                x1[h] = v.excl_index[iAtom[h] + 1];
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-        {
-            const int cnt  = x1[h] - x0[h];
-            int       incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int t = __shfl_up_sync(full, incl, o);
-                if (lane >= o)
-                {
-                    incl += t;
-                }
-            }
-            const int tot = __shfl_sync(full, incl, 31);
-            if (nex + tot <= kExclStage)
-            {
-                const int off = nex + incl - cnt;
-                // the partners four at a time: their list entries, then their grid slots
-                for (int x = x0[h]; x < x1[h]; x += 4)
-                {
-                    int jAtom[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                    {
-                        jAtom[u] = x + u < x1[h] ? v.excl_list[x + u] : -1;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                    {
-                        if (x + u < x1[h])
-                        {
-                            sm.ex_j[off + (x + u - x0[h])] = (jAtom[u] == iAtom[h]) ? -1 : v.cells[jAtom[u]];
-                            sm.ex_i[off + (x + u - x0[h])] = (unsigned char)(h * 32 + lane);
-                        }
-                    }
-                }
-            }
-            nex += tot;
+            sm.jl[p] = rec_cj[p];
+            sm.jm[p] = rec_m[p];
         }
     }
-    const bool ex_staged = nex <= kExclStage;
+    int ex_off = 0;
+    if (warp < 2)
     {
-        const int  shift = code & 0xff;
-        const int  nj    = code >> 8;
-        const int  ncj4  = (nj + kJg - 1) / kJg;
-        const bool excludeSubDiagonal = (shift == kCentral);
-        if (lane < kNcl)
-        {
-            sm.diag_pos[lane] = -1;
-        }
-        for (int w = lane; w < 2 * kMaxCj4PerEntry / 32; w += 32)
-        {
-            sm.need[w] = 0u;
-        }
-        // the j-list is sorted on cluster index; short lists go to shared memory (four records per
-        // lane loaded at a time) for the group writes and the exclusion lookups
-        const bool staged = nj <= kEmitStage;
-        if (staged)
-        {
-            for (int p0 = 0; p0 < nj; p0 += 128)
-            {
-                int           c[4];
-                unsigned char m[4];
+        const int cnt  = x1 - x0;
+        int       incl = cnt;
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                {
-                    const int p = p0 + u * 32 + lane;
-                    c[u]        = p < nj ? rec_cj[p] : 0;
-                    m[u]        = p < nj ? rec_m[p] : 0;
-                }
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(full, incl, o);
+            if (lane >= o)
+            {
+                incl += t;
+            }
+        }
+        ex_off = incl - cnt;
+        if (lane == 31)
+        {
+            sm.ex_count[warp] = incl;
+        }
+    }
+    __syncthreads();
+    // the exclusions as (i-slot, partner grid slot) pairs when they fit; else the entry walks the exclusion lists
+    const int  nex       = sm.ex_count[0] + sm.ex_count[1];
+    const bool ex_staged = nex <= kExclStage;
+    if (ex_staged && warp < 2)
+    {
+        const int off = ex_off + (warp == 1 ? sm.ex_count[0] : 0);
+        // the partners four at a time: their list entries, then their grid slots
+        for (int x = x0; x < x1; x += 4)
+        {
+            int jAtom[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                {
-                    const int p = p0 + u * 32 + lane;
-                    if (p < nj)
-                    {
-                        sm.jl[p] = c[u];
-                        sm.jm[p] = m[u];
-                    }
-                }
+            for (int u = 0; u < 4; u++)
+            {
+                jAtom[u] = x + u < x1 ? v.excl_list[x + u] : -1;
             }
-        }
-        __syncwarp();
-        const int*           jlist = staged ? sm.jl : rec_cj;
-        const unsigned char* mlist = staged ? sm.jm : rec_m;
-        for (int g = lane; g < ncj4; g += 32)
-        {
-            Cj4      c;
-            unsigned im = 0u;
 #pragma unroll
-            for (int off = 0; off < kJg; off++)
+            for (int u = 0; u < 4; u++)
             {
-                const int p = g * kJg + off;
-                c.cj[off]   = p < nj ? jlist[p] : 0;
-                im |= p < nj ? (unsigned)mlist[p] << (off * kNcl) : 0u;
-            }
-            c.imei[0].imask    = im;
-            c.imei[0].excl_ind = 0;
-            c.imei[1]          = c.imei[0];
-            v.cj4[cj4_out + g] = c;
-            reinterpret_cast<uint2*>(v.imask_outer)[cj4_out + g] = make_uint2(im, im);
-            v.grp_pairs[cj4_out + g] = (unsigned char)__popc(im);
-        }
-        // the diagonal j-clusters (the i-cell's own clusters, central shift)
-        if (excludeSubDiagonal)
-        {
-            for (int p = lane; p < nj; p += 32)
-            {
-                const int cj = jlist[p];
-                if ((cj >> 3) == ci)
+                if (x + u < x1)
                 {
-                    sm.diag_pos[cj & (kNcl - 1)] = p;
-                    atomicOr(&sm.need[(2 * (p / kJg)) / 32], 3u << ((2 * (p / kJg)) % 32));
+                    sm.ex_j[off + (x + u - x0)] = (jAtom[u] == iAtom) ? -1 : v.cells[jAtom[u]];
+                    sm.ex_i[off + (x + u - x0)] = (unsigned char)(warp * 32 + lane);
                 }
             }
         }
-        int basei = 0;  // first exclusion mask of this entry
-        // the mask of a flagged (cj4, half) slot: masks are allocated to the flagged slots in order
-        auto excl_of_slot = [&](int slot) {
-            int x = basei;
-            for (int w = 0; w < slot / 32; w++)
-            {
-                x += __popc(sm.need[w]);
-            }
-            return x + __popc(sm.need[slot / 32] & ((1u << (slot % 32)) - 1u));
-        };
-        __syncwarp();
-        __threadfence_block();
-        if (lane == 0)
+    }
+    const int*           jlist = staged ? sm.jl : rec_cj;
+    const unsigned char* mlist = staged ? sm.jm : rec_m;
+    for (int g = tid; g < ncj4; g += kThreads)
+    {
+        Cj4      c;
+        unsigned im = 0u;
+#pragma unroll
+        for (int off = 0; off < kJg; off++)
         {
-            Sci e;
-            e.sci          = ci;
-            e.shift        = shift;
-            e.cj4_start    = cj4_out;
-            e.cj4_end      = cj4_out + ncj4;
-            v.sci[sci_out] = e;
+            const int p = g * kJg + off;
+            c.cj[off]   = p < nj ? jlist[p] : 0;
+            im |= p < nj ? (unsigned)mlist[p] << (off * kNcl) : 0u;
         }
-        // --- topology exclusions (setExclusionsForIEntry, GPU list) ---
-        const int  cjFirst     = jlist[0];
-        const int  cjLast      = jlist[nj - 1];
-        const bool diagRemoved = excludeSubDiagonal;
-        // pass A: flag (cj4, half) pairs that need an exclusion mask; pass B (rep 1): clear the bits
-        for (int rep = 0; rep < 2; rep++)
+        c.imei[0].imask    = im;
+        c.imei[0].excl_ind = 0;
+        c.imei[1]          = c.imei[0];
+        v.cj4[cj4_out + g] = c;
+        reinterpret_cast<uint2*>(v.imask_outer)[cj4_out + g] = make_uint2(im, im);
+        v.grp_pairs[cj4_out + g] = (unsigned char)__popc(im);
+    }
+    // the diagonal j-clusters (the i-cell's own clusters, central shift)
+    if (excludeSubDiagonal)
+    {
+        for (int p = tid; p < nj; p += kThreads)
         {
-            // one excluded atom pair (i-slot i of the cell, partner at grid slot jIndex)
-            auto exclude = [&](int i, int jIndex) {
-                if (diagRemoved && jIndex <= ci * kSc + i)
-                {
-                    return;
-                }
-                const int jCluster = jIndex / kCl;
-                if (jCluster < cjFirst || jCluster > cjLast)
-                {
-                    return;
-                }
-                int a = 0, b = nj - 1, index = -1;
-                while (a <= b)
-                {
-                    const int m  = (a + b) >> 1;
-                    const int cm = jlist[m];
-                    if (cm == jCluster)
-                    {
-                        index = m;
-                        break;
-                    }
-                    if (cm < jCluster)
-                    {
-                        a = m + 1;
-                    }
-                    else
-                    {
-                        b = m - 1;
-                    }
-                }
-                const int iCluster = i / kCl;
-                if (index < 0 || !((mlist[index] >> iCluster) & 1u))
-                {
-                    return;
-                }
-                const unsigned pairMask = 1u << ((index % kJg) * kNcl + iCluster);
-                const int      innerI   = i & (kCl - 1);
-                const int      innerJ   = jIndex & (kCl - 1);
-                const int      jHalf    = innerJ / (kCl / kSplit);
-                const int      slot     = 2 * (index / kJg) + jHalf;
-                if (rep == 0)
-                {
-                    atomicOr(&sm.need[slot / 32], 1u << (slot % 32));
-                }
-                else
-                {
-                    const int ei = excl_of_slot(slot);
-                    atomicAnd(&v.excl[ei].pair[(innerJ & (kCl / kSplit - 1)) * kCl + innerI], ~pairMask);
-                }
-            };
-            if (ex_staged)
+            const int cj = jlist[p];
+            if ((cj >> 3) == ci)
             {
-                for (int t = lane; t < nex; t += 32)
-                {
-                    if (sm.ex_j[t] >= 0)
-                    {
-                        exclude(sm.ex_i[t], sm.ex_j[t]);
-                    }
-                }
+                sm.diag_pos[cj & (kNcl - 1)] = p;
+                atomicOr(&sm.need[(2 * (p / kJg)) / 32], 3u << ((2 * (p / kJg)) % 32));
+            }
+        }
+    }
+    if (tid == 0)
+    {
+        Sci r;
+        r.sci       = ci;
+        r.shift     = shift;
+        r.cj4_start = cj4_out;
+        r.cj4_end   = cj4_out + ncj4;
+        v.sci[e]    = r;
+    }
+    __syncthreads();
+    // --- topology exclusions (setExclusionsForIEntry, GPU list) ---
+    const int cjFirst = jlist[0];
+    const int cjLast  = jlist[nj - 1];
+    // list position of one excluded atom pair (i-slot i of the cell, partner at grid slot jIndex), -1: not in the entry
+    auto position = [&](int i, int jIndex) {
+        if (excludeSubDiagonal && jIndex <= ci * kSc + i)
+        {
+            return -1;
+        }
+        const int jCluster = jIndex / kCl;
+        if (jCluster < cjFirst || jCluster > cjLast)
+        {
+            return -1;
+        }
+        int a = 0, b = nj - 1;
+        while (a <= b)
+        {
+            const int m  = (a + b) >> 1;
+            const int cm = jlist[m];
+            if (cm == jCluster)
+            {
+                return ((mlist[m] >> (i / kCl)) & 1u) ? m : -1;
+            }
+            if (cm < jCluster)
+            {
+                a = m + 1;
             }
             else
             {
-                for (int i = lane; i < kSc; i += 32)
-                {
-                    const int iAtom = v.atom_indices[ci * kSc + i];
-                    if (iAtom < 0)
-                    {
-                        continue;
-                    }
-                    for (int x = v.excl_index[iAtom]; x < v.excl_index[iAtom + 1]; x++)
-                    {
-                        const int jAtom = v.excl_list[x];
-                        if (jAtom != iAtom)
-                        {
-                            exclude(i, v.cells[jAtom]);
-                        }
-                    }
-                }
-            }
-            if (rep == 0)
-            {
-                // allocate the flagged masks, all interacting
-                __syncwarp();
-                int nneed = 0;
-                for (int w = 0; w < (2 * ncj4 + 31) / 32; w++)
-                {
-                    nneed += __popc(sm.need[w]);
-                }
-                if (lane == 0 && nneed > 0)
-                {
-                    basei = atomicAdd(&v.hdr->num_excl, nneed);
-                }
-                basei = __shfl_sync(full, basei, 0);
-                if (basei + nneed > v.hdr->excl_capacity)
-                {
-                    if (lane == 0)
-                    {
-                        set_status(v.hdr, kStatusExclOverflow);
-                    }
-                    return;
-                }
-                int run = basei;
-                for (int w = 0; w < (2 * ncj4 + 31) / 32; w++)
-                {
-                    unsigned bits = sm.need[w];
-                    while (bits)
-                    {
-                        const int b = __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        const int slot = w * 32 + b;
-                        v.excl[run].pair[lane] = 0xffffffffu;
-                        if (lane == 0)
-                        {
-                            v.cj4[cj4_out + slot / 2].imei[slot % 2].excl_ind = run;
-                        }
-                        run++;
-                    }
-                }
-                __syncwarp();
-                __threadfence_block();
-                // self and Newton exclusions of the diagonal cluster pairs
-                // (setSelfAndNewtonExclusionsGpu): clear j <= i
-                for (int dj = 0; dj < kNcl; dj++)
-                {
-                    const int pos = sm.diag_pos[dj];
-                    if (pos < 0)
-                    {
-                        continue;
-                    }
-                    const int off = pos % kJg;
-                    // lane = (jIndexInPart, i): word jIndexInPart*8 + i
-                    const int jip = lane >> 3, ii = lane & 7;
-                    for (int part = 0; part < kSplit; part++)
-                    {
-                        const int jOffset = part * (kCl / kSplit);
-                        if (ii >= jOffset + jip)
-                        {
-                            const int ei = excl_of_slot(2 * (pos / kJg) + part);
-                            atomicAnd(&v.excl[ei].pair[jip * kCl + ii], ~(1u << (off * kNcl + dj)));
-                        }
-                    }
-                }
-                __syncwarp();
+                b = m - 1;
             }
         }
+        return -1;
+    };
+    // the (cj4, half) slot of list position index and grid slot jIndex
+    auto slot_of = [&](int index, int jIndex) {
+        return 2 * (index / kJg) + (jIndex & (kCl - 1)) / (kCl / kSplit);
+    };
+    auto flag = [&](int slot) { atomicOr(&sm.need[slot / 32], 1u << (slot % 32)); };
+    // the mask of a flagged slot: masks are allocated to the flagged slots in order
+    auto excl_of_slot = [&](int slot) {
+        return sm.base + sm.first[slot / 32] + __popc(sm.need[slot / 32] & ((1u << (slot % 32)) - 1u));
+    };
+    auto exclude = [&](int i, int jIndex, int index) {
+        const unsigned pairMask = 1u << ((index % kJg) * kNcl + i / kCl);
+        const int      innerJ   = jIndex & (kCl - 1);
+        atomicAnd(&v.excl[excl_of_slot(slot_of(index, jIndex))].pair[(innerJ & (kCl / kSplit - 1)) * kCl + (i & (kCl - 1))],
+                  ~pairMask);
+    };
+    // without staging: f(i-slot, grid slot of the partner) for every exclusion
+    auto walk = [&](auto f) {
+        for (int i = tid; i < kSc; i += kThreads)
+        {
+            const int a = v.atom_indices[ci * kSc + i];
+            if (a < 0)
+            {
+                continue;
+            }
+            for (int x = v.excl_index[a]; x < v.excl_index[a + 1]; x++)
+            {
+                const int jAtom = v.excl_list[x];
+                if (jAtom != a)
+                {
+                    f(i, v.cells[jAtom]);
+                }
+            }
+        }
+    };
+    // flag the (cj4, half) pairs that need an exclusion mask; staged positions are kept in the thread's own slots
+    int kept[(kExclStage + kThreads - 1) / kThreads];
+    if (ex_staged)
+    {
+#pragma unroll
+        for (int u = 0; u < (kExclStage + kThreads - 1) / kThreads; u++)
+        {
+            const int t = tid + u * kThreads;
+            kept[u]     = t < nex && sm.ex_j[t] >= 0 ? position(sm.ex_i[t], sm.ex_j[t]) : -1;
+            if (kept[u] >= 0)
+            {
+                flag(slot_of(kept[u], sm.ex_j[t]));
+            }
+        }
+    }
+    else
+    {
+        walk([&](int i, int jIndex) {
+            const int index = position(i, jIndex);
+            if (index >= 0)
+            {
+                flag(slot_of(index, jIndex));
+            }
+        });
+    }
+    __syncthreads();
+    // allocate the flagged masks
+    if (warp == 0)
+    {
+        constexpr int kPer = kWords / 32;
+        int           own  = 0;
+#pragma unroll
+        for (int u = 0; u < kPer; u++)
+        {
+            own += __popc(sm.need[lane * kPer + u]);
+        }
+        int incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int t = __shfl_up_sync(full, incl, o);
+            if (lane >= o)
+            {
+                incl += t;
+            }
+        }
+        int run = incl - own;
+#pragma unroll
+        for (int u = 0; u < kPer; u++)
+        {
+            sm.first[lane * kPer + u] = run;
+            run += __popc(sm.need[lane * kPer + u]);
+        }
+        if (lane == 31)
+        {
+            sm.masks = incl;
+            sm.base  = incl > 0 ? atomicAdd(&v.hdr->num_excl, incl) : 0;
+        }
+    }
+    __syncthreads();
+    if (sm.masks == 0)
+    {
+        return;
+    }
+    if (sm.base + sm.masks > v.hdr->excl_capacity)
+    {
+        if (tid == 0)
+        {
+            set_status(v.hdr, kStatusExclOverflow);
+        }
+        return;
+    }
+    // all interacting
+    for (int w = warp; w < (2 * ncj4 + 31) / 32; w += kEmitWarps)
+    {
+        unsigned bits = sm.need[w];
+        int      run  = sm.base + sm.first[w];
+        while (bits)
+        {
+            const int slot = w * 32 + __ffs(bits) - 1;
+            bits &= bits - 1;
+            v.excl[run].pair[lane] = 0xffffffffu;
+            if (lane == 0)
+            {
+                v.cj4[cj4_out + slot / 2].imei[slot % 2].excl_ind = run;
+            }
+            run++;
+        }
+    }
+    __syncthreads();
+    // self and Newton exclusions of the diagonal cluster pairs (setSelfAndNewtonExclusionsGpu): clear j <= i;
+    // lane = (jIndexInPart, i): word jIndexInPart * 8 + i
+    for (int k = warp; k < kNcl * kSplit; k += kEmitWarps)
+    {
+        const int dj = k / kSplit, part = k % kSplit;
+        const int pos = sm.diag_pos[dj];
+        const int jip = lane >> 3, ii = lane & 7;
+        if (pos >= 0 && ii >= part * (kCl / kSplit) + jip)
+        {
+            atomicAnd(&v.excl[excl_of_slot(2 * (pos / kJg) + part)].pair[jip * kCl + ii],
+                      ~(1u << (pos % kJg * kNcl + dj)));
+        }
+    }
+    if (ex_staged)
+    {
+#pragma unroll
+        for (int u = 0; u < (kExclStage + kThreads - 1) / kThreads; u++)
+        {
+            const int t = tid + u * kThreads;
+            if (kept[u] >= 0)
+            {
+                exclude(sm.ex_i[t], sm.ex_j[t], kept[u]);
+            }
+        }
+    }
+    else
+    {
+        walk([&](int i, int jIndex) {
+            const int index = position(i, jIndex);
+            if (index >= 0)
+            {
+                exclude(i, jIndex, index);
+            }
+        });
     }
 }
 
@@ -1112,8 +1125,7 @@ cudaError_t launch_search_write(const DeviceView& v, int num_entries, cudaStream
 {
     if (num_entries > 0)
     {
-        const int blocks = (num_entries + kWarpsPerBlock - 1) / kWarpsPerBlock;
-        launch_pdl(k_search_emit, blocks, 32 * kWarpsPerBlock, 0, s, v);
+        launch_pdl(k_search_emit, num_entries, 32 * kEmitWarps, 0, s, v);
     }
     return cudaGetLastError();
 }

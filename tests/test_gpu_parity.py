@@ -137,6 +137,22 @@ def test_search_windows_match_oracle(molecules, edge, rlist):
     calc.close()
 
 
+@pytest.mark.parametrize("reach,molecules,edge,rlist", [(1, 300, 2.08, 1.0), (3, 300, 2.08, 1.0), (9, 1500, 3.56, 1.7)])
+def test_exclusion_masks_match_oracle(reach, molecules, edge, rlist):
+    """Exclusions with the `reach` neighbours on either side in atom order: cells with fewer and with more than the
+    256 exclusions that the list writer stages, and lists longer than the 512 j-clusters that it stages."""
+    s = systems.spc_water(molecules, edge, seed=17)
+    lists = [[j for j in range(max(0, a - reach), min(s.n, a + reach + 1))] for a in range(s.n)]
+    s.excl_index = np.concatenate([[0], np.cumsum([len(t) for t in lists])]).astype(np.int32)
+    s.excl_list = np.concatenate(lists).astype(np.int32)
+    calc, o = _pair(s, rlist=rlist)
+    pg, po = calc.pairlist(), o.pairlist()
+    np.testing.assert_array_equal(pg["sci"], po["sci"])
+    assert np.array_equal(canonical_pairs(pg["sci"], pg["cj4"], pg["excl"]),
+                          canonical_pairs(po["sci"], po["cj4"], po["excl"]))
+    calc.close()
+
+
 def test_balancing_leaves_forces_unchanged():
     s = systems.water_small()
     calc, _o = _pair(s)
