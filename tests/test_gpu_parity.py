@@ -66,6 +66,28 @@ def test_grid_bit_exact(name):
     np.testing.assert_array_equal(g["bb"][used], r["bb"][used])
 
 
+@pytest.mark.parametrize("form", ["water", "layers", "slab", "point", "zeros"])
+def test_grid_sort_forms(form):
+    """The z sort by bins and, where a bin overflows (layers, a thin slab, one height), by the whole column; ties in
+    every dimension, which the atom index decides; coordinates of both zeros."""
+    s = systems.lj_fcc(cells=9, lattice=0.5256, seed=2) if form != "water" else systems.spc_water(2000, 3.92, seed=3)
+    if form == "slab":
+        s.x[:, 2] *= 0.03
+    elif form == "point":
+        s.x[:, 2] = 1.25
+    elif form == "zeros":
+        s.x[::3, 2] = np.where(np.arange(len(s.x[::3])) % 2, -0.0, 0.0)
+        s.x[::2, 0] = -0.0
+    opts = nblib.NBKernelOptions(pairlist_cutoff=0.4, rcoulomb=0.35)
+    calc = nblib.ForceCalculator(s, opts)
+    o = O.Oracle(s, coulomb=0, rc=0.35, rlist=0.4)
+    o.grid()
+    g, r = calc.grid(), o.grid_arrays()
+    for k in ("cxy_ind", "num_clusters", "atom_indices", "cells", "bbcz", "xq"):
+        np.testing.assert_array_equal(g[k], r[k], err_msg=k)
+    calc.close()
+
+
 @pytest.mark.parametrize("name", list(SYSTEMS))
 def test_pairlist_bit_exact_as_sorted_sets(name):
     s = SYSTEMS[name]()
