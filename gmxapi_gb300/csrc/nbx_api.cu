@@ -22,7 +22,7 @@ namespace nbx
 {
 cudaError_t launch_search_count(const DeviceView& v, cudaStream_t s);
 cudaError_t launch_search_write(const DeviceView& v, int num_entries, cudaStream_t s);
-cudaError_t launch_balance(const DeviceView& v, int min_ci_balanced, cudaStream_t s);
+cudaError_t launch_balance(const DeviceView& v, int num_entries, int min_ci_balanced, cudaStream_t s);
 } // namespace nbx
 
 using namespace nbx;
@@ -393,7 +393,7 @@ int search_launch_write(nbx_handle* h)
         PhaseTimer t(h, 3);
         if (e == cudaSuccess) e = launch_search_write(v, h->h_hdr->num_sci, h->stream);
         // split long entries and order them large-first (the GPU list's load balancing)
-        if (e == cudaSuccess) e = launch_balance(v, h->min_ci_balanced, h->stream);
+        if (e == cudaSuccess) e = launch_balance(v, h->h_hdr->num_sci, h->min_ci_balanced, h->stream);
     }
     if (e == cudaSuccess && h->use_prune)
     {

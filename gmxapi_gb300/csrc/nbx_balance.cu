@@ -21,6 +21,8 @@
 // write pieces -> sort into the final list, all sizes from the list header.
 #include "nbx_internal.cuh"
 
+#include <algorithm>
+
 namespace nbx
 {
 namespace
@@ -45,61 +47,77 @@ __device__ __forceinline__ int balance_target(const ListHeader* hdr, int min_ci_
     return t > kMinTarget ? (int)t : kMinTarget;
 }
 
-// Walks entry e's cj4 groups (their cluster-pair counts, the bits of imei[0].imask, written by
-// the search) and returns its number of pieces; with kWrite the pieces are stored from out[0].
-template<bool kWrite>
-__device__ int split_entry(const unsigned char* __restrict__ grp_pairs, Sci e, int nsp_max, Sci* out)
+// Cuts entry e into pieces, one warp, a cj4 group per lane, and returns their number; piece(start, end) is called
+// with each, in order, by all lanes.  With P the prefix sum of the groups' cluster pairs (grp_pairs, the bits of
+// imei[0].imask, written by the search) the open piece that starts at s is cut before the first group j with
+// nsp_max - nsp < nsp + pairs(j) - nsp_max, nsp = P[j] - P[s]: P[j] + P[j + 1] > 2 (nsp_max + P[s]), found by a ballot.
+// The last two pieces are evened out by moving one group.
+template<class Piece>
+__device__ __forceinline__ int split_entry(const unsigned char* __restrict__ grp_pairs, Sci e, int nsp_max,
+                                           const Piece& piece)
 {
-    const int j4len = e.cj4_end - e.cj4_start;
+    const unsigned full  = 0xffffffffu;
+    const int      lane  = threadIdx.x & 31;
+    const int      j4len = e.cj4_end - e.cj4_start;
     if (!(nsp_max > 0 && j4len > 1 && j4len * kNcl * kJg > nsp_max))
     {
-        if (kWrite)
-        {
-            out[0] = e;
-        }
+        piece(e.cj4_start, e.cj4_end);
         return 1;
     }
-    int n   = 1;
-    int nsp = 0, nsp_sci = 0, nsp_cj4_e = 0, nsp_cj4 = 0;
-    int prev_start = e.cj4_start;  // start of the open piece
-    int last_start = e.cj4_start, last_end = e.cj4_start;  // previous closed piece
-    for (int j = e.cj4_start; j < e.cj4_end; j++)
+    int n     = 1;
+    int start = e.cj4_start, p_start = 0;          // the open piece and P at its start
+    int prev_start = e.cj4_start, prev_pairs = 0;  // the last closed piece (it ends at start) and its pairs
+    int last_pairs = 0, last_in_prev = 0;          // pairs of the group before the chunk, of the closed piece's last group
+    int carry = 0;
+    for (int c0 = e.cj4_start; c0 < e.cj4_end; c0 += 32)
     {
-        const int nsp_cj4_p = nsp_cj4;
-        nsp_cj4             = grp_pairs[j];
-        if (nsp > 0 && nsp_max - nsp < nsp + nsp_cj4 - nsp_max)
+        const int j     = c0 + lane;
+        const int pairs = j < e.cj4_end ? grp_pairs[j] : 0;
+        int       incl  = pairs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
         {
-            if (kWrite)
+            const int t = __shfl_up_sync(full, incl, o);
+            if (lane >= o)
             {
-                Sci p       = e;
-                p.cj4_start = prev_start;
-                p.cj4_end   = j;
-                out[n - 1]  = p;
+                incl += t;
             }
-            last_start = prev_start;
-            last_end   = j;
-            prev_start = j;
-            n++;
-            nsp_sci   = nsp;
-            nsp_cj4_e = nsp_cj4_p;
-            nsp       = 0;
         }
-        nsp += nsp_cj4;
-    }
-    if (kWrite)
-    {
-        Sci p       = e;
-        p.cj4_start = prev_start;
-        p.cj4_end   = e.cj4_end;
-        out[n - 1]  = p;
-        // even out the last two pieces by moving one cj4 group
-        if (n >= 2 && nsp_sci - nsp_cj4_e >= nsp + nsp_cj4_e)
+        incl += carry;
+        const int below  = incl - pairs;
+        int       before = __shfl_up_sync(full, pairs, 1);  // pairs of group j - 1
+        before           = lane == 0 ? last_pairs : before;
+        for (;;)
         {
-            out[n - 2].cj4_end   = last_end - 1;
-            out[n - 1].cj4_start = last_end - 1;
+            const unsigned cut =
+                    __ballot_sync(full, j < e.cj4_end && below > p_start && below + incl > 2 * (nsp_max + p_start));
+            if (cut == 0u)
+            {
+                break;
+            }
+            const int src = __ffs(cut) - 1;
+            if (n > 1)
+            {
+                piece(prev_start, start);
+            }
+            prev_start   = start;
+            start        = c0 + src;
+            const int ps = __shfl_sync(full, below, src);
+            prev_pairs   = ps - p_start;
+            last_in_prev = __shfl_sync(full, before, src);
+            p_start      = ps;
+            n++;
         }
+        last_pairs = __shfl_sync(full, pairs, 31);
+        carry      = __shfl_sync(full, incl, 31);
     }
-    (void)last_start;
+    if (n > 1)
+    {
+        const int cut = prev_pairs - last_in_prev >= carry - p_start + last_in_prev ? start - 1 : start;
+        piece(prev_start, cut);
+        start = cut;
+    }
+    piece(start, e.cj4_end);
     return n;
 }
 
@@ -131,20 +149,25 @@ __global__ void k_balance_count(DeviceView v, int min_ci_balanced)
     }
     const int nsp_max = balance_target(hdr, min_ci_balanced);
     const int nsci    = hdr->num_sci;
-    const int e       = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e == 0)
+    const int t       = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0)
     {
         v.hdr->nsp_max         = nsp_max;
         v.hdr->num_sci_unsplit = nsci;
     }
-    for (int k = e; k < kSortChunks * kSizeClasses; k += gridDim.x * blockDim.x)
+    for (int k = t; k < kSortChunks * kSizeClasses; k += gridDim.x * blockDim.x)
     {
         sort_hist(v)[k] = 0;
     }
     // nothing is split: every entry is one piece, at its own place
+    const int e = t >> 5;
     if (nsp_max > 0 && e < nsci)
     {
-        v.sci_pieces[e] = split_entry<false>(v.grp_pairs, v.sci[e], nsp_max, nullptr);
+        const int n = split_entry(v.grp_pairs, v.sci[e], nsp_max, [](int, int) {});
+        if ((t & 31) == 0)
+        {
+            v.sci_pieces[e] = n;
+        }
     }
 }
 
@@ -250,19 +273,36 @@ __global__ void k_balance_write(DeviceView v)
     {
         return;
     }
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e < hdr->num_sci_unsplit)
+    // entries per chunk and class for the sort
+    const int m     = largest_class(hdr, hdr->num_sci_split);
+    const int chunk = sort_chunk(hdr->num_sci_split);
+    auto      put   = [&](int p, const Sci& e, int start, int end) {
+        const int len = end - start;
+        v.sci_tmp[p]  = Sci{ e.sci, e.shift, start, end };
+        atomicAdd(&sort_hist(v)[p / chunk * kSizeClasses + (len < m ? len : m)], 1);
+    };
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (hdr->nsp_max == 0)
     {
-        const int first = hdr->nsp_max > 0 ? v.sci_pieces[e] : e;
-        const int count = split_entry<true>(v.grp_pairs, v.sci[e], hdr->nsp_max, v.sci_tmp + first);
-        // entries per chunk and class for the sort
-        const int m     = largest_class(hdr, hdr->num_sci_split);
-        const int chunk = sort_chunk(hdr->num_sci_split);
-        for (int p = first; p < first + count; p++)
+        if (t < hdr->num_sci_unsplit)
         {
-            const int len = v.sci_tmp[p].cj4_end - v.sci_tmp[p].cj4_start;
-            atomicAdd(&sort_hist(v)[p / chunk * kSizeClasses + (len < m ? len : m)], 1);
+            const Sci e = v.sci[t];
+            put(t, e, e.cj4_start, e.cj4_end);
         }
+        return;
+    }
+    const int i = t >> 5;
+    if (i < hdr->num_sci_unsplit)
+    {
+        const Sci e = v.sci[i];
+        int       p = v.sci_pieces[i];
+        split_entry(v.grp_pairs, e, hdr->nsp_max, [&](int start, int end) {
+            if ((t & 31) == 0)
+            {
+                put(p, e, start, end);
+            }
+            p++;
+        });
     }
 }
 
@@ -383,10 +423,12 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_entries(DeviceView v)
 
 } // namespace
 
-cudaError_t launch_balance(const DeviceView& v, int min_ci_balanced, cudaStream_t s)
+cudaError_t launch_balance(const DeviceView& v, int num_entries, int min_ci_balanced, cudaStream_t s)
 {
+    // a warp per entry: a thread per entry walked its groups one after the other (45k atoms, 1165 entries of 40
+    // groups: writing 11.3 us, now 6.4 us; counting 4.7 us as before)
     const int tb     = 256;
-    const int blocks = (v.sci_cap + tb - 1) / tb;
+    const int blocks = std::max((num_entries + tb / 32 - 1) / (tb / 32), 1);
     launch_pdl(k_balance_count, blocks, tb, 0, s, v, min_ci_balanced);
     launch_pdl(k_balance_scan, 1, 1024, 0, s, v);
     launch_pdl(k_balance_write, blocks, tb, 0, s, v);
