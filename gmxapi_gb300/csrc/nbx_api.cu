@@ -51,8 +51,12 @@ struct nbx_handle
     double* d_out = nullptr;  // energies[2] + virial[9]
     unsigned long long* d_count = nullptr;
     ListHeader* h_hdr = nullptr;  // pinned copy for reading sizes
-    double*     h_out = nullptr;  // pinned copy of the energies and virial (11 doubles)
+    double*     h_out = nullptr;  // pinned copy of the energies and virial (11 doubles) and the list status
     double*     d_hout = nullptr; // h_out's device address when the device can write it directly
+    unsigned*   d_status = nullptr; // where this call's kernels report the list status (in d_hout), or nullptr
+    float*      h_stage = nullptr;  // pinned coordinates and forces that stand in for pageable host arrays
+    float*      d_stage = nullptr;  // its device address
+    size_t      stage_f = 0;        // first force in h_stage (floats)
     bool        x_host = false;   // this call's coordinates / forces are host memory used in place
     bool        f_host = false;
     // adjoint scratch, allocated on the first backward call
@@ -477,7 +481,7 @@ int compute_async(nbx_handle* h, const float* d_x, float* d_f, double* d_e, doub
             collect_timings(h, false);
         }
     }
-    if (e == cudaSuccess) e = launch_reduce_f(v, d_f, d_e, d_vir, h->stream, h->f_host);
+    if (e == cudaSuccess) e = launch_reduce_f(v, d_f, d_e, d_vir, h->stream, h->f_host, h->d_status);
     h->force_launches += 1;
     h->launches += 3 + (v.vdw_mod == NBX_VDW_LJPME && energy ? 1 : 0) + (h->fep_on ? 1 : 0);
     return cuda_check(h, e, "compute");
@@ -488,15 +492,85 @@ int compute_async(nbx_handle* h, const float* d_x, float* d_f, double* d_e, doub
 // addressing), or nullptr: then the array is staged by copies.  Kernels then read the
 // coordinates from and write the forces to host memory over the host link, overlapping
 // the transfer with the kernels that use it.
-void* mapped_device_ptr(const void* p)
+void* mapped_device_ptr(const void* p, bool* pageable = nullptr)
 {
     cudaPointerAttributes a{};
+    if (pageable)
+    {
+        *pageable = false;
+    }
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
     {
         cudaGetLastError();
         return nullptr;
     }
+    if (pageable)
+    {
+        *pageable = a.type == cudaMemoryTypeUnregistered;
+    }
     return (a.type == cudaMemoryTypeHost && a.devicePointer) ? a.devicePointer : nullptr;
+}
+
+// Pageable coordinates and forces of up to this many atoms go through pinned memory that the kernels use in place: a
+// copy on the CPU against one by the driver on the stream.  Beside mapped arrays, coordinates cost 3 / 8.5 / 13 us at
+// 6 000 / 24 000 / 60 000 atoms by the CPU, 9.4 / 11.4 / 12.7 us by the driver; forces, which the CPU reads back from
+// memory, 3.7 / 16 us at 6 000 / 24 000 atoms against 9.5 / 10 us.
+constexpr int kStageAtoms      = 32768;
+constexpr int kStageForceAtoms = 12288;
+
+void alloc_stage(nbx_handle* h)
+{
+    if (h->n > kStageAtoms || !h->d_hout)
+    {
+        return;
+    }
+    h->stage_f = ((size_t)3 * h->n + 63) / 64 * 64;
+    if (cudaMallocHost(&h->h_stage, sizeof(float) * (h->n <= kStageForceAtoms ? 2 : 1) * h->stage_f) != cudaSuccess)
+    {
+        cudaGetLastError();
+        h->h_stage = nullptr;
+        return;
+    }
+    h->d_stage = static_cast<float*>(mapped_device_ptr(h->h_stage));
+}
+
+// Where the kernels of a host-array call read its coordinates: the array itself when it is mapped pinned memory, the
+// staging memory, or d_x after a copy on the stream (always with in_place false).
+cudaError_t host_coordinates(nbx_handle* h, const float* x, bool in_place, const float** d_x)
+{
+    const size_t bytes = sizeof(float) * 3 * h->n;
+    bool         page  = false;
+    *d_x               = in_place ? static_cast<const float*>(mapped_device_ptr(x, &page)) : nullptr;
+    if (page && h->d_stage)
+    {
+        std::memcpy(h->h_stage, x, bytes);
+        *d_x = h->d_stage;
+    }
+    if (*d_x)
+    {
+        return cudaSuccess;
+    }
+    *d_x = h->d_x;
+    return cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, h->stream);
+}
+
+// Where they write its forces; nullptr: to d_f, copied on the stream.
+float* host_forces(nbx_handle* h, float* f)
+{
+    bool         page = false;
+    float* const d_f  = static_cast<float*>(mapped_device_ptr(f, &page));
+    return page && h->d_stage && h->n <= kStageForceAtoms ? h->d_stage + h->stage_f : d_f;
+}
+
+// Waits for a host-array call; then the staged forces, when d_f is the staging memory.
+cudaError_t finish_host_call(nbx_handle* h, float* f, const float* d_f)
+{
+    const cudaError_t e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess && d_f && d_f == h->d_stage + h->stage_f)
+    {
+        std::memcpy(f, h->h_stage + h->stage_f, sizeof(float) * 3 * h->n);
+    }
+    return e;
 }
 
 bool valid_box(const float* box)
@@ -587,7 +661,8 @@ const char* nbx_last_error(const nbx_handle* h)
     return h ? h->err.c_str() : g_create_error.c_str();
 }
 
-int nbx_create(const nbx_system_desc* sys, const nbx_options* opts_in, int device, nbx_handle** out)
+// nbx_create without what only host-array calls use (the systems of a batch have none).
+static int create_handle(const nbx_system_desc* sys, const nbx_options* opts_in, int device, nbx_handle** out)
 {
     if (!sys || !out)
     {
@@ -860,7 +935,7 @@ int nbx_create(const nbx_system_desc* sys, const nbx_options* opts_in, int devic
     if (e == cudaSuccess) e = dalloc(h, &h->d_out, 11);
     if (e == cudaSuccess) e = dalloc(h, &h->d_count, 1);
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_hdr, sizeof(ListHeader));
-    if (e == cudaSuccess) e = cudaMallocHost(&h->h_out, 11 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMallocHost(&h->h_out, 12 * sizeof(double));
     if (e == cudaSuccess) h->d_hout = static_cast<double*>(mapped_device_ptr(h->h_out));
     if (e == cudaSuccess) e = cudaMemcpyAsync(q, sys->q, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(t, sys->type, sizeof(int) * n, cudaMemcpyHostToDevice, h->stream);
@@ -893,6 +968,16 @@ int nbx_create(const nbx_system_desc* sys, const nbx_options* opts_in, int devic
     return NBX_OK;
 }
 
+int nbx_create(const nbx_system_desc* sys, const nbx_options* opts_in, int device, nbx_handle** out)
+{
+    const int rc = create_handle(sys, opts_in, device, out);
+    if (rc == NBX_OK)
+    {
+        alloc_stage(*out);
+    }
+    return rc;
+}
+
 int nbx_destroy(nbx_handle* h)
 {
     if (!h)
@@ -912,6 +997,7 @@ int nbx_destroy(nbx_handle* h)
     {
         cudaFreeHost(h->h_hdr);
         cudaFreeHost(h->h_out);
+        cudaFreeHost(h->h_stage);
     }
     for (auto& p : h->ev_pending)
     {
@@ -992,42 +1078,49 @@ int nbx_compute(nbx_handle* h, const float* x, float* f, double* energies, doubl
     }
     cudaSetDevice(h->device);
     const size_t bytes = sizeof(float) * 3 * h->n;
-    // mapped pinned arrays are read / written by the kernels in place; others are copied
-    const float* d_x = static_cast<const float*>(mapped_device_ptr(x));
-    float*       d_f = static_cast<float*>(mapped_device_ptr(f));
-    if (!d_x)
-    {
-        const int rc = cuda_check(h, cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, h->stream),
-                                  "nbx_compute H2D");
-        if (rc != NBX_OK)
-        {
-            return rc;
-        }
-        d_x = h->d_x;
-    }
-    // host arrays: forces are overwritten (GmxForceCalculator::compute), whatever nbx_set_force_accumulate says
-    const int accumulate = h->v.accumulate_f;
-    h->v.accumulate_f    = 0;
-    h->x_host = d_x != h->d_x;
-    h->f_host = d_f != nullptr;
-    int rc = compute_async(h, d_x, d_f ? d_f : h->d_f, energies ? h->d_out : nullptr, virial ? h->d_out + 2 : nullptr);
-    h->v.accumulate_f = accumulate;
-    h->x_host = h->f_host = false;
+    const float* d_x   = nullptr;
+    int          rc    = cuda_check(h, host_coordinates(h, x, true, &d_x), "nbx_compute H2D");
     if (rc != NBX_OK)
     {
         return rc;
     }
-    cudaError_t e = d_f ? cudaSuccess : cudaMemcpyAsync(f, h->d_f, bytes, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess && (energies || virial))
+    float* const  d_f   = host_forces(h, f);
+    // energies, virial and list status: written by the finishing kernel into the pinned h_out when the device can
+    // address it, else copied
+    double* const d_out = h->d_hout ? h->d_hout : h->d_out;
+    // host arrays: forces are overwritten (GmxForceCalculator::compute), whatever nbx_set_force_accumulate says
+    const int accumulate = h->v.accumulate_f;
+    h->v.accumulate_f    = 0;
+    h->x_host   = d_x != h->d_x;
+    h->f_host   = d_f != nullptr;
+    h->d_status = h->d_hout ? reinterpret_cast<unsigned*>(h->d_hout + 11) : nullptr;
+    rc = compute_async(h, d_x, d_f ? d_f : h->d_f, energies ? d_out : nullptr, virial ? d_out + 2 : nullptr);
+    h->v.accumulate_f = accumulate;
+    h->x_host = h->f_host = false;
+    h->d_status = nullptr;
+    if (rc != NBX_OK)
     {
-        e = cudaMemcpyAsync(h->h_out, h->d_out, 11 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        cudaStreamSynchronize(h->stream);  // the staging memory may still be read
+        return rc;
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h->h_hdr, h->v.hdr, sizeof(ListHeader), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaError_t e = d_f ? cudaSuccess : cudaMemcpyAsync(f, h->d_f, bytes, cudaMemcpyDeviceToHost, h->stream);
+    if (!h->d_hout)
+    {
+        if (e == cudaSuccess && (energies || virial))
+        {
+            e = cudaMemcpyAsync(h->h_out, h->d_out, 11 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        }
+        if (e == cudaSuccess)
+        {
+            e = cudaMemcpyAsync(h->h_out + 11, &h->v.hdr->status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream);
+        }
+    }
+    if (e == cudaSuccess) e = finish_host_call(h, f, d_f);
     if ((rc = cuda_check(h, e, "nbx_compute D2H")) != NBX_OK)
     {
         return rc;
     }
+    h->h_hdr->status = *reinterpret_cast<const unsigned*>(h->h_out + 11);
     if (energies)
     {
         energies[0] = h->h_out[0];
@@ -1156,21 +1249,15 @@ int nbx_md_step(nbx_handle* h, long long step, const float* x, float* f, double*
     }
     cudaSetDevice(h->device);
     const size_t bytes = sizeof(float) * 3 * h->n;
-    // mapped pinned arrays are read / written by the kernels in place, except the
-    // coordinates of a search step (the gridding passes read them several times)
+    // not in place on a search step: the gridding passes read the coordinates several times
     const bool   search = !h->have_list || step % std::max(1, h->opts.nstlist) == 0;
-    const float* d_x    = search ? nullptr : static_cast<const float*>(mapped_device_ptr(x));
-    float*       d_f    = static_cast<float*>(mapped_device_ptr(f));
-    if (!d_x)
+    const float* d_x    = nullptr;
+    int          rc     = cuda_check(h, host_coordinates(h, x, !search, &d_x), "nbx_md_step H2D");
+    if (rc != NBX_OK)
     {
-        const int rc = cuda_check(h, cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, h->stream),
-                                  "nbx_md_step H2D");
-        if (rc != NBX_OK)
-        {
-            return rc;
-        }
-        d_x = h->d_x;
+        return rc;
     }
+    float* const d_f = host_forces(h, f);
     const int accumulate = h->v.accumulate_f;  // host arrays: forces are overwritten
     h->v.accumulate_f    = 0;
     // energies and virial: written by the finishing kernel into the pinned h_out when the
@@ -1178,12 +1265,13 @@ int nbx_md_step(nbx_handle* h, long long step, const float* x, float* f, double*
     double* d_out = h->d_hout ? h->d_hout : h->d_out;
     h->x_host     = d_x != h->d_x;
     h->f_host     = d_f != nullptr;
-    int     rc    = nbx_md_step_device(h, step, d_x, d_f ? d_f : h->d_f, energies ? d_out : nullptr,
+    rc            = nbx_md_step_device(h, step, d_x, d_f ? d_f : h->d_f, energies ? d_out : nullptr,
                                        virial ? d_out + 2 : nullptr);
     h->v.accumulate_f = accumulate;
     h->x_host = h->f_host = false;
     if (rc != NBX_OK)
     {
+        cudaStreamSynchronize(h->stream);  // the staging memory may still be read
         return rc;
     }
     cudaError_t e = d_f ? cudaSuccess : cudaMemcpyAsync(f, h->d_f, bytes, cudaMemcpyDeviceToHost, h->stream);
@@ -1191,7 +1279,7 @@ int nbx_md_step(nbx_handle* h, long long step, const float* x, float* f, double*
     {
         e = cudaMemcpyAsync(h->h_out, h->d_out, 11 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) e = finish_host_call(h, f, d_f);
     if ((rc = cuda_check(h, e, "nbx_md_step D2H")) != NBX_OK)
     {
         return rc;
@@ -2308,7 +2396,7 @@ int nbx_batch_create(int num_systems, const nbx_system_desc* systems, const nbx_
     for (int i = 0; i < num_systems && e == cudaSuccess; i++)
     {
         nbx_handle* h  = nullptr;
-        int         rc = nbx_create(&systems[i], &b->opts, device, &h);
+        int         rc = create_handle(&systems[i], &b->opts, device, &h);
         if (rc != NBX_OK)
         {
             std::string msg = "system " + std::to_string(i) + ": " + nbx_last_error(nullptr);

@@ -242,9 +242,14 @@ constexpr int kReduceAtoms   = 4;
 constexpr int kReduceThreads = 256;
 
 __global__ void __launch_bounds__(kReduceThreads)
-        k_reduce_f(DeviceView v, float* __restrict__ f, int do_virial, double* d_energies, double* d_virial, int stage)
+        k_reduce_f(DeviceView v, float* __restrict__ f, int do_virial, double* d_energies, double* d_virial, int stage,
+                   unsigned* d_status)
 {
     pdl_begin();
+    if (d_status && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        *d_status = v.hdr->status;
+    }
     float w[9];
 #pragma unroll
     for (int k = 0; k < 9; k++)
@@ -620,11 +625,12 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_f(const DeviceView& v, float* d_f, double* d_e, double* d_vir, cudaStream_t s, bool stage)
+cudaError_t launch_reduce_f(const DeviceView& v, float* d_f, double* d_e, double* d_vir, cudaStream_t s, bool stage,
+                            unsigned* d_status)
 {
     const int per_block = kReduceThreads * kReduceAtoms;
     launch_pdl(k_reduce_f, (v.n + per_block - 1) / per_block, kReduceThreads, 0, s, v, d_f, d_vir ? 1 : 0, d_e,
-               d_vir, stage ? 1 : 0);
+               d_vir, stage ? 1 : 0, d_status);
     return cudaGetLastError();
 }
 
@@ -856,7 +862,8 @@ extern "C" int nbx_compute_noalloc(const nbx_noalloc_args* a, float* d_f, double
             launch_k_force<false, false, 0>(v, blocks, smem, s, ctr);
         }
         launch_pdl(k_reduce_f, (v.n + kReduceThreads * kReduceAtoms - 1) / (kReduceThreads * kReduceAtoms),
-                   kReduceThreads, 0, s, v, d_f, d_virial ? 1 : 0, nullptr, nullptr, 0);
+                   kReduceThreads, 0, s, v, d_f, d_virial ? 1 : 0, nullptr, nullptr, 0,
+                        static_cast<unsigned*>(nullptr));
         if (energy)
         {
             launch_pdl(k_finish, 1, 32, 0, s, v, d_energies, d_virial);

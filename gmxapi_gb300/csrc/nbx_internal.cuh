@@ -479,9 +479,10 @@ cudaError_t launch_force_x2(const DeviceView& v, bool energy, cudaStream_t s, in
 cudaError_t launch_force_x2_lj(const DeviceView& v, int lj, bool energy, cudaStream_t s, int num_sms, int* counter);
 // forces to atom order (+ virial); with d_e / d_vir the last block also finishes the energies
 // and virial (the accumulators must have been cleared by launch_convert_x(clear))
-// (stage: write the forces through shared memory as contiguous floats, for f in host memory)
+// (stage: write the forces through shared memory as contiguous floats, for f in host memory); d_status (or
+// nullptr) receives the status bits of the list header
 cudaError_t launch_reduce_f(const DeviceView& v, float* d_f, double* d_e, double* d_vir, cudaStream_t s,
-                            bool stage = false);
+                            bool stage = false, unsigned* d_status = nullptr);
 cudaError_t launch_pair_count(const DeviceView& v, unsigned long long* d_out, cudaStream_t s);
 cudaError_t measure_fp32_peak(double* tflops);
 cudaError_t launch_batch_prune(const BatchSys* sys, const int* entry_prefix, int nsys, float outer2, float inner2,

@@ -81,3 +81,29 @@ def test_one_mapped_array_and_one_pageable(pinned):
         assert np.allclose(b.energies, a.energies, rtol=1e-9, atol=0.0), step
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("molecules", [1, 333, 4096, 4097, 10922, 10923])
+@pytest.mark.parametrize("energies", [True, False])
+def test_pageable_host_arrays_match_device_arrays(molecules, energies):
+    """Pageable arrays on either side of the sizes up to which forces (12,288 atoms) and coordinates (32,768) are staged, mixed
+    with mapped ones, overwritten and read again on the next call: the forces of the device call to 1e-6."""
+    s = systems.spc_water(molecules, max(2.2, (molecules * 0.0299) ** (1 / 3)), seed=14)
+    c = nblib.ForceCalculator(s, _opts())
+    ft, fp = _pinned(np.zeros_like(s.x, np.float32))
+    x = s.x.astype(np.float32).copy()
+    f = np.full_like(x, 7.0)
+    for k in range(3):
+        x += np.float32(0.002 * (k - 1))
+        d = torch.from_numpy(x).cuda()
+        df = torch.empty_like(d)
+        ev = torch.zeros(11, dtype=torch.float64, device="cuda")
+        c.compute_device(d.data_ptr(), df.data_ptr(), ev.data_ptr(), ev.data_ptr() + 16)
+        c.synchronize()
+        want = df.cpu().numpy().astype(np.float64)
+        for out in (f, fp):
+            c.compute(x, forces=out, energies=energies)
+            assert rel_rms(out.astype(np.float64), want) <= 1e-6
+            if energies:
+                assert np.allclose(c.energies, ev[:2].cpu().numpy(), rtol=1e-9, atol=0.0)
+    c.close()
