@@ -726,12 +726,15 @@ __global__ void k_batch_set_q(const BatchSys* __restrict__ sys, BatchMap map, co
     }
 }
 
+constexpr int kLossThreads = 256;
+
 // Loss sum |F - F_target|^2 (FP64) and its gradient 2 (F - F_target) per coordinate.
 __global__ void k_match_loss(const float* __restrict__ f, const float* __restrict__ ft, size_t n3, float* gF,
                              double* loss)
 {
     pdl_begin();
-    double acc = 0.0;
+    __shared__ double sum[kLossThreads / 32];
+    double            acc = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x)
     {
         const float d = f[i] - ft[i];
@@ -742,9 +745,21 @@ __global__ void k_match_loss(const float* __restrict__ f, const float* __restric
     {
         acc += __shfl_xor_sync(0xffffffffu, acc, o);
     }
-    if ((threadIdx.x & 31) == 0 && acc != 0.0)
+    if ((threadIdx.x & 31) == 0)
     {
-        atomicAdd(loss, acc);
+        sum[threadIdx.x >> 5] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        for (int w = 1; w < kLossThreads / 32; w++)
+        {
+            acc += sum[w];
+        }
+        if (acc != 0.0)
+        {
+            atomicAdd(loss, acc);
+        }
     }
 }
 
@@ -850,6 +865,9 @@ __global__ void k_lb_table(const double* __restrict__ sig, const double* __restr
     }
 }
 
+constexpr int kLbThreads = 256;
+constexpr int kLbTerms   = 12;  // 55 types, what two tables in 48 KB allow
+
 // Its adjoint: d L / d sigma_k and d L / d epsilon_k from d L / d table (one block; every type's
 // sums run over its row and column in a fixed order).  d epsilon_ij / d epsilon_i is written
 // epsilon_j / (2 epsilon_ij), as the derivative of the square root of the product.
@@ -874,15 +892,39 @@ __global__ void k_lb_table_backward(const double* __restrict__ sig, const double
         ge[m] = g6 * 24.0 * s6 + g12 * 48.0 * s6 * s6;
     }
     __syncthreads();
+    // the terms of row k (sigma_k, epsilon_k as the first index) and column k (as the second) in place of the
+    // derivatives, a thread each: square roots and quotients in FP64 one after the other took most of 10.8 us
+    double ts[kLbTerms], te[kLbTerms];
+#pragma unroll
+    for (int u = 0; u < kLbTerms; u++)
+    {
+        const int m = threadIdx.x + u * kLbThreads;
+        if (m < nt * nt)
+        {
+            const int k = m / nt, j = m - k * nt;
+            ts[u]       = 0.5 * gs[m] + 0.5 * gs[j * nt + k];
+            te[u]       = (ge[m] + ge[j * nt + k]) * (eps[j] / (2.0 * sqrt(eps[k] * eps[j])));
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLbTerms; u++)
+    {
+        const int m = threadIdx.x + u * kLbThreads;
+        if (m < nt * nt)
+        {
+            gs[m] = ts[u];
+            ge[m] = te[u];
+        }
+    }
+    __syncthreads();
     for (int k = threadIdx.x; k < nt; k += blockDim.x)
     {
         double as = 0.0, ae = 0.0;
         for (int j = 0; j < nt; j++)
         {
-            const double eij = sqrt(eps[k] * eps[j]);
-            // row k (sigma_k, epsilon_k as the first index) and column k (as the second)
-            as += 0.5 * gs[k * nt + j] + 0.5 * gs[j * nt + k];
-            ae += (ge[k * nt + j] + ge[j * nt + k]) * (eps[j] / (2.0 * eij));
+            as += gs[k * nt + j];
+            ae += ge[k * nt + j];
         }
         gsig[k] = as;
         geps[k] = ae;
@@ -905,7 +947,7 @@ cudaError_t launch_lb_table(const double* sig, const double* eps, int nt, double
 cudaError_t launch_lb_table_backward(const double* sig, const double* eps, int nt, const double* gtable,
                                      double* gsig, double* geps, cudaStream_t s)
 {
-    launch_pdl(k_lb_table_backward, 1, 256, 2 * sizeof(double) * nt * nt, s, sig, eps, nt, gtable, gsig, geps);
+    launch_pdl(k_lb_table_backward, 1, kLbThreads, 2 * sizeof(double) * nt * nt, s, sig, eps, nt, gtable, gsig, geps);
     return cudaGetLastError();
 }
 
@@ -1012,7 +1054,9 @@ cudaError_t launch_match_loss(const float* d_f, const float* d_ft, size_t n3, fl
                               int num_sms, cudaStream_t s)
 {
     cudaMemsetAsync(d_loss, 0, sizeof(double), s);
-    launch_pdl(k_match_loss, num_sms * 4, 256, 0, s, d_f, d_ft, n3, d_gF, d_loss);
+    const size_t need = (n3 + kLossThreads - 1) / kLossThreads;
+    launch_pdl(k_match_loss, (int)std::max<size_t>(1, std::min<size_t>(need, num_sms * 4)), kLossThreads, 0, s, d_f, d_ft,
+               n3, d_gF, d_loss);
     return cudaGetLastError();
 }
 

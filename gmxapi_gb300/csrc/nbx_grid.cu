@@ -595,6 +595,32 @@ __global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear
 {
     pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    // every load before the first store, which may alias it
+    int a = -1, k = t;
+    if (atom_order)
+    {
+        if (t < v.n)
+        {
+            k = v.cells[t];
+            a = (unsigned)k < (unsigned)(v.g.cells_capacity * kSc) ? t : -1;
+        }
+    }
+    else if (t < v.hdr->num_cells * kSc)
+    {
+        a = v.atom_indices[k];
+    }
+    float c[3], q = 0.0f;
+    int   code = 0, type = 0;
+    if (a >= 0)
+    {
+        for (int d = 0; d < 3; d++)
+        {
+            c[d] = x[3 * a + d];
+        }
+        q    = v.xq[k].w;
+        code = v.image[a];
+        type = v.tgrid[k];
+    }
     if (clear)
     {
         if (t < v.g.cells_capacity * kSc)
@@ -603,9 +629,9 @@ __global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear
         }
         if (blockIdx.x == 0)
         {
-            for (int k = threadIdx.x; k < kNShift * 3; k += blockDim.x)
+            for (int i = threadIdx.x; i < kNShift * 3; i += blockDim.x)
             {
-                v.fshift[k] = 0.0;
+                v.fshift[i] = 0.0;
             }
             if (threadIdx.x < 2)
             {
@@ -622,44 +648,17 @@ __global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear
             }
         }
     }
-    int a, k;
-    if (atom_order)
+    if (a >= 0)
     {
-        a = t;
-        if (a >= v.n)
+        for (int d = 0; d < 3; d++)
         {
-            return;
+            const int s = (int)(signed char)((code >> (8 * d)) & 0xff);
+            c[d]        = (s == 0) ? c[d] : c[d] + (float)s * v.g.box[d];
         }
-        k = v.cells[a];
-        if ((unsigned)k >= (unsigned)(v.g.cells_capacity * kSc))
-        {
-            return;
-        }
+        v.xq[k] = make_float4(c[0], c[1], c[2], q);
+        // the cluster-packed copy (charges and types too: they may change between searches)
+        write_packed_slot(v.xqp, k, c[0], c[1], c[2], q, type);
     }
-    else
-    {
-        k = t;
-        if (k >= v.hdr->num_cells * kSc)
-        {
-            return;
-        }
-        a = v.atom_indices[k];
-        if (a < 0)
-        {
-            return;
-        }
-    }
-    const float4 old  = v.xq[k];
-    const int    code = v.image[a];
-    float        c[3];
-    for (int d = 0; d < 3; d++)
-    {
-        const int s = (int)(signed char)((code >> (8 * d)) & 0xff);
-        c[d]        = (s == 0) ? x[3 * a + d] : x[3 * a + d] + (float)s * v.g.box[d];
-    }
-    v.xq[k] = make_float4(c[0], c[1], c[2], old.w);
-    // the cluster-packed copy (charges and types too: they may change between searches)
-    write_packed_slot(v.xqp, k, c[0], c[1], c[2], old.w, v.tgrid[k]);
 }
 
 // After a search: the cluster-packed copy of every grid slot, fillers included (the coordinate
