@@ -340,3 +340,36 @@ def test_filed_atoms_match_oracle(pm, layout, grid):
         assert np.abs(p.virial - vir).max() <= ENERGY_RTOL * np.abs(vir).max()
         x = np.roll(x, 5, axis=0)
     p.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32768, 32769])
+def test_gather_shapes_give_the_field_of_the_grid(n):
+    """Direct gather with four threads per atom (up to 32,768 atoms) and with one, beyond: against the sum over the
+    64 points in FP64 from the engine's own splines, on a random potential; atoms without charge get nothing.  The
+    float sum of 64 products of weights that add up to 1 (derivatives: to 2 in magnitude) errs by at most 66 roundings
+    of the largest product sum, 8e-6 of max |f|."""
+    from gmxapi_gb300 import pme
+
+    rng = np.random.default_rng(n)
+    grid, box = (20, 24, 30), [2.1, 2.5, 2.9]
+    p = pme.Pme(box, grid, 3.1)
+    x = (rng.uniform(-0.5, 1.5, (n, 3)) * box).astype(np.float32)
+    q = rng.uniform(-1, 1, n).astype(np.float32)
+    q[::5] = 0.0
+    phi = rng.standard_normal(grid).astype(np.float32)
+    dx, dq, dp = (torch.from_numpy(np.ascontiguousarray(t)).cuda() for t in (x, q, phi))
+    f = torch.zeros((n, 3), dtype=torch.float32, device="cuda")
+    idx = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    th, dth = (torch.zeros((3, n, 4), dtype=torch.float32, device="cuda") for _ in range(2))
+    p.splines_device(n, dx.data_ptr(), idx.data_ptr(), th.data_ptr(), dth.data_ptr())
+    p.gather_device(n, dx.data_ptr(), dq.data_ptr(), dp.data_ptr(), f.data_ptr())
+    torch.cuda.synchronize()
+    idx, th, dth = idx.cpu().numpy(), th.cpu().numpy().astype(np.float64), dth.cpu().numpy().astype(np.float64)
+    g = [(idx[:, d, None] + np.arange(4)) % grid[d] for d in range(3)]
+    v = phi.astype(np.float64)[g[0][:, :, None, None], g[1][:, None, :, None], g[2][:, None, None, :]]
+    want = np.empty((n, 3))
+    for d in range(3):
+        w = [dth[k] if k == d else th[k] for k in range(3)]
+        want[:, d] = -q * np.einsum("nxyz,nx,ny,nz->n", v, *w) * grid[d] / box[d]
+    assert np.abs(f.cpu().numpy() - want).max() <= 8e-6 * max(np.abs(want).max(), 1e-6)
+    p.close()
