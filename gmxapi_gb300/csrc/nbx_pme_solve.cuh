@@ -36,12 +36,11 @@ struct PmeTotals
 // serialise in L2.
 constexpr int kSolveReplicas = 32;
 
-// The block's energy / virial sums: per warp in float, per block in FP64 added to one of the replicas.
-// Blocks of at most 256 threads, a multiple of 32.
-__device__ __forceinline__ void solve_add(const float acc[7], double* partials)
+// The block's energy / virial sums: per warp in float (solve_add_warp), after a block barrier per block in
+// FP64 added to one of the replicas (solve_add_block).  Blocks of at most 256 threads, a multiple of 32.
+__device__ __forceinline__ void solve_add_warp(const float acc[7], double (*red)[8])
 {
-    __shared__ double red[7][8];
-    const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = 0; k < 7; k++)
     {
         float v = acc[k];
@@ -54,16 +53,27 @@ __device__ __forceinline__ void solve_add(const float acc[7], double* partials)
             red[k][warp] = (double)v;
         }
     }
-    __syncthreads();
+}
+
+__device__ __forceinline__ void solve_add_block(const double (*red)[8], double* partials)
+{
     if (threadIdx.x < 7)
     {
         double v = 0.0;
-        for (int w = 0; w < nwarps; w++)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++)
         {
             v += red[threadIdx.x][w];
         }
         atomicAdd(&partials[(blockIdx.x % kSolveReplicas) * 8 + threadIdx.x], v);
     }
+}
+
+__device__ __forceinline__ void solve_add(const float acc[7], double* partials)
+{
+    __shared__ double red[7][8];
+    solve_add_warp(acc, red);
+    __syncthreads();
+    solve_add_block(red, partials);
 }
 
 // One warp: the replicas' sums (complete: of an earlier kernel, or behind a completion counter), which
