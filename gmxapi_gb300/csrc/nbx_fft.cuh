@@ -11,7 +11,8 @@
 // last stage), twiddles from a table of the n roots exp(-2 pi i k / n) computed on the host in
 // double.  Axis passes: along z two real lines form one complex line (a + i b) and are separated
 // after the transform; along y and x a block loads a tile of 8 consecutive z-frequencies (coalesced
-// rows) and each warp transforms one column.
+// rows) and each warp transforms one column.  This is the path of the lengths that have no
+// transform in registers (FftLen, nbx_fft_len.cuh).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -9,9 +9,10 @@
 //   RF      qq*(1/r + k_rf r^2 - c_rf),
 // and the forces on j are the negated forces on i (half list).
 //
-// This file holds the one-pair-per-lane kernel (k_force: the autotuner's tile 0), the force reduction, the allocation-free entry and the launch dispatch; the
-// default kernel is the packed two-pairs-per-lane core of nbx_force_x2.cuh / nbx_pair_x2.cuh, which shares the work queue, the exclusion work items and the
-// reduction below.
+// This file holds the one-pair-per-lane kernel (k_force: tile 0), the force reduction, the
+// allocation-free entry and the launch dispatch; the default kernel is the packed two-pairs-per-lane
+// core of nbx_force_x2.cuh / nbx_pair_x2.cuh, which shares the work queue, the exclusion work items
+// and the reduction below.
 //
 // GB300 design (not the reference's 8x8-thread blocks):
 //  - persistent warps take list entries from an atomic work queue;
@@ -30,7 +31,7 @@
 //    would be systematic) and reduced in FP64; the Coulomb energies of
 //    excluded pairs and the self terms are summed in FP64 (rigid molecules
 //    repeat the same pair geometry, so their float rounding would not average
-//    out) by work items of 128 atoms interleaved with the list entries in the
+//    out) by work items of 32 or 128 atoms interleaved with the list entries in the
 //    same queue (k_excl_energy, a separate kernel, only for LJ-PME);
 //  - a force evaluation is three launches: k_convert_x (clears the
 //    accumulators), k_force or k_force_x2, k_reduce_f (its last block writes

@@ -8,9 +8,10 @@
 // The reference's pigeonhole sort (sort_atoms) keeps every run of occupied
 // holes ordered on (coordinate, atom index) and the hole index is monotonic in
 // the coordinate, so its result is the atoms ordered on (coordinate, index),
-// reversed for a backwards sort.  Here that order comes from a bitonic sort
-// (columns, z) and from rank computation inside a warp (32-atom y slabs and
-// 16-atom x halves).  All coordinate arithmetic is plain IEEE single precision
+// reversed for a backwards sort.  Here that order comes from counting the
+// smaller keys of small sets in shared memory: bins of a column's height (z; a
+// bitonic sort of the whole column where a bin overflows), 32-atom slabs (y) and
+// their halves (x).  All coordinate arithmetic is plain IEEE single precision
 // (this file is compiled with --fmad=false) so the grid, and therefore the
 // pair list, is bit-identical to the reference's.
 #include "nbx_internal.cuh"
