@@ -242,6 +242,8 @@ __device__ __forceinline__ void finish_sums(const DeviceView& v, double* d_energ
 constexpr int kReduceAtoms   = 4;
 constexpr int kReduceThreads = 256;
 
+// kAtoms atoms a thread.
+template<int kAtoms>
 __global__ void __launch_bounds__(kReduceThreads)
         k_reduce_f(DeviceView v, float* __restrict__ f, int do_virial, double* d_energies, double* d_virial, int stage,
                    unsigned* d_status)
@@ -257,19 +259,43 @@ __global__ void __launch_bounds__(kReduceThreads)
     {
         w[k] = 0.0f;
     }
+    // the shift-force part of the virial, sum_s shift_s (x) fshift_s, in the first block beside the others'
+    // gathers (in the last block it ended the kernel: 288 000 atoms with energies 399.9 us, now 397.8 us): one
+    // warp per component (8 warps, component 8 on warp 0), the 45 shifts over the lanes, a shuffle reduction
+    if (d_virial && blockIdx.x == 0)
+    {
+        const int lane = threadIdx.x & 31;
+        for (int c = threadIdx.x >> 5; c < 9; c += kReduceThreads / 32)
+        {
+            double t = 0.0;
+            for (int sh = lane; sh < kNShift; sh += 32)
+            {
+                t += (double)v.shiftvec[3 * sh + c / 3] * v.fshift[3 * sh + c % 3];
+            }
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                t += __shfl_xor_sync(0xffffffffu, t, o);
+            }
+            if (lane == 0)
+            {
+                atomicAdd(&v.virial[c], t);
+                __threadfence();
+            }
+        }
+    }
     // all gathers first, then the stores: stores through f may alias the loads, so loads
     // written after a store would wait for it
-    const int a0 = (blockIdx.x * kReduceThreads) * kReduceAtoms + threadIdx.x;
-    int       ks[kReduceAtoms];
+    const int a0 = (blockIdx.x * kReduceThreads) * kAtoms + threadIdx.x;
+    int       ks[kAtoms];
 #pragma unroll
-    for (int r = 0; r < kReduceAtoms; r++)
+    for (int r = 0; r < kAtoms; r++)
     {
         const int a = a0 + r * kReduceThreads;
         ks[r]       = a < v.n ? v.cells[a] : -1;
     }
-    float4 fa[kReduceAtoms], xa[kReduceAtoms];
+    float4 fa[kAtoms], xa[kAtoms];
 #pragma unroll
-    for (int r = 0; r < kReduceAtoms; r++)
+    for (int r = 0; r < kAtoms; r++)
     {
         if (ks[r] >= 0)
         {
@@ -284,7 +310,7 @@ __global__ void __launch_bounds__(kReduceThreads)
     {
         // the virial of the nonbonded forces only (before any accumulation into f)
 #pragma unroll
-        for (int r = 0; r < kReduceAtoms; r++)
+        for (int r = 0; r < kAtoms; r++)
         {
             if (ks[r] >= 0)
             {
@@ -306,9 +332,9 @@ __global__ void __launch_bounds__(kReduceThreads)
     {
         // the block's forces through shared memory, written as contiguous floats: whole
         // sectors when f is host memory written over the host link
-        __shared__ float sf[3 * kReduceThreads * kReduceAtoms];
+        __shared__ float sf[3 * kReduceThreads * kAtoms];
 #pragma unroll
-        for (int r = 0; r < kReduceAtoms; r++)
+        for (int r = 0; r < kAtoms; r++)
         {
             if (ks[r] >= 0)
             {
@@ -319,8 +345,8 @@ __global__ void __launch_bounds__(kReduceThreads)
             }
         }
         __syncthreads();
-        const int base  = blockIdx.x * kReduceThreads * kReduceAtoms;
-        const int count = 3 * min(kReduceThreads * kReduceAtoms, v.n - base);
+        const int base  = blockIdx.x * kReduceThreads * kAtoms;
+        const int count = 3 * min(kReduceThreads * kAtoms, v.n - base);
         float*    fb    = f + 3 * (size_t)base;
         for (int i = threadIdx.x; i < count; i += kReduceThreads)
         {
@@ -331,9 +357,9 @@ __global__ void __launch_bounds__(kReduceThreads)
     {
         if (v.accumulate_f)
         {
-            float old[kReduceAtoms][3];
+            float old[kAtoms][3];
 #pragma unroll
-            for (int r = 0; r < kReduceAtoms; r++)
+            for (int r = 0; r < kAtoms; r++)
             {
                 if (ks[r] >= 0)
                 {
@@ -344,7 +370,7 @@ __global__ void __launch_bounds__(kReduceThreads)
                 }
             }
 #pragma unroll
-            for (int r = 0; r < kReduceAtoms; r++)
+            for (int r = 0; r < kAtoms; r++)
             {
                 fa[r].x += old[r][0];
                 fa[r].y += old[r][1];
@@ -352,7 +378,7 @@ __global__ void __launch_bounds__(kReduceThreads)
             }
         }
 #pragma unroll
-        for (int r = 0; r < kReduceAtoms; r++)
+        for (int r = 0; r < kAtoms; r++)
         {
             if (ks[r] >= 0)
             {
@@ -411,30 +437,6 @@ __global__ void __launch_bounds__(kReduceThreads)
     if (last)
     {
         __threadfence();
-        // the shift-force part of the virial, sum_s shift_s (x) fshift_s: one warp per component
-        // (8 warps, component 8 on warp 0), the 45 shifts over the lanes, a shuffle reduction
-        __shared__ double sv[9];
-        if (d_virial)
-        {
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            for (int c = warp; c < 9; c += kReduceThreads / 32)
-            {
-                double t = 0.0;
-                for (int sh = lane; sh < kNShift; sh += 32)
-                {
-                    t += (double)v.shiftvec[3 * sh + c / 3] * __ldcg(&v.fshift[3 * sh + c % 3]);
-                }
-                for (int o = 16; o > 0; o >>= 1)
-                {
-                    t += __shfl_xor_sync(0xffffffffu, t, o);
-                }
-                if (lane == 0)
-                {
-                    sv[c] = t + __ldcg(&v.virial[c]);
-                }
-            }
-        }
-        __syncthreads();
         if (d_energies && threadIdx.x < 2)
         {
             d_energies[threadIdx.x] = __ldcg(&v.energy[threadIdx.x])
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(kReduceThreads)
         }
         if (d_virial && threadIdx.x < 9)
         {
-            d_virial[threadIdx.x] = -0.5 * sv[threadIdx.x];
+            d_virial[threadIdx.x] = -0.5 * __ldcg(&v.virial[threadIdx.x]);
         }
     }
 }
@@ -629,9 +631,20 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
 cudaError_t launch_reduce_f(const DeviceView& v, float* d_f, double* d_e, double* d_vir, cudaStream_t s, bool stage,
                             unsigned* d_status)
 {
-    const int per_block = kReduceThreads * kReduceAtoms;
-    launch_pdl(k_reduce_f, (v.n + per_block - 1) / per_block, kReduceThreads, 0, s, v, d_f, d_vir ? 1 : 0, d_e,
-               d_vir, stage ? 1 : 0, d_status);
+    // without energies an atom a thread (3 000 / 24 000 / 45 000 / 288 000 atoms: the evaluation 20.2 / 39.5 / 65.0 /
+    // 313.7 us with four, 19.6 / 38.3 / 64.0 / 313.2 us with one); with them every block ends in FP64 sums, and
+    // fewer blocks are better (57.7 / 88.8 / 389.4 us with four, 59.4 / 90.7 / 391.5 us with one)
+    if (!d_e && !d_vir)
+    {
+        launch_pdl(k_reduce_f<1>, (v.n + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, s, v, d_f,
+                   d_vir ? 1 : 0, d_e, d_vir, stage ? 1 : 0, d_status);
+    }
+    else
+    {
+        const int per_block = kReduceThreads * kReduceAtoms;
+        launch_pdl(k_reduce_f<kReduceAtoms>, (v.n + per_block - 1) / per_block, kReduceThreads, 0, s, v, d_f,
+                   d_vir ? 1 : 0, d_e, d_vir, stage ? 1 : 0, d_status);
+    }
     return cudaGetLastError();
 }
 
@@ -862,7 +875,7 @@ extern "C" int nbx_compute_noalloc(const nbx_noalloc_args* a, float* d_f, double
         {
             launch_k_force<false, false, 0>(v, blocks, smem, s, ctr);
         }
-        launch_pdl(k_reduce_f, (v.n + kReduceThreads * kReduceAtoms - 1) / (kReduceThreads * kReduceAtoms),
+        launch_pdl(k_reduce_f<kReduceAtoms>, (v.n + kReduceThreads * kReduceAtoms - 1) / (kReduceThreads * kReduceAtoms),
                    kReduceThreads, 0, s, v, d_f, d_virial ? 1 : 0, nullptr, nullptr, 0,
                         static_cast<unsigned*>(nullptr));
         if (energy)
