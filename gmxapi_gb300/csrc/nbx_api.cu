@@ -554,19 +554,24 @@ cudaError_t host_coordinates(nbx_handle* h, const float* x, bool in_place, const
     return cudaMemcpyAsync(h->d_x, x, bytes, cudaMemcpyHostToDevice, h->stream);
 }
 
+bool stages_forces(const nbx_handle* h)
+{
+    return h->d_stage && h->n <= kStageForceAtoms;
+}
+
 // Where they write its forces; nullptr: to d_f, copied on the stream.
 float* host_forces(nbx_handle* h, float* f)
 {
     bool         page = false;
     float* const d_f  = static_cast<float*>(mapped_device_ptr(f, &page));
-    return page && h->d_stage && h->n <= kStageForceAtoms ? h->d_stage + h->stage_f : d_f;
+    return page && stages_forces(h) ? h->d_stage + h->stage_f : d_f;
 }
 
 // Waits for a host-array call; then the staged forces, when d_f is the staging memory.
 cudaError_t finish_host_call(nbx_handle* h, float* f, const float* d_f)
 {
     const cudaError_t e = cudaStreamSynchronize(h->stream);
-    if (e == cudaSuccess && d_f && d_f == h->d_stage + h->stage_f)
+    if (e == cudaSuccess && stages_forces(h) && d_f == h->d_stage + h->stage_f)
     {
         std::memcpy(f, h->h_stage + h->stage_f, sizeof(float) * 3 * h->n);
     }
