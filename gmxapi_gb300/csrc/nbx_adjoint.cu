@@ -764,7 +764,7 @@ __global__ void k_match_loss(const float* __restrict__ f, const float* __restric
 }
 
 // Upstream force gradients to grid order; clears the output accumulators.
-// Per grid slot: the coordinates of this evaluation into xq (as k_convert_x, with the box shifts of
+// Per grid slot: the coordinates of this evaluation into xq and xqp (as k_convert_x, with the box shifts of
 // the last search) when x is given, the upstream force gradient (and the type) in grid order, a cleared dL/dx
 // accumulator; block 0 also clears the work queue and the FP64 type-pair gradient table (in place
 // of separate memsets).
@@ -788,21 +788,31 @@ __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const f
     {
         return;
     }
-    const int a = v.atom_indices[k];
+    const int   a = v.atom_indices[k];
+    const int   t = v.tgrid[k];
+    float       g[3] = { 0.0f, 0.0f, 0.0f };
+    if (a >= 0)
+    {
+        for (int d = 0; d < 3; d++)
+        {
+            g[d] = gF[3 * a + d];
+        }
+    }
     if (x && a >= 0)
     {
-        const float4 old  = v.xq[k];
-        const int    code = v.image[a];
-        float        c[3];
+        const float q    = v.xq[k].w;
+        const int   code = v.image[a];
+        float       c[3];
         for (int d = 0; d < 3; d++)
         {
             const int sh = (int)(signed char)((code >> (8 * d)) & 0xff);
             c[d]         = (sh == 0) ? x[3 * a + d] : x[3 * a + d] + (float)sh * v.g.box[d];
         }
-        v.xq[k] = make_float4(c[0], c[1], c[2], old.w);
+        v.xq[k] = make_float4(c[0], c[1], c[2], q);
+        // the cluster-packed copy follows: a full prune tests the atoms of xq against those of xqp
+        write_packed_slot(v.xqp, k, c[0], c[1], c[2], q, t);
     }
-    const float t = __int_as_float(v.tgrid[k]);
-    gnb[k] = (a >= 0) ? make_float4(gF[3 * a], gF[3 * a + 1], gF[3 * a + 2], t) : make_float4(0.0f, 0.0f, 0.0f, t);
+    gnb[k] = make_float4(g[0], g[1], g[2], __int_as_float(t));
     dnb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 

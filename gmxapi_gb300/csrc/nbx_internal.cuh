@@ -194,8 +194,8 @@ struct DeviceView
     int*    cells;         // [N]
     float4* xq;            // [cap*64]
     int*    tgrid;         // [cap*64]
-    // the same atoms cluster-packed for the packed force kernel: per cluster of 8 atoms one
-    // 160-byte record x[8], y[8], z[8], q[8], type[8] (int bits) with atom a at position
+    // the same atoms cluster-packed for the packed force kernel and the full prune, written wherever xq's
+    // coordinates are: per cluster of 8 atoms one 160-byte record x[8], y[8], z[8], q[8], type[8] (int bits) with atom a at position
     // 2 (a & 3) + (a >> 2), so atoms a and a + 4 are adjacent
     float*  xqp;           // [cap*64*5]
     float4* bb;            // [cap*8*2] lower, upper

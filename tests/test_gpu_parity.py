@@ -241,6 +241,28 @@ def test_fresh_prune_masks_forms(name, inner):
     calc.close()
 
 
+@pytest.mark.parametrize("name", ["water_small_box", "lj_liquid"])
+def test_fresh_prune_after_backward_pass(name):
+    """A full prune after an adjoint pass at other coordinates than the last evaluation's tests both sides
+    of every pair at the adjoint's: inner masks as the oracle's there."""
+    torch = pytest.importorskip("torch")
+    s = SYSTEMS[name]()
+    calc, o = _pair(s, rlist_inner=0.95, prune=10)
+    o.prune(fresh=True)
+    calc.compute(s.x)
+    x = systems.perturb(s.x, np.random.default_rng(6), 0.05)
+    dx = torch.from_numpy(np.ascontiguousarray(x, np.float32).reshape(-1)).cuda()
+    gx, gf = torch.zeros_like(dx), torch.ones_like(dx)
+    torch.cuda.synchronize()
+    calc.backward_device(dx.data_ptr(), gf.data_ptr(), None, gx.data_ptr(), None, None)
+    calc.prune_device(-1)
+    calc.synchronize()
+    o.set_x(x)
+    o.prune(fresh=True)
+    assert _masks(calc.pairlist(), False) == _masks(o.pairlist(), False)
+    calc.close()
+
+
 @pytest.mark.parametrize("name", list(SYSTEMS))
 @pytest.mark.parametrize("coulomb", [nblib.CoulombType.Pme, nblib.CoulombType.ReactionField])
 def test_forces_energies_virial_vs_oracle(name, coulomb):
