@@ -897,6 +897,7 @@ struct nbx_pme
     float2*      cgrid     = nullptr;  // half-complex grid [nx][ny][nz/2+1]
     float*       bsp       = nullptr;  // spline moduli x | y | z
     double*      sums      = nullptr;  // solve sums [kSolveReplicas][8]: energy + 6 virial terms, zero between solves
+    bool         summed    = false;    // a solve has added to the sums and no totals were taken yet
     unsigned*    done      = nullptr;  // blocks of the running solve that have written their partials
     int          num_sms   = 1;
     nbx::FftPlan3 fft{};  // the hand-written 3D real <-> half-complex transform (nbx_fft.cu)
@@ -1065,8 +1066,32 @@ cudaError_t launch_gather_bricks(nbx_pme* p, const float* d_x, const float* d_q,
     return e;
 }
 
+// Before a solve that adds to the sums: clears what an earlier call left there that ended between its solve and
+// its gather, which takes the totals and clears them.
+cudaError_t begin_sums(nbx_pme* p)
+{
+    if (!p->summed)
+    {
+        return cudaSuccess;
+    }
+    const cudaError_t e = cudaMemsetAsync(p->sums, 0, sizeof(double) * 8 * nbx::kSolveReplicas, p->stream);
+    if (e == cudaSuccess)
+    {
+        p->summed = false;
+    }
+    return e;
+}
+
 cudaError_t launch_solve(nbx_pme* p, float2* cgrid, double* d_energy, double* d_virial)
 {
+    if (d_energy || d_virial)
+    {
+        const cudaError_t e = begin_sums(p);
+        if (e != cudaSuccess)
+        {
+            return e;
+        }
+    }
     const double vol     = (double)p->box[0] * p->box[1] * p->box[2];
     const int    nc      = (int)complex_points(p);
     const int    cap     = (d_energy || d_virial) ? kSolveEnergyBlocksPerSm * p->num_sms : kSolveMaxBlocks;
@@ -1097,6 +1122,15 @@ bool fused_x_solve(const nbx_pme* p)
 
 cudaError_t launch_x_solve(nbx_pme* p, double* d_energy, double* d_virial)
 {
+    if (d_energy || d_virial)
+    {
+        const cudaError_t e = begin_sums(p);
+        if (e != cudaSuccess)
+        {
+            return e;
+        }
+        p->summed = true;
+    }
     const double vol    = (double)p->box[0] * p->box[1] * p->box[2];
     const float  factor = (float)(M_PI * M_PI) / (p->beta * p->beta);
     const float  elfac  = (float)nbx::one_4pi_eps0() / p->epsilon_r;
@@ -1560,8 +1594,13 @@ int pme_forces(nbx_pme* p, int natoms, const float* d_x, const float* d_q, float
     {
         tot = { p->sums, d_energy, d_virial };
     }
-    return cuda_status(p, p->by_bricks ? launch_gather_bricks(p, d_x, d_q, p->grid, d_f, tot)
-                                       : launch_gather(p, natoms, d_x, d_q, p->grid, d_f, tot));
+    const cudaError_t e = p->by_bricks ? launch_gather_bricks(p, d_x, d_q, p->grid, d_f, tot)
+                                       : launch_gather(p, natoms, d_x, d_q, p->grid, d_f, tot);
+    if (e == cudaSuccess && tot.partials)
+    {
+        p->summed = false;
+    }
+    return cuda_status(p, e);
 }
 
 } // namespace nbx

@@ -342,6 +342,52 @@ def test_filed_atoms_match_oracle(pm, layout, grid):
     p.close()
 
 
+@pytest.mark.parametrize("n,grid", [(300, (32, 32, 32)), (300, (31, 29, 33)), (17001, (32, 32, 32))])
+@pytest.mark.parametrize("then", ["compute", "solve"])
+def test_call_ended_before_its_gather_leaves_nothing_behind(pm, n, grid, then):
+    """An evaluation with energies whose second half (the gather, which takes the energy totals) never runs, as
+    when the short-range forces of a step fail in between: the next evaluation or solve gives its own energy, not
+    the sum of both.  (Charges are spread by float atomics in any order: a few roundings of 6e-8 per point.)"""
+    import ctypes
+
+    from gmxapi_gb300 import _lib
+
+    box = (2.9, 3.1, 3.3)
+    rng = np.random.default_rng(3)
+    x = (rng.random((n, 3)) * np.array(box)).astype(np.float32)
+    q = rng.normal(0.0, 0.4, n).astype(np.float32)
+    p = pm.Pme(box, grid, 3.0, device=0)
+    f0 = p.compute(x, q)
+    e0, v0 = p.energy, p.virial
+    half = getattr(_lib.load(), "_ZN3nbx13pme_potentialEP7nbx_pmeiPKfS3_PdS4_P11CUstream_st")
+    half.argtypes = [ctypes.c_void_p, ctypes.c_int] + 5 * [ctypes.c_void_p]
+    dx, dq = torch.from_numpy(x).cuda(), torch.from_numpy(q).cuda()
+    e = torch.zeros(10, dtype=torch.float64, device="cuda")
+    stream = torch.cuda.Stream()
+    p.set_stream(stream.cuda_stream)
+    torch.cuda.synchronize()
+    assert half(p.h, n, dx.data_ptr(), dq.data_ptr(), e.data_ptr(), e[1:].data_ptr(), stream.cuda_stream) == 0
+    if then == "compute":
+        f1 = p.compute(x, q)
+        assert rel_rms(f1, f0) <= 1e-6
+        energy, vir = p.energy, p.virial
+    else:
+        c = torch.zeros((grid[0], grid[1], grid[2] // 2 + 1, 2), device="cuda")
+        c[1, 2, 3, 0] = 1.0
+        got = torch.zeros((2, 10), dtype=torch.float64, device="cuda")
+        fresh = pm.Pme(box, grid, 3.0, device=0)
+        for handle, row in ((p, got[0]), (fresh, got[1])):
+            d = c.clone()
+            torch.cuda.synchronize()
+            handle.solve_device(d.data_ptr(), row.data_ptr(), row[1:].data_ptr())
+            handle.synchronize()
+        (energy, e0), (vir, v0) = got[:, 0].tolist(), got[:, 1:].cpu().numpy()
+        fresh.close()
+    assert energy == pytest.approx(e0, rel=1e-6)
+    np.testing.assert_allclose(vir, v0, rtol=0, atol=1e-6 * np.abs(v0).max())
+    p.close()
+
+
 @pytest.mark.parametrize("n", [1, 31, 32768, 32769])
 def test_gather_shapes_give_the_field_of_the_grid(n):
     """Direct gather with four threads per atom (up to 32,768 atoms) and with one, beyond: against the sum over the
