@@ -31,6 +31,7 @@
 #include "nbx_pme_solve.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -906,6 +907,7 @@ struct nbx_pme
     // filing of the atoms by grid brick (launch_file), allocated when the first call that takes it runs
     Bricks bricks{};
     int    brick_atoms = 0;      // atoms the filing arrays are sized for
+    std::vector<void*> old_bricks;  // smaller arrays, which captured graphs may still use
     bool   filed       = false;  // atoms are filed and the counts not yet cleared by a gather
     bool   by_bricks   = false;  // the last pme_potential went by bricks, and so does its gather
     std::string  err;
@@ -970,18 +972,22 @@ bool use_bricks(const nbx_pme* p, int natoms)
 void free_bricks(nbx_pme* p)
 {
     cudaFree(p->bricks.frac);
+    for (void* b : p->old_bricks)
+    {
+        cudaFree(b);
+    }
+    p->old_bricks.clear();
     p->bricks      = Bricks{};
     p->brick_atoms = 0;
     p->filed       = false;
 }
 
 // The filing arrays (one allocation) for natoms atoms; false when there is no memory for them: then the
-// direct path runs.
+// direct path runs and the arrays that were there stay.
 bool alloc_bricks(nbx_pme* p, int natoms)
 {
-    free_bricks(p);
-    Bricks& b   = p->bricks;
-    size_t  nbr = 1;
+    Bricks b{};
+    size_t nbr = 1;
     for (int k = 0; k < 3; k++)
     {
         b.nb[k] = (p->d.n[k] + kBrick - 1) / kBrick;
@@ -1003,18 +1009,31 @@ bool alloc_bricks(nbx_pme* p, int natoms)
         e = cudaFuncSetAttribute(k_pme_spread_bricks, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(SpreadWarp) * kBrickWarps));
     }
+    // arrays that are replaced go on to serve the graphs that were captured with them: their counts have to be
+    // zero, as a gather leaves them
+    if (e == cudaSuccess && p->bricks.frac && p->filed)
+    {
+        e = cudaMemsetAsync(p->bricks.count, 0, sizeof(int) * (nbr + 1), p->stream);
+    }
     if (e != cudaSuccess)
     {
         cudaGetLastError();
-        free_bricks(p);
+        cudaFree(b.frac);
         return false;
     }
+    if (p->bricks.frac)
+    {
+        p->old_bricks.push_back(p->bricks.frac);
+    }
+    p->bricks      = b;
     p->brick_atoms = natoms;
+    p->filed       = false;
     return true;
 }
 
 // As alloc_bricks, when the arrays there are too small; nothing is allocated while the stream is being
-// captured (the direct path runs then).
+// captured (the direct path runs then).  The arrays grow by at least half, so that all the replaced ones together
+// hold at most twice as many atoms as the present ones.
 bool ensure_bricks(nbx_pme* p, int natoms)
 {
     if (p->brick_atoms >= natoms)
@@ -1027,8 +1046,7 @@ bool ensure_bricks(nbx_pme* p, int natoms)
         cudaGetLastError();
         return false;
     }
-    cudaStreamSynchronize(p->stream);
-    return alloc_bricks(p, natoms);
+    return alloc_bricks(p, (int)std::max<long long>(natoms, std::min(3LL * p->brick_atoms / 2, (long long)INT_MAX)));
 }
 
 cudaError_t launch_spread_bricks(nbx_pme* p, int natoms, const float* d_x, const float* d_q, float* grid)

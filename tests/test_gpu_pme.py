@@ -388,6 +388,60 @@ def test_call_ended_before_its_gather_leaves_nothing_behind(pm, n, grid, then):
     p.close()
 
 
+@pytest.mark.parametrize("warm", [True, False])
+def test_captured_evaluation_survives_larger_calls(pm, warm):
+    """A captured evaluation replayed after calls with more atoms, which need larger filing arrays; captured
+    with its arrays in place (warm) or without any (the direct path).  As before the capture, up to the order of
+    the float atomics."""
+    box, grid = (2.9, 3.1, 3.3), (32, 32, 32)
+    rng = np.random.default_rng(23)
+    p = pm.Pme(box, grid, 3.0, device=0)
+    stream = torch.cuda.Stream()
+    p.set_stream(stream.cuda_stream)
+
+    def inputs(n):
+        x = (rng.random((n, 3)) * np.array(box)).astype(np.float32)
+        q = rng.normal(0.0, 0.4, n).astype(np.float32)
+        return x, q, dev(x), dev(q), torch.zeros((n, 3), device="cuda"), torch.zeros(10, dtype=torch.float64, device="cuda")
+
+    def call(a):
+        p.compute_device(len(a[0]), a[2].data_ptr(), a[3].data_ptr(), a[4].data_ptr(), a[5].data_ptr(),
+                         a[5][1:].data_ptr())
+
+    small, large, larger = inputs(17001), inputs(26001), inputs(40001)
+    torch.cuda.synchronize()
+    if warm:
+        call(small)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        small[4].zero_()
+        call(small)
+    for a in (large, larger, small):
+        want, energy, _ = P.compute(a[0], a[1], box, grid, 3.0, single=True)
+        for replay in ((False, True) if a is small else (False,)):
+            torch.cuda.synchronize()
+            if replay:
+                small[5].zero_()
+                torch.cuda.synchronize()
+                graph.replay()
+            else:
+                a[4].zero_()
+                torch.cuda.synchronize()
+                call(a)
+            torch.cuda.synchronize()
+            assert rel_rms(a[4].cpu().numpy(), want) <= FORCE_RTOL
+            assert a[5][0].item() == pytest.approx(energy, rel=ENERGY_RTOL)
+        # after every larger call the graph again
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want, energy, _ = P.compute(small[0], small[1], box, grid, 3.0, single=True)
+        assert rel_rms(small[4].cpu().numpy(), want) <= FORCE_RTOL
+        assert small[5][0].item() == pytest.approx(energy, rel=ENERGY_RTOL)
+    p.close()
+
+
 @pytest.mark.parametrize("n", [1, 31, 32768, 32769])
 def test_gather_shapes_give_the_field_of_the_grid(n):
     """Direct gather with four threads per atom (up to 32,768 atoms) and with one, beyond: against the sum over the
