@@ -157,11 +157,11 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     {
         rinv6 = mul2(rinv6, make_float2(intA, intB));
     }
-    const float2 rinv8  = mul2(rinv6, rinv2);
-    const float2 rinv14 = mul2(rinv6, rinv8);
-    const float2 fdisp  = make_float2(ljA.x * rinv8.x, ljB.x * rinv8.y);
-    const float2 frep   = make_float2(ljA.y * rinv14.x, ljB.y * rinv14.y);
-    const float2 phi_lj = sub2(frep, fdisp);
+    // C / r^n as products that stay finite down to the smallest distance where C is 0 (r^-14 alone overflows
+    // below 1.8 pm), and rounded once where the two terms cancel
+    const float2 vdisp  = make_float2(ljA.x * rinv6.x, ljB.x * rinv6.y);
+    const float2 vrep   = mul2(make_float2(ljA.y * rinv6.x, ljB.y * rinv6.y), rinv6);
+    const float2 phi_lj = mul2(sub2(vrep, vdisp), rinv2);
     float2       psi, dpsi, hq = f2(0.0f);  // Coulomb phi / qq, 2 r^2 times its s-derivative, energy / qq
     if (kEwald)
     {
@@ -169,11 +169,12 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
         const float2 t    = make_float2(fast_rcp(tt.x), fast_rcp(tt.y));
         const float2 earg = mul2(f2(k.nbeta2l2), r2);
         const float2 expm = make_float2(fast_ex2(earg.x), fast_ex2(earg.y));
-        const float2 tp   = mul2(mul2(t, erfc_poly2(t)), rinv);  // erfc(beta r) / r = tp expm
-        psi               = mul2(mul2(expm, add2(tp, f2(k.c2b))), rinv2);
+        const float2 tp   = mul2(t, erfc_poly2(t));  // erfc(beta r) = tp expm
+        psi               = mul2(mul2(expm, fma2(tp, rinv, f2(k.c2b))), rinv2);
         if (kGE)
         {
-            hq = fma2(tp, expm, make_float2(inA ? -intA * k.sh_ewald : 0.0f, inB ? -intB * k.sh_ewald : 0.0f));
+            hq = fma2(mul2(tp, expm), rinv,
+                      make_float2(inA ? -intA * k.sh_ewald : 0.0f, inB ? -intB * k.sh_ewald : 0.0f));
         }
         if (kExcl)
         {
@@ -204,8 +205,8 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     const float2 gy   = sub2(make_float2(i2.z, i2.w), f2(gj.y));
     const float2 gz   = sub2(make_float2(i3.x, i3.y), f2(gj.z));
     const float2 gr   = fma2(gz, dz, fma2(gy, dy, mul2(gx, dx)));
-    // 2 phi' (g.r), phi' = (qq dpsi + 8 fdisp - 14 frep) / (2 r^2)
-    const float2 dphi = fma2(qq, dpsi, fma2(f2(-14.0f), frep, mul2(f2(8.0f), fdisp)));
+    // 2 phi' (g.r), phi' = (qq dpsi + (8 vdisp - 14 vrep) / r^2) / (2 r^2)
+    const float2 dphi = fma2(qq, dpsi, mul2(fma2(f2(-14.0f), vrep, mul2(f2(8.0f), vdisp)), rinv2));
     float2       coef = mul2(mul2(dphi, rinv2), gr);
     float2       wq   = mul2(psi, gr);  // dL/d(q_i q_j) / epsfac
     if (kGE)
@@ -227,8 +228,9 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     dj.z   = add2(dj.z, uz);
     dj.q   = fma2(wq, qi, dj.q);
     // dL/d(6C6) and dL/d(12C12) of the pairs, by i type
-    float2 d6  = mul2(gr, rinv8);
-    float2 d12 = mul2(gr, rinv14);
+    const float2 gr6 = mul2(gr, rinv6);
+    float2       d6  = mul2(gr6, rinv2);
+    float2       d12 = mul2(gr6, mul2(rinv6, rinv2));
     if (kGE)
     {
         const bool   cA = inA && (!kExcl || intA != 0.0f), cB = inB && (!kExcl || intB != 0.0f);

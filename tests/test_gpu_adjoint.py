@@ -122,6 +122,36 @@ def test_adjoint_linear_loss_matches_fp64_autograd(name, coulomb):
     print(name, coulomb, errs)
 
 
+@pytest.mark.parametrize("distance", [1.2e-3, 1.7e-3, 0.02])
+def test_adjoint_of_close_charges_without_lj(distance):
+    """Two charges whose type has no LJ terms, so close that r^-14 alone is beyond the largest float: the
+    coordinate and charge gradients of every atom are those of the FP64 functional."""
+    s = _with_plain_type(systems.lj_liquid(n=600, ntypes=2, seed=31))
+    inside = (s.x > 0.3).all(1) & (s.x < 1.5).all(1)  # the close pair is not wrapped apart
+    plain = np.flatnonzero((s.type == 1) & inside)[:2]
+    s.x[plain[1]] = s.x[plain[0]] + np.array([distance, 0.0, 0.0], np.float32)
+    rng = np.random.default_rng(3)
+    g_f, g_e = rng.normal(size=(s.n, 3)), np.array([0.3, -0.2])
+    g = _gpu(s, COULOMB_EWALD, g_f, g_e)
+    r = _fp64(s, COULOMB_EWALD, g_f, g_e)
+    others = np.setdiff1d(np.arange(s.n), plain)
+    for atoms in (plain, others):
+        assert rel_rms(g["gx"][atoms], r["gx"][atoms]) < GX_RTOL
+        assert rel_rms(g["gq"][atoms], r["gq"][atoms]) < GQ_RTOL
+
+
+def _with_plain_type(s):
+    """The system with no LJ terms for its last type."""
+    t = systems.System(**{**s.__dict__})
+    t.x = s.x.copy()
+    t.epsilon = s.epsilon.copy()
+    t.epsilon[-1] = 0.0
+    sij = 0.5 * (s.sigma[:, None] + s.sigma[None, :])
+    eij = np.sqrt(t.epsilon[:, None] * t.epsilon[None, :])
+    t.nbfp = systems.nbfp_from_c6c12(4.0 * eij * sij**6, 4.0 * eij * sij**12)
+    return t
+
+
 def test_adjoint_force_matching_loss_matches_fp64_autograd():
     """Loss sum |F - F_target|^2 with F_target at parameters perturbed by up to 5 %."""
     s = CASES["liquid2000"]()
