@@ -128,6 +128,11 @@ struct AdjJ
     float  hi[kBig ? 2 : 1][4], lo[kBig ? 2 : 1][4];
 };
 
+__device__ __forceinline__ float2 pick2(bool a, bool b, float2 v)
+{
+    return make_float2(a ? v.x : 0.0f, b ? v.y : 0.0f);
+}
+
 // One step: i-cluster c against the lane's j-atom.  okA / okB: the pair's mask bit (and, on the diagonal,
 // j > i); intA / intB: its exclusion bit as 0 / 1.
 template<bool kEwald, bool kGE, bool kBig, bool kExcl>
@@ -146,9 +151,8 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     r2                = make_float2(fmaxf(r2.x, kMinDist2), fmaxf(r2.y, kMinDist2));
     float2       rinv = make_float2(fast_rsqrt(r2.x), fast_rsqrt(r2.y));
     rinv              = fma2(rinv, fma2(mul2(r2, f2(-0.5f)), mul2(rinv, rinv), f2(0.5f)), rinv);
-    // 1/r = 0 for pairs out of range: every term below then vanishes, but for the constants, which have
-    // their own masks
-    rinv               = make_float2(inA ? rinv.x : 0.0f, inB ? rinv.y : 0.0f);
+    // pairs out of range add zeros: 1/r = 0, and no upstream gradient (0 times one that is not finite is not 0)
+    rinv               = pick2(inA, inB, rinv);
     const float2 rinv2 = mul2(rinv, rinv);
     const float2 ljA   = *reinterpret_cast<const float2*>(nbfp_b + (tA << 7) + tjb);
     const float2 ljB   = *reinterpret_cast<const float2*>(nbfp_b + (tB << 7) + tjb);
@@ -173,8 +177,7 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
         psi               = mul2(mul2(expm, fma2(tp, rinv, f2(k.c2b))), rinv2);
         if (kGE)
         {
-            hq = fma2(mul2(tp, expm), rinv,
-                      make_float2(inA ? -intA * k.sh_ewald : 0.0f, inB ? -intB * k.sh_ewald : 0.0f));
+            hq = fma2(mul2(tp, expm), rinv, make_float2(-intA * k.sh_ewald, -intB * k.sh_ewald));
         }
         if (kExcl)
         {
@@ -190,20 +193,19 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     else
     {
         const float2 r3 = kExcl ? mul2(mul2(rinv, rinv2), make_float2(intA, intB)) : mul2(rinv, rinv2);
-        psi             = add2(r3, make_float2(inA ? k.nk_rf2 : 0.0f, inB ? k.nk_rf2 : 0.0f));
+        psi             = add2(r3, f2(k.nk_rf2));
         dpsi            = mul2(f2(-3.0f), r3);
         if (kGE)
         {
-            const float2 h = fma2(f2(k.k_rf), r2, sub2(mul2(rinv, make_float2(intA, intB)), f2(k.c_rf)));
-            hq             = make_float2(inA ? h.x : 0.0f, inB ? h.y : 0.0f);
+            hq = fma2(f2(k.k_rf), r2, sub2(mul2(rinv, make_float2(intA, intB)), f2(k.c_rf)));
         }
     }
     const float2 qi   = make_float2(i1.z, i1.w);
     const float2 qq   = mul2(qi, f2(qje));
     const float2 phi  = fma2(qq, psi, phi_lj);
-    const float2 gx   = sub2(make_float2(i2.x, i2.y), f2(gj.x));
-    const float2 gy   = sub2(make_float2(i2.z, i2.w), f2(gj.y));
-    const float2 gz   = sub2(make_float2(i3.x, i3.y), f2(gj.z));
+    const float2 gx   = pick2(inA, inB, sub2(make_float2(i2.x, i2.y), f2(gj.x)));
+    const float2 gy   = pick2(inA, inB, sub2(make_float2(i2.z, i2.w), f2(gj.y)));
+    const float2 gz   = pick2(inA, inB, sub2(make_float2(i3.x, i3.y), f2(gj.z)));
     const float2 gr   = fma2(gz, dz, fma2(gy, dy, mul2(gx, dx)));
     // 2 phi' (g.r), phi' = (qq dpsi + (8 vdisp - 14 vrep) / r^2) / (2 r^2)
     const float2 dphi = fma2(qq, dpsi, mul2(fma2(f2(-14.0f), vrep, mul2(f2(8.0f), vdisp)), rinv2));
@@ -211,8 +213,8 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     float2       wq   = mul2(psi, gr);  // dL/d(q_i q_j) / epsfac
     if (kGE)
     {
-        coef = sub2(coef, fma2(f2(k.gE_c), mul2(qq, psi), mul2(f2(k.gE_lj), phi_lj)));
-        wq   = fma2(f2(k.gE_c), hq, wq);
+        coef = sub2(coef, pick2(inA, inB, fma2(f2(k.gE_c), mul2(qq, psi), mul2(f2(k.gE_lj), phi_lj))));
+        wq   = add2(wq, pick2(inA, inB, mul2(f2(k.gE_c), hq)));
     }
     const float2 ux = fma2(phi, gx, mul2(coef, dx));
     const float2 uy = fma2(phi, gy, mul2(coef, dy));
@@ -233,12 +235,14 @@ __device__ __forceinline__ void adj_step(const AdjConsts& k, const char* __restr
     float2       d12 = mul2(gr6, mul2(rinv6, rinv2));
     if (kGE)
     {
-        const bool   cA = inA && (!kExcl || intA != 0.0f), cB = inB && (!kExcl || intB != 0.0f);
-        const float2 e6 = fma2(rinv6, f2(1.0f / 6.0f), make_float2(cA ? k.cpot6 : 0.0f, cB ? k.cpot6 : 0.0f));
-        const float2 e12 =
-                fma2(mul2(rinv6, rinv6), f2(1.0f / 12.0f), make_float2(cA ? k.cpot12 : 0.0f, cB ? k.cpot12 : 0.0f));
-        d6  = fma2(f2(k.gE_lj), e6, d6);
-        d12 = fma2(f2(k.gE_lj), e12, d12);
+        d6  = fma2(f2(k.gE_lj), fma2(rinv6, f2(1.0f / 6.0f), f2(k.cpot6)), d6);
+        d12 = fma2(f2(k.gE_lj), fma2(mul2(rinv6, rinv6), f2(1.0f / 12.0f), f2(k.cpot12)), d12);
+    }
+    if (kGE || kExcl)
+    {
+        const bool cA = inA && (!kExcl || intA != 0.0f), cB = inB && (!kExcl || intB != 0.0f);
+        d6            = pick2(cA, cB, d6);
+        d12           = pick2(cA, cB, d12);
     }
     const int row = lane >> 2;
     float     h[4], r[4];
@@ -263,12 +267,57 @@ struct AdjTypes
     float s6[kBig ? 2 : 1][4], s12[kBig ? 2 : 1][4];
 };
 
+// The type terms of one j-cluster pair by pair, for the i-clusters `rem`: what the products with one-hot matrices
+// cannot sum, since a term that is not finite (an upstream gradient that is not, or atoms so close that r^-14
+// overflows) times their zeros reaches every type pair.  Such a term goes to its own type pair here, as every other
+// of the j-cluster.  sums: the warp's FP64 type-pair sums (element 0 of lane 0).
+template<bool kGE>
+__device__ __noinline__ void adj_types_by_pair(const AdjWarp& w, double* sums, const float4 xj, const float4 gj,
+                                               unsigned rem, unsigned mj, unsigned xA, unsigned xB, int diag, float rc2,
+                                               float gE_lj, float cpot6, float cpot12)
+{
+    const int lane = threadIdx.x & 31, j = lane >> 2, ip = lane & 3, tj = __float_as_int(gj.w);
+    for (; rem; rem &= rem - 1)
+    {
+        const int    c  = __ffs(rem) - 1;
+        const float4 i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
+        for (int h = 0; h < 2; h++)
+        {
+            const float dx = (h ? i0.y : i0.x) - xj.x, dy = (h ? i0.w : i0.z) - xj.y, dz = (h ? i1.y : i1.x) - xj.z;
+            float       r2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
+            const bool  in = ((mj >> c) & 1u) && !(c == diag && j <= ip + 4 * h) && (((h ? xB : xA) >> c) & 1u);
+            if (!in || !(r2 < rc2))
+            {
+                continue;
+            }
+            r2                = fmaxf(r2, kMinDist2);
+            float rinv        = fast_rsqrt(r2);
+            rinv              = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
+            const float rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
+            const float gx = (h ? i2.y : i2.x) - gj.x, gy = (h ? i2.w : i2.z) - gj.y, gz = (h ? i3.y : i3.x) - gj.z;
+            const float gr6 = (gx * dx + gy * dy + gz * dz) * rinv6;
+            float       d6 = gr6 * rinv2, d12 = gr6 * (rinv6 * rinv2);
+            if (kGE)
+            {
+                d6  = fmaf(gE_lj, fmaf(rinv6, 1.0f / 6.0f, cpot6), d6);
+                d12 = fmaf(gE_lj, fmaf(rinv6 * rinv6, 1.0f / 12.0f, cpot12), d12);
+            }
+            // the element of adj_flush that is (i type a, j type b)
+            const int a = __float_as_int(h ? i3.w : i3.z), b = tj;
+            double*   s = sums + 64 * (4 * (a >> 3) + (a & 1) + 2 * (b >> 3)) + 4 * (b & 7) + ((a & 7) >> 1);
+            atomicAdd(s, -(double)d6);
+            atomicAdd(s + 32, (double)d12);
+        }
+    }
+}
+
 // All set cluster pairs of one cj4 group.  m: the mask of the lane's half; u: both halves' masks; wA / wB:
 // the lane's exclusion words (i-atoms ip and ip + 4).
 template<bool kEwald, bool kGE, bool kBig, bool kExcl>
 __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w,
                                           float4* __restrict__ dnb, int cj_lane, unsigned m, unsigned u, unsigned wA,
-                                          unsigned wB, int sci, bool central, int lane, AdjTypes<kBig>& types)
+                                          unsigned wB, int sci, bool central, int lane, double* gsum,
+                                          AdjTypes<kBig>& types)
 {
     const unsigned full = 0xffffffffu;
     const int      j = lane >> 2, ip = lane & 3;
@@ -284,9 +333,9 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         const float4   xj   = w.jx[jm * kCl + j], gj = w.jg[jm * kCl + j];
         const int      tj   = __float_as_int(gj.w);
         const float    qje  = xj.w * k.epsfac;
-        // an empty slot has no pairs: two empty slots coincide, and the huge powers of their 1/r must not meet
-        // the zeros of the one-hot factors
+        // an empty slot has no pairs (two empty slots coincide)
         const unsigned mj   = tj == k.filler ? 0u : m >> (jm * kNcl);
+        const unsigned set  = rem;
         const unsigned xA   = wA >> (jm * kNcl), xB = wB >> (jm * kNcl);
         const int      diag = kExcl && central ? cj - sci * kNcl : -1;  // the diagonal i-cluster, if in 0 .. 7
         AdjJ<kBig>     dj;
@@ -340,6 +389,17 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         keep.y += __shfl_xor_sync(full, send.y, 2);
         float one = (o1 ? keep.y : keep.x) + __shfl_xor_sync(full, o1 ? keep.x : keep.y, 1);
         atomicAdd(reinterpret_cast<float*>(&dnb[cj * kCl + j]) + ip, -one);
+        float total = 0.0f;
+#pragma unroll
+        for (int n = 0; n < (kBig ? 2 : 1); n++)
+        {
+            total += (dj.hi[n][0] + dj.hi[n][1]) + (dj.hi[n][2] + dj.hi[n][3]);
+        }
+        if (__any_sync(full, !isfinite(total)))
+        {
+            adj_types_by_pair<kGE>(w, gsum - lane, xj, gj, set, mj, xA, xB, diag, k.rc2, k.gE_lj, k.cpot6, k.cpot12);
+            continue;
+        }
         // type pairs: D of row j turns into the B fragment (k = j-atoms ip and ip + 4, n = i type lane >> 2)
         // of the product with the one-hot j types
         const int   t0 = __shfl_sync(full, tj, 4 * ip), t1 = __shfl_sync(full, tj, 16 + 4 * ip);
@@ -459,14 +519,14 @@ __device__ __forceinline__ void adj_entry(const AdjConsts& k, const AdjPtrs& p, 
         if ((ime.y | ime.w) == 0)
         {
             adj_group<kEwald, kGE, kBig, false>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, ~0u, ~0u, s.sci, central,
-                                                lane, types);
+                                                lane, gsum, types);
         }
         else
         {
             const unsigned* pair = p.excl[lane < 16 ? ime.y : ime.w].pair;
             const int       at   = ((lane >> 2) & 3) * kCl + (lane & 3);
             adj_group<kEwald, kGE, kBig, true>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, pair[at], pair[at + 4], s.sci,
-                                               central, lane, types);
+                                               central, lane, gsum, types);
         }
     }
     // the i-side sums: lane (c, ip) adds the eight j-lanes' slots of the atoms ip and ip + 4

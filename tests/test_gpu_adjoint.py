@@ -152,6 +152,90 @@ def _with_plain_type(s):
     return t
 
 
+def _backward(s, g_f, coulomb=COULOMB_EWALD, g_e=None):
+    """(dL/dx, dL/dq, dL/d type table summed over both orders of a pair) of the engine's adjoint alone."""
+    opts = NBKernelOptions(coulomb_type=CoulombType.Pme if coulomb == COULOMB_EWALD else CoulombType.ReactionField,
+                           pairlist_cutoff=RLIST, rcoulomb=RC, epsilon_rf=1.0 if coulomb == COULOMB_EWALD else 0.0)
+    eng = DifferentiableNonbonded(s, opts)
+    x = torch.tensor(s.x, dtype=torch.float32, device=DEV)
+    g = torch.tensor(g_f, dtype=torch.float32, device=DEV)
+    ge = None if g_e is None else torch.tensor(g_e, dtype=torch.float64, device=DEV)
+    gx, gq = torch.zeros_like(x), torch.zeros(s.n, device=DEV)
+    tab = torch.zeros((s.ntypes, s.ntypes, 2), dtype=torch.float64, device=DEV)
+    eng.search(x)
+    torch.cuda.synchronize()
+    eng.calc.backward_device(x.data_ptr(), g.data_ptr(), None if ge is None else ge.data_ptr(), gx.data_ptr(),
+                             gq.data_ptr(), tab.data_ptr())
+    eng.calc.synchronize()
+    out = gx.cpu().numpy(), gq.cpu().numpy(), (tab + tab.transpose(0, 1)).cpu().numpy()
+    eng.close()
+    return out
+
+
+def _within(s, atom, reach):
+    d = s.x.astype(np.float64) - s.x[atom].astype(np.float64)
+    d -= np.round(d / s.box) * s.box
+    return np.einsum("ij,ij->i", d, d) < reach**2
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("ntypes,coulomb", [(3, COULOMB_EWALD), (3, COULOMB_RF), (12, COULOMB_EWALD), (8, COULOMB_EWALD)])
+def test_adjoint_of_a_gradient_that_is_not_finite(ntypes, coulomb, bad):
+    """One atom's upstream gradient that is not finite reaches the atoms within the cut-off and the type pairs of that
+    atom's type, and nothing else: atoms and type pairs without it are as with that gradient zero (the float sums of
+    an atom or a type pair in another order: 2e-6 of the largest)."""
+    s = systems.lj_liquid(n=900, ntypes=ntypes, seed=41)
+    atom = 17
+    rng = np.random.default_rng(4)
+    g_f = rng.normal(size=(s.n, 3))
+    g_f[atom] = 0.0
+    gx0, gq0, tab0 = _backward(s, g_f, coulomb)
+    g_f[atom] = (0.5, bad, -0.25)
+    gx, gq, tab = _backward(s, g_f, coulomb)
+    near, far = _within(s, atom, RC - 1e-4), ~_within(s, atom, RC + 1e-4)
+    assert not np.isfinite(gx[near]).all(axis=1).any()
+    assert np.abs(gx[far] - gx0[far]).max() <= 2e-6 * np.abs(gx0).max()
+    assert np.abs(gq[far] - gq0[far]).max() <= 2e-6 * np.abs(gq0).max()
+    clean = np.ones((ntypes, ntypes), bool)
+    clean[s.type[atom], :] = clean[:, s.type[atom]] = False
+    for k in range(2):
+        assert np.abs(tab[..., k] - tab0[..., k])[clean].max() <= 2e-6 * np.abs(tab0[..., k]).max()
+
+
+@pytest.mark.parametrize("ntypes,g_e", [(3, None), (3, [0.3, -0.2]), (12, None)])
+def test_adjoint_type_pairs_beside_an_overlapping_pair(ntypes, g_e):
+    """Two LJ atoms so close that their r^-14 is beyond the largest float: every other type pair's gradient is the FP64
+    functional's."""
+    s = systems.lj_liquid(n=600, ntypes=ntypes, seed=43)
+    s.x = s.x.copy()
+    inside = (s.x > 0.3).all(1) & (s.x < 1.5).all(1)
+    a = np.flatnonzero((s.type == 0) & inside)[0]
+    b = np.flatnonzero((s.type == 1) & inside)[0]
+    s.x[b] = s.x[a] + np.array([1.2e-3, 0.0, 0.0], np.float32)
+    # no other atom at the new place: its gradient terms there would hide the rest
+    near = _within(s, a, 0.15)
+    near[[a, b]] = False
+    keep = np.flatnonzero(~near)
+    s = systems.System(**{**s.__dict__, "x": s.x[keep], "q": s.q[keep], "type": s.type[keep],
+                          "excl_index": np.arange(len(keep) + 1, dtype=np.int32),
+                          "excl_list": np.arange(len(keep), dtype=np.int32)})
+    rng = np.random.default_rng(5)
+    g_f = rng.normal(size=(s.n, 3))
+    _, _, tab = _backward(s, g_f, COULOMB_EWALD, g_e)
+    o = orc.Oracle(s, coulomb=COULOMB_EWALD, rc=RC, rlist=RLIST)
+    ref = AllPairsFP64(s, RC, o.beta, orc.lib().orc_one_4pi_eps0(), coulomb=COULOMB_EWALD)
+    nbfp = torch.tensor(np.asarray(s.nbfp, np.float64).reshape(ntypes, ntypes, 2), requires_grad=True)
+    f, e = ref.forces_energies(torch.tensor(s.x, dtype=torch.float64, requires_grad=True),
+                               torch.tensor(s.q, dtype=torch.float64), nbfp)
+    loss = (torch.tensor(g_f) * f).sum() + (0.0 if g_e is None else (torch.tensor(g_e) * e).sum())
+    (want,) = torch.autograd.grad(loss, nbfp)
+    want = (want + want.transpose(0, 1)).numpy()
+    clean = np.ones((ntypes, ntypes), bool)
+    clean[0, 1] = clean[1, 0] = False
+    for k in range(2):
+        assert rel_rms(tab[..., k][clean], want[..., k][clean]) < GPARAM_RTOL
+
+
 def test_adjoint_force_matching_loss_matches_fp64_autograd():
     """Loss sum |F - F_target|^2 with F_target at parameters perturbed by up to 5 %."""
     s = CASES["liquid2000"]()
