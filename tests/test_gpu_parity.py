@@ -461,6 +461,29 @@ def test_lj_modifiers_same_from_both_tiles(name, mod, coulomb, shift):
     calc.close()
 
 
+@pytest.mark.parametrize("mod", [nblib.VdwModifier.ForceSwitch, nblib.VdwModifier.PotSwitch, nblib.VdwModifier.LjPme])
+@pytest.mark.parametrize("coulomb", [nblib.CoulombType.Pme, nblib.CoulombType.ReactionField])
+def test_lj_modifier_forces_as_accurate_from_both_tiles(mod, coulomb):
+    """Forces without energies: the packed kernel's error against the FP64 sum is no larger than the
+    one-pair-per-lane kernel's (2 % for the order of the float atomics, which moves either by less than 1 %)."""
+    from gmxapi_gb300 import pme
+
+    s = SYSTEMS["water3000"]()
+    lj_pme = mod == nblib.VdwModifier.LjPme
+    calc = nblib.ForceCalculator(s, nblib.NBKernelOptions(
+        coulomb_type=coulomb, pairlist_cutoff=1.0, rcoulomb=0.9, vdw_modifier=mod, rvdw_switch=0.0 if lj_pme else 0.7))
+    o = O.Oracle(s, rc=0.9, rlist=1.0)
+    f64, _ = O.fp64_allpairs(s, coulomb=int(coulomb), rc=0.9, beta=o.beta if coulomb == 0 else None,
+                             vdw_modifier=int(mod), rvdw_switch=0.0 if lj_pme else 0.7,
+                             beta_lj=pme.ewald_coefficient_lj(0.9, 1e-3) if lj_pme else 0.0)
+    err = []
+    for tile in (0, 1):
+        calc.set_force_kernel(tile, 2, 2)
+        err.append(rel_rms(calc.compute(s.x, energies=False), f64))
+    calc.close()
+    assert err[1] <= 1.02 * err[0], err
+
+
 def test_switch_modifiers_rejected_where_unsupported():
     s = systems.lj_liquid(n=600, ntypes=4, seed=3)
     with pytest.raises(nblib.InputException):
