@@ -315,7 +315,7 @@ __device__ __noinline__ void adj_types_by_pair(const AdjWarp& w, double* sums, c
 // the lane's exclusion words (i-atoms ip and ip + 4).
 template<bool kEwald, bool kGE, bool kBig, bool kExcl>
 __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w,
-                                          float4* __restrict__ dnb, int cj_lane, unsigned m, unsigned u, unsigned wA,
+                                          float4* dnb, int cj_lane, unsigned m, unsigned u, unsigned wA,
                                           unsigned wB, int sci, bool central, int lane, double* gsum,
                                           AdjTypes<kBig>& types)
 {
@@ -621,8 +621,8 @@ __device__ __forceinline__ void adj_flush(const DeviceView& v, const double* gsu
 
 template<bool kEwald, bool kGE, bool kBig>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
-        k_backward(DeviceView v, const float4* __restrict__ gnb, float4* dnb, double* gnbfp, int* work_counter,
-                   const double* __restrict__ gE)
+        k_backward(DeviceView v, const float4* gnb, float4* dnb, double* gnbfp, int* work_counter,
+                   const double* gE)
 {
     pdl_begin();
     extern __shared__ float4 adj_dyn[];
@@ -666,8 +666,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
 // gradient sums; per-system upstream energy gradients gE[2 s], gE[2 s + 1]).
 template<bool kEwald, bool kGE, bool kBig>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
-        k_batch_backward(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
-                         double* gnbfp, int* work_counter, const double* __restrict__ gE)
+        k_batch_backward(DeviceView cv, const BatchSys* __restrict__ sys, const int* prefix, int nsys,
+                         double* gnbfp, int* work_counter, const double* gE)
 {
     pdl_begin();
     extern __shared__ float4 adj_dyn[];
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocksPerSm)
 }
 
 // Batched upstream gradients to grid order, outputs cleared.
-__global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, BatchMap map, const float* __restrict__ gF,
+__global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, BatchMap map, const float* gF,
                                     int* counter,
                                     double* gnbfp, int n_gnbfp)
 {
@@ -739,7 +739,7 @@ __global__ void k_batch_adj_prepare(const BatchSys* __restrict__ sys, BatchMap m
 
 // Batched atom-order outputs, dL/dq with the self-energy term.
 __global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ sys, BatchMap map,
-                                   const double* __restrict__ gE,
+                                   const double* gE,
                                    float* gx, float* gq)
 {
     pdl_begin();
@@ -769,7 +769,7 @@ __global__ void k_batch_adj_finish(DeviceView cv, const BatchSys* __restrict__ s
 }
 
 // Charges of all systems (concatenated atom order) into xq.w and each system's q.
-__global__ void k_batch_set_q(const BatchSys* __restrict__ sys, BatchMap map, const float* __restrict__ q)
+__global__ void k_batch_set_q(const BatchSys* __restrict__ sys, BatchMap map, const float* q)
 {
     pdl_begin();
     const int2      part = map.slots[blockIdx.x];
@@ -791,7 +791,7 @@ __global__ void k_batch_set_q(const BatchSys* __restrict__ sys, BatchMap map, co
 constexpr int kLossThreads = 256;
 
 // Loss sum |F - F_target|^2 (FP64) and its gradient 2 (F - F_target) per coordinate.
-__global__ void k_match_loss(const float* __restrict__ f, const float* __restrict__ ft, size_t n3, float* gF,
+__global__ void k_match_loss(const float* f, const float* ft, size_t n3, float* gF,
                              double* loss)
 {
     pdl_begin();
@@ -830,7 +830,7 @@ __global__ void k_match_loss(const float* __restrict__ f, const float* __restric
 // the last search) when x is given, the upstream force gradient (and the type) in grid order, a cleared dL/dx
 // accumulator; block 0 also clears the work queue and the FP64 type-pair gradient table (in place
 // of separate memsets).
-__global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const float* __restrict__ gF, float4* gnb,
+__global__ void k_adj_prepare(DeviceView v, const float* x, const float* gF, float4* gnb,
                               float4* dnb, int* counter, double* gnbfp, int n_gnbfp)
 {
     pdl_begin();
@@ -881,8 +881,8 @@ __global__ void k_adj_prepare(DeviceView v, const float* __restrict__ x, const f
 // Atom-order outputs; dL/dq also gets the self-energy term.  Block 0 also copies the type-pair
 // gradients out of the padded (nt+1)^2 table into the caller's nt^2 one when gout is given (the
 // adjoint kernel has finished: no separate launch).
-__global__ void k_adj_finish(DeviceView v, const float4* __restrict__ dnb, const double* __restrict__ gE, float* gx,
-                             float* gq, const double* __restrict__ gpad, double* gout)
+__global__ void k_adj_finish(DeviceView v, const float4* dnb, const double* gE, float* gx,
+                             float* gq, const double* gpad, double* gout)
 {
     pdl_begin();
     if (gout && blockIdx.x == 0)
@@ -921,7 +921,7 @@ __global__ void k_adj_finish(DeviceView v, const float4* __restrict__ dnb, const
 // Lorentz-Berthelot type table {6 C6, 12 C12} from per-type sigma and epsilon (one block):
 // sigma_ij = (sigma_i + sigma_j) / 2, epsilon_ij = sqrt(epsilon_i epsilon_j), C6 = 4 eps s^6,
 // C12 = 4 eps s^12 (the combination nblib applies, api/nblib/gmxsetup.cpp:143-166).
-__global__ void k_lb_table(const double* __restrict__ sig, const double* __restrict__ eps, int nt, double* table)
+__global__ void k_lb_table(const double* sig, const double* eps, int nt, double* table)
 {
     pdl_begin();
     for (int m = threadIdx.x; m < nt * nt; m += blockDim.x)
@@ -943,8 +943,8 @@ constexpr int kLbTerms   = 12;  // 55 types, what two tables in 48 KB allow
 // Its adjoint: d L / d sigma_k and d L / d epsilon_k from d L / d table (one block; every type's
 // sums run over its row and column in a fixed order).  d epsilon_ij / d epsilon_i is written
 // epsilon_j / (2 epsilon_ij), as the derivative of the square root of the product.
-__global__ void k_lb_table_backward(const double* __restrict__ sig, const double* __restrict__ eps, int nt,
-                                    const double* __restrict__ gt, double* gsig, double* geps)
+__global__ void k_lb_table_backward(const double* sig, const double* eps, int nt,
+                                    const double* gt, double* gsig, double* geps)
 {
     pdl_begin();
     extern __shared__ double lbs[];  // [2][nt * nt]: d L / d sigma_ij, d L / d epsilon_ij
@@ -1139,7 +1139,7 @@ cudaError_t launch_set_nbfp(const DeviceView& v, const float* d_nbfp, cudaStream
 
 // Charges and LJ parameters for force matching: q (atom order) into xq.w and the
 // nbfp table (with the all-zero filler type); the self energy follows the charges.
-__global__ void k_set_q(DeviceView v, const float* __restrict__ q)
+__global__ void k_set_q(DeviceView v, const float* q)
 {
     pdl_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1154,7 +1154,7 @@ __global__ void k_set_q(DeviceView v, const float* __restrict__ q)
     }
 }
 
-__global__ void k_set_nbfp(float2* nbfp, const float* __restrict__ src, int nt)
+__global__ void k_set_nbfp(float2* nbfp, const float* src, int nt)
 {
     pdl_begin();
     const int m   = blockIdx.x * blockDim.x + threadIdx.x;

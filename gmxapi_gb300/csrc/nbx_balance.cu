@@ -53,7 +53,7 @@ __device__ __forceinline__ int balance_target(const ListHeader* hdr, int min_ci_
 // nsp_max - nsp < nsp + pairs(j) - nsp_max, nsp = P[j] - P[s]: P[j] + P[j + 1] > 2 (nsp_max + P[s]), found by a ballot.
 // The last two pieces are evened out by moving one group.
 template<class Piece>
-__device__ __forceinline__ int split_entry(const unsigned char* __restrict__ grp_pairs, Sci e, int nsp_max,
+__device__ __forceinline__ int split_entry(const unsigned char* grp_pairs, Sci e, int nsp_max,
                                            const Piece& piece)
 {
     const unsigned full  = 0xffffffffu;

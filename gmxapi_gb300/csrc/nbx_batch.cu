@@ -46,7 +46,7 @@ __global__ void k_batch_prefix(const BatchSys* sys, int nsys, int* prefix, unsig
 // nbnxn_atomdata_copy_x_to_nbat_x for all systems; also clears the grid-order force accumulators and, with
 // sums, the evaluation's FP64 sums and work counter (n8 8-byte words), so no memset is needed.
 __global__ void __launch_bounds__(kBatchPart) k_batch_convert(const BatchSys* __restrict__ sys, BatchMap map,
-                                                              const float* __restrict__ x, double* sums, int n8)
+                                                              const float* x, double* sums, int n8)
 {
     pdl_begin();
     const int2      part = map.slots[blockIdx.x];
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kBatchPart) k_batch_excl_energy(DeviceView cv,
 // the entry's system slots.
 template<bool kEnergy, bool kEwald, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-        k_batch_force(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
+        k_batch_force(DeviceView cv, const BatchSys* __restrict__ sys, const int* prefix, int nsys,
                       int* work_counter, double* energies, double* fshift)
 {
     pdl_begin();
@@ -203,7 +203,7 @@ constexpr int kBatchReduceAtoms = 4;
 
 // f (concatenated, atom order) and per-system sum x (x) f, float partials reduced in FP64.
 __global__ void __launch_bounds__(kBatchPart) k_batch_reduce(const BatchSys* __restrict__ sys, BatchMap map,
-                                                             float* __restrict__ f, double* virial, int do_virial)
+                                                             float* f, double* virial, int do_virial)
 {
     pdl_begin();
     const int2      part = map.atoms4[blockIdx.x];

@@ -13,7 +13,7 @@ namespace
 
 template<bool kEnergy, int kCoul, int kThreads, int kMinBlocks, int kDepth>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-        k_batch_force_x2(DeviceView cv, const BatchSys* __restrict__ sys, const int* __restrict__ prefix, int nsys,
+        k_batch_force_x2(DeviceView cv, const BatchSys* __restrict__ sys, const int* prefix, int nsys,
                          int* work_counter, double* energies, double* fshift)
 {
     pdl_begin();

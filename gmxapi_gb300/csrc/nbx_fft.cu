@@ -46,8 +46,8 @@ __device__ __forceinline__ void load_roots(float2* W, const FftAxis& ax)
 
 // z forward: lines 2p and 2p + 1 of the real grid as one complex line a + i b, transformed, then
 // A_k = (Z_k + conj Z_{n-k}) / 2 and B_k = (Z_k - conj Z_{n-k}) / 2i for k = 0 .. n/2.
-__global__ void __launch_bounds__(kZWarps * 32) k_fft_z_r2c(FftAxis ax, const float* __restrict__ real,
-                                                            float2* __restrict__ cplx, int nlines)
+__global__ void __launch_bounds__(kZWarps * 32) k_fft_z_r2c(FftAxis ax, const float* real,
+                                                            float2* cplx, int nlines)
 {
     pdl_begin();
     extern __shared__ float2 fsm[];
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(kZWarps * 32) k_fft_z_r2c(FftAxis ax, const fl
 // imaginary parts are lines 2p and 2p + 1 of the real grid.  The imaginary parts of A_0 and B_0
 // (and of A_{n/2}, B_{n/2} for even n) are dropped, as a complex-to-real transform that assumes a
 // Hermitian line does.
-__global__ void __launch_bounds__(kZWarps * 32) k_fft_z_c2r(FftAxis ax, const float2* __restrict__ cplx,
-                                                            float* __restrict__ real, int nlines)
+__global__ void __launch_bounds__(kZWarps * 32) k_fft_z_c2r(FftAxis ax, const float2* cplx,
+                                                            float* real, int nlines)
 {
     pdl_begin();
     extern __shared__ float2 fsm[];
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kZWarps * 32) k_fft_z_c2r(FftAxis ax, const fl
 // z-frequencies t*T .. t*T + T-1 of all n points of the line (rows of T consecutive elements:
 // coalesced), warp c transforms column c, the tile is written back.
 template<bool kInv>
-__global__ void __launch_bounds__(kFftTile * 32) k_fft_strided(FftAxis ax, float2* __restrict__ data, int elem_stride,
+__global__ void __launch_bounds__(kFftTile * 32) k_fft_strided(FftAxis ax, float2* data, int elem_stride,
                                                                int outer_stride, int ntiles, int nzc)
 {
     pdl_begin();

@@ -218,7 +218,7 @@ constexpr int kCols   = 8;  // z-frequencies per block of the strided passes
 // A_k = (Z_k + conj Z_{n-k}) / 2 and B_k = (Z_k - conj Z_{n-k}) / 2i for k = 0 .. n/2.
 template<int R1, int R2>
 __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
-        k_z_r2c(const float2* __restrict__ roots, const float* __restrict__ real, float2* __restrict__ cplx, int nlines)
+        k_z_r2c(const float2* __restrict__ roots, const float* real, float2* cplx, int nlines)
 {
     pdl_begin();
     using S              = Shape<R1, R2>;
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
 // B_{n/2} for even n) are dropped, as a complex-to-real transform that assumes a Hermitian line does.
 template<int R1, int R2>
 __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
-        k_z_c2r(const float2* __restrict__ roots, const float2* __restrict__ cplx, float* __restrict__ real, int nlines)
+        k_z_c2r(const float2* __restrict__ roots, const float2* cplx, float* real, int nlines)
 {
     pdl_begin();
     using S              = Shape<R1, R2>;
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(round32(kZPairs* Shape<R1, R2>::threads))
 // z-frequencies t kCols .. t kCols + kCols - 1.
 template<int R1, int R2, bool kInv>
 __global__ void __launch_bounds__(round32(kCols* Shape<R1, R2>::threads))
-        k_strided(const float2* __restrict__ roots, float2* __restrict__ data, int elem_stride, int outer_stride,
+        k_strided(const float2* __restrict__ roots, float2* data, int elem_stride, int outer_stride,
                   int ntiles, int nzc)
 {
     pdl_begin();
@@ -512,7 +512,7 @@ struct Plane
 
 template<int R1, int R2>
 __global__ void __launch_bounds__(Plane<R1, R2>::threads)
-        k_plane_r2c(const float2* __restrict__ roots, const float* __restrict__ real, float2* __restrict__ cplx)
+        k_plane_r2c(const float2* __restrict__ roots, const float* real, float2* cplx)
 {
     pdl_begin();
     using S = Shape<R1, R2>;
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(Plane<R1, R2>::threads)
 
 template<int R1, int R2>
 __global__ void __launch_bounds__(Plane<R1, R2>::threads)
-        k_plane_c2r(const float2* __restrict__ roots, const float2* __restrict__ cplx, float* __restrict__ real)
+        k_plane_c2r(const float2* __restrict__ roots, const float2* cplx, float* real)
 {
     pdl_begin();
     using S = Shape<R1, R2>;

@@ -245,7 +245,7 @@ constexpr int kReduceThreads = 256;
 // kAtoms atoms a thread.
 template<int kAtoms>
 __global__ void __launch_bounds__(kReduceThreads)
-        k_reduce_f(DeviceView v, float* __restrict__ f, int do_virial, double* d_energies, double* d_virial, int stage,
+        k_reduce_f(DeviceView v, float* f, int do_virial, double* d_energies, double* d_virial, int stage,
                    unsigned* d_status)
 {
     pdl_begin();

@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_fill(DeviceView v, unsign
 // clear: also zero what a force evaluation accumulates into (the grid-order forces,
 // shift forces, energies, virial, the work queue and the reduction's completion
 // counter), in place of separate memsets before the force kernel.
-__global__ void k_convert_x(DeviceView v, const float* __restrict__ x, int clear, int atom_order)
+__global__ void k_convert_x(DeviceView v, const float* x, int clear, int atom_order)
 {
     pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -12,11 +12,14 @@ struct nbx_pme;
 namespace nbx
 {
 
-// Every kernel is launched as a programmatic dependent of the kernel before it on its stream: its blocks
-// may take their places while that kernel still runs, and wait in pdl_begin (the first statement of
-// every kernel, before any access to memory) until it has ended and its writes are visible.  An
+// Every kernel of an evaluation is launched as a programmatic dependent of the kernel before it on its
+// stream: its blocks may take their places while that kernel still runs, and wait in pdl_begin (their first
+// statement, before any access to memory) until it has ended and its writes are visible.  An
 // evaluation is a chain of kernels of a few microseconds, so their launch latencies and block start-up
 // were a large part of it (3,000 atoms: 3 kernels for the forces, 7 for PME).
+// What an earlier kernel may write is not constant for as long as such a kernel is resident: pointers to it
+// are not __restrict__ (the compiler could move their loads above the wait, and const ones through the
+// non-coherent path), only those to tables that the host writes before any launch.
 __device__ __forceinline__ void pdl_begin()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -59,8 +59,8 @@ __device__ __forceinline__ float put_in_box(float x, float L)
 }
 
 __global__ void __launch_bounds__(kLfThreads) k_leapfrog(int n, float dt, const float* __restrict__ inv_mass,
-                                                         float* __restrict__ x, float* __restrict__ v,
-                                                         const float* __restrict__ f, float3 box, int wrap,
+                                                         float* x, float* v,
+                                                         const float* f, float3 box, int wrap,
                                                          double* partials, unsigned* done, double* ekin_out)
 {
     nbx::pdl_begin();

@@ -83,7 +83,7 @@ struct AtomSplines
     float dth[3][kOrder];
 };
 
-__device__ __forceinline__ void atom_splines(const PmeDims& d, const float* __restrict__ x, int a, AtomSplines& s)
+__device__ __forceinline__ void atom_splines(const PmeDims& d, const float* x, int a, AtomSplines& s)
 {
     for (int k = 0; k < 3; k++)
     {
@@ -99,7 +99,7 @@ __device__ __forceinline__ int wrap_once(int i, int n)
 }
 
 // Spline data in the reference's test layout: idx [N][3], theta/dtheta [3][N][4].
-__global__ void k_pme_splines(PmeDims d, int natoms, const float* __restrict__ x, int* idx, float* theta,
+__global__ void k_pme_splines(PmeDims d, int natoms, const float* x, int* idx, float* theta,
                               float* dtheta)
 {
     nbx::pdl_begin();
@@ -154,8 +154,8 @@ __device__ __forceinline__ void spread_row_v4(float* row, int gz0, int nz, const
 
 // x point ix of an atom: adds its 4 x 4 (y, z) weights to the grid.
 template<bool kVec>
-__device__ __forceinline__ void spread_quarter(const PmeDims& d, int a, int ix, const float* __restrict__ x,
-                                               const float* __restrict__ q, float* grid)
+__device__ __forceinline__ void spread_quarter(const PmeDims& d, int a, int ix, const float* x,
+                                               const float* q, float* grid)
 {
     const float qa = q[a];
     if (qa == 0.0f)
@@ -197,7 +197,7 @@ __device__ __forceinline__ void spread_quarter(const PmeDims& d, int a, int ix, 
 
 // Four threads per atom (one x point each).
 template<bool kVec>
-__global__ void k_pme_spread(PmeDims d, int natoms, const float* __restrict__ x, const float* __restrict__ q,
+__global__ void k_pme_spread(PmeDims d, int natoms, const float* x, const float* q,
                              float* grid)
 {
     nbx::pdl_begin();
@@ -243,8 +243,8 @@ __device__ __forceinline__ int brick_count(const Bricks& b)
 }
 
 // Files the atoms by brick and clears the grid (no block adds to it before this kernel has ended).
-__global__ void __launch_bounds__(256) k_pme_file(PmeDims d, Bricks b, int natoms, const float* __restrict__ x,
-                                                  const float* __restrict__ q, float4* grid4, int n4)
+__global__ void __launch_bounds__(256) k_pme_file(PmeDims d, Bricks b, int natoms, const float* x,
+                                                  const float* q, float4* grid4, int n4)
 {
     nbx::pdl_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -307,7 +307,7 @@ struct SpreadWarp
 };
 
 __global__ void __launch_bounds__(32 * kBrickWarps)
-        k_pme_spread_bricks(PmeDims d, Bricks b, const float* __restrict__ x, const float* __restrict__ q, float* grid)
+        k_pme_spread_bricks(PmeDims d, Bricks b, const float* x, const float* q, float* grid)
 {
     nbx::pdl_begin();
     extern __shared__ float4 spread_smem[];
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_pme_solve_lj(PmeDims d, float
 }
 
 // Force of one atom of charge qa from the potential grid (do_fspline + gather_f_bsplines), added to f.
-__device__ __forceinline__ void gather_atom(const PmeDims& d, int a, float qa, const float* __restrict__ x,
-                                            const float* __restrict__ grid, float* f)
+__device__ __forceinline__ void gather_atom(const PmeDims& d, int a, float qa, const float* x,
+                                            const float* grid, float* f)
 {
     AtomSplines s;
     atom_splines(d, x, a, s);
@@ -634,7 +634,7 @@ __device__ __forceinline__ void gather_atom(const PmeDims& d, int a, float qa, c
             float        sz = 0.0f, sdz = 0.0f;
             for (int iz = 0; iz < kOrder; iz++)
             {
-                const float g = __ldg(&row[gz[iz]]);
+                const float g = row[gz[iz]];
                 sz            = fmaf(s.th[2][iz], g, sz);
                 sdz           = fmaf(s.dth[2][iz], g, sdz);
             }
@@ -650,8 +650,8 @@ __device__ __forceinline__ void gather_atom(const PmeDims& d, int a, float qa, c
 
 // kLanes 4: four threads per atom, one x point each; 1: a thread per atom.
 template<int kLanes>
-__global__ void k_pme_gather(PmeDims d, int natoms, const float* __restrict__ x, const float* __restrict__ q,
-                             const float* __restrict__ grid, float* f, PmeTotals tot)
+__global__ void k_pme_gather(PmeDims d, int natoms, const float* x, const float* q,
+                             const float* grid, float* f, PmeTotals tot)
 {
     nbx::pdl_begin();
     if (tot.partials && blockIdx.x == 0 && threadIdx.x < 32)
@@ -691,7 +691,7 @@ __global__ void k_pme_gather(PmeDims d, int natoms, const float* __restrict__ x,
 #pragma unroll
             for (int iz = 0; iz < kOrder; iz++)
             {
-                const float g = __ldg(&row[gz[iz]]);
+                const float g = row[gz[iz]];
                 sz            = fmaf(s.th[2][iz], g, sz);
                 sdz           = fmaf(s.dth[2][iz], g, sdz);
             }
@@ -719,8 +719,8 @@ __global__ void k_pme_gather(PmeDims d, int natoms, const float* __restrict__ x,
 // The same by bricks: a block per brick reads the brick's 11 x 11 x 12 points into shared memory and
 // takes its filed atoms, one per thread; the counts are cleared for the next call.
 __global__ void __launch_bounds__(kGatherThreads, 10)
-        k_pme_gather_bricks(PmeDims d, Bricks b, const float* __restrict__ x, const float* __restrict__ q,
-                            const float* __restrict__ grid, float* f, PmeTotals tot)
+        k_pme_gather_bricks(PmeDims d, Bricks b, const float* x, const float* q,
+                            const float* grid, float* f, PmeTotals tot)
 {
     nbx::pdl_begin();
     __shared__ float tile[kTileFloats];
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kGatherThreads, 10)
         const int    tx = row / kTile, ty = row - tx * kTile;
         const int    gx = brick_point(bx * kBrick, tx, d.n[0]), gy = brick_point(by * kBrick, ty, d.n[1]);
         const int    gz = brick_point(bz * kBrick, z4, d.n[2]);
-        const float4 g  = __ldg(reinterpret_cast<const float4*>(grid + ((size_t)gx * d.n[1] + gy) * d.n[2] + gz));
+        const float4 g  = *reinterpret_cast<const float4*>(grid + ((size_t)gx * d.n[1] + gy) * d.n[2] + gz);
         float2*      t  = reinterpret_cast<float2*>(tile + tx * kTileSx + ty * kTileSy + z4);
         t[0]            = make_float2(g.x, g.y);
         t[1]            = make_float2(g.z, g.w);

@@ -54,7 +54,7 @@ __device__ __forceinline__ float exact_r2(float dx, float dy, float dz)
 
 // The smallest squared distance between the 8 atoms at xi (shifted by s*) and the 4 at xj, each
 // rounded as the CPU restatement rounds it.
-__device__ __noinline__ float exact_min_r2(const float4* __restrict__ xi, const float4* __restrict__ xj, float sx,
+__device__ __noinline__ float exact_min_r2(const float4* xi, const float4* xj, float sx,
                                            float sy, float sz)
 {
     unsigned m = 0xffffffffu;
