@@ -1197,11 +1197,11 @@ int nbx_md_step_device(nbx_handle* h, long long step, const float* d_x, float* d
 namespace nbx
 {
 
-int md_forces(nbx_handle* h, const float* d_x, float* d_f, double* d_e, int force_grid)
+int md_forces(nbx_handle* h, const float* d_x, float* d_f, double* d_e, bool share)
 {
-    h->v.force_grid = force_grid;
-    const int rc    = compute_async(h, d_x, d_f, d_e, nullptr);
-    h->v.force_grid = 0;
+    h->v.force_share = share ? 1 : 0;
+    const int rc     = compute_async(h, d_x, d_f, d_e, nullptr);
+    h->v.force_share = 0;
     return rc;
 }
 

@@ -141,8 +141,8 @@ cudaError_t launch_x2(const DeviceView& v, cudaStream_t s, int num_sms, int* cou
     {
         return e;
     }
-    launch_pdl(k_force_x2<kEnergy, kCoul, kDepth, kBlocks, kLj>, v.force_grid ? v.force_grid : num_sms * kBlocks,
-               kForceThreads, smem, s, v, counter);
+    const int blocks = v.force_share ? num_sms * kBlocks * 3 / 4 : num_sms * kBlocks;
+    launch_pdl(k_force_x2<kEnergy, kCoul, kDepth, kBlocks, kLj>, blocks, kForceThreads, smem, s, v, counter);
     return cudaGetLastError();
 }
 

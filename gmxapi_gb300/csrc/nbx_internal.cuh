@@ -272,7 +272,7 @@ struct DeviceView
     int pair_core;
     int stage_depth;
     int force_blocks;  // resident blocks of 256 threads per SM for the packed kernel (2, 3)
-    int force_grid;    // blocks of the packed kernel; 0: all that are resident
+    int force_share;   // 1: the packed kernel leaves a quarter of its block slots to a kernel beside it
 };
 
 // The system of batch entry e: the last system whose entry prefix sum is <= e.
@@ -464,9 +464,9 @@ cudaError_t launch_convert_x(const DeviceView& v, const float* d_x, cudaStream_t
 cudaError_t launch_search(const DeviceView& v, cudaStream_t s);
 cudaError_t launch_prune(const DeviceView& v, int fresh, int part, int nparts, cudaStream_t s);
 // The parts of nbx_md_step_device: the lists of a step (*searched: by a search, which puts d_x in the box), and its
-// forces, with force_grid blocks in the packed force kernel (0: all that are resident).
+// forces, the packed force kernel without a quarter of its blocks when share is set.
 int md_lists(nbx_handle* h, long long step, const float* d_x, bool* searched);
-int md_forces(nbx_handle* h, const float* d_x, float* d_f, double* d_e, int force_grid);
+int md_forces(nbx_handle* h, const float* d_x, float* d_f, double* d_e, bool share);
 // The parts of nbx_pme_compute_device: the potential on the grid, on stream s, and the forces, on the handle's.
 int pme_potential(nbx_pme* p, int natoms, const float* d_x, const float* d_q, double* d_energy, double* d_virial,
                   cudaStream_t s);

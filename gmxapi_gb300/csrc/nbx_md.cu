@@ -435,7 +435,7 @@ int nbx_md_run_device(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long f
 namespace
 {
 
-// Up to this many atoms the force kernel beside a mesh part leaves a quarter of its block slots free: the mesh
+// Up to this many atoms the (packed) force kernel beside a mesh part leaves a quarter of its block slots free: the mesh
 // kernels are as long as it and bound by latency.  20 steps of 10 976 / 32 000 / 55 296 / 87 808 / 364 500 atoms:
 // 1142 / 1601 / 2017 / 2750 / 10097 us so, 1139 / 1663 / 2116 / 2665 / 9672 us with all of its blocks.
 constexpr int kSharedSmAtoms = 65536;
@@ -464,7 +464,7 @@ int step_with_mesh(nbx_handle* h, nbx_pme* pme, nbx_leapfrog* lf, long long step
     }
     if (e == cudaSuccess && rc == NBX_OK)
     {
-        rc = nbx::md_forces(h, d_x, d_f, row, natoms <= kSharedSmAtoms ? lf->num_sms * 3 / 2 : 0);
+        rc = nbx::md_forces(h, d_x, d_f, row, natoms <= kSharedSmAtoms);
     }
     // the side stream joins also when something failed
     if (e == cudaSuccess) e = cudaStreamWaitEvent(main, lf->potential, 0);

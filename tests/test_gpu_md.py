@@ -178,6 +178,78 @@ def test_md_run_forces_match_separate_calls(md, cells):
     ref.close()
 
 
+@pytest.mark.parametrize("cells", [12, 26])
+def test_md_run_of_moving_atoms_matches_separate_calls(md, cells):
+    """13 steps of atoms that move 0.003 nm a step (a search in between), mesh part beside the short-range forces,
+    against the same parts called one after the other on one stream.  Positions differ by their rounding (1e-6 nm a
+    step at 14 nm), which the soft potential turns into 1e-4 of the forces; a mesh part that saw the coordinates
+    before or after a step would be off by 1e-3 and more."""
+    from gmxapi_gb300 import nblib, systems
+
+    s = systems.lj_fcc(cells=cells, lattice=0.5256, charge=0.3, seed=21)
+    s.nbfp = (0.01 * np.asarray(s.nbfp)).astype(np.float32)
+    rng = np.random.default_rng(4)
+    v0 = rng.uniform(-1.5, 1.5, (s.n, 3)).astype(np.float32)
+    masses = np.full(s.n, systems.ARGON_MASS, np.float32)
+    opts = nblib.NBKernelOptions(pairlist_cutoff=1.1, rcoulomb=0.9, nstlist=10, compute_virial_and_energy=True)
+    run = md.MdRunner(s, masses, opts, dt=0.002, velocities=v0)
+    rows = run.run(13, nstcalcenergy=6)
+    ref = md.MdRunner(s, masses, opts, dt=0.002, velocities=v0)
+    for obj in (ref.pme, ref.lf):
+        obj.set_stream(ref.stream.cuda_stream)
+    e = torch.zeros((13, 3), dtype=torch.float64, device="cuda")
+    for step in range(13):
+        ref.calc.md_step_device(step, ref.x.data_ptr(), ref.f.data_ptr(), e[step].data_ptr(), None)
+        ref.pme.compute_device(s.n, ref.x.data_ptr(), ref.q.data_ptr(), ref.f.data_ptr(), e[step, 2:].data_ptr(), None)
+        ref.lf.integrate_device(0.002, ref.x.data_ptr(), ref.v.data_ptr(), ref.f.data_ptr(), None)
+    torch.cuda.synchronize()
+    assert rel_rms(run.f.cpu().numpy(), ref.f.cpu().numpy()) <= 3e-4
+    assert rel_rms(run.velocities(), ref.velocities()) <= 1e-5
+    box = np.asarray(s.box, np.float64)
+    d = run.positions().astype(np.float64) - ref.positions()
+    assert np.abs(d - np.round(d / box) * box).max() <= 2e-5
+    np.testing.assert_allclose(rows[:, :3], e.cpu().numpy()[::6], rtol=1e-5)
+    run.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("blocks_per_sm", [2, 3])
+@pytest.mark.parametrize("share", [True, False])
+def test_shared_force_launch_leaves_a_quarter_of_its_blocks(md, share, blocks_per_sm, tmp_path):
+    """The grid of the short-range forces of a step with PME (three quarters of the packed kernel's block slots up to
+    65,536 atoms, all of them beyond), for both of its shapes, as the profiler records it."""
+    import ctypes
+    import json
+
+    from gmxapi_gb300 import _lib, nblib, systems
+
+    s = systems.lj_fcc(cells=6, lattice=0.5256, charge=0.3, seed=21)
+    calc = nblib.ForceCalculator(s, nblib.NBKernelOptions(pairlist_cutoff=1.0, rcoulomb=0.9))
+    calc.set_force_kernel(1, 2, blocks_per_sm)
+    stream = torch.cuda.Stream()
+    calc.set_stream(stream.cuda_stream)
+    forces = getattr(_lib.load(), "_ZN3nbx9md_forcesEP10nbx_handlePKfPfPdb")
+    forces.argtypes = 4 * [ctypes.c_void_p] + [ctypes.c_bool]
+    x = torch.from_numpy(s.x.reshape(-1).copy()).cuda()
+    f = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    for _ in range(2):  # the first session of a process may record nothing
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            assert forces(calc.h, x.data_ptr(), f.data_ptr(), None, share) == 0
+            torch.cuda.synchronize()
+    path = str(tmp_path / "step.json")
+    prof.export_chrome_trace(path)
+    with open(path) as fh:
+        kernels = [e for e in json.load(fh)["traceEvents"] if e.get("cat") == "kernel"]
+    if not kernels:
+        pytest.skip("no kernel records from the profiler")
+    grids = {e["args"]["grid"][0] for e in kernels if "k_force_x2" in e["name"]}
+    slots = torch.cuda.get_device_properties(0).multi_processor_count * blocks_per_sm
+    assert grids == {slots * 3 // 4 if share else slots}
+    assert rel_rms(f.cpu().numpy(), calc.compute(s.x, energies=False).reshape(-1)) <= 1e-6
+    calc.close()
+
+
 def test_md_nve_energy_drift(md):
     """2,000 steps (4 ps) of NVE argon-like atoms with charges (LJ + Ewald + PME), started from
     the lattice at 120 K: total-energy drift bounded."""
