@@ -64,6 +64,7 @@ __device__ __forceinline__ float wrap_coord(float v, float L, ListHeader* hdr, i
 
 constexpr int kGridThreads    = 256;   // 45k atoms in blocks of 1024 x 4 filled 11 of the SMs: 8.3 us, now 4.3 us
 constexpr int kMaxSmemCols    = 8192;  // column counters kept in shared memory up to this many columns
+constexpr int kOneAtomCols    = 4096;  // columns up to which a thread takes one atom
 
 // Wrap into the box, column index, and each atom's slot within its column.
 // Column counts are gathered per block in shared memory; each block then
@@ -686,8 +687,10 @@ cudaError_t launch_grid(const DeviceView& v, float* d_x, int write_back, cudaStr
     cudaMemsetAsync(v.cxy_na, 0, sizeof(int) * (v.g.ncol + 1), s);
     const int tb = 256;
     const size_t smem   = v.g.ncol <= kMaxSmemCols ? sizeof(int) * (size_t)v.g.ncol : 0;
-    // an atom per thread fills the GPU soonest; with many columns a block's counters are worth more atoms
-    if (v.g.ncol <= 4 * kGridThreads)
+    // an atom per thread fills the GPU soonest; with many columns a block's counters are worth more atoms: gridding
+    // takes 38.2 / 59.2 / 79.6 us with one and 40.7 / 61.8 / 82.7 us with eight at 1156 / 2401 / 3600 columns, 155.2 /
+    // 138.8 and 154.3 / 136.3 us at 7225 / 5476
+    if (v.g.ncol <= kOneAtomCols)
     {
         launch_pdl(k_wrap_column<1>, (v.n + kGridThreads - 1) / kGridThreads, kGridThreads, smem, s, v, d_x, write_back);
     }

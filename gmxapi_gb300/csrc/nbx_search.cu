@@ -88,7 +88,7 @@ constexpr int kEmitStage = 512;  // j-lists up to this length are staged in shar
                                  // exclusion lookups
 
 constexpr int kShiftSlots   = kCentral + 1;  // shifts 0 .. central, the visiting order
-constexpr int kManyCells    = 4096;          // i-cells from which a cell takes two warps
+constexpr int kManyCells    = 1200;          // grid capacity from which a cell takes two warps
 constexpr int kCellWindow   = 128;           // candidate j-cells in shared memory at a time
 static_assert(kShiftSlots <= kMaxEntriesPerCell && kShiftSlots <= 32, "one lane and one entry code per shift");
 
@@ -1107,8 +1107,10 @@ cudaError_t launch_search_count(const DeviceView& v, cudaStream_t s)
     // num_subpairs .. rec_need: accumulated by the count pass or set by balancing
     cudaMemsetAsync(&v.hdr->num_subpairs, 0,
                     offsetof(ListHeader, rec_need) + sizeof(int) - offsetof(ListHeader, num_subpairs), s);
-    // two warps a cell once the cells alone fill the GPU (960k atoms, 15.6k cells: the search step 1671 us, with
-    // four 1686 us), four while a cell's latency counts (45k atoms: 235 us, with two 240 us)
+    // two warps a cell once the cells alone fill the GPU, four while a cell's latency counts.  The host knows the
+    // grid's capacity, not its cells; at 100 / 50 / 25 atoms per nm^3 and a capacity of 1018 the pass takes
+    // 23.0 / 20.0 / 18.0 us with four and 28.1 / 22.1 / 20.0 us with two, at 1365 27.2 / 24.4 / 24.1 and 24.2 / 21.0 /
+    // 20.0 us, at 4474 53.6 / 42.9 / 44.5 and 48.6 / 36.5 / 37.3 us (at 2653 and 3008, 100 per nm^3, equal)
     if (cap > kManyCells)
     {
         launch_pdl(k_search_count<2>, cap, 64, 0, s, v);

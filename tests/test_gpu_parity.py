@@ -159,6 +159,41 @@ def test_search_windows_match_oracle(molecules, edge, rlist):
     calc.close()
 
 
+@pytest.mark.parametrize("edge,columns", [(71.7, 64 * 64), (74.0, 65 * 65), (204.0, 91 * 91)])
+def test_many_columns_match_oracle(edge, columns):
+    """A flat box whose atoms are gridded one per thread (up to 4096 columns), eight per thread (beyond) and without
+    column counters in shared memory (more than 8192): grid and list as the oracle's."""
+    n, rng = 60000, np.random.default_rng(12)
+    box = np.array([edge, edge, 0.25], np.float32)
+    s = systems.System(x=(rng.random((n, 3)) * box).astype(np.float32), box=box, q=np.zeros(n, np.float32),
+                       type=np.zeros(n, np.int32), ntypes=1, nbfp=systems.nbfp_from_c6c12(np.array([[1e-3]]), np.array([[1e-6]])),
+                       excl_index=np.arange(n + 1, dtype=np.int32), excl_list=np.arange(n, dtype=np.int32), name="flat")
+    calc, o = _pair(s, rc=0.2, rlist=0.24)
+    g, r = calc.grid(), o.grid_arrays()
+    assert g["ncx"] * g["ncy"] == columns
+    for k in ("cxy_ind", "num_clusters", "atom_indices", "cells", "bbcz", "xq"):
+        np.testing.assert_array_equal(g[k], r[k], err_msg=k)
+    pg, po = calc.pairlist(), o.pairlist()
+    assert np.array_equal(canonical_pairs(pg["sci"], pg["cj4"], pg["excl"]),
+                          canonical_pairs(po["sci"], po["cj4"], po["excl"]))
+    calc.close()
+
+
+@pytest.mark.parametrize("molecules,four_warps", [(23400, True), (24000, False)])
+def test_search_count_shapes_match_oracle(molecules, four_warps):
+    """Grids just below and above the capacity of 1200 cells from which the count pass takes two warps a cell instead of
+    four: the same entries in the same order with the same pairs."""
+    s = systems.spc_water(molecules, (molecules * 0.0299) ** (1 / 3), seed=3)
+    calc, o = _pair(s)
+    g = calc.grid()
+    assert (s.n // 64 + g["ncx"] * g["ncy"] <= 1200) == four_warps
+    pg, po = calc.pairlist(), o.pairlist()
+    np.testing.assert_array_equal(pg["sci"], po["sci"])
+    assert np.array_equal(canonical_pairs(pg["sci"], pg["cj4"], pg["excl"]),
+                          canonical_pairs(po["sci"], po["cj4"], po["excl"]))
+    calc.close()
+
+
 @pytest.mark.parametrize("reach,molecules,edge,rlist", [(1, 300, 2.08, 1.0), (3, 300, 2.08, 1.0), (9, 1500, 3.56, 1.7)])
 def test_exclusion_masks_match_oracle(reach, molecules, edge, rlist):
     """Exclusions with the `reach` neighbours on either side in atom order: cells with fewer and with more than the
