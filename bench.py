@@ -691,7 +691,8 @@ PME_SPACING = 0.12
 def measure_pme(dev: int, calc=None, frames=None, flush=None, stream=None, steps: int = 20) -> dict:
     """Smooth-PME reciprocal space for the same 288k-atom box (120^3 grid at 0.12 nm, beta
     from rc 0.9 / rtol 1e-5, pme_order 4): the whole reciprocal step with energy and
-    virial, the spread and gather stages alone, the full electrostatics step (cluster-pair
+    virial, the transforms alone, the spread and gather entries (which take the atoms
+    directly, where the whole step files them by grid brick), the full electrostatics step (cluster-pair
     real space + PME) on one stream, the host-array call, parity against the PME oracle
     and the oracle's own time on the host.  Each timed pass follows a 256 MB L2 flush."""
     import torch
@@ -748,6 +749,14 @@ def measure_pme(dev: int, calc=None, frames=None, flush=None, stream=None, steps
     gather = timed(lambda k: p.gather_device(n, frames[k % nf].data_ptr(), q.data_ptr(), g.data_ptr(),
                                              f.data_ptr()))
 
+    cg = torch.zeros((grid[0], grid[1], grid[2] // 2 + 1, 2), dtype=torch.float32, device=frames.device)
+
+    def transforms(k):
+        p.fft_device(1, g.data_ptr(), cg.data_ptr())
+        p.fft_device(-1, g.data_ptr(), cg.data_ptr())
+
+    ffts = timed(transforms)
+
     def electrostatics(k):
         x = frames[k % nf].data_ptr()
         calc.compute_device(x, f.data_ptr(), ev[1:].data_ptr(), ev[3:].data_ptr())
@@ -779,12 +788,15 @@ def measure_pme(dev: int, calc=None, frames=None, flush=None, stream=None, steps
         "grid": list(grid), "beta": beta, "atoms": n,
         "ms_energy_virial": full, "ms_forces_only": forces_only,
         "atoms_per_s": n / (full * 1e-3),
-        "stages_ms": {"spread": spread, "gather": gather,
-                      "ffts_solve_memset": forces_only - spread - gather},
-        "spread": {"weighted_adds_per_s": n * 64 / (spread * 1e-3),
-                   "vector_reductions_per_s": red_ops / (spread * 1e-3),
-                   "note": "64 weighted grid adds per atom as 16-byte red.global.add.v4.f32; the 6.9 MB "
-                           "grid stays in L2, so the bound is L2 reduction throughput, not HBM"},
+        "stages_ms": {"transforms_alone": ffts, "file_spread_solve_gather": forces_only - ffts,
+                      "note": "transforms: nbx_pme_fft_device both ways (the step does the solve inside its x pass); "
+                              "the rest of a step without energies"},
+        "entries_ms": {"spread_device": spread, "gather_device": gather,
+                       "spread_weighted_adds_per_s": n * 64 / (spread * 1e-3),
+                       "spread_vector_reductions_per_s": red_ops / (spread * 1e-3),
+                       "note": "nbx_pme_spread_device and nbx_pme_gather_device take the atoms directly (64 weighted "
+                               "grid adds per atom as 16-byte red.global.add.v4.f32, bound by L2 reductions); the "
+                               "step above files them by grid brick and launches neither kernel"},
         "electrostatics_step_ms": step_ms,
         "electrostatics_note": "cluster-pair LJ + Ewald real space (F+E+virial) then PME (F+E+virial) "
                                "on one stream, list fixed",
@@ -798,8 +810,8 @@ def measure_pme(dev: int, calc=None, frames=None, flush=None, stream=None, steps
 
 
 def measure_md(dev: int, steps: int = 200, warmup: int = 20) -> dict:
-    """GPU-resident MD steps (nbx_md_run_device): cluster-pair LJ + Ewald real space, PME
-    reciprocal space and leap-frog on one stream, for 296,352 argon-like atoms with charges
+    """GPU-resident MD steps (nbx_md_run_device): cluster-pair LJ + Ewald real space beside the
+    grid part of PME, and leap-frog, for 296,352 argon-like atoms with charges
     +-0.1 e (fcc start at 120 K, box 22.08 nm, rc 0.9, rlist 1.0, nstlist 10, dynamic pruning to
     rlist_inner 0.92 every 4 steps in 2 rolling parts as mdrun does on a GPU, PME grid at 0.12 nm,
     dt 2 fs), energies every 100 steps.  Reports the step time and the NVE drift (the inner radius

@@ -578,7 +578,7 @@ cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int n
     {
         // an atom's exclusions are a chain of dependent loads: one atom per lane while that leaves fewer items
         // than the list has entries (24k atoms: about 750 beside 6,700), four where items would only add
-        // queue traffic
+        // queue traffic (24k to 180k water atoms: within 0.7 % of each other on either side of the line)
         kv.excl_atoms  = v.n < 65536 ? 32 : kExclChunkAtoms;
         kv.excl_chunks = (v.n + kv.excl_atoms - 1) / kv.excl_atoms;
     }

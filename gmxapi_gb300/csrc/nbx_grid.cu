@@ -353,7 +353,9 @@ constexpr int kBinMean       = 26;  // keys a bin is made for
 constexpr int kBinSortMax    = 32 * kMaxBins;
 
 // Sorts the n atoms of a column on z through bins of equal height (monotone in z, so that the sorted bins make the
-// sorted column); false, with nothing written, when a bin overflows (layers).
+// sorted column); false, with nothing written, when a bin overflows (layers, boxes partly empty along z: gridding of
+// 96 000 / 288 000 atoms in a third of their box 65 / 48 us, with the sort of the whole column alone 74 / 76 us; evenly
+// spread 24 / 31 and 43 / 70 us).
 __device__ bool bin_sort(const DeviceView& v, int base, int n, unsigned long long* keys, int* bin_n)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

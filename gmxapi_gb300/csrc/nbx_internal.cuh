@@ -475,10 +475,10 @@ int pme_forces(nbx_pme* p, int natoms, const float* d_x, const float* d_q, float
 
 cudaError_t launch_force(const DeviceView& v, bool energy, cudaStream_t s, int num_sms, cudaEvent_t ev0 = nullptr,
                          cudaEvent_t ev1 = nullptr);
-// the packed-core force kernel (v.pair_core 1; potential-shift or plain cut-off LJ), with the
+// the packed-core force kernel (v.pair_core 1) for potential-shift and plain cut-off LJ, with the
 // v.stage_depth j-stage buffers and v.force_blocks blocks per SM
 cudaError_t launch_force_x2(const DeviceView& v, bool energy, cudaStream_t s, int num_sms, int* counter);
-// the same with lj 1 force switch, 2 potential switch, 3 LJ-PME
+// the same kernel in its default shape with lj 1 force switch, 2 potential switch, 3 LJ-PME
 cudaError_t launch_force_x2_lj(const DeviceView& v, int lj, bool energy, cudaStream_t s, int num_sms, int* counter);
 // forces to atom order (+ virial); with d_e / d_vir the last block also finishes the energies
 // and virial (the accumulators must have been cleared by launch_convert_x(clear))

@@ -436,8 +436,9 @@ namespace
 {
 
 // Up to this many atoms the (packed) force kernel beside a mesh part leaves a quarter of its block slots free: the mesh
-// kernels are as long as it and bound by latency.  20 steps of 10 976 / 32 000 / 55 296 / 87 808 / 364 500 atoms:
-// 1142 / 1601 / 2017 / 2750 / 10097 us so, 1139 / 1663 / 2116 / 2665 / 9672 us with all of its blocks.
+// kernels are as long as it and bound by latency.  20 steps of 10 976 / 32 000 / 55 296 / 62 500 / 87 808 / 364 500
+// atoms at 27.5 per nm^3: 1063 / 1480 / 1908 / 2127 / 2693 / 9988 us so, 1081 / 1559 / 1983 / 2101 / 2553 / 9523 us with
+// all of its blocks; of 62 500 / 70 304 / 87 808 at 62.5 per nm^3: 2390 / 2581 / 3040 and 2397 / 2645 / 2910 us.
 constexpr int kSharedSmAtoms = 65536;
 
 // Forces of one step with PME: the mesh potential (spread, transforms, solve) on the side stream beside the

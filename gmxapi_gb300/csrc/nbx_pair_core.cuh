@@ -297,7 +297,9 @@ __device__ __forceinline__ void process_half(const DeviceView& v, const SysPtrs&
             }
             else if (kLj != 0)
             {
-                // force / potential switch from rvdw_switch to rc (kernel_ref_inner.h:168-200)
+                // force / potential switch from rvdw_switch to rc (kernel_ref_inner.h:168-200); as there, an
+                // excluded pair beyond rvdw_switch keeps the force switch's polynomial in its force, while its
+                // energy does not count
                 const float r   = r2 * rinv;
                 const float rsw = fmaxf(r - v.rvdw_switch, 0.0f);
                 const float rs2 = rsw * rsw;

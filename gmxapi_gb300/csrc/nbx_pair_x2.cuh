@@ -326,7 +326,8 @@ __device__ __forceinline__ void pair_phys_x2(const PairConstsX2& k, const char* 
     if (kLj == 1 || kLj == 2)
     {
         // force / potential switch from rvdw_switch to rc (kernel_ref_inner.h:168-200); r = 0 for pairs out of
-        // range
+        // range.  As there, an excluded pair beyond rvdw_switch keeps the force switch's polynomial in its force,
+        // while its energy does not count
         const float2 r   = mul2(r2, rinv);
         const float2 rsw = make_float2(fmaxf(r.x - k.rvdw_switch, 0.0f), fmaxf(r.y - k.rvdw_switch, 0.0f));
         const float2 rs2 = mul2(rsw, rsw);

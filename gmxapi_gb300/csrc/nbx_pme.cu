@@ -959,9 +959,11 @@ cudaError_t launch_spread(nbx_pme* p, int natoms, const float* d_x, const float*
 
 // Whether nbx_pme_compute_device files the atoms by brick.  The extra pass over the atoms has to pay, and
 // a brick's tile has to be worth its flush: at 85 atoms a brick (water at 0.12 nm) file + spread + gather
-// take 6.5 + 17.7 + 16.0 us at 288k atoms with cold caches, spread + gather directly 45.9 + 17.2 us; at
-// 18 atoms a brick (argon) the direct path stays.  Rows are flushed in aligned blocks of 4
-// points, and a tile may wrap once per dimension.
+// take 6.5 + 17.7 + 16.0 us at 288k atoms with cold caches, spread + gather directly 45.9 + 17.2 us.  Whole
+// evaluations by bricks and directly: water of 16 500 atoms 21.5 and 25.2 us, of 13 200 22.9 and 23.3, of 7 500 21.1 and
+// 16.6; crystals at 44 to 55 atoms a brick 25.1 and 33.5 us (32 000 atoms), 54.5 and 60.2 (131 072), at 22 atoms a
+// brick 26.1 and 31.4 (23 328) but 51.0 and 47.2 (55 296), 87.2 and 75.8 (131 072); atoms in random order at 32 a brick
+// 124 and 140 us (300 000).  Rows are flushed in aligned blocks of 4 points, and a tile may wrap once per dimension.
 bool use_bricks(const nbx_pme* p, int natoms)
 {
     const int* n = p->d.n;
@@ -1183,8 +1185,9 @@ cudaError_t launch_gather(nbx_pme* p, int natoms, const float* d_x, const float*
     if (natoms > 0)
     {
         // four threads per atom while a thread per atom leaves the GPU waiting for its 64 loads: 3 000 atoms 6.8 ->
-        // 4.6 us, 32 000 8.7 -> 7.7 us; from then on the splines, computed four times, cost more (20 steps of 87 808
-        // atoms 2588 us with a thread per atom, 2691 us with four)
+        // 4.6 us, 32 000 8.7 -> 7.7 us; from then on the splines, computed four times, cost more (20 steps of 32 000 /
+        // 42 592 / 55 296 / 62 500 atoms 1508 / 1697 / 1915 / 2144 us with a thread per atom, 1503 / 1697 / 1946 /
+        // 2212 us with four)
         if (natoms <= kGatherLanesAtoms)
         {
             nbx::launch_pdl(k_pme_gather<4>, (4 * natoms + 127) / 128, 128, 0, p->stream, p->d, natoms, d_x, d_q, grid,

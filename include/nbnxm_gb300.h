@@ -114,7 +114,8 @@ int nbx_update_pairlist(nbx_handle* h, const float* x);
  * nonbonded kernel -> atomdata_add_nbat_f_to_f.  Host arrays; forces are overwritten.
  * energies (double[2]) and virial (double[9]) may be NULL.  An array in pinned host memory mapped
  * into the device's address space (cudaMallocHost, cudaHostAlloc, cudaHostRegister) is read or
- * written by the kernels in place; other host memory is staged through device buffers. */
+ * written by the kernels in place; other host memory goes through the handle's pinned memory (coordinates up to
+ * 32,768 atoms, forces up to 12,288) or is copied to and from device buffers. */
 int nbx_compute(nbx_handle* h, const float* x, float* f, double* energies, double* virial);
 
 /* ---- device-resident interface (pointers into device memory, asynchronous on the handle's stream) ---- */

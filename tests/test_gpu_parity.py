@@ -519,6 +519,39 @@ def test_lj_modifier_forces_as_accurate_from_both_tiles(mod, coulomb):
     assert err[1] <= 1.02 * err[0], err
 
 
+@pytest.mark.parametrize("tile", [0, 1])
+@pytest.mark.parametrize("mod", [nblib.VdwModifier.ForceSwitch, nblib.VdwModifier.PotSwitch])
+def test_excluded_pairs_beyond_the_switch_vs_oracle(mod, tile):
+    """Excluded LJ pairs farther apart than rvdw_switch: forces and energies as the oracle's (with the force switch the
+    reference keeps the switching polynomial in an excluded pair's force, not in the energy)."""
+    from scipy.spatial import cKDTree
+
+    s = systems.lj_liquid(n=1500, ntypes=4, seed=19)
+    pairs = cKDTree(s.x % s.box[0], boxsize=float(s.box[0])).query_pairs(0.8, output_type="ndarray")
+    d = s.x[pairs[:, 0]].astype(np.float64) - s.x[pairs[:, 1]]
+    r = np.linalg.norm(d - np.round(d / s.box) * s.box, axis=1)
+    pairs = pairs[(r > 0.5)][::97]
+    partners = [{a} for a in range(s.n)]
+    for a, b in pairs:
+        partners[a].add(int(b))
+        partners[b].add(int(a))
+    s.excl_index = np.concatenate(([0], np.cumsum([len(p) for p in partners]))).astype(np.int32)
+    s.excl_list = np.array([b for p in partners for b in sorted(p)], np.int32)
+    calc = nblib.ForceCalculator(s, nblib.NBKernelOptions(
+        coulomb_type=nblib.CoulombType.Pme, pairlist_cutoff=1.0, rcoulomb=0.9, compute_virial_and_energy=True,
+        vdw_modifier=mod, rvdw_switch=0.4))
+    calc.set_force_kernel(tile, 2, 2)
+    o = O.Oracle(s, rc=0.9, rlist=1.0, vdw_modifier=int(mod), rvdw_switch=0.4)
+    o.grid()
+    o.search()
+    o.force(True)
+    f = calc.compute(s.x)
+    assert rel_rms(f, o.forces()) <= FORCE_RTOL
+    eo = o.energies()
+    assert np.all(np.abs(calc.energies - eo) <= ENERGY_RTOL * np.abs(eo) + 1e-9), (calc.energies, eo)
+    calc.close()
+
+
 def test_switch_modifiers_rejected_where_unsupported():
     s = systems.lj_liquid(n=600, ntypes=4, seed=3)
     with pytest.raises(nblib.InputException):
