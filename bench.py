@@ -1062,7 +1062,7 @@ def run_ours(args) -> None:
         "pairs_computed_per_eval": pairs_avg, "useful_pairs_per_eval": up,
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": FORCE_KERNEL_DRAM_BYTES,
-                     "kernel": "nbx::k_force<energy, ewald>",
+                     "kernel": "nbx::k_force_x2<energy, ewald>",
                      "note": f"{FLOPS_PER_PAIR_VF} flops per computed pair (nrnb.cpp:106) x "
                              f"{pairs_avg:.4g} computed pairs / {avg_force_ms:.4f} ms average launch; "
                              "the launch also holds the excluded-pair and self energy work items; "

@@ -636,7 +636,7 @@ struct EmitSmem
 // of the diagonal j-clusters and topology exclusions), allocate the flagged masks all interacting,
 // clear j <= i on the diagonal (setSelfAndNewtonExclusionsGpu) and the excluded atom pairs
 // (setExclusionsForIEntry).  A chain of dependent loads and short loops: with one warp an entry 27.8 us at 45k
-// and 90 us at 960k atoms, with two 12.6 and 76 us (with four 12.6 and 82 us).
+// and 90 us at 960k atoms, with two 12.6 and 69 us (with four 12.6 and 82 us).
 __global__ void __launch_bounds__(32 * kEmitWarps) k_search_emit(DeviceView v)
 {
     pdl_begin();
