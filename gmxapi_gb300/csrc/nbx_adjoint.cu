@@ -268,57 +268,12 @@ struct AdjTypes
     float s6[kBig ? 2 : 1][4], s12[kBig ? 2 : 1][4];
 };
 
-// The type terms of one j-cluster pair by pair, for the i-clusters `rem`: what the products with one-hot matrices
-// cannot sum, since a term that is not finite (an upstream gradient that is not, or atoms so close that r^-14
-// overflows) times their zeros reaches every type pair.  Such a term goes to its own type pair here, as every other
-// of the j-cluster.  sums: the warp's FP64 type-pair sums (element 0 of lane 0).
-template<bool kGE>
-__device__ __noinline__ void adj_types_by_pair(const AdjWarp& w, double* sums, const float4 xj, const float4 gj,
-                                               unsigned rem, unsigned mj, unsigned xA, unsigned xB, int diag, float rc2,
-                                               float gE_lj, float cpot6, float cpot12)
-{
-    const int lane = threadIdx.x & 31, j = lane >> 2, ip = lane & 3, tj = __float_as_int(gj.w);
-    for (; rem; rem &= rem - 1)
-    {
-        const int    c  = __ffs(rem) - 1;
-        const float4 i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
-        for (int h = 0; h < 2; h++)
-        {
-            const float dx = (h ? i0.y : i0.x) - xj.x, dy = (h ? i0.w : i0.z) - xj.y, dz = (h ? i1.y : i1.x) - xj.z;
-            float       r2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
-            const bool  in = ((mj >> c) & 1u) && !(c == diag && j <= ip + 4 * h) && (((h ? xB : xA) >> c) & 1u);
-            if (!in || !(r2 < rc2))
-            {
-                continue;
-            }
-            r2                = fmaxf(r2, kMinDist2);
-            float rinv        = fast_rsqrt(r2);
-            rinv              = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
-            const float rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
-            const float gx = (h ? i2.y : i2.x) - gj.x, gy = (h ? i2.w : i2.z) - gj.y, gz = (h ? i3.y : i3.x) - gj.z;
-            const float gr6 = (gx * dx + gy * dy + gz * dz) * rinv6;
-            float       d6 = gr6 * rinv2, d12 = gr6 * (rinv6 * rinv2);
-            if (kGE)
-            {
-                d6  = fmaf(gE_lj, fmaf(rinv6, 1.0f / 6.0f, cpot6), d6);
-                d12 = fmaf(gE_lj, fmaf(rinv6 * rinv6, 1.0f / 12.0f, cpot12), d12);
-            }
-            // the element of adj_flush that is (i type a, j type b)
-            const int a = __float_as_int(h ? i3.w : i3.z), b = tj;
-            double*   s = sums + 64 * (4 * (a >> 3) + (a & 1) + 2 * (b >> 3)) + 4 * (b & 7) + ((a & 7) >> 1);
-            atomicAdd(s, -(double)d6);
-            atomicAdd(s + 32, (double)d12);
-        }
-    }
-}
-
 // All set cluster pairs of one cj4 group.  m: the mask of the lane's half; u: both halves' masks; wA / wB:
 // the lane's exclusion words (i-atoms ip and ip + 4).
 template<bool kEwald, bool kGE, bool kBig, bool kExcl>
 __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __restrict__ nbfp_b, AdjWarp& w,
                                           float4* dnb, int cj_lane, unsigned m, unsigned u, unsigned wA,
-                                          unsigned wB, int sci, bool central, int lane, double* gsum,
-                                          AdjTypes<kBig>& types)
+                                          unsigned wB, int sci, bool central, int lane, AdjTypes<kBig>& types)
 {
     const unsigned full = 0xffffffffu;
     const int      j = lane >> 2, ip = lane & 3;
@@ -336,7 +291,6 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         const float    qje  = xj.w * k.epsfac;
         // an empty slot has no pairs (two empty slots coincide)
         const unsigned mj   = tj == k.filler ? 0u : m >> (jm * kNcl);
-        const unsigned set  = rem;
         const unsigned xA   = wA >> (jm * kNcl), xB = wB >> (jm * kNcl);
         const int      diag = kExcl && central ? cj - sci * kNcl : -1;  // the diagonal i-cluster, if in 0 .. 7
         AdjJ<kBig>     dj;
@@ -390,17 +344,6 @@ __device__ __forceinline__ void adj_group(const AdjConsts& k, const char* __rest
         keep.y += __shfl_xor_sync(full, send.y, 2);
         float one = (o1 ? keep.y : keep.x) + __shfl_xor_sync(full, o1 ? keep.x : keep.y, 1);
         atomicAdd(reinterpret_cast<float*>(&dnb[cj * kCl + j]) + ip, -one);
-        float total = 0.0f;
-#pragma unroll
-        for (int n = 0; n < (kBig ? 2 : 1); n++)
-        {
-            total += (dj.hi[n][0] + dj.hi[n][1]) + (dj.hi[n][2] + dj.hi[n][3]);
-        }
-        if (__any_sync(full, !isfinite(total)))
-        {
-            adj_types_by_pair<kGE>(w, gsum - lane, xj, gj, set, mj, xA, xB, diag, k.rc2, k.gE_lj, k.cpot6, k.cpot12);
-            continue;
-        }
         // type pairs: D of row j turns into the B fragment (k = j-atoms ip and ip + 4, n = i type lane >> 2)
         // of the product with the one-hot j types
         const int   t0 = __shfl_sync(full, tj, 4 * ip), t1 = __shfl_sync(full, tj, 16 + 4 * ip);
@@ -447,6 +390,61 @@ template<bool kBig>
 __host__ __device__ constexpr int adj_sum_copies()
 {
     return kBig ? 1 : kAdjWarps;
+}
+
+// The type terms of one list entry pair by pair: what the products with one-hot matrices cannot sum, since a term that
+// is not finite (an upstream gradient that is not, or atoms so close that r^-14 overflows) times their zeros reaches
+// every type pair.  Such a term goes to its own type pair here, as every other of the entry.  Lane (j, ip) as in
+// adj_step; sums: the warp's FP64 type-pair sums (element 0 of lane 0).
+template<bool kGE>
+__device__ __noinline__ void adj_types_by_pair(const AdjWarp& w, double* sums, const AdjPtrs& p, const Sci& s, float rc2,
+                                               float gE_lj, float cpot6, float cpot12, int filler)
+{
+    const int lane = threadIdx.x & 31, j = lane >> 2, ip = lane & 3;
+    for (int g = s.cj4_start; g < s.cj4_end; g++)
+    {
+        const Imei     im = p.cj4[g].imei[j >> 2];
+        const unsigned wA = p.excl[im.excl_ind].pair[(j & 3) * kCl + ip], wB = p.excl[im.excl_ind].pair[(j & 3) * kCl + ip + 4];
+        for (int b = 0; b < 32; b++)
+        {
+            const int cj = p.cj4[g].cj[b / kNcl], c = b % kNcl, at = cj * kCl + j;
+            if (!((im.imask >> b) & 1u))
+            {
+                continue;
+            }
+            const float4 xj = p.xq[at], gj = p.gnb[at];
+            const int    tj = __float_as_int(gj.w);
+            const bool   diag = s.shift == kCentral && cj == s.sci * kNcl + c;
+            const float4 i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
+            for (int h = 0; h < 2; h++)
+            {
+                const float dx = (h ? i0.y : i0.x) - xj.x, dy = (h ? i0.w : i0.z) - xj.y, dz = (h ? i1.y : i1.x) - xj.z;
+                float       r2 = fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx)));
+                // (the diagonal cluster pair counts j > i only)
+                if (tj == filler || !(r2 < rc2) || !(((h ? wB : wA) >> b) & 1u) || (diag && j <= ip + 4 * h))
+                {
+                    continue;
+                }
+                r2                = fmaxf(r2, kMinDist2);
+                float rinv        = fast_rsqrt(r2);
+                rinv              = fmaf(rinv, fmaf(-0.5f * r2, rinv * rinv, 0.5f), rinv);
+                const float rinv2 = rinv * rinv, rinv6 = rinv2 * rinv2 * rinv2;
+                const float gx = (h ? i2.y : i2.x) - gj.x, gy = (h ? i2.w : i2.z) - gj.y, gz = (h ? i3.y : i3.x) - gj.z;
+                const float gr6 = (gx * dx + gy * dy + gz * dz) * rinv6;
+                float       d6 = gr6 * rinv2, d12 = gr6 * (rinv6 * rinv2);
+                if (kGE)
+                {
+                    d6  = fmaf(gE_lj, fmaf(rinv6, 1.0f / 6.0f, cpot6), d6);
+                    d12 = fmaf(gE_lj, fmaf(rinv6 * rinv6, 1.0f / 12.0f, cpot12), d12);
+                }
+                // the element of adj_flush that is (i type a, j type tj)
+                const int a = __float_as_int(h ? i3.w : i3.z);
+                double*   e = sums + 64 * (4 * (a >> 3) + (a & 1) + 2 * (tj >> 3)) + 4 * (tj & 7) + ((a & 7) >> 1);
+                atomicAdd(e, -(double)d6);
+                atomicAdd(e + 32, (double)d12);
+            }
+        }
+    }
 }
 
 // One list entry.  gsum: the lane's FP64 type-pair sums (shared memory, stride 32).
@@ -520,14 +518,14 @@ __device__ __forceinline__ void adj_entry(const AdjConsts& k, const AdjPtrs& p, 
         if ((ime.y | ime.w) == 0)
         {
             adj_group<kEwald, kGE, kBig, false>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, ~0u, ~0u, s.sci, central,
-                                                lane, gsum, types);
+                                                lane, types);
         }
         else
         {
             const unsigned* pair = p.excl[lane < 16 ? ime.y : ime.w].pair;
             const int       at   = ((lane >> 2) & 3) * kCl + (lane & 3);
             adj_group<kEwald, kGE, kBig, true>(k, nbfp_b, w, p.dnb, cj_lane, m, m0 | m1, pair[at], pair[at + 4], s.sci,
-                                               central, lane, gsum, types);
+                                               central, lane, types);
         }
     }
     // the i-side sums: lane (c, ip) adds the eight j-lanes' slots of the atoms ip and ip + 4
@@ -551,6 +549,21 @@ __device__ __forceinline__ void adj_entry(const AdjConsts& k, const AdjPtrs& p, 
         const int at = s.sci * kSc + c * kCl + ip;
         red_add_v4(&p.dnb[at], t0.x, t0.z, t1.x, t1.z);
         red_add_v4(&p.dnb[at + 4], t0.y, t0.w, t1.y, t1.w);
+    }
+    float total = 0.0f;
+#pragma unroll
+    for (int n = 0; n < (kBig ? 2 : 1); n++)
+    {
+#pragma unroll
+        for (int i = 0; i < (kBig ? 4 : 2); i++)
+        {
+            total += types.s6[n][i] + types.s12[n][i];
+        }
+    }
+    if (__any_sync(full, !isfinite(total)))
+    {
+        adj_types_by_pair<kGE>(w, gsum - lane, p, s, k.rc2, k.gE_lj, k.cpot6, k.cpot12, k.filler);
+        return;
     }
 #pragma unroll
     for (int n = 0; n < (kBig ? 2 : 1); n++)
