@@ -395,27 +395,29 @@ __host__ __device__ constexpr int adj_sum_copies()
 // The type terms of one list entry pair by pair: what the products with one-hot matrices cannot sum, since a term that
 // is not finite (an upstream gradient that is not, or atoms so close that r^-14 overflows) times their zeros reaches
 // every type pair.  Such a term goes to its own type pair here, as every other of the entry.  Lane (j, ip) as in
-// adj_step; sums: the warp's FP64 type-pair sums (element 0 of lane 0).
+// adj_step; sums: the warp's FP64 type-pair sums (element 0 of lane 0).  (Arguments by value: an address taken of the
+// caller's variables would put them, and through the shift vectors the whole DeviceView, into local memory.)
 template<bool kGE>
-__device__ __noinline__ void adj_types_by_pair(const AdjWarp& w, double* sums, const AdjPtrs& p, const Sci& s, float rc2,
-                                               float gE_lj, float cpot6, float cpot12, int filler)
+__device__ __noinline__ void adj_types_by_pair(const AdjWarp* w, double* sums, const Cj4* cj4, const Excl* excl,
+                                               const float4* xq, const float4* gnb, int sci, int shift, int cj4_start,
+                                               int cj4_end, float rc2, float gE_lj, float cpot6, float cpot12, int filler)
 {
     const int lane = threadIdx.x & 31, j = lane >> 2, ip = lane & 3;
-    for (int g = s.cj4_start; g < s.cj4_end; g++)
+    for (int g = cj4_start; g < cj4_end; g++)
     {
-        const Imei     im = p.cj4[g].imei[j >> 2];
-        const unsigned wA = p.excl[im.excl_ind].pair[(j & 3) * kCl + ip], wB = p.excl[im.excl_ind].pair[(j & 3) * kCl + ip + 4];
+        const Imei     im = cj4[g].imei[j >> 2];
+        const unsigned wA = excl[im.excl_ind].pair[(j & 3) * kCl + ip], wB = excl[im.excl_ind].pair[(j & 3) * kCl + ip + 4];
         for (int b = 0; b < 32; b++)
         {
-            const int cj = p.cj4[g].cj[b / kNcl], c = b % kNcl, at = cj * kCl + j;
+            const int cj = cj4[g].cj[b / kNcl], c = b % kNcl, at = cj * kCl + j;
             if (!((im.imask >> b) & 1u))
             {
                 continue;
             }
-            const float4 xj = p.xq[at], gj = p.gnb[at];
+            const float4 xj = xq[at], gj = gnb[at];
             const int    tj = __float_as_int(gj.w);
-            const bool   diag = s.shift == kCentral && cj == s.sci * kNcl + c;
-            const float4 i0 = w.irec[c][0][ip], i1 = w.irec[c][1][ip], i2 = w.irec[c][2][ip], i3 = w.irec[c][3][ip];
+            const bool   diag = shift == kCentral && cj == sci * kNcl + c;
+            const float4 i0 = w->irec[c][0][ip], i1 = w->irec[c][1][ip], i2 = w->irec[c][2][ip], i3 = w->irec[c][3][ip];
             for (int h = 0; h < 2; h++)
             {
                 const float dx = (h ? i0.y : i0.x) - xj.x, dy = (h ? i0.w : i0.z) - xj.y, dz = (h ? i1.y : i1.x) - xj.z;
@@ -562,7 +564,8 @@ __device__ __forceinline__ void adj_entry(const AdjConsts& k, const AdjPtrs& p, 
     }
     if (__any_sync(full, !isfinite(total)))
     {
-        adj_types_by_pair<kGE>(w, gsum - lane, p, s, k.rc2, k.gE_lj, k.cpot6, k.cpot12, k.filler);
+        adj_types_by_pair<kGE>(&w, gsum - lane, p.cj4, p.excl, p.xq, p.gnb, s.sci, s.shift, s.cj4_start, s.cj4_end, k.rc2,
+                               k.gE_lj, k.cpot6, k.cpot12, k.filler);
         return;
     }
 #pragma unroll
