@@ -30,9 +30,9 @@
 // of P_j^T D, which is added in FP32 over the entry and in FP64 beyond it.  (Float atomics on per-warp
 // tables in shared memory, which this replaces, are compare-and-swap loops.)  Against 64 bits the sigma and
 // epsilon gradients are off by 0.1-2e-7 (1 to 15 types), with those tables by 3-5.6e-7.
-// The kernel is bound by the latency of dependent arithmetic at 16 warps per SM (issue 53 %, FMA pipe 44 %, L1 70 %).
-// 24,000-atom 8-type liquid: 91.5 us with one pair per lane and table atomics, 54.5 us now; a gradient step of 16
-// liquids of 2,000 to 50,000 atoms 1276 and 941 us.
+// The kernel is bound by the latency of dependent arithmetic at 16 warps per SM (issue 53 %, FMA pipe 44 %, L1 72 %).
+// 24,000-atom 8-type liquid: 91.5 us with one pair per lane and table atomics, 52.4 us now; a gradient step of 16
+// liquids of 2,000 to 50,000 atoms 1276 and 923 us.
 #include "nbx_internal.cuh"
 #include "nbx_pair_x2.cuh"
 
